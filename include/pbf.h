@@ -125,8 +125,8 @@ typedef struct pbf_stats_t {
   double solver_residual;     /* learned solver: mean clamped density error at its last check */
   uint32_t tiles;             /* 32-particle tiles of the last list fill that wrote staging (0: none) */
   uint32_t tiles_staged;      /* of those, the tiles the staged gathers read from shared memory */
-  uint32_t lists_slot_order;  /* fast math: 1 if the last list fill walked the bins in slot order (few lists
-                                 at the cap), 0 if in the reference's order */
+  uint32_t lists_slot_order;  /* fast math: 1 if at most 1 in 64 lists had reached the cap in the fill before the
+                                 last one (or that was the first after an upload), 0 if more had; exact math: 0 */
 } pbf_stats_t;
 
 typedef struct pbf_ctx pbf_ctx;
@@ -184,8 +184,7 @@ int pbf_set_params(pbf_ctx* ctx, const pbf_params* p);
 int pbf_get_params(const pbf_ctx* ctx, pbf_params* p);
 
 /* Host AoS float3 state in; x* = x (particles.h:184-199).  v may be NULL (zero).
- * Fast math: also starts the list-order choice afresh (slot order first), so
- * steps from an uploaded state do not depend on what the context ran before. */
+ * Steps from an uploaded state do not depend on what the context ran before. */
 int pbf_upload(pbf_ctx* ctx, const float* x_aos, const float* v_aos, size_t n);
 /* Download in the reference's particle order; any pointer may be NULL. */
 int pbf_download(pbf_ctx* ctx, float* x_aos, float* v_aos, float* rho, float* lambda);
@@ -229,7 +228,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps);
  *  sorted_keys [N]  bin id of each sorted entry
  *  bin_begin/bin_end [B]  lower/upper bound of every bin (neighbors.h:137-148)
  * Any pointer may be NULL.  idx is in the reference's order (x offset outer)
- * whatever order the fast fill walked in (pbf_stats_t.lists_slot_order). */
+ * whatever order the fast path keeps its lists in. */
 int pbf_get_neighbors(pbf_ctx* ctx, int32_t* idx, int32_t* count);
 int pbf_get_bins(pbf_ctx* ctx, uint32_t* sorted_keys, uint32_t* sorted_ids,
                  uint32_t* bin_begin, uint32_t* bin_end);

@@ -452,6 +452,13 @@ __global__ void k_reorder(int n, const unsigned long long* __restrict__ pairs, c
   if (lamS) lamS[b] = lamH[a];  // FULL: lambda; fused step: last step's lambda sum, when kept
 }
 
+// Device words of the fast path's fill (FillWord): the lists that reached the
+// cap in the last fill, its particle count, and whether at most 1 in
+// kSlotCappedShare lists had reached the cap in the fill before it (1 after an
+// upload).  k_runs, the launch before the fill, moves them on.
+enum FillWord { kFillCapped = 0, kFillCount = 1, kFillFewCapped = 2, kFillWords = 3 };
+constexpr uint32_t kSlotCappedShare = 64;
+
 // Runs of bit-identical x* among consecutive sorted slots (particles piled
 // onto one point, e.g. clamped into a box corner by a collapsing scene):
 // run_end[i] = the first slot j > i whose x* differs from slot j - 1's, or the
@@ -460,8 +467,14 @@ __global__ void k_reorder(int n, const unsigned long long* __restrict__ pairs, c
 // crowded (may be null): the histogram's flag; zero means no bin is large
 // enough for the fill to read the runs, and the launch returns at once.
 constexpr int kRunBlock = 1024;
+// fw (fast math, may be null): the fill words, moved on to the fill that follows.
 __global__ void __launch_bounds__(kRunBlock) k_runs(int n, const float4* __restrict__ pst, uint32_t* run_end,
-                                                    const uint32_t* __restrict__ crowded) {
+                                                    const uint32_t* __restrict__ crowded, uint32_t* fw) {
+  if (fw && blockIdx.x == 0 && threadIdx.x == 0) {
+    fw[kFillFewCapped] = (uint64_t)fw[kFillCapped] * kSlotCappedShare <= (uint64_t)fw[kFillCount] ? 1u : 0u;
+    fw[kFillCapped] = 0u;
+    fw[kFillCount] = (uint32_t)n;
+  }
   if (crowded && *crowded == 0u) return;
   __shared__ uint32_t wfirst[kRunBlock / 32];  // first run start of every warp's 32 slots
   const int i = blockIdx.x * kRunBlock + threadIdx.x;
@@ -619,20 +632,15 @@ __device__ __forceinline__ void axis_bins(float c, float s, int (&out)[3]) {
   for (int i = 0; i < 3; ++i) out[i] = pbf::dev_axis_bin(pbf::xadd(c, pbf::xmul((float)(i - 1), s)), s);
 }
 
-// The 27 visits of one particle, in the reference's order (x offset outer,
-// z inner) or, slot, z offset outer and x inner: the bins then come in
-// ascending keys, so a warp's lanes read neighbouring slots together in the
-// gathers.  slot records where each visit's entries start (sc[visit
-// k*9 + j*3 + i]).  Stops at the cap and returns the list's length.  The
-// order is a run-time choice in one loop: two compiled walks made the fill
-// of a settled dam (crowded bins) 10-25% slower.
+// The 27 visits of one particle in the reference's order (x offset outer, z
+// inner).  Stops at the cap and returns the list's length.
 template <bool STAGE>
 __device__ __forceinline__ int fill_walk(float px, float py, float pz, const int (&bx)[3], const int (&by)[3],
                                          const int (&bz)[3], float s, float skip_eps, const pbf::Region& R,
                                          float s2, int cap, uint32_t self, const uint32_t* __restrict__ cell_start,
                                          const float4* __restrict__ pst, const uint32_t* __restrict__ run_end,
                                          int32_t* row, uint32_t* err, const FillStage& S, const int* soff,
-                                         bool& stray, bool slot, uint8_t* sc) {
+                                         bool& stray) {
   const bool finite = isfinite(px) && isfinite(py) && isfinite(pz);
   // per-axis distance from the particle to its own bin's faces, less the margin
   const float lo[3] = {fmaxf(px - ((float)bx[1] * s - s) - skip_eps, 0.f),
@@ -642,11 +650,9 @@ __device__ __forceinline__ int fill_walk(float px, float py, float pz, const int
                        fmaxf(((float)(by[1] + 1) * s - s) - py - skip_eps, 0.f),
                        fmaxf(((float)(bz[1] + 1) * s - s) - pz - skip_eps, 0.f)};
   int count = 0;
-  for (int u = 0; u < 3; u++) {
+  for (int i = 0; i < 3; i++) {
     for (int j = 0; j < 3; j++) {
-      for (int w = 0; w < 3; w++) {
-        const int i = slot ? w : u, k = slot ? u : w;
-        if (slot) sc[k * 9 + j * 3 + i] = (uint8_t)count;
+      for (int k = 0; k < 3; k++) {
         const float ex = i == 0 ? lo[0] : (i == 2 ? hi[0] : 0.f);
         const float ey = j == 0 ? lo[1] : (j == 2 ? hi[1] : 0.f);
         const float ez = k == 0 ? lo[2] : (k == 2 ? hi[2] : 0.f);
@@ -661,44 +667,21 @@ __device__ __forceinline__ int fill_walk(float px, float py, float pz, const int
   return count;
 }
 
-// Beside each list of the fast path (seg, kSegWords words per slot): where
-// each of the 27 visits' entries start, in visit order (z offset outer), then
-// kSegReferenceOrder when the list is in the reference's order (the cap is at
-// most 64, so a byte holds an offset).
-constexpr int kSegWords = 8;
-constexpr uint8_t kSegReferenceOrder = 0xFF;
+// The lists at the cap of one warp, added to fw[kFillCapped] with one atomic
+// (the warp's live lanes call it together).
+__device__ __forceinline__ void count_capped(uint32_t* fw, bool capped) {
+  const unsigned act = __activemask();
+  const unsigned cm = __ballot_sync(act, capped);
+  if (cm && (int)(threadIdx.x & 31) == __ffs(act) - 1) atomicAdd(&fw[kFillCapped], (uint32_t)__popc(cm));
+}
 
-// The fast path's choice of list order, in device words (FillWord): the
-// lists that reached the cap in the fill under way, the slot-order lists
-// queued for the reference's walk, the order of the next fill (1 = slot
-// order), the redo kernel's block ticket, and the order the last fill used.
-// The cap keeps the first entries in the reference's order, so a slot-order
-// list that reaches it is walked again in that order (k_fill_redo).  Once
-// more than 1 / kSlotCappedShare of the lists reach the cap (a dam that has
-// settled), the fill walks in the reference's order, where the cap costs
-// nothing, until the share drops again.  At 1 in 16 or 1 in 8 the re-walks
-// cost more than the slot order saves in the gathers.
-enum FillWord {
-  kFillCapped = 0,
-  kFillQueued = 1,
-  kFillSlotOrder = 2,
-  kFillTicket = 3,
-  kFillLastOrder = 4,
-  kFillWords = 5
-};
-constexpr uint32_t kSlotCappedShare = 64;
-
-// The list of slot b (a thread's share of k_fill2).  SLOT (fast math): in
-// the order fw chose, the visits' starts or the reference-order mark in seg,
-// a slot-order list that reached the cap queued for k_fill_redo; else in the
-// reference's order.
-template <bool STAGE, bool SLOT>
+// The list of slot b in the reference's order (a thread's share of k_fill2).
+// fw (fast math): the lists at the cap are counted.
+template <bool STAGE>
 __device__ __forceinline__ void fill_thread(int b, const Dev& P, int n, size_t stride, const float4* __restrict__ pst,
                                             const uint32_t* __restrict__ cell_start,
                                             const uint32_t* __restrict__ run_end, int32_t* nbr, int32_t* cnt,
-                                            uint32_t* err, const TileIO& T, uint32_t* seg, uint32_t* fw,
-                                            int32_t* queue) {
-  __shared__ __align__(16) uint8_t seg_smem[SLOT ? kFillBlock : 1][4 * kSegWords];
+                                            uint32_t* err, const TileIO& T, uint32_t* fw) {
   if (!STAGE && b >= n) return;
   if (STAGE && (b & ~(kTile - 1)) >= n) return;  // a whole warp past the end: no tile (warp-uniform)
   const bool live = b < n;
@@ -762,88 +745,208 @@ __device__ __forceinline__ void fill_thread(int b, const Dev& P, int n, size_t s
     if (!live) return;
   }
   const FillStage S{staged, xmn, xmx, ymn, zmn, ny, nz, row16};
-  const bool slot = SLOT && fw[kFillSlotOrder] != 0;
-  uint8_t* sc = SLOT ? seg_smem[threadIdx.x] : nullptr;
   const int count = fill_walk<STAGE>(xp.x, xp.y, xp.z, bx, by, bz, s, P.skip_eps, R, P.s2, cap, (uint32_t)b,
-                                     cell_start, pst, run_end, row, err, S, soff, stray, slot, sc);
+                                     cell_start, pst, run_end, row, err, S, soff, stray);
   cnt[b] = count;
-  if (SLOT) {
-    const bool capped = count >= cap;
-    // warp-aggregated counts: the lists at the cap, the slot-order ones among them queued
-    const unsigned act = __activemask(), lane_lt = (1u << (threadIdx.x & 31)) - 1u;
-    const int leader = __ffs(act) - 1;
-    const unsigned cm = __ballot_sync(act, capped), qm = __ballot_sync(act, slot && capped);
-    uint32_t qbase = 0;
-    if ((int)(threadIdx.x & 31) == leader) {
-      if (cm) atomicAdd(&fw[kFillCapped], (uint32_t)__popc(cm));
-      if (qm) qbase = atomicAdd(&fw[kFillQueued], (uint32_t)__popc(qm));
-    }
-    qbase = __shfl_sync(act, qbase, leader);
-    if (slot && capped) {
-      queue[qbase + __popc(qm & lane_lt)] = b;
-      if (STAGE) stray = true;  // the tile walks the int32 lists
-    }
-    if (slot) {  // (a fill in the reference's order leaves seg alone: the export reads its order word)
-      sc[27] = capped ? kSegReferenceOrder : 0;
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(seg_smem[threadIdx.x]);
-#pragma unroll
-      for (int v = 0; v < kSegWords; ++v) seg[(size_t)b * kSegWords + v] = w[v];
-    }
-  }
+  if (fw) count_capped(fw, count >= cap);
   // a bin outside the tile's box (float re-hash at a bin face): the tile walks the int32 lists
   if (STAGE && stray) T.nruns[tile] = 0;
 }
 
-template <bool STAGE, bool SLOT>
+template <bool STAGE>
 __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t stride, const float4* __restrict__ pst,
                                                       const uint32_t* __restrict__ cell_start,
                                                       const uint32_t* __restrict__ run_end, int32_t* nbr,
-                                                      int32_t* cnt, uint32_t* err, TileIO T, uint32_t* seg,
-                                                      uint32_t* fw, int32_t* queue) {
-  fill_thread<STAGE, SLOT>(blockIdx.x * kFillBlock + threadIdx.x, P, n, stride, pst, cell_start, run_end, nbr, cnt,
-                           err, T, seg, fw, queue);
+                                                      int32_t* cnt, uint32_t* err, TileIO T, uint32_t* fw) {
+  fill_thread<STAGE>(blockIdx.x * kFillBlock + threadIdx.x, P, n, stride, pst, cell_start, run_end, nbr, cnt, err, T,
+                     fw);
 }
 
-// The queued slot-order lists that reached the cap, walked again in the
-// reference's order (int32 lists; their seg already says so).  Then the last
-// block to finish picks the next fill's order from the share of lists at the
-// cap and clears the counts.  No thread returns early: every block reaches
-// the ticket.
-__global__ void __launch_bounds__(kFillBlock) k_fill_redo(Dev P, int n, size_t stride, const float4* __restrict__ pst,
-                                                          const uint32_t* __restrict__ cell_start,
-                                                          const uint32_t* __restrict__ run_end, int32_t* nbr,
-                                                          int32_t* cnt, uint32_t* err, const int32_t* __restrict__ queue,
-                                                          uint32_t* fw) {
-  const uint32_t queued = fw[kFillQueued];
-  for (uint32_t t = blockIdx.x * kFillBlock + threadIdx.x; t < queued; t += gridDim.x * kFillBlock) {
-    const int b = queue[t];
-    const float4 xp = pst[b];
-    const pbf::Region R = pbf::region_of(P, b);
-    int bx[3], by[3], bz[3];
-    axis_bins(xp.x, P.s, bx);
-    axis_bins(xp.y, P.s, by);
-    axis_bins(xp.z, P.s, bz);
-    const FillStage none{};
-    bool stray = false;
-    cnt[b] = fill_walk<false>(xp.x, xp.y, xp.z, bx, by, bz, P.s, P.skip_eps, R, P.s2, P.cap, (uint32_t)b,
-                              cell_start, pst, run_end, nbr + pbf::list_base(b, stride), err, none, nullptr,
-                              stray, false, nullptr);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&fw[kFillTicket], 1u) == gridDim.x - 1) {
-      __threadfence();
-      const uint32_t capped = atomicAdd(&fw[kFillCapped], 0u);
-      fw[kFillLastOrder] = fw[kFillSlotOrder];
-      fw[kFillSlotOrder] = (uint64_t)capped * kSlotCappedShare <= (uint64_t)n ? 1u : 0u;
-      fw[kFillCapped] = 0;
-      fw[kFillQueued] = 0;
-      fw[kFillTicket] = 0;
+// ---- the fast path's fill: tests first, lists after ----
+// A particle's 27 bins are 9 rows of three (x offsets), each one run of
+// consecutive slots.  A thread tests a row's candidates with no branch, four
+// loads in flight, one bit of the outcome per candidate (the sign of
+// d^2 - s^2, shifted into a mask word), and keeps the rows' masks in shared
+// memory; then it writes its list from the set bits, entry j of every lane in
+// the same iteration, whole 32-byte chunks at a time.  k_fill2's walk appends
+// inside the test loop: a warp pays for the append at almost every candidate,
+// because some lane accepts it, and its 4-byte stores touch a sector each.
+// The entries come in slot order (z offset outer, x inner: ascending keys), so
+// a warp's lanes read neighbouring slots together in the gathers.  A list
+// with more candidates than the cap keeps the reference's first `cap` (x
+// offset outer): the bits of the visits past it are cleared before the list
+// is written, no candidate is tested again.
+// The mask path takes particles whose 27 bins are the integer neighbours of
+// their own (the reference's float re-hash of coord +- s decides), inside the
+// grid, no row longer than kMaskRow candidates.  The others are walked in the
+// reference's order (fill_walk), which stops at the cap: in a crowded region
+// that is early.
+// Bound by instruction issue (70% of the slots; 27 of 32 lanes active) with
+// the L1 data path at 62% (a 16-byte load moves 512 bytes to the registers
+// even where the lanes read one record).  Measured against the walk that
+// appended in its test loop and its second launch for the capped lists: 1M dam
+// 0.497 + 0.092 -> 0.378 ms, 65k 0.062 + 0.060 -> 0.042 ms, 500k squeezed to
+// 92% of the lists at the cap 0.295 + 0.515 -> 0.311 ms; warp instructions at
+// 1M 446M -> 269M.
+constexpr int kMaskBlock = 64;
+constexpr int kMaskWords = 3, kMaskRow = 32 * kMaskWords;  // mask words and candidates of a row
+constexpr int kMaskUnits = 9 * kMaskWords;                 // mask words of a particle; at most 32
+constexpr int kMaskOver = 3;  // records the four-candidate loop may read past a row's end (their bits are dropped)
+
+// Words that have bits left to write.
+__device__ __forceinline__ uint32_t units_of(const uint32_t (*m)[kMaskBlock]) {
+  uint32_t u = 0;
+#pragma unroll
+  for (int w = 0; w < kMaskUnits; ++w) u |= m[w][threadIdx.x] ? 1u << w : 0u;
+  return u;
+}
+
+// Keep the first `cap` candidates of the reference's order (x offset outer, z
+// inner; within a bin ascending slots), clear the others' bits.
+__device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t key0, uint32_t (*m)[kMaskBlock],
+                                         const uint32_t* __restrict__ cell_start) {
+  int rem = cap;
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 3; ++j)
+      for (int k = 0; k < 3; ++k) {
+        const int r = k * 3 + j;
+        const uint32_t rk = key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)k + (uint32_t)(j * R.dimx);
+        const uint32_t a0 = cell_start[rk];
+        const int lo = (int)(cell_start[rk + i] - a0), hi = (int)(cell_start[rk + i + 1] - a0);
+        for (int w = lo >> 5; w < kMaskWords && 32 * w < hi; ++w) {
+          const int l = max(lo - 32 * w, 0), e = min(hi - 32 * w, 32);
+          const uint32_t range = (e == 32 ? 0xffffffffu : (1u << e) - 1u) & ~((1u << l) - 1u);
+          const uint32_t all = m[r * kMaskWords + w][threadIdx.x];
+          uint32_t keep = all & range;
+          int extra = __popc(keep) - rem;
+          rem = max(-extra, 0);
+          if (extra > 0) {
+            for (; extra > 0; --extra) keep &= ~(0x80000000u >> __clz(keep));
+            m[r * kMaskWords + w][threadIdx.x] = (all & ~range) | keep;
+          }
+        }
+      }
+}
+
+__global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t stride,
+                                                           const float4* __restrict__ pst,
+                                                           const uint32_t* __restrict__ cell_start,
+                                                           const uint32_t* __restrict__ run_end, int32_t* nbr,
+                                                           int32_t* cnt, uint32_t* err, uint8_t* ref_order,
+                                                           uint32_t* fw) {
+  __shared__ uint32_t mask[kMaskUnits][kMaskBlock];
+  __shared__ uint32_t first[9][kMaskBlock];  // the rows' first slots
+  const int b = blockIdx.x * kMaskBlock + threadIdx.x;
+  if (b >= n) return;
+  const int tid = threadIdx.x;
+  const float4 xp = pst[b];
+  const float s = P.s, s2 = P.s2;
+  const pbf::Region R = pbf::region_of(P, b);
+  int bx[3], by[3], bz[3];
+  axis_bins(xp.x, s, bx);
+  axis_bins(xp.y, s, by);
+  axis_bins(xp.z, s, bz);
+  const bool finite = isfinite(xp.x) && isfinite(xp.y) && isfinite(xp.z);
+  bool masks = finite && bx[1] - bx[0] == 1 && bx[2] - bx[1] == 1 && by[1] - by[0] == 1 && by[2] - by[1] == 1 &&
+               bz[1] - bz[0] == 1 && bz[2] - bz[1] == 1 && bx[0] >= 0 && by[0] >= 0 && bz[0] >= 0 &&
+               bx[2] < R.dimx && by[2] < R.dimy && bz[2] < R.dimz;
+  const uint32_t key0 =
+      R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)bz[0] + ((uint32_t)by[0] * (uint32_t)R.dimx + (uint32_t)bx[0]);
+  int count = 0;
+  uint32_t units = 0;  // mask words that are not empty
+  if (masks) {
+    // per-axis distance to the neighbour rows, less the margin (fill_visit's skip, for a whole row)
+    const float ylo = fmaxf(xp.y - ((float)by[1] * s - s) - P.skip_eps, 0.f);
+    const float yhi = fmaxf(((float)(by[1] + 1) * s - s) - xp.y - P.skip_eps, 0.f);
+    const float zlo = fmaxf(xp.z - ((float)bz[1] * s - s) - P.skip_eps, 0.f);
+    const float zhi = fmaxf(((float)(bz[1] + 1) * s - s) - xp.z - P.skip_eps, 0.f);
+    for (int r = 0; r < 9; ++r) {
+      const int k = r / 3, j = r - 3 * k;
+      const float ey = j == 0 ? ylo : (j == 2 ? yhi : 0.f), ez = k == 0 ? zlo : (k == 2 ? zhi : 0.f);
+      const uint32_t rk = key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)k + (uint32_t)(j * R.dimx);
+      uint32_t a0 = 0;
+      int len = 0;
+      if (!(ey * ey + ez * ez > s2)) {
+        a0 = cell_start[rk];
+        len = (int)(cell_start[rk + 3] - a0);
+      }
+      first[r][tid] = a0;
+      if (len > kMaskRow) {
+        masks = false;
+        break;
+      }
+      const float4* p = pst + a0;
+#pragma unroll 1
+      for (int w = 0; w < kMaskWords; ++w, p += 32) {
+        const int rest = min(len - 32 * w, 32);
+        uint32_t m = 0;
+        if (rest > 0) {
+          int c = 0;
+#pragma unroll 1
+          for (; c < rest; c += 4) {
+            const float4 q0 = __ldg(p + c), q1 = __ldg(p + c + 1), q2 = __ldg(p + c + 2), q3 = __ldg(p + c + 3);
+            auto test = [&](const float4& q) {  // the sign bit of d^2 - s^2 (a NaN's is clear)
+              const float d2 = pbf::mag2<true>(pbf::xsub(xp.x, q.x), pbf::xsub(xp.y, q.y), pbf::xsub(xp.z, q.z));
+              m = __funnelshift_l(__float_as_uint(pbf::xsub(d2, s2)), m, 1);
+            };
+            test(q0);
+            test(q1);
+            test(q2);
+            test(q3);
+          }
+          m = __brev(m << (32 - c));  // candidate t at bit t
+          if (rest < 32) m &= (1u << rest) - 1u;
+          const uint32_t self = (uint32_t)b - a0 - 32u * (uint32_t)w;
+          if (r == 4 && self < 32u) m &= ~(1u << self);
+        }
+        mask[r * kMaskWords + w][tid] = m;
+        count += __popc(m);
+        units |= m ? 1u << (r * kMaskWords + w) : 0u;
+      }
     }
   }
+  int32_t* row = nbr + pbf::list_base(b, stride);
+  const int cap = P.cap;
+  if (masks) {
+    if (count > cap) {
+      keep_capped(cap, R, key0, mask, cell_start);
+      count = cap;
+      units = units_of(mask);
+    }
+    uint32_t m = 0, at = 0;
+    for (int e0 = 0; e0 < count; e0 += pbf::kListChunk) {
+      int32_t e[pbf::kListChunk];
+#pragma unroll
+      for (int t = 0; t < pbf::kListChunk; ++t) {
+        if (e0 + t < count) {
+          if (m == 0u) {  // the next word that has bits
+            const int u = __ffs(units) - 1;
+            units &= units - 1u;
+            const int r = (u * 11) >> 5;  // u / kMaskWords
+            m = mask[u][tid];
+            at = first[r][tid] + 32u * (uint32_t)(u - kMaskWords * r);
+          }
+          e[t] = (int32_t)(at + (uint32_t)__ffs(m) - 1u);
+          m &= m - 1u;
+        } else {
+          e[t] = 0;  // past the count: never read as an entry
+        }
+      }
+      int4* dst = reinterpret_cast<int4*>(row + pbf::list_off(e0));
+      dst[0] = make_int4(e[0], e[1], e[2], e[3]);
+      dst[1] = make_int4(e[4], e[5], e[6], e[7]);
+    }
+  } else {
+    const FillStage none{};
+    bool stray = false;
+    count = fill_walk<false>(xp.x, xp.y, xp.z, bx, by, bz, s, P.skip_eps, R, s2, cap, (uint32_t)b, cell_start, pst,
+                             run_end, row, err, none, nullptr, stray);
+  }
+  cnt[b] = count;
+  ref_order[b] = masks ? 0 : 1;
+  count_capped(fw, count >= cap);
 }
-
+static_assert(kMaskWords == 3 && kMaskUnits <= 32, "the words' division by 3 and their bit set");
 // ---- density (particles.h:292-313) ----
 // Per-stage form: writes rho into vel.w.  A particle sitting on a neighbour is
 // nudged (particles.h:303-305); the reference writes position_stars_[p] in
@@ -2282,35 +2385,44 @@ __global__ void __launch_bounds__(kBlock) k_stats(Dev P, int b0, int b1, size_t 
 }
 
 // Neighbour lists in reference index space, [N][cap], -1 past count.
-// seg (fast math, whose last fill walked in slot order when *last_order is
-// 1): each slot-order list is written back in the reference's order, visit
-// by visit (x offset outer, z inner; within a visit the entries keep their
-// ascending slots), from where the fill recorded each visit starts.
+// ref_order (may be null: every list is in the reference's order): a list
+// whose byte is 0 holds its entries in another order.  Its bins are the 27 at
+// integer offsets of the particle's own, so an entry's visit follows from the
+// two bin keys (key, per slot), and its place in the reference's list is the
+// number of entries of an earlier visit, or of the same visit and a lower slot.
 __global__ void k_export_neighbors(int n, size_t stride, int cap, const int32_t* __restrict__ nbr,
                                    const int32_t* __restrict__ cnt, const uint32_t* __restrict__ orig,
-                                   int32_t* idx_out, int32_t* cnt_out, const uint32_t* __restrict__ seg,
-                                   const uint32_t* __restrict__ last_order) {
+                                   int32_t* idx_out, int32_t* cnt_out, const uint8_t* __restrict__ ref_order,
+                                   const uint32_t* __restrict__ key, Dev P) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   const size_t o = orig[b];
   const int c = cnt[b];
   if (cnt_out) cnt_out[o] = c;
   if (!idx_out) return;
-  const uint8_t* sc = seg && *last_order ? reinterpret_cast<const uint8_t*>(seg + (size_t)b * kSegWords) : nullptr;
-  if (sc == nullptr || sc[27] == kSegReferenceOrder) {
-    for (int k = 0; k < cap; ++k)
-      idx_out[o * cap + k] = k < c ? (int32_t)orig[nbr[pbf::list_at(b, stride, k)]] : -1;
+  for (int k = c; k < cap; ++k) idx_out[o * cap + k] = -1;
+  if (ref_order == nullptr || ref_order[b]) {
+    for (int k = 0; k < c; ++k) idx_out[o * cap + k] = (int32_t)orig[nbr[pbf::list_at(b, stride, k)]];
     return;
   }
-  int e = 0;
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j)
-      for (int k = 0; k < 3; ++k) {
-        const int v = k * 9 + j * 3 + i;  // visit v's entries: [sc[v], sc[v+1]) of the slot-order list
-        for (int t = sc[v], t1 = v < 26 ? sc[v + 1] : c; t < t1; ++t)
-          idx_out[o * cap + e++] = (int32_t)orig[nbr[pbf::list_at(b, stride, t)]];
-      }
-  for (; e < cap; ++e) idx_out[o * cap + e] = -1;
+  const pbf::Region R = pbf::region_of(P, b);
+  const int plane = R.dimx * R.dimy, half = (plane - 1) / 2;  // |dy * dimx + dx| <= half: at least 3 bins per axis
+  const int own = (int)key[b];
+  int place[64];  // the visit of every entry (c <= 64)
+  for (int k = 0; k < c; ++k) {
+    const int d = (int)key[nbr[pbf::list_at(b, stride, k)]] - own;
+    const int dz = d > half ? 1 : (d < -half ? -1 : 0);
+    const int r = d - dz * plane;
+    const int dy = r > 1 ? 1 : (r < -1 ? -1 : 0);
+    place[k] = (r - dy * R.dimx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
+  }
+  for (int k = 0; k < c; ++k) {
+    const int q = nbr[pbf::list_at(b, stride, k)];
+    int rank = 0;
+    for (int t = 0; t < c; ++t)
+      rank += place[t] < place[k] || (place[t] == place[k] && nbr[pbf::list_at(b, stride, t)] < q) ? 1 : 0;
+    idx_out[o * cap + rank] = (int32_t)orig[q];
+  }
 }
 
 }  // namespace
@@ -2333,10 +2445,9 @@ struct pbf_ctx {
   cudaStream_t side = nullptr;  // captures the body of the learned solver's conditional loop
   bool capture_failed = false;  // a step's conditional loop could not be captured whole
   bool lists_valid = false;
-  bool lists_slot_order = false;  // fast math: seg says, per list, which order it is in
-  uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's order choice (FillWord)
-  int32_t* redo_queue = nullptr;   // [C] slot-order lists that reached the cap
-  uint32_t* seg = nullptr;        // [C][kSegWords] where the fast fill's visits start
+  bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
+  uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
+  uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order
 
   float4 *posH = nullptr, *pstH = nullptr, *velH = nullptr, *scrH = nullptr;
   float4 *posS = nullptr, *pstS = nullptr, *velS = nullptr, *scrS = nullptr, *xl = nullptr, *velT = nullptr;
@@ -2849,47 +2960,35 @@ void launch_sort_to_pairs(pbf_ctx* ctx) {
 }
 
 void launch_fill(pbf_ctx* ctx, const float4* pst) {
+  const bool fast = ctx->params.exact_math == 0;
+  uint32_t* fw = fast ? ctx->fill_words : nullptr;
   {
     Launch L(ctx, "runs");
     k_runs<<<blocks_for(ctx->n, kRunBlock), kRunBlock, 0, ctx->stream>>>((int)ctx->n, pst, ctx->run_end,
-                                                                         ctx->cell_count + ctx->nbins);
+                                                                         ctx->cell_count + ctx->nbins, fw);
   }
-  // fast math: lists in slot order while few reach the cap (the gathers' sums
-  // in any order are within the fast path's tolerance), the capped ones
-  // walked again in the reference's order; exact math: the reference's order
-  const bool slot = ctx->params.exact_math == 0;
-  ctx->lists_slot_order = slot;
-  {
-    Launch L(ctx, "fill_neighbors");
-    auto fill = [&](auto stage, auto order) {
-      k_fill2<decltype(stage)::value, decltype(order)::value>
-          <<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, ctx->stream>>>(
-              ctx->dev, (int)ctx->n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err,
-              tile_io(ctx), ctx->seg, ctx->fill_words, ctx->redo_queue);
-    };
-    using T_ = std::true_type;
-    using F_ = std::false_type;
-    if (any_staged(ctx)) {
-      if (slot) fill(T_{}, T_{}); else fill(T_{}, F_{});
-    } else {
-      if (slot) fill(F_{}, T_{}); else fill(F_{}, F_{});
-    }
-  }
-  if (slot) {
-    Launch L(ctx, "fill_redo");
-    const int grid = std::max(1, std::min(blocks_for(ctx->n, kFillBlock), 4 * ctx->sms));
-    k_fill_redo<<<grid, kFillBlock, 0, ctx->stream>>>(ctx->dev, (int)ctx->n, ctx->lstride, pst, ctx->cell_start,
-                                                      ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, ctx->redo_queue,
-                                                      ctx->fill_words);
-  }
+  // fast math: lists in slot order (the gathers' sums in any order are within
+  // the fast path's tolerance); exact math and the staged gathers' 16-bit
+  // lists: the reference's order
+  const bool staged = any_staged(ctx);
+  ctx->lists_slot_order = fast && !staged;
+  Launch L(ctx, "fill_neighbors");
+  const int n = (int)ctx->n;
+  if (ctx->lists_slot_order)
+    k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, ctx->stream>>>(
+        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, ctx->ref_order,
+        fw);
+  else if (staged)
+    k_fill2<true><<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, ctx->stream>>>(
+        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
+  else
+    k_fill2<false><<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, ctx->stream>>>(
+        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
 }
 
-// An upload starts the fast fill's order choice afresh: slot order first, no
-// lists counted.  The steps from an uploaded state then do not depend on what
-// the context ran before.
+// An upload forgets the fills before it: no lists counted at the cap.
 int reset_fill_order(pbf_ctx* ctx) {
   CK(cudaMemsetAsync(ctx->fill_words, 0, kFillWords * sizeof(uint32_t), ctx->stream));
-  CK(cudaMemsetAsync(ctx->fill_words + kFillSlotOrder, 1, 1, ctx->stream));
   return PBF_OK;
 }
 
@@ -3338,12 +3437,12 @@ int launches_per_step(const pbf_ctx* ctx) {
   // kernels only (the memsets are not), as launched eagerly (a captured
   // learned step runs its plain iterations in a conditional graph node and
   // launches fewer once converged): ext/predict/hash + 3 scan + radix
-  // passes x (histogram, 3 scan, scatter) + reorder + runs + fill + [fast
-  // math: fill redo] + K x (density/lambda, [exact: lambda fix-up], delta-p)
+  // passes x (histogram, 3 scan, scatter) + reorder + runs + fill +
+  // K x (density/lambda, [exact: lambda fix-up], delta-p)
   // + (K==0: velocity) + 2 if gamma + 4 (visc, vort, apply, visc)
   const int sort = 5 * ctx->radix_passes;
-  const int fill = ctx->params.exact_math ? 2 : 3;  // runs, fill, [redo]
-  if (persist_on(ctx)) return 1 + 3 + sort + 1 + fill + 1;  // ... reorder, runs, fill, redo, the persistent step
+  const int fill = 2;  // runs, fill
+  if (persist_on(ctx)) return 1 + 3 + sort + 1 + fill + 1;  // ... reorder, runs, fill, the persistent step
   const int K = ctx->params.solve_steps;
   const int tail = (ctx->params.gamma != 0.0f ? 2 : 0) + 4;
   if (ctx->params.solver == 1 && !ctx->params.exact_math && !(ctx->params.residual_tol > 0.0f)) {
@@ -3423,8 +3522,8 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
   ctx->lstride = list_stride(p->neighbor_cap);
   ctx->lstride_cap = ctx->lstride;
   const size_t cap = ctx->lstride;
-  if ((rc = dalloc(ctx, &ctx->posH, C)) || (rc = dalloc(ctx, &ctx->pstH, C)) || (rc = dalloc(ctx, &ctx->velH, C)) ||
-      (rc = dalloc(ctx, &ctx->scrH, C)) || (rc = dalloc(ctx, &ctx->posS, C)) || (rc = dalloc(ctx, &ctx->pstS, C + 1)) ||
+  if ((rc = dalloc(ctx, &ctx->posH, C)) || (rc = dalloc(ctx, &ctx->pstH, C + kMaskOver)) || (rc = dalloc(ctx, &ctx->velH, C)) ||
+      (rc = dalloc(ctx, &ctx->scrH, C)) || (rc = dalloc(ctx, &ctx->posS, C)) || (rc = dalloc(ctx, &ctx->pstS, C + 1 + kMaskOver)) ||
       (rc = dalloc(ctx, &ctx->velS, C + 1)) || (rc = dalloc(ctx, &ctx->scrS, C)) || (rc = dalloc(ctx, &ctx->xl, C + 1)) ||
       (rc = dalloc(ctx, &ctx->velT, C + 1)) || (rc = dalloc(ctx, &ctx->lamH, C)) || (rc = dalloc(ctx, &ctx->lamS, C)) ||
       (rc = dalloc(ctx, &ctx->origH, C)) || (rc = dalloc(ctx, &ctx->origS, C)) || (rc = dalloc(ctx, &ctx->key, C)) ||
@@ -3438,9 +3537,8 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
       (rc = dalloc(ctx, &ctx->scan_part, (size_t)ctx->nscan_parts)) || (rc = dalloc(ctx, &ctx->err, 1)) ||
       (rc = dalloc(ctx, &ctx->nudge, 1)) ||
       (rc = dalloc(ctx, &ctx->pairs, C)) || (rc = dalloc(ctx, &ctx->pairs_sorted, C)) || (rc = dalloc(ctx, &ctx->nbr, pbf::list_entries(C, cap))) ||
-      (rc = dalloc(ctx, &ctx->seg, C * kSegWords)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
-      (rc = dalloc(ctx, &ctx->redo_queue, C)) ||
-            (rc = dalloc(ctx, &ctx->cnt, C)) || (rc = dalloc(ctx, &ctx->stage, 6 * C)) ||
+      (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
+      (rc = dalloc(ctx, &ctx->cnt, C)) || (rc = dalloc(ctx, &ctx->stage, 6 * C)) ||
       (rc = dalloc(ctx, &ctx->stage_i, std::max(C * cap + C, pbf::list_entries(C, cap)))) ||
       (rc = dalloc(ctx, &ctx->acc, 8)) ||
       (rc = dalloc(ctx, &ctx->maxerr, 1)) || (rc = dalloc(ctx, &ctx->hits, 1)) ||
@@ -3467,10 +3565,8 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
     fail(ctx, PBF_ERR_CUDA, "initialisation failed");
     return bail(PBF_ERR_CUDA);
   }
-  // the first fill walks in slot order (the byte sets word kFillSlotOrder to 1)
   if (cudaMemsetAsync(ctx->err, 0, sizeof(uint32_t), ctx->stream) != cudaSuccess ||
       cudaMemsetAsync(ctx->fill_words, 0, kFillWords * sizeof(uint32_t), ctx->stream) != cudaSuccess ||
-      cudaMemsetAsync(ctx->fill_words + kFillSlotOrder, 1, 1, ctx->stream) != cudaSuccess ||
       cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
     fail(ctx, PBF_ERR_CUDA, "initialisation failed");
     return bail(PBF_ERR_CUDA);
@@ -4199,8 +4295,8 @@ int pbf_get_neighbors(pbf_ctx* ctx, int32_t* idx, int32_t* count) {
   int32_t* dc = ctx->stage_i + n * cap;
   k_export_neighbors<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, ctx->lstride, (int)cap, ctx->nbr, ctx->cnt,
                                                                  ctx->origH, di, dc,
-                                                                 ctx->lists_slot_order ? ctx->seg : nullptr,
-                                                                 ctx->fill_words + kFillLastOrder);
+                                                                 ctx->lists_slot_order ? ctx->ref_order : nullptr,
+                                                                 ctx->keyH, ctx->dev);
   if (int rc = check_launch(ctx, "export_neighbors")) return rc;
   if (idx) CK(cudaMemcpyAsync(idx, di, n * cap * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   if (count) CK(cudaMemcpyAsync(count, dc, n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
@@ -4270,7 +4366,7 @@ static int stats_range(pbf_ctx* ctx, size_t b0, size_t b1, bool clear_flags, pbf
     out->solver_iterations = (uint32_t)ctx->params.solve_steps;
     out->solver_residual = -1.0;
   }
-  if (!ctx->params.exact_math) CK(cudaMemcpy(&out->lists_slot_order, ctx->fill_words + kFillLastOrder,
+  if (!ctx->params.exact_math) CK(cudaMemcpy(&out->lists_slot_order, ctx->fill_words + kFillFewCapped,
                                              sizeof(uint32_t), cudaMemcpyDeviceToHost));
   if (any_staged(ctx) && ctx->n) {  // the tiles of the last list fill
     const size_t tiles = (ctx->n + kTile - 1) / kTile;
@@ -4977,7 +5073,7 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
     std::swap(vin, vout);
   }
   k_noalloc_gather<<<g, kBlock, 0, s>>>(nn, vin, d_x, sorted_x, sorted_id);
-  k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end, nullptr);
+  k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end, nullptr, nullptr);
   k_noalloc_fill<<<g, kBlock, 0, s>>>(d, nn, sorted_x, sorted_id, cell_start, run_end, d_nbr, d_cnt, err);
   if (d_flags) e = cudaMemcpyAsync(d_flags, err, 4, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaGetLastError();
