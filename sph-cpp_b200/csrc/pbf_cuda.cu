@@ -203,8 +203,12 @@ __global__ void k_predict(Dev P, int n, const float4* __restrict__ pos, const fl
   pst[a] = make_float4(s.x, s.y, s.z, 0.0f);
 }
 
-// Bins holding more particles than this walk their candidates run by run.
-constexpr uint32_t kRunBin = 512;
+// Bins holding more particles than this walk their candidates run by run.  A
+// run waits for the load before it, so short runs lose to the tests' four
+// loads in flight: the fill of the 1M dam at steps 150 / 200 / 250 / 290 takes
+// 0.72 / 1.27 / 2.83 / 2.81 ms at 512, 0.56 / 1.26 / 2.63 / 2.78 at 1,024,
+// 0.56 / 1.07 / 2.25 / 2.14 at 4,096.
+constexpr uint32_t kRunBin = 4096;
 
 // calculate_bins (neighbors.h:120-125) + bin histogram; the radix sort's
 // input (key, pair) goes to the particle's reference index.  The word after
@@ -453,11 +457,15 @@ __global__ void k_reorder(int n, const unsigned long long* __restrict__ pairs, c
 }
 
 // Device words of the fast path's fill (FillWord): the lists that reached the
-// cap in the last fill, its particle count, and whether at most 1 in
+// cap in the last fill, its particle count, whether at most 1 in
 // kSlotCappedShare lists had reached the cap in the fill before it (1 after an
-// upload).  k_runs, the launch before the fill, moves them on.
-enum FillWord { kFillCapped = 0, kFillCount = 1, kFillFewCapped = 2, kFillWords = 3 };
+// upload), the warps of particles k_fill_masks left to k_fill_rest and how
+// many of those are taken.  k_runs, the launch before the fill, moves them on.
+enum FillWord { kFillCapped = 0, kFillCount, kFillFewCapped, kFillRest, kFillTaken, kFillWords };
 constexpr uint32_t kSlotCappedShare = 64;
+
+// Dev::walk of a list whose entries are all walked (lists hold at most 64).
+constexpr uint8_t kWalkAll = 0xFF;
 
 // Runs of bit-identical x* among consecutive sorted slots (particles piled
 // onto one point, e.g. clamped into a box corner by a collapsing scene):
@@ -474,6 +482,8 @@ __global__ void __launch_bounds__(kRunBlock) k_runs(int n, const float4* __restr
     fw[kFillFewCapped] = (uint64_t)fw[kFillCapped] * kSlotCappedShare <= (uint64_t)fw[kFillCount] ? 1u : 0u;
     fw[kFillCapped] = 0u;
     fw[kFillCount] = (uint32_t)n;
+    fw[kFillRest] = 0u;
+    fw[kFillTaken] = 0u;
   }
   if (crowded && *crowded == 0u) return;
   __shared__ uint32_t wfirst[kRunBlock / 32];  // first run start of every warp's 32 slots
@@ -509,6 +519,31 @@ __global__ void __launch_bounds__(kRunBlock) k_runs(int n, const float4* __restr
   run_end[i] = e;
 }
 
+
+// Up to 32 candidates from p on (1 <= many), tested with no branch: bit t of
+// the result is d^2 < s2 of candidate t.  Four loads in flight; the sign of
+// d^2 - s2 is shifted into the mask (a NaN's is clear).  Reads whole groups of
+// four, kMaskOver records past the last at most (their bits are dropped).
+constexpr int kMaskOver = 3;
+__device__ __forceinline__ uint32_t test_chunk(const float4* __restrict__ p, int many, float px, float py, float pz,
+                                               float s2) {
+  uint32_t m = 0;
+  int c = 0;
+#pragma unroll 1
+  for (; c < many; c += 4) {
+    const float4 q0 = __ldg(p + c), q1 = __ldg(p + c + 1), q2 = __ldg(p + c + 2), q3 = __ldg(p + c + 3);
+    auto test = [&](const float4& q) {
+      const float d2 = pbf::mag2<true>(pbf::xsub(px, q.x), pbf::xsub(py, q.y), pbf::xsub(pz, q.z));
+      m = __funnelshift_l(__float_as_uint(pbf::xsub(d2, s2)), m, 1);
+    };
+    test(q0);
+    test(q1);
+    test(q2);
+    test(q3);
+  }
+  m = __brev(m << (32 - c));
+  return many < 32 ? m & ((1u << many) - 1u) : m;
+}
 
 // One crowded bin [q0, q1) of the list fill, run by run: one distance test per
 // run of bit-identical x*; on a hit the run's slots are appended in order, the
@@ -602,22 +637,14 @@ __device__ __forceinline__ int fill_visit(int cx, int cy, int cz, bool at_offset
   const uint32_t q0 = cell_start[nb], q1 = cell_start[nb + 1];
   if (q1 - q0 > kRunBin) {
     count = fill_runs(px, py, pz, s2, cap, self, q0, q1, pst, run_end, row, staged ? S.row16 : nullptr, off, count);
-  } else if (q0 <= self && self < q1) {  // the particle's own bin: skip itself
-    for (uint32_t q = q0; q < q1; ++q) {
-      const float4 xq = pst[q];
-      const float d2 = pbf::mag2<true>(pbf::xsub(px, xq.x), pbf::xsub(py, xq.y), pbf::xsub(pz, xq.z));
-      if (d2 < s2 && q != self && count < cap) {
-        if (staged) S.row16[count] = (uint16_t)((int)q + off);
-        row[pbf::list_off(count++)] = (int32_t)q;
-      }
-    }
-  } else {  // another bin (all but one of the 27, at the same offset for every lane)
-    for (uint32_t q = q0; q < q1; ++q) {
-      const float4 xq = pst[q];
-      const float d2 = pbf::mag2<true>(pbf::xsub(px, xq.x), pbf::xsub(py, xq.y), pbf::xsub(pz, xq.z));
-      if (d2 < s2 && count < cap) {
-        if (staged) S.row16[count] = (uint16_t)((int)q + off);
-        row[pbf::list_off(count++)] = (int32_t)q;
+  } else {
+    for (uint32_t q = q0; q < q1 && count < cap; q += 32) {
+      uint32_t m = test_chunk(pst + q, (int)min(q1 - q, 32u), px, py, pz, s2);
+      if (self - q < 32u) m &= ~(1u << (self - q));  // the particle itself
+      for (; m && count < cap; m &= m - 1u) {
+        const uint32_t c = q + (uint32_t)__ffs(m) - 1u;
+        if (staged) S.row16[count] = (uint16_t)((int)c + off);
+        row[pbf::list_off(count++)] = (int32_t)c;
       }
     }
   }
@@ -748,7 +775,10 @@ __device__ __forceinline__ void fill_thread(int b, const Dev& P, int n, size_t s
   const int count = fill_walk<STAGE>(xp.x, xp.y, xp.z, bx, by, bz, s, P.skip_eps, R, P.s2, cap, (uint32_t)b,
                                      cell_start, pst, run_end, row, err, S, soff, stray);
   cnt[b] = count;
-  if (fw) count_capped(fw, count >= cap);
+  if (fw) {
+    P.walk[b] = kWalkAll;
+    count_capped(fw, count >= cap);
+  }
   // a bin outside the tile's box (float re-hash at a bin face): the tile walks the int32 lists
   if (STAGE && stray) T.nruns[tile] = 0;
 }
@@ -767,10 +797,9 @@ __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t strid
 // consecutive slots.  A thread tests a row's candidates with no branch, four
 // loads in flight, one bit of the outcome per candidate (the sign of
 // d^2 - s^2, shifted into a mask word), and keeps the rows' masks in shared
-// memory; then it writes its list from the set bits, entry j of every lane in
-// the same iteration, whole 32-byte chunks at a time.  k_fill2's walk appends
-// inside the test loop: a warp pays for the append at almost every candidate,
-// because some lane accepts it, and its 4-byte stores touch a sector each.
+// memory; then it writes its list from the set bits, the near entries (see
+// walk_count) before the others, entry j of every lane in the same iteration,
+// whole 32-byte chunks at a time.
 // The entries come in slot order (z offset outer, x inner: ascending keys), so
 // a warp's lanes read neighbouring slots together in the gathers.  A list
 // with more candidates than the cap keeps the reference's first `cap` (x
@@ -778,9 +807,9 @@ __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t strid
 // is written, no candidate is tested again.
 // The mask path takes particles whose 27 bins are the integer neighbours of
 // their own (the reference's float re-hash of coord +- s decides), inside the
-// grid, no row longer than kMaskRow candidates.  The others are walked in the
-// reference's order (fill_walk), which stops at the cap: in a crowded region
-// that is early.
+// grid, no row longer than kMaskRow candidates.  The others are left to
+// k_fill_rest, which walks them in the reference's order and stops at the cap:
+// in a crowded region that is early.
 // Bound by instruction issue (70% of the slots; 27 of 32 lanes active) with
 // the L1 data path at 62% (a 16-byte load moves 512 bytes to the registers
 // even where the lanes read one record).  Measured against the walk that
@@ -791,20 +820,11 @@ __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t strid
 constexpr int kMaskBlock = 64;
 constexpr int kMaskWords = 3, kMaskRow = 32 * kMaskWords;  // mask words and candidates of a row
 constexpr int kMaskUnits = 9 * kMaskWords;                 // mask words of a particle; at most 32
-constexpr int kMaskOver = 3;  // records the four-candidate loop may read past a row's end (their bits are dropped)
-
-// Words that have bits left to write.
-__device__ __forceinline__ uint32_t units_of(const uint32_t (*m)[kMaskBlock]) {
-  uint32_t u = 0;
-#pragma unroll
-  for (int w = 0; w < kMaskUnits; ++w) u |= m[w][threadIdx.x] ? 1u << w : 0u;
-  return u;
-}
 
 // Keep the first `cap` candidates of the reference's order (x offset outer, z
 // inner; within a bin ascending slots), clear the others' bits.
 __device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t key0, uint32_t (*m)[kMaskBlock],
-                                         const uint32_t* __restrict__ cell_start) {
+                                         uint32_t (*near)[kMaskBlock], const uint32_t* __restrict__ cell_start) {
   int rem = cap;
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
@@ -822,7 +842,9 @@ __device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t
           rem = max(-extra, 0);
           if (extra > 0) {
             for (; extra > 0; --extra) keep &= ~(0x80000000u >> __clz(keep));
-            m[r * kMaskWords + w][threadIdx.x] = (all & ~range) | keep;
+            keep |= all & ~range;
+            m[r * kMaskWords + w][threadIdx.x] = keep;
+            near[r * kMaskWords + w][threadIdx.x] &= keep;
           }
         }
       }
@@ -830,17 +852,18 @@ __device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t
 
 __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t stride,
                                                            const float4* __restrict__ pst,
-                                                           const uint32_t* __restrict__ cell_start,
-                                                           const uint32_t* __restrict__ run_end, int32_t* nbr,
-                                                           int32_t* cnt, uint32_t* err, uint8_t* ref_order,
-                                                           uint32_t* fw) {
-  __shared__ uint32_t mask[kMaskUnits][kMaskBlock];
+                                                           const uint32_t* __restrict__ cell_start, int32_t* nbr,
+                                                           int32_t* cnt, uint8_t* ref_order, uint32_t* fw,
+                                                           uint2* rest) {
+  __shared__ uint32_t mask[kMaskUnits][kMaskBlock];  // within s
+  __shared__ uint32_t near[kMaskUnits][kMaskBlock];  // ... and within the near radius
   __shared__ uint32_t first[9][kMaskBlock];  // the rows' first slots
+  __shared__ uint8_t length[9][kMaskBlock];  // ... and candidates
   const int b = blockIdx.x * kMaskBlock + threadIdx.x;
   if (b >= n) return;
   const int tid = threadIdx.x;
   const float4 xp = pst[b];
-  const float s = P.s, s2 = P.s2;
+  const float s = P.s, s2 = P.s2, near2 = P.near2;
   const pbf::Region R = pbf::region_of(P, b);
   int bx[3], by[3], bz[3];
   axis_bins(xp.x, s, bx);
@@ -852,42 +875,54 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
                bx[2] < R.dimx && by[2] < R.dimy && bz[2] < R.dimz;
   const uint32_t key0 =
       R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)bz[0] + ((uint32_t)by[0] * (uint32_t)R.dimx + (uint32_t)bx[0]);
-  int count = 0;
-  uint32_t units = 0;  // mask words that are not empty
+  int count = 0, walk = 0;
+  uint32_t near_units = 0, far_units = 0;  // mask words that have near entries, others
   if (masks) {
     // per-axis distance to the neighbour rows, less the margin (fill_visit's skip, for a whole row)
     const float ylo = fmaxf(xp.y - ((float)by[1] * s - s) - P.skip_eps, 0.f);
     const float yhi = fmaxf(((float)(by[1] + 1) * s - s) - xp.y - P.skip_eps, 0.f);
     const float zlo = fmaxf(xp.z - ((float)bz[1] * s - s) - P.skip_eps, 0.f);
     const float zhi = fmaxf(((float)(bz[1] + 1) * s - s) - xp.z - P.skip_eps, 0.f);
+#pragma unroll
     for (int r = 0; r < 9; ++r) {
       const int k = r / 3, j = r - 3 * k;
       const float ey = j == 0 ? ylo : (j == 2 ? yhi : 0.f), ez = k == 0 ? zlo : (k == 2 ? zhi : 0.f);
       const uint32_t rk = key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)k + (uint32_t)(j * R.dimx);
-      uint32_t a0 = 0;
-      int len = 0;
+      uint32_t a0 = 0, a1 = 0;
       if (!(ey * ey + ez * ez > s2)) {
         a0 = cell_start[rk];
-        len = (int)(cell_start[rk + 3] - a0);
+        a1 = cell_start[rk + 3];
       }
       first[r][tid] = a0;
-      if (len > kMaskRow) {
-        masks = false;
-        break;
-      }
+      length[r][tid] = (uint8_t)min(a1 - a0, 255u);
+      masks = masks && a1 - a0 <= (uint32_t)kMaskRow;
+    }
+  }
+  // a warp with particles left to k_fill_rest is queued: its number and their lanes
+  {
+    const unsigned act = __activemask();
+    const unsigned left = __ballot_sync(act, !masks);
+    if (left && (int)(tid & 31) == __ffs(act) - 1) rest[atomicAdd(&fw[kFillRest], 1u)] = make_uint2((uint32_t)b >> 5, left);
+  }
+  if (!masks) return;
+  {
+    for (int r = 0; r < 9; ++r) {
+      const uint32_t a0 = first[r][tid];
+      const int len = length[r][tid];
       const float4* p = pst + a0;
 #pragma unroll 1
       for (int w = 0; w < kMaskWords; ++w, p += 32) {
         const int rest = min(len - 32 * w, 32);
-        uint32_t m = 0;
+        uint32_t m = 0, mn = 0;
         if (rest > 0) {
           int c = 0;
 #pragma unroll 1
           for (; c < rest; c += 4) {
             const float4 q0 = __ldg(p + c), q1 = __ldg(p + c + 1), q2 = __ldg(p + c + 2), q3 = __ldg(p + c + 3);
-            auto test = [&](const float4& q) {  // the sign bit of d^2 - s^2 (a NaN's is clear)
+            auto test = [&](const float4& q) {  // the sign bits of d^2 - s^2 and d^2 - near^2 (a NaN's are clear)
               const float d2 = pbf::mag2<true>(pbf::xsub(xp.x, q.x), pbf::xsub(xp.y, q.y), pbf::xsub(xp.z, q.z));
               m = __funnelshift_l(__float_as_uint(pbf::xsub(d2, s2)), m, 1);
+              mn = __funnelshift_l(__float_as_uint(pbf::xsub(d2, near2)), mn, 1);
             };
             test(q0);
             test(q1);
@@ -898,55 +933,246 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
           if (rest < 32) m &= (1u << rest) - 1u;
           const uint32_t self = (uint32_t)b - a0 - 32u * (uint32_t)w;
           if (r == 4 && self < 32u) m &= ~(1u << self);
+          mn = __brev(mn << (32 - c)) & m;
         }
-        mask[r * kMaskWords + w][tid] = m;
+        const int u = r * kMaskWords + w;
+        mask[u][tid] = m;
+        near[u][tid] = mn;
         count += __popc(m);
-        units |= m ? 1u << (r * kMaskWords + w) : 0u;
+        walk += __popc(mn);
+        near_units |= mn ? 1u << u : 0u;
+        far_units |= m != mn ? 1u << u : 0u;
       }
     }
   }
   int32_t* row = nbr + pbf::list_base(b, stride);
   const int cap = P.cap;
-  if (masks) {
-    if (count > cap) {
-      keep_capped(cap, R, key0, mask, cell_start);
-      count = cap;
-      units = units_of(mask);
+  if (count > cap) {
+    keep_capped(cap, R, key0, mask, near, cell_start);
+    count = cap;
+    walk = 0;
+    near_units = far_units = 0;
+    for (int u = 0; u < kMaskUnits; ++u) {
+      const uint32_t all = mask[u][tid], mn = near[u][tid];
+      walk += __popc(mn);
+      near_units |= mn ? 1u << u : 0u;
+      far_units |= all != mn ? 1u << u : 0u;
     }
-    uint32_t m = 0, at = 0;
-    for (int e0 = 0; e0 < count; e0 += pbf::kListChunk) {
-      int32_t e[pbf::kListChunk];
+  }
+  uint32_t m = 0, at = 0, units = near_units;
+  bool far = false;
+  for (int e0 = 0; e0 < count; e0 += pbf::kListChunk) {
+    int32_t e[pbf::kListChunk];
 #pragma unroll
-      for (int t = 0; t < pbf::kListChunk; ++t) {
-        if (e0 + t < count) {
-          if (m == 0u) {  // the next word that has bits
-            const int u = __ffs(units) - 1;
-            units &= units - 1u;
-            const int r = (u * 11) >> 5;  // u / kMaskWords
-            m = mask[u][tid];
-            at = first[r][tid] + 32u * (uint32_t)(u - kMaskWords * r);
+    for (int t = 0; t < pbf::kListChunk; ++t) {
+      if (e0 + t < count) {
+        if (m == 0u) {  // the next word that has bits, the near entries' words first
+          if (units == 0u) {
+            units = far_units;
+            far = true;
           }
-          e[t] = (int32_t)(at + (uint32_t)__ffs(m) - 1u);
-          m &= m - 1u;
-        } else {
-          e[t] = 0;  // past the count: never read as an entry
+          const int u = __ffs(units) - 1;
+          units &= units - 1u;
+          const int r = (u * 11) >> 5;  // u / kMaskWords
+          m = far ? mask[u][tid] & ~near[u][tid] : near[u][tid];
+          at = first[r][tid] + 32u * (uint32_t)(u - kMaskWords * r);
         }
+        e[t] = (int32_t)(at + (uint32_t)__ffs(m) - 1u);
+        m &= m - 1u;
+      } else {
+        e[t] = 0;  // past the count: never read as an entry
       }
-      int4* dst = reinterpret_cast<int4*>(row + pbf::list_off(e0));
-      dst[0] = make_int4(e[0], e[1], e[2], e[3]);
-      dst[1] = make_int4(e[4], e[5], e[6], e[7]);
     }
-  } else {
-    const FillStage none{};
-    bool stray = false;
-    count = fill_walk<false>(xp.x, xp.y, xp.z, bx, by, bz, s, P.skip_eps, R, s2, cap, (uint32_t)b, cell_start, pst,
-                             run_end, row, err, none, nullptr, stray);
+    int4* dst = reinterpret_cast<int4*>(row + pbf::list_off(e0));
+    dst[0] = make_int4(e[0], e[1], e[2], e[3]);
+    dst[1] = make_int4(e[4], e[5], e[6], e[7]);
   }
   cnt[b] = count;
-  ref_order[b] = masks ? 0 : 1;
+  P.walk[b] = (uint8_t)walk;
+  ref_order[b] = 0;
   count_capped(fw, count >= cap);
 }
+
+// One particle's list in the reference's order, by a whole warp: lane v looks
+// up visit v's bin, then the bins' candidates are tested 32 at a time and the
+// hits appended in order.  k_fill_rest takes it for a few particles of a warp:
+// a single lane's walk is a chain of dependent loads, 27 bins long (about
+// 60 us, the whole launch where one particle of a million sits on a bin face).
+// -1: a bin holds more than kCooperativeBin particles, where 32 tests a step
+// with nothing in flight behind them are slower than the lane's walk.
+constexpr uint32_t kCooperativeBin = 512;
+__device__ __forceinline__ int fill_cooperative(const Dev& P, int b, size_t stride, const float4* __restrict__ pst,
+                                                const uint32_t* __restrict__ cell_start, int32_t* nbr, uint32_t* err) {
+  const int lane = threadIdx.x & 31;
+  const float4 xp = pst[b];
+  const pbf::Region R = pbf::region_of(P, b);
+  uint32_t q0 = 0, q1 = 0;
+  if (lane < 27) {
+    auto bin = [&](float c, int o) { return pbf::dev_axis_bin(pbf::xadd(c, pbf::xmul((float)(o - 1), P.s)), P.s); };
+    const int cx = bin(xp.x, lane / 9), cy = bin(xp.y, lane / 3 % 3), cz = bin(xp.z, lane % 3);
+    if (!isfinite(xp.x) || !isfinite(xp.y) || !isfinite(xp.z) || cx < 0 || cy < 0 || cz < 0 || cx >= R.dimx ||
+        cy >= R.dimy || cz >= R.dimz) {
+      atomicOr(err, PBF_FLAG_KEY_RANGE);
+    } else {
+      const uint32_t key =
+          R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)cz + ((uint32_t)cy * (uint32_t)R.dimx + (uint32_t)cx);
+      q0 = cell_start[key];
+      q1 = cell_start[key + 1];
+    }
+  }
+  if (__any_sync(0xffffffffu, q1 - q0 > kCooperativeBin)) return -1;
+  int32_t* row = nbr + pbf::list_base(b, stride);
+  int count = 0;
+  for (int v = 0; v < 27 && count < P.cap; ++v) {
+    const uint32_t e = __shfl_sync(0xffffffffu, q1, v);
+    for (uint32_t q = __shfl_sync(0xffffffffu, q0, v); q < e && count < P.cap; q += 32) {
+      const uint32_t c = q + (uint32_t)lane;
+      bool hit = false;
+      if (c < e && c != (uint32_t)b) {
+        const float4 xq = pst[c];
+        hit = pbf::mag2<true>(pbf::xsub(xp.x, xq.x), pbf::xsub(xp.y, xq.y), pbf::xsub(xp.z, xq.z)) < P.s2;
+      }
+      const unsigned hits = __ballot_sync(0xffffffffu, hit);
+      const int at = count + __popc(hits & ((1u << lane) - 1u));
+      if (hit && at < P.cap) row[pbf::list_off(at)] = (int32_t)c;
+      count += __popc(hits);
+    }
+  }
+  return min(count, P.cap);
+}
+
+// The particles k_fill_masks left, in the reference's order.  Blocks take the
+// queued warps as they come, four at a time (the walks differ in length by
+// orders of magnitude).  A queued warp keeps its own lanes, and a block's
+// warps are neighbours: they read the same candidates together (queued
+// particle by particle, or taken warp by warp, the walk of a collapsed dam took
+// 25-40% longer).
+constexpr int kRestCooperative = 4;
+__global__ void __launch_bounds__(kFillBlock) k_fill_rest(Dev P, int n, size_t stride, const float4* __restrict__ pst,
+                                                          const uint32_t* __restrict__ cell_start,
+                                                          const uint32_t* __restrict__ run_end, int32_t* nbr,
+                                                          int32_t* cnt, uint32_t* err, uint8_t* ref_order,
+                                                          uint32_t* fw, const uint2* __restrict__ rest) {
+  constexpr int kWarps = kFillBlock / 32;
+  __shared__ uint32_t taken;
+  const uint32_t total = fw[kFillRest];
+  const int lane = threadIdx.x & 31;
+  while (total > 0u) {  // the same for the whole block
+    __syncthreads();
+    if (threadIdx.x == 0) taken = atomicAdd(&fw[kFillTaken], (uint32_t)kWarps);
+    __syncthreads();
+    if (taken >= total) return;
+    const uint32_t t = taken + (threadIdx.x >> 5);
+    const uint2 w = t < total ? rest[t] : make_uint2(0u, 0u);
+    const bool mine = w.y >> lane & 1u;
+    const int b = (int)(w.x * 32u) + lane;
+    int count = 0;
+    bool walk = mine;
+    if (__popc(w.y) <= kRestCooperative) {
+      for (unsigned m = w.y; m; m &= m - 1u) {
+        const int l = __ffs(m) - 1;
+        const int c = fill_cooperative(P, (int)(w.x * 32u) + l, stride, pst, cell_start, nbr, err);
+        if (l == lane && c >= 0) {
+          count = c;
+          walk = false;
+        }
+      }
+    }
+    if (walk) {
+      const float4 xp = pst[b];
+      int bx[3], by[3], bz[3];
+      axis_bins(xp.x, P.s, bx);
+      axis_bins(xp.y, P.s, by);
+      axis_bins(xp.z, P.s, bz);
+      const FillStage none{};
+      bool stray = false;
+      count = fill_walk<false>(xp.x, xp.y, xp.z, bx, by, bz, P.s, P.skip_eps, pbf::region_of(P, b), P.s2, P.cap,
+                               (uint32_t)b, cell_start, pst, run_end, nbr + pbf::list_base(b, stride), err, none,
+                               nullptr, stray);
+    }
+    __syncwarp();
+    if (mine) {
+      cnt[b] = count;
+      P.walk[b] = kWalkAll;
+      ref_order[b] = 1;
+    }
+    const unsigned capped = __ballot_sync(0xffffffffu, mine && count >= P.cap);
+    if (lane == 0 && capped) atomicAdd(&fw[kFillCapped], (uint32_t)__popc(capped));
+  }
+}
 static_assert(kMaskWords == 3 && kMaskUnits <= 32, "the words' division by 3 and their bit set");
+// ---- near entries ----
+// The lists reach to s (1.2 h in the reference) because x* moves during the
+// iterations, but every kernel of the step is zero beyond h: at rest 45% of
+// the entries add exact zeros.  The fill puts the entries within h +
+// kNearMargin * h first, and a gather walks only those (Dev::walk) as long as
+// no other entry can have come within h: two particles further apart than
+// that at the fill have to cover the margin together.  Every position update
+// adds its move to the particle's path (x*.w); a particle whose path passes
+// half the margin marks the 27 bins around its own, and the lists there are
+// walked whole from the next launch on.  (An unmarked list's entries past the
+// near ones would add zeros, so a mark more or less changes no bit.)
+// kNearSlack is left out of the path's bound for rounding: the squared
+// distances' (3e-7 of h^2), the path's sum and rsqrt's.
+// A margin of 0.05 h keeps 0.67 of a disordered list.  1M dam, all 54 entries
+// against the near 32: density/lambda 0.117 -> 0.077 ms, delta-p 0.095 -> 0.068,
+// viscosity 0.168 -> 0.104, vorticity 0.163 -> 0.109, apply 0.090 -> 0.060, the
+// final viscosity 0.130 -> 0.088; step 100 of it, where 6% of the particles pass
+// half the margin: 0.371 -> 0.285 ms for the step's three density passes.
+constexpr float kNearMargin = 0.05f, kNearSlack = 0.0005f;
+
+// Entries of list b that a gather walks.
+__device__ __forceinline__ int walk_count(const Dev& P, int b, const int32_t* __restrict__ cnt) {
+  return min((int)P.walk[b], cnt[b]);
+}
+
+// Marks the lists that may hold slot b, those of the 27 bins around its own,
+// to be walked whole, for every lane whose `mark` is set (the whole warp calls
+// it; one lane a bin).  A bin's particles share the 27, so the first of them
+// marks for all: the word of the bin's histogram, used up by the scan, carries
+// the flag until the next step clears it.  16 slots a store; the slots beside
+// a bin's own are marked too.  A bin of more than kMaskRow particles needs no
+// mark: its particles' own rows are longer, their lists walked whole anyway.
+__device__ __forceinline__ void mark_neighbourhoods(const Dev& P, int b, bool mark) {
+  constexpr uint32_t kMarked = 0x80000000u;
+  if (__any_sync(0xffffffffu, mark)) {
+    uint32_t key = 0;
+    if (mark) {
+      key = P.slot_key[b];
+      mark = !(*(volatile uint32_t*)(P.cell_mark + key) & kMarked) && !(atomicOr(P.cell_mark + key, kMarked) & kMarked);
+    }
+    const int lane = threadIdx.x & 31;
+    for (unsigned m = __ballot_sync(0xffffffffu, mark); m; m &= m - 1u) {
+      const int src = __ffs(m) - 1;
+      const int bb = __shfl_sync(0xffffffffu, b, src);
+      const uint32_t own = __shfl_sync(0xffffffffu, key, src);
+      if (lane < 27) {
+        const pbf::Region R = pbf::region_of(P, bb);
+        const int plane = R.dimx * R.dimy, k = (int)(own - R.key0);
+        const int z = k / plane, y = (k - z * plane) / R.dimx, x = k - z * plane - y * R.dimx;
+        const int cx = x + lane % 3 - 1, cy = y + lane / 3 % 3 - 1, cz = z + lane / 9 - 1;
+        if (cx >= 0 && cy >= 0 && cz >= 0 && cx < R.dimx && cy < R.dimy && cz < R.dimz) {
+          const uint32_t c = R.key0 + (uint32_t)plane * (uint32_t)cz + (uint32_t)(cy * R.dimx + cx);
+          const uint32_t q0 = P.cell_start[c], q1 = P.cell_start[c + 1];
+          if (q1 - q0 <= (uint32_t)kMaskRow)
+            for (uint32_t q = q0 & ~15u; q < q1; q += 16)
+              *reinterpret_cast<uint4*>(P.walk + q) =
+                  make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        }
+      }
+    }
+  }
+}
+
+// The path of a particle after its move from old (old.w: the path so far) to
+// s; mark: it has passed the bound with this move (a NaN passes it).
+__device__ __forceinline__ float moved(const Dev& P, float4 old, float3 s, bool& mark) {
+  const float dx = s.x - old.x, dy = s.y - old.y, dz = s.z - old.z;
+  const float path = old.w + sqrtf(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+  mark = old.w <= P.near_move && !(path <= P.near_move);
+  return path;
+}
+
 // ---- density (particles.h:292-313) ----
 // Per-stage form: writes rho into vel.w.  A particle sitting on a neighbour is
 // nudged (particles.h:303-305); the reference writes position_stars_[p] in
@@ -1035,7 +1261,7 @@ __global__ void __launch_bounds__(kBlock) k_lambda(Dev P, int n, size_t stride, 
 // nudged positions, which is what a separate lambda stage after the density
 // stage sees.
 template <bool X>
-__device__ __forceinline__ void density_lambda_one(const Dev& P, int b, size_t stride, const int32_t* __restrict__ nbr,
+__device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t stride, const int32_t* __restrict__ nbr,
                                                    const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                    float4* xl, float4* vel, float* lam, uint32_t* nudge) {
   float4 xp = pst[b];
@@ -1065,6 +1291,7 @@ __device__ __forceinline__ void density_lambda_one(const Dev& P, int b, size_t s
   xl[b] = make_float4(xp.x, xp.y, xp.z, l);
   vel[b].w = rho;
   lam[b] = l;
+  return nudged;
 }
 
 template <bool X>
@@ -1156,38 +1383,40 @@ __device__ __forceinline__ void density_lambda_tile(int tile, const Dev& P, cons
   const pbf::Group G = pbf::group_at<GL>(n, tile);
   const int b = G.b;
   const float4 xp = pst[b];
-  const int c = G.live ? cnt[b] : 0;
   const DensitySums S = density_sums<GL, MODE == kDlRecord, STAGED, COH>(
-      F, G, nbr + pbf::list_base(b, stride), STAGED ? nbr16 + (size_t)b * stride : nullptr, c, STAGED ? staged : n,
-      STAGED ? stage : pst, xp);
+      F, G, nbr + pbf::list_base(b, stride), STAGED ? nbr16 + (size_t)b * stride : nullptr,
+      G.live ? walk_count(P, b, cnt) : 0, STAGED ? staged : n, STAGED ? stage : pst, xp);
   const float rho = fmaf(F.m_poly, S.sw, F.m_w0);
   if (MODE == kDlCheck && G.live && G.lane == 0) err += fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
-  if (!G.live || G.lane != 0) return;
-  const float L2 = F.lam_grad * F.lam_grad;
-  const float sc = L2 * S.s2;  // sum |grad_q C|^2
-  const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));  // |grad_p C|^2
-  const bool close = S.dmin < 4e-16f;
-  const float nh = S.nh;
-  if (close) {  // a neighbour (almost) on top: the reference-ordered path decides the nudge
-    density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
-  } else {
-    const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
-    const float l = -C / (sc + g2 + F.lambda_eps);
-    xl[b] = make_float4(xp.x, xp.y, xp.z, l);
-    vel[b].w = rho;
-    lam[b] = l;
-  }
-  if (MODE == kDlRecord) {
-    if (io.first) {
-      float f[pbf::kMlpIn];
-      pbf::raw_features(P, pbf::region_of(P, b), F, f, c, rho, sc, g2, (int)nh, io.lamprev[b], vel[b], xp);
-#pragma unroll
-      for (int k = 0; k < pbf::kMlpIn; ++k) io.feats[(size_t)b * pbf::kMlpIn + k] = f[k];
-      io.lamsum[b] = lam[b];
+  bool mark = false;  // nudged: a move the delta-p pass already sees
+  if (G.live && G.lane == 0) {
+    const float L2 = F.lam_grad * F.lam_grad;
+    const float sc = L2 * S.s2;  // sum |grad_q C|^2
+    const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));  // |grad_p C|^2
+    const bool close = S.dmin < 4e-16f;
+    const float nh = S.nh;
+    if (close) {  // a neighbour (almost) on top: the reference-ordered path decides the nudge
+      mark = density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
     } else {
-      io.lamsum[b] += lam[b];
+      const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
+      const float l = -C / (sc + g2 + F.lambda_eps);
+      xl[b] = make_float4(xp.x, xp.y, xp.z, l);
+      vel[b].w = rho;
+      lam[b] = l;
+    }
+    if (MODE == kDlRecord) {
+      if (io.first) {
+        float f[pbf::kMlpIn];
+        pbf::raw_features(P, pbf::region_of(P, b), F, f, cnt[b], rho, sc, g2, (int)nh, io.lamprev[b], vel[b], xp);
+#pragma unroll
+        for (int k = 0; k < pbf::kMlpIn; ++k) io.feats[(size_t)b * pbf::kMlpIn + k] = f[k];
+        io.lamsum[b] = lam[b];
+      } else {
+        io.lamsum[b] += lam[b];
+      }
     }
   }
+  mark_neighbourhoods(P, b, mark);
 }
 
 // The residual check runs on a persistent grid walking the tiles, so that
@@ -1252,7 +1481,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kl_residual_probe(De
     G.b = G.live ? slot : 0;
     const int b = G.b;
     const float4 xp = pst[b];
-    const int c = G.live ? cnt[b] : 0;
+    const int c = G.live ? walk_count(P, b, cnt) : 0;
     const DensitySums S = density_sums<GL, false>(F, G, nbr + pbf::list_base(b, stride), nullptr, c, n, pst, xp);
     if (G.live && G.lane == 0) err += fmaxf(fmaf(fmaf(F.m_poly, S.sw, F.m_w0), F.inv_rho0, -1.0f), 0.0f);
   }
@@ -1353,37 +1582,40 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kl_features(Dev P, F
   const pbf::Group G = pbf::group_of<GL>(n);
   const int b = G.b;
   const float4 xp = pst[b];
-  const int c = G.live ? cnt[b] : 0;
-  const DensitySums S = density_sums<GL, true>(F, G, nbr + pbf::list_base(b, stride), nullptr, c, n, pst, xp);
-  if (!G.live || G.lane != 0) return;
-  const float rho = fmaf(F.m_poly, S.sw, F.m_w0);
-  const float L2 = F.lam_grad * F.lam_grad;
-  const float sc = L2 * S.s2;
-  const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));
-  const bool close = S.dmin < 4e-16f;
-  const float nh = S.nh;
-  const float4 v = vel[b];
-  float f[pbf::kMlpIn];
-  pbf::raw_features(P, pbf::region_of(P, b), F, f, c, rho, sc, g2, (int)nh, lamprev[b], v, xp);
-  uint32_t row[pbf::kMlpInPad / 2];
+  const DensitySums S = density_sums<GL, true>(F, G, nbr + pbf::list_base(b, stride), nullptr,
+                                               G.live ? walk_count(P, b, cnt) : 0, n, pst, xp);
+  bool mark = false;  // nudged: a move the delta-p pass already sees
+  if (G.live && G.lane == 0) {
+    const float rho = fmaf(F.m_poly, S.sw, F.m_w0);
+    const float L2 = F.lam_grad * F.lam_grad;
+    const float sc = L2 * S.s2;
+    const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));
+    const bool close = S.dmin < 4e-16f;
+    const float nh = S.nh;
+    const float4 v = vel[b];
+    float f[pbf::kMlpIn];
+    pbf::raw_features(P, pbf::region_of(P, b), F, f, cnt[b], rho, sc, g2, (int)nh, lamprev[b], v, xp);
+    uint32_t row[pbf::kMlpInPad / 2];
 #pragma unroll
-  for (int k = 0; k < pbf::kMlpIn; k += 2)
-    row[k / 2] = pbf::pack_bf16x2((f[k] - M.feat_mean[k]) * M.feat_inv_std[k],
-                                  (f[k + 1] - M.feat_mean[k + 1]) * M.feat_inv_std[k + 1]);
-  row[6] = 0u;
-  row[7] = pbf::pack_bf16x2(0.0f, close ? 1.0f : 0.0f);
-  uint4* dst = reinterpret_cast<uint4*>(featb + (size_t)b * pbf::kMlpInPad);
-  dst[0] = make_uint4(row[0], row[1], row[2], row[3]);
-  dst[1] = make_uint4(row[4], row[5], row[6], row[7]);
-  if (close) {
-    density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
-    return;
+    for (int k = 0; k < pbf::kMlpIn; k += 2)
+      row[k / 2] = pbf::pack_bf16x2((f[k] - M.feat_mean[k]) * M.feat_inv_std[k],
+                                    (f[k + 1] - M.feat_mean[k + 1]) * M.feat_inv_std[k + 1]);
+    row[6] = 0u;
+    row[7] = pbf::pack_bf16x2(0.0f, close ? 1.0f : 0.0f);
+    uint4* dst = reinterpret_cast<uint4*>(featb + (size_t)b * pbf::kMlpInPad);
+    dst[0] = make_uint4(row[0], row[1], row[2], row[3]);
+    dst[1] = make_uint4(row[4], row[5], row[6], row[7]);
+    if (close) {
+      mark = density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
+    } else {
+      const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
+      const float l1 = -C / (sc + g2 + F.lambda_eps);
+      xl[b] = make_float4(xp.x, xp.y, xp.z, l1);
+      vel[b] = make_float4(v.x, v.y, v.z, rho);
+      lam[b] = l1;
+    }
   }
-  const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
-  const float l1 = -C / (sc + g2 + F.lambda_eps);
-  xl[b] = make_float4(xp.x, xp.y, xp.z, l1);
-  vel[b] = make_float4(v.x, v.y, v.z, rho);
-  lam[b] = l1;
+  mark_neighbourhoods(P, b, mark);
 }
 
 // The network on the 5th-generation tensor cores (see pbf_mlp_tc.cuh): a
@@ -1886,7 +2118,7 @@ __device__ __forceinline__ void dp_update_tile(int tile, const Dev& P, const Fas
   const pbf::Group G = pbf::group_at<GL>(n, tile);
   const int b = G.b;
   const float4 xp = xl[b];
-  const int c = G.live ? cnt[b] : 0;
+  const int c = G.live ? walk_count(P, b, cnt) : 0;
   float ax = 0.f, ay = 0.f, az = 0.f;
   const float lp = xp.w;
   pbf::walk1<GL, STAGED, false, COH>(nbr + pbf::list_base(b, stride),
@@ -1904,17 +2136,20 @@ __device__ __forceinline__ void dp_update_tile(int tile, const Dev& P, const Fas
   ax = pbf::gsum<GL>(ax);
   ay = pbf::gsum<GL>(ay);
   az = pbf::gsum<GL>(az);
-  if (!G.live || G.lane != 0) return;
-  if (lamsum) lamsum[b] += xp.w;
-  const float3 s = pbf::boundary(P, pbf::region_of(P, b),
-                                 make_float3(pbf::xadd(xp.x, F.dp_scale * ax), pbf::xadd(xp.y, F.dp_scale * ay),
-                                                pbf::xadd(xp.z, F.dp_scale * az)));
-  const float4 ns = make_float4(s.x, s.y, s.z, 0.0f);
-  pst[b] = ns;
-  if (LAST) {
-    const float3 v = velocity_of(P, ns, pos[b]);
-    vel[b] = make_float4(v.x, v.y, v.z, vel[b].w);
+  bool mark = false;
+  if (G.live && G.lane == 0) {
+    if (lamsum) lamsum[b] += xp.w;
+    const float3 s = pbf::boundary(P, pbf::region_of(P, b),
+                                   make_float3(pbf::xadd(xp.x, F.dp_scale * ax), pbf::xadd(xp.y, F.dp_scale * ay),
+                                               pbf::xadd(xp.z, F.dp_scale * az)));
+    const float4 ns = make_float4(s.x, s.y, s.z, moved(P, pst[b], s, mark));
+    pst[b] = ns;
+    if (LAST) {
+      const float3 v = velocity_of(P, ns, pos[b]);
+      vel[b] = make_float4(v.x, v.y, v.z, vel[b].w);
+    }
   }
+  mark_neighbourhoods(P, b, mark);
 }
 
 // COND launches (the learned solver's extra iterations) use a persistent grid
@@ -1956,7 +2191,7 @@ __global__ void __launch_bounds__(kStageThreads) ks_dp_update(Dev P, Fast F, int
 // wvis (fast, direct walks): the weights W(r)/rho_q per list entry, written
 // by the first pass and read by the final one (pbf::gwalk2w, pbf::gwalkw).
 template <bool FINAL, int GL, bool STAGED = false, bool COH = false>
-__device__ __forceinline__ void viscosity_tile(int tile, const Fast& F, int n, size_t stride,
+__device__ __forceinline__ void viscosity_tile(int tile, const Dev& P, const Fast& F, int n, size_t stride,
                                                const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
                                                const float4* __restrict__ pst, const float4* __restrict__ vin,
                                                float4* vout, float4* posH, float4* pstH,
@@ -1965,7 +2200,7 @@ __device__ __forceinline__ void viscosity_tile(int tile, const Fast& F, int n, s
   const pbf::Group G = pbf::group_at<GL>(n, tile);
   const int b = G.b;
   const float4 xp = pst[b], vp = vin[b];
-  const int c = G.live ? cnt[b] : 0;
+  const int c = G.live ? walk_count(P, b, cnt) : 0;
   float ax = 0.f, ay = 0.f, az = 0.f;
   auto weight = [&](float4 xq, float4 vq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
@@ -2013,7 +2248,7 @@ __global__ void __launch_bounds__(kBlock) kf_viscosity(Dev P, Fast F, int n, siz
                                                        float4* vout, float4* posH, float4* pstH,
                                                        const uint32_t* __restrict__ origS, uint32_t* origH,
                                                        __half* wvis) {
-  viscosity_tile<FINAL, GL>(blockIdx.x, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, wvis);
+  viscosity_tile<FINAL, GL>(blockIdx.x, P, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, wvis);
 }
 
 template <bool FINAL>
@@ -2029,21 +2264,21 @@ __global__ void __launch_bounds__(kStageThreads) ks_viscosity(Dev P, Fast F, int
   const int tile = blockIdx.x;
   const int staged = stage_tile<true>(T, tile, pst, sa, vin, sb);
   if (staged >= 0)
-    viscosity_tile<FINAL, 4, true>(tile, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, nullptr,
+    viscosity_tile<FINAL, 4, true>(tile, P, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, nullptr,
                                    Src{T.nbr16, sa, sb, staged});
   else
-    viscosity_tile<FINAL, 4>(tile, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, nullptr);
+    viscosity_tile<FINAL, 4>(tile, P, F, n, stride, nbr, cnt, pst, vin, vout, posH, pstH, origS, origH, nullptr);
 }
 
 template <int GL, bool STAGED = false, bool COH = false>
-__device__ __forceinline__ void vorticity_tile(int tile, const Fast& F, int n, size_t stride,
+__device__ __forceinline__ void vorticity_tile(int tile, const Dev& P, const Fast& F, int n, size_t stride,
                                                const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
                                                const float4* __restrict__ pst, const float4* __restrict__ vel,
                                                float4* scr, float4* xl, Src src = Src{nullptr, nullptr, nullptr, 0}) {
   const pbf::Group G = pbf::group_at<GL>(n, tile);
   const int b = G.b;
   const float4 xp = pst[b], vp = vel[b];
-  const int c = G.live ? cnt[b] : 0;
+  const int c = G.live ? walk_count(P, b, cnt) : 0;
   float wx = 0.f, wy = 0.f, wz = 0.f;
   pbf::walk2<GL, STAGED, false, COH>(nbr + pbf::list_base(b, stride),
                                      STAGED ? src.nbr16 + (size_t)b * stride : nullptr, c, STAGED ? src.dummy : n,
@@ -2072,7 +2307,7 @@ __global__ void __launch_bounds__(kBlock) kf_vorticity(Dev P, Fast F, int n, siz
                                                        const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
                                                        const float4* __restrict__ pst, const float4* __restrict__ vel,
                                                        float4* scr, float4* xl) {
-  vorticity_tile<GL>(blockIdx.x, F, n, stride, nbr, cnt, pst, vel, scr, xl);
+  vorticity_tile<GL>(blockIdx.x, P, F, n, stride, nbr, cnt, pst, vel, scr, xl);
 }
 
 __global__ void __launch_bounds__(kStageThreads) ks_vorticity(Dev P, Fast F, int n, size_t stride,
@@ -2085,13 +2320,13 @@ __global__ void __launch_bounds__(kStageThreads) ks_vorticity(Dev P, Fast F, int
   const int tile = blockIdx.x;
   const int staged = stage_tile<true>(T, tile, pst, sa, vel, sb);
   if (staged >= 0)
-    vorticity_tile<4, true>(tile, F, n, stride, nbr, cnt, pst, vel, scr, xl, Src{T.nbr16, sa, sb, staged});
+    vorticity_tile<4, true>(tile, P, F, n, stride, nbr, cnt, pst, vel, scr, xl, Src{T.nbr16, sa, sb, staged});
   else
-    vorticity_tile<4>(tile, F, n, stride, nbr, cnt, pst, vel, scr, xl);
+    vorticity_tile<4>(tile, P, F, n, stride, nbr, cnt, pst, vel, scr, xl);
 }
 
 template <int GL, bool STAGED = false, bool COH = false>
-__device__ __forceinline__ void apply_vorticity_tile(int tile, const Fast& F, int n, size_t stride,
+__device__ __forceinline__ void apply_vorticity_tile(int tile, const Dev& P, const Fast& F, int n, size_t stride,
                                                      const int32_t* __restrict__ nbr,
                                                      const int32_t* __restrict__ cnt,
                                                      const float4* __restrict__ xl, const float4* __restrict__ scr,
@@ -2099,7 +2334,7 @@ __device__ __forceinline__ void apply_vorticity_tile(int tile, const Fast& F, in
   const pbf::Group G = pbf::group_at<GL>(n, tile);
   const int b = G.b;
   const float4 xp = xl[b];
-  const int c = G.live ? cnt[b] : 0;
+  const int c = G.live ? walk_count(P, b, cnt) : 0;
   float ex = 0.f, ey = 0.f, ez = 0.f;
   pbf::walk1<GL, STAGED, false, COH>(nbr + pbf::list_base(b, stride),
                                      STAGED ? src.nbr16 + (size_t)b * stride : nullptr, c, STAGED ? src.dummy : n,
@@ -2131,7 +2366,7 @@ __global__ void __launch_bounds__(kBlock) kf_apply_vorticity(Dev P, Fast F, int 
                                                              const int32_t* __restrict__ cnt,
                                                              const float4* __restrict__ xl,
                                                              const float4* __restrict__ scr, float4* vel) {
-  apply_vorticity_tile<GL>(blockIdx.x, F, n, stride, nbr, cnt, xl, scr, vel);
+  apply_vorticity_tile<GL>(blockIdx.x, P, F, n, stride, nbr, cnt, xl, scr, vel);
 }
 
 __global__ void __launch_bounds__(kStageThreads) ks_apply_vorticity(Dev P, Fast F, int n, size_t stride,
@@ -2144,9 +2379,9 @@ __global__ void __launch_bounds__(kStageThreads) ks_apply_vorticity(Dev P, Fast 
   const int tile = blockIdx.x;
   const int staged = stage_tile<false>(T, tile, xl, stage, nullptr, nullptr);
   if (staged >= 0)
-    apply_vorticity_tile<4, true>(tile, F, n, stride, nbr, cnt, xl, scr, vel, Src{T.nbr16, stage, nullptr, staged});
+    apply_vorticity_tile<4, true>(tile, P, F, n, stride, nbr, cnt, xl, scr, vel, Src{T.nbr16, stage, nullptr, staged});
   else
-    apply_vorticity_tile<4>(tile, F, n, stride, nbr, cnt, xl, scr, vel);
+    apply_vorticity_tile<4>(tile, P, F, n, stride, nbr, cnt, xl, scr, vel);
 }
 
 // ---- the persistent step (batches of scenes) ----
@@ -2312,17 +2547,17 @@ __global__ void __launch_bounds__(kPersistThreads, 12)
                                                            A.vel, nullptr);
           break;
         case kPVisc:
-          viscosity_tile<false, kPGLVisc, false, true>(tile, F, n, stride, A.nbr, A.cnt, A.pst, A.vel, A.velT,
+          viscosity_tile<false, kPGLVisc, false, true>(tile, P, F, n, stride, A.nbr, A.cnt, A.pst, A.vel, A.velT,
                                                        nullptr, nullptr, nullptr, nullptr, A.wvis);
           break;
         case kPVort:
-          vorticity_tile<kPGLVort, false, true>(tile, F, n, stride, A.nbr, A.cnt, A.pst, A.velT, A.scr, A.xl);
+          vorticity_tile<kPGLVort, false, true>(tile, P, F, n, stride, A.nbr, A.cnt, A.pst, A.velT, A.scr, A.xl);
           break;
         case kPApply:
-          apply_vorticity_tile<kPGLApply, false, true>(tile, F, n, stride, A.nbr, A.cnt, A.xl, A.scr, A.velT);
+          apply_vorticity_tile<kPGLApply, false, true>(tile, P, F, n, stride, A.nbr, A.cnt, A.xl, A.scr, A.velT);
           break;
         default:
-          viscosity_tile<true, kPGLVisc, false, true>(tile, F, n, stride, A.nbr, A.cnt, A.pst, A.velT, A.velH,
+          viscosity_tile<true, kPGLVisc, false, true>(tile, P, F, n, stride, A.nbr, A.cnt, A.pst, A.velT, A.velH,
                                                       A.posH, A.pstH, A.origS, A.origH, A.wvis);
           break;
       }
@@ -2447,7 +2682,9 @@ struct pbf_ctx {
   bool lists_valid = false;
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
-  uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order
+  uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order, near entries first
+  uint2* rest = nullptr;           // [C / 32] warps of particles k_fill_masks leaves to k_fill_rest: number, lanes
+  uint8_t* walk = nullptr;         // [C, rounded up to whole 16-byte words] Dev::walk
 
   float4 *posH = nullptr, *pstH = nullptr, *velH = nullptr, *scrH = nullptr;
   float4 *posS = nullptr, *pstS = nullptr, *velS = nullptr, *scrS = nullptr, *xl = nullptr, *velT = nullptr;
@@ -2639,6 +2876,12 @@ int make_dev(pbf_ctx* ctx, const pbf_params& p, Dev& d, int64_t dims[3]) {
     for (int a = 0; a < 3; ++a) mx = std::fmax(mx, std::fabs(p.boundary_max[a]) + 2.0f * s);
     d.skip_eps = 64.0f * std::ldexp(1.0f, std::ilogb(mx) - 23);
   }
+  {
+    // near entries (walk_count): within h + kNearMargin * h at the fill, when that is short of s
+    const float near = h + kNearMargin * h;
+    d.near2 = near < s ? near * near : d.s2;
+    d.near_move = near < s ? (0.5f * kNearMargin - kNearSlack) * h : FLT_MAX;
+  }
   d.dimx = (int)dims[0];
   d.dimy = (int)dims[1];
   d.dimz = (int)dims[2];
@@ -2705,6 +2948,14 @@ int upload_scenes(pbf_ctx* ctx) {
   ctx->dev.scene_first = ctx->d_scene_first;
   ctx->dev.nscenes = (int)ctx->scenes.size();
   return PBF_OK;
+}
+
+// The list arrays Dev carries.
+void bind_lists(pbf_ctx* ctx) {
+  ctx->dev.walk = ctx->walk;
+  ctx->dev.slot_key = ctx->keyH;
+  ctx->dev.cell_start = ctx->cell_start;
+  ctx->dev.cell_mark = ctx->cell_count;
 }
 
 template <typename T>
@@ -2972,18 +3223,29 @@ void launch_fill(pbf_ctx* ctx, const float4* pst) {
   // lists: the reference's order
   const bool staged = any_staged(ctx);
   ctx->lists_slot_order = fast && !staged;
-  Launch L(ctx, "fill_neighbors");
   const int n = (int)ctx->n;
-  if (ctx->lists_slot_order)
-    k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, ctx->stream>>>(
-        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, ctx->ref_order,
-        fw);
-  else if (staged)
-    k_fill2<true><<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, ctx->stream>>>(
-        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
-  else
-    k_fill2<false><<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, ctx->stream>>>(
-        ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
+  cudaStream_t s = ctx->stream;
+  if (!ctx->lists_slot_order) {
+    Launch L(ctx, "fill_neighbors");
+    const int grid = blocks_for(ctx->n, kFillBlock);
+    if (staged)
+      k_fill2<true><<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr,
+                                                ctx->cnt, ctx->err, tile_io(ctx), fw);
+    else
+      k_fill2<false><<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end,
+                                                 ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
+    return;
+  }
+  {
+    Launch L(ctx, "fill_neighbors");
+    k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start,
+                                                                      ctx->nbr, ctx->cnt, ctx->ref_order, fw,
+                                                                      ctx->rest);
+  }
+  Launch L(ctx, "fill_rest");
+  const int grid = std::min(blocks_for(ctx->n, kFillBlock), 16 * ctx->sms);  // a warp or more for every queued one
+  k_fill_rest<<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr,
+                                          ctx->cnt, ctx->err, ctx->ref_order, fw, ctx->rest);
 }
 
 // An upload forgets the fills before it: no lists counted at the cap.
@@ -3437,12 +3699,12 @@ int launches_per_step(const pbf_ctx* ctx) {
   // kernels only (the memsets are not), as launched eagerly (a captured
   // learned step runs its plain iterations in a conditional graph node and
   // launches fewer once converged): ext/predict/hash + 3 scan + radix
-  // passes x (histogram, 3 scan, scatter) + reorder + runs + fill +
+  // passes x (histogram, 3 scan, scatter) + reorder + runs + fill + [fast math: rest] +
   // K x (density/lambda, [exact: lambda fix-up], delta-p)
   // + (K==0: velocity) + 2 if gamma + 4 (visc, vort, apply, visc)
   const int sort = 5 * ctx->radix_passes;
-  const int fill = 2;  // runs, fill
-  if (persist_on(ctx)) return 1 + 3 + sort + 1 + fill + 1;  // ... reorder, runs, fill, the persistent step
+  const int fill = ctx->params.exact_math || any_staged(ctx) ? 2 : 3;  // runs, fill, [rest]
+  if (persist_on(ctx)) return 1 + 3 + sort + 1 + fill + 1;  // ... reorder, runs, fill, rest, the persistent step
   const int K = ctx->params.solve_steps;
   const int tail = (ctx->params.gamma != 0.0f ? 2 : 0) + 4;
   if (ctx->params.solver == 1 && !ctx->params.exact_math && !(ctx->params.residual_tol > 0.0f)) {
@@ -3537,7 +3799,7 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
       (rc = dalloc(ctx, &ctx->scan_part, (size_t)ctx->nscan_parts)) || (rc = dalloc(ctx, &ctx->err, 1)) ||
       (rc = dalloc(ctx, &ctx->nudge, 1)) ||
       (rc = dalloc(ctx, &ctx->pairs, C)) || (rc = dalloc(ctx, &ctx->pairs_sorted, C)) || (rc = dalloc(ctx, &ctx->nbr, pbf::list_entries(C, cap))) ||
-      (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
+      (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->walk, (C + 15) / 16 * 16)) || (rc = dalloc(ctx, &ctx->rest, (C + 31) / 32)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
       (rc = dalloc(ctx, &ctx->cnt, C)) || (rc = dalloc(ctx, &ctx->stage, 6 * C)) ||
       (rc = dalloc(ctx, &ctx->stage_i, std::max(C * cap + C, pbf::list_entries(C, cap)))) ||
       (rc = dalloc(ctx, &ctx->acc, 8)) ||
@@ -3556,6 +3818,7 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
       (rc = dalloc(ctx, &ctx->w2b, pbf::kMlpH * pbf::kMlpH)) || (rc = dalloc(ctx, &ctx->w2tb, pbf::kMlpH * pbf::kMlpH)))
     return bail(rc);
   ctx->wvis = reinterpret_cast<__half*>(ctx->stage_i);
+  bind_lists(ctx);
   if (!ctx->scenes.empty() &&
       ((rc = dalloc(ctx, &ctx->d_regions, ctx->regions.size())) ||
        (rc = dalloc(ctx, &ctx->d_scene_first, ctx->scene_first.size())) || (rc = upload_scenes(ctx))))
@@ -3617,6 +3880,7 @@ int pbf_set_params(pbf_ctx* ctx, const pbf_params* p) {
     ctx->lists_valid = false;
   ctx->params = *p;
   ctx->dev = d;
+  bind_lists(ctx);
   ctx->fast = pbf::make_fast(d);
   ctx->lstride = lstride;
   std::memcpy(ctx->dims, dims, sizeof(dims));

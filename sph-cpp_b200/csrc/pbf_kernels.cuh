@@ -74,6 +74,15 @@ struct Dev {
   // others (halo particles) as they are; span_end = 0xffffffff is every particle
   const uint32_t* span_orig;
   uint32_t span_end;
+  // fast math's lists, near entries first (k_fill_masks): the squared near
+  // radius, how far a particle may move before its neighbourhood is marked,
+  // the entries every list is walked for (kWalkAll: all), the bin key of every
+  // sorted slot, the bins' first slots and the bins' marks
+  float near2, near_move;
+  uint8_t* walk;
+  const uint32_t* slot_key;
+  const uint32_t* cell_start;
+  uint32_t* cell_mark;
 };
 
 // Whether the particle in home slot `i` is inside the stage's span.
