@@ -183,17 +183,16 @@ def kernel_bytes(name: str, n: int, nbar: float, K: int, nbins: int) -> float:
     per = {
         "ext_predict_hash": 16 + 16 + 16 + 16 + 4 + 4,           # x, v in; v, x*, key, rank out (+ histogram in L2)
         "scan_reduce": 4.0 * nbins / n,
-        "scan_partials": 8.0 * nbins / n / 4096,                # one partial sum per scan tile of 4096 bins, read and written
         "scan_apply": 8.0 * nbins / n,
-        "radix_hist": 4 + 2048.0 * 4 / 4096,                    # key in; per-tile digit counts out
-        "radix_scan": 2048.0 * 4 / 4096,                        # digit counts (3 launches, per launch)
-        "radix_scatter": 4 + 8 + 4 + 8,                         # key, pair in; key, pair out
+        "arrivals": 4 + 4 + 4 + 8,                              # key, arrival number, orig in; (orig, slot) out
+        "order_crowded": 4.0 / n,                               # the count of crowded bins
         "warm_features": 16 + L + 16 + 16 + 4 + 16 + 32,       # x*, list, v, last lambda in; (x*, l1), v, bf16 features out
         "warm_mlp": 32 + 16 + 16 + 4 + 4,                       # features, (x*, l1) in; (x*, lambda), lambda, sum out
         "residual_check": 16 + L + 16 + 4 + 4,                  # as density_lambda
-        "reorder": 8 + 4 + 3 * 16 + 3 * 16 + 4 + 4,             # pair, key, (x, x*, v) in and out, orig, key
+        "reorder": 8 + 4 + 3 * 16 + 3 * 16 + 4 + 4,             # arrival, key, (x, x*, v) in and out, orig, key
         "runs": 16 + 4,                                         # x* in (the previous slot's is a cache hit); run end out
-        "fill_neighbors": 16 + 4 * nbar + 4 + 8.0 * nbins / n + 1,  # own x*, list + count out, bin starts, order byte
+        "fill_neighbors": 16 + 4 * nbar + 4 + 8.0 * nbins / n + 2,  # own x*, list + counts out, bin starts, order byte
+        "fill_rest": 4.0 / n,                                   # the count of particles the mask fill left
         "density_lambda": 16 + L + 16 + 4 + 4,                  # x* in; list; (x*, lambda), rho, lambda out
         "lambda_fixup": 16 + L + 16 + 4,                        # exact math after a nudge: x* in, list; (x*, lambda), lambda out
         "dp_update": 16 + L + 16 + (32.0 / K),                  # (x*, lambda) in; list; x* out; last: x in, v out

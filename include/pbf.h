@@ -448,7 +448,7 @@ void pbf_group_destroy(pbf_group* g);
  * as pbf_find_neighbors + pbf_get_neighbors) for a caller-owned device point
  * set, using only a file-scope device array of PBF_NOALLOC_SCRATCH_BYTES that
  * every GPU loading the library holds until the process exits.  The sort is
- * the regular path's stable radix sort (linear in n however the points crowd
+ * the regular path's stable cell sort (linear in n however the points crowd
  * into bins) and crowded bins are walked run by run over bit-identical
  * positions, so no input makes the search quadratic in a bin's population
  * beyond the distance tests the reference itself makes.

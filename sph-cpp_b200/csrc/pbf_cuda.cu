@@ -9,13 +9,14 @@
 //   working buffers in the current step's sorted order
 //     posS, pstS, velS, origS, velT, xl = (x*, lambda) or (x*, |omega|)
 //   grid:   cell_count[B], cell_start[B+1] (begin/end of every bin),
-//           key/rank per particle, pairs[C] = (reference index << 32 | slot)
-//   lists:  nbr[cap][C] int32 slot indices (column-major: one warp reads one
-//           128-byte line per list entry), cnt[C]
+//           key and arrival number per particle, arrivals[C] = (reference
+//           index, slot)
+//   lists:  nbr: int32 slot indices in warp tiles (pbf::list_base), cnt[C],
+//           walk[C] = the entries a gather walks
 //
 // One step (pbf_step) is one CUDA graph of:
-//   memset counts -> ext+predict+hash+histogram -> 3-pass scan -> scatter ->
-//   per-cell stable fix-up -> reorder -> fill lists ->
+//   memset counts -> ext+predict+hash+histogram -> 2-pass scan -> arrivals ->
+//   crowded bins -> reorder -> runs -> fill lists (+ the rest) ->
 //   K x [density+lambda, delta-p+x* update (+ velocity on the last)] ->
 //   viscosity -> vorticity -> vorticity apply -> viscosity + x = x*.
 // Particles are kept in cell order between steps, so neighbours of a warp's
@@ -61,26 +62,12 @@ constexpr int kScanTile = kScanThreads * kScanItems;
 
 inline int blocks_for(size_t n, int b = kBlock) { return (int)((n + b - 1) / b); }
 
-// Digit histogram entries of the radix sort for up to `capacity` particles
-// (2^kRadixBits digits per 2^kRadixTileLog2-element tile); the constants are
-// checked against the kernels' below.
-constexpr int kRadixBitsHost = 11, kRadixTileHost = 4096;
-inline size_t radix_entries(size_t capacity) {
-  return ((capacity + kRadixTileHost - 1) / kRadixTileHost) * ((size_t)1 << kRadixBitsHost);
-}
 // Neighbor list rows are kListAlign-entry multiples long, so the fast gathers
 // read whole vectors of indices (the entries past a particle's count are
 // replaced by a dummy slot, one past the last particle, whose every kernel
 // term is exactly zero).
 constexpr int kListAlign = 32;
 inline size_t list_stride(int cap) { return ((size_t)cap + kListAlign - 1) / kListAlign * kListAlign; }
-
-// Passes to sort keys < nbins.
-inline int radix_passes_for(int nbins) {
-  int bits = 0;
-  while (bits < 31 && ((int64_t)1 << bits) < (int64_t)nbins) ++bits;
-  return (bits + kRadixBitsHost - 1) / kRadixBitsHost;
-}
 
 // ============================================================================
 // Kernels
@@ -210,42 +197,50 @@ __global__ void k_predict(Dev P, int n, const float4* __restrict__ pos, const fl
 // 0.56 / 1.07 / 2.25 / 2.14 at 4,096.
 constexpr uint32_t kRunBin = 4096;
 
-// calculate_bins (neighbors.h:120-125) + bin histogram; the radix sort's
-// input (key, pair) goes to the particle's reference index.  The word after
-// the histogram (cell_count[nbins]) is raised when a bin passes kRunBin
-// particles: only then does the list fill need the runs (k_runs).  The lanes
-// of a warp with the same key add to its count once (a settled dam piles
-// hundreds of thousands of particles into one bin, whose count would
-// otherwise take one atomic per particle, one after another).
-__device__ __forceinline__ void hash_out(const Dev& P, int a, uint32_t k, const uint32_t* __restrict__ orig,
-                                         uint32_t* key, uint32_t* cell_count, uint32_t* key_ref,
-                                         unsigned long long* pair_ref) {
+// Bins of more than this many particles are ordered by k_order_crowded, the
+// others by counting within the bin (k_reorder).
+constexpr uint32_t kCountBin = 1024;
+
+// The words after the bin histogram (cleared with it): kCrowdedRuns is raised
+// when a bin passes kRunBin particles (only then does the list fill need the
+// runs, k_runs), kCrowdedBins counts the bins past kCountBin.
+enum CrowdedWord { kCrowdedRuns = 0, kCrowdedBins = 1, kCrowdedWords = 2 };
+
+// calculate_bins (neighbors.h:120-125) + bin histogram; rank = the particle's
+// arrival number in its bin (any order).  The lanes of a warp with the same
+// key add to its count once (a settled dam piles hundreds of thousands of
+// particles into one bin, whose count would otherwise take one atomic per
+// particle, one after another).
+__device__ __forceinline__ void hash_out(int nbins, int a, uint32_t k, uint32_t* key, uint32_t* rank,
+                                         uint32_t* cell_count, uint32_t* crowded) {
   key[a] = k;
+  const int lane = threadIdx.x & 31;
   const unsigned same = __match_any_sync(__activemask(), k);
-  if ((threadIdx.x & 31) == (unsigned)(__ffs(same) - 1)) {
-    const uint32_t add = (uint32_t)__popc(same), old = atomicAdd(&cell_count[k], add);
-    if (old <= kRunBin && old + add > kRunBin) atomicOr(&cell_count[P.nbins], 1u);
+  const int leader = __ffs(same) - 1;
+  uint32_t old = 0;
+  if (lane == leader) {
+    const uint32_t add = (uint32_t)__popc(same);
+    old = atomicAdd(&cell_count[k], add);
+    if (old <= kRunBin && old + add > kRunBin) atomicOr(&cell_count[nbins + kCrowdedRuns], 1u);
+    if (old <= kCountBin && old + add > kCountBin) crowded[atomicAdd(&cell_count[nbins + kCrowdedBins], 1u)] = k;
   }
-  const uint32_t o = orig[a];
-  key_ref[o] = k;
-  pair_ref[o] = ((unsigned long long)o << 32) | (unsigned long long)(uint32_t)a;
+  rank[a] = __shfl_sync(same, old, leader) + (uint32_t)__popc(same & ((1u << lane) - 1u));
 }
 
-__global__ void k_hash(Dev P, int n, const float4* __restrict__ pst, const uint32_t* __restrict__ orig,
-                       uint32_t* key, uint32_t* cell_count, uint32_t* key_ref, unsigned long long* pair_ref,
-                       uint32_t* err) {
+__global__ void k_hash(Dev P, int n, const float4* __restrict__ pst, uint32_t* key, uint32_t* rank,
+                       uint32_t* cell_count, uint32_t* crowded, uint32_t* err) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   const float4 s = pst[a];
   uint32_t k;
   if (!pbf::bin_of(P, pbf::region_of(P, a), s.x, s.y, s.z, k)) atomicOr(err, PBF_FLAG_KEY_RANGE);
-  hash_out(P, a, k, orig, key, cell_count, key_ref, pair_ref);
+  hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
 // Fused apply_external_forces + predict_positions + calculate_bins + histogram.
 __global__ void k_ext_predict_hash(Dev P, int n, const float4* __restrict__ pos, float4* vel, float4* pst,
-                                   const uint32_t* __restrict__ orig, uint32_t* key, uint32_t* cell_count,
-                                   uint32_t* key_ref, unsigned long long* pair_ref, uint32_t* err) {
+                                   uint32_t* key, uint32_t* rank, uint32_t* cell_count, uint32_t* crowded,
+                                   uint32_t* err) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   float4 v = vel[a];
@@ -256,7 +251,7 @@ __global__ void k_ext_predict_hash(Dev P, int n, const float4* __restrict__ pos,
   pst[a] = make_float4(s.x, s.y, s.z, 0.0f);
   uint32_t k;
   if (!pbf::bin_of(P, R, s.x, s.y, s.z, k)) atomicOr(err, PBF_FLAG_KEY_RANGE);
-  hash_out(P, a, k, orig, key, cell_count, key_ref, pair_ref);
+  hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
 // ---- exclusive scan of cell_count[0..m-1] (+ total at [m]) -> cell_start ----
@@ -300,25 +295,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __
   if (threadIdx.x == 0) partial[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_partials(uint32_t* partial, int np) {
-  __shared__ uint32_t ws[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (int base = 0; base < np; base += kScanThreads) {
-    const int i = base + threadIdx.x;
-    const uint32_t v = i < np ? partial[i] : 0u;
-    uint32_t total;
-    const uint32_t ex = block_exclusive_scan(v, ws, total);
-    const uint32_t c = carry;
-    if (i < np) partial[i] = ex + c;
-    __syncthreads();
-    if (threadIdx.x == 0) carry = c + total;
-    __syncthreads();
-  }
-}
-
 // out[0..m] (m+1 entries): exclusive prefix of in[0..m-1], out[m] = total.
+// Every block adds up the tiles' sums before its own (310 at 1M particles): a
+// launch that scanned them took 2 us of every step.
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in, int m,
                                                              const uint32_t* __restrict__ partial,
                                                              uint32_t* out) {
@@ -331,8 +310,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
     v[i] = base + i < (size_t)m ? in[base + i] : 0u;
     s += v[i];
   }
+  uint32_t before = 0;
+  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kScanThreads) before += partial[i];
   uint32_t total;
-  uint32_t run = block_exclusive_scan(s, ws, total) + partial[blockIdx.x];
+  block_exclusive_scan(before, ws, total);
+  before = total;
+  __syncthreads();  // ws is written again
+  uint32_t run = block_exclusive_scan(s, ws, total) + before;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     if (base + i <= (size_t)m) out[base + i] = run;
@@ -340,118 +324,103 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
   }
 }
 
-// ---- stable LSD radix sort of (bin key, pair) ----
-// The hash kernels write every particle's key and pair (reference index << 32
-// | home slot) at its reference index, so the input is in reference-index
-// order and a stable sort by key orders every bin by reference index: the
-// permutation of the reference's stable sort_by_key (neighbors.h:130-132).
-// kRadixBits-bit digits, least significant first; each pass is a per-tile
-// digit histogram (digit-major: hist[d * tiles + tile]), an exclusive scan of
-// it (the scan kernels above) and a stable scatter.  The work is O(n) per pass
-// however the particles crowd into bins.
-constexpr int kRadixBits = 11;
-constexpr int kRadixDigits = 1 << kRadixBits;
-constexpr int kRadixThreads = 256;
-constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kRadixItems = 16;
-constexpr int kRadixTile = kRadixThreads * kRadixItems;  // elements per tile (block)
-static_assert(kRadixBits == kRadixBitsHost && kRadixTile == kRadixTileHost, "radix buffer sizing");
-
-__device__ __forceinline__ uint32_t radix_digit(uint32_t key, int shift) {
-  return (key >> shift) & (uint32_t)(kRadixDigits - 1);
+// ---- the cell sort ----
+// The reference's stable sort_by_key (neighbors.h:130-132) orders every bin by
+// reference index.  The bin histogram and its scan place every bin, so only
+// the order within bins is left to find, and bins are small (14 particles at
+// rest): k_arrivals writes every particle's reference index and slot at its
+// bin's start plus its arrival number, and k_reorder counts the smaller
+// indices in the bin.  Bins of more than kCountBin particles, where that
+// count would be quadratic, are ordered by k_order_crowded: linear in the bin
+// plus a bitmap of all indices.  A stable radix sort of (key, index) and its
+// scans took 10 launches, 51 us a step at 65k particles and 73 us at 1M; what
+// takes their place (k_arrivals, k_order_crowded's launch, the count) 5 and
+// 10 us.  Bound by the scattered 8-byte stores of k_arrivals and, in
+// k_reorder, by the state's bytes.
+__global__ void k_arrivals(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
+                           const uint32_t* __restrict__ orig, const uint32_t* __restrict__ cell_start,
+                           uint2* arrivals) {
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a >= n) return;
+  arrivals[cell_start[key[a]] + rank[a]] = make_uint2(orig ? orig[a] : (uint32_t)a, (uint32_t)a);
 }
 
-__global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* __restrict__ keys, int n, int shift,
-                                                             int tiles, uint32_t* hist) {
-  __shared__ uint32_t cnt[kRadixDigits];
-  for (int d = threadIdx.x; d < kRadixDigits; d += kRadixThreads) cnt[d] = 0u;
-  __syncthreads();
-  const size_t base = (size_t)blockIdx.x * kRadixTile;
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < kRadixTile; i += kRadixThreads) {  // warp-uniform trip count
-    const size_t j = base + i;
-    const bool live = j < (size_t)n;
-    const uint32_t d = live ? radix_digit(keys[j], shift) : (uint32_t)kRadixDigits;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);  // one shared-memory add per distinct digit
-    if (live && (peers & ((1u << lane) - 1u)) == 0u) atomicAdd(&cnt[d], (uint32_t)__popc(peers));
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < kRadixDigits; d += kRadixThreads) hist[(size_t)d * tiles + blockIdx.x] = cnt[d];
-}
-
-// Stable scatter of one tile.  Warp w owns elements [w*32*kRadixItems,
-// (w+1)*32*kRadixItems) of the tile, walked item by item (element = item*32 +
-// lane): equal digits in one item are ranked by lane (__match_any_sync) and a
-// per-warp running count per digit carries the rank across items; the warps'
-// counts then become exclusive prefixes over the warps, so ranks follow the
-// element order across the tile, and tiles follow each other through the
-// scanned histogram.  keys_out may be null (last pass).
-__global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t* __restrict__ keys_in,
-                                                                const unsigned long long* __restrict__ vals_in,
-                                                                int n, int shift, int tiles,
-                                                                const uint32_t* __restrict__ offsets,
-                                                                uint32_t* keys_out, unsigned long long* vals_out) {
-  __shared__ uint16_t wcnt[kRadixWarps * kRadixDigits];  // counts <= 32*kRadixItems, prefixes <= kRadixTile
-  for (int d = threadIdx.x; d < kRadixWarps * kRadixDigits; d += kRadixThreads) wcnt[d] = 0;
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  uint16_t* mine = wcnt + warp * kRadixDigits;
-  const size_t wbase = (size_t)blockIdx.x * kRadixTile + (size_t)warp * 32 * kRadixItems;
-  uint32_t dig[kRadixItems], rk[kRadixItems];
-#pragma unroll
-  for (int it = 0; it < kRadixItems; ++it) {
-    const size_t j = wbase + (size_t)it * 32 + lane;
-    const bool live = j < (size_t)n;
-    const uint32_t d = live ? radix_digit(keys_in[j], shift) : (uint32_t)kRadixDigits;
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t base = live ? (uint32_t)mine[d] : 0u;
-    __syncwarp();
-    if (live && (peers & lt) == 0u) mine[d] = (uint16_t)(base + (uint32_t)__popc(peers));
-    __syncwarp();
-    dig[it] = d;
-    rk[it] = base + (uint32_t)__popc(peers & lt);
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < kRadixDigits; d += kRadixThreads) {
-    uint32_t run = 0;
-#pragma unroll
-    for (int w = 0; w < kRadixWarps; ++w) {
-      const uint32_t c = wcnt[w * kRadixDigits + d];
-      wcnt[w * kRadixDigits + d] = (uint16_t)run;
-      run += c;
+// Crowded bins, a block each: the bin's reference indices as bits, the bits'
+// prefix sums, and every particle's place from the two.  bits: `regions`
+// regions of 2 * words words (words = the bitmap of n indices), one per block.
+constexpr int kOrderThreads = 1024;
+__global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, const uint32_t* __restrict__ crowded_bins,
+                                                                 const uint32_t* __restrict__ crowded,
+                                                                 const uint32_t* __restrict__ cell_start,
+                                                                 const uint2* __restrict__ arrivals, uint32_t* bits,
+                                                                 uint32_t* place) {
+  __shared__ uint32_t ws[32];
+  const uint32_t bins = *crowded_bins;
+  uint32_t* mine = bits + 2 * (size_t)words * blockIdx.x;
+  uint32_t* before = mine + words;
+  for (uint32_t i = blockIdx.x; i < bins; i += gridDim.x) {
+    const uint32_t s = cell_start[crowded[i]], e = cell_start[crowded[i] + 1];
+    for (int w = threadIdx.x; w < words; w += kOrderThreads) __stcg(mine + w, 0u);
+    __syncthreads();
+#pragma unroll 8
+    for (uint32_t j = s + threadIdx.x; j < e; j += kOrderThreads) {
+      const uint32_t o = __ldg(&arrivals[j].x);
+      atomicOr(mine + (o >> 5), 1u << (o & 31u));
     }
+    __syncthreads();
+    uint32_t run = 0;
+    for (int w0 = 0; w0 < words; w0 += kOrderThreads) {
+      const int w = w0 + (int)threadIdx.x;
+      uint32_t total;
+      const uint32_t ex = block_exclusive_scan(w < words ? (uint32_t)__popc(__ldcg(mine + w)) : 0u, ws, total);
+      if (w < words) before[w] = run + ex;
+      run += total;
+      __syncthreads();  // ws is written again
+    }
+#pragma unroll 8
+    for (uint32_t j = s + threadIdx.x; j < e; j += kOrderThreads) {
+      const uint32_t o = __ldg(&arrivals[j].x);
+      place[j] = s + before[o >> 5] + (uint32_t)__popc(__ldcg(mine + (o >> 5)) & ((1u << (o & 31u)) - 1u));
+    }
+    __syncthreads();
   }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < kRadixItems; ++it) {
-    const size_t j = wbase + (size_t)it * 32 + lane;
-    if (j >= (size_t)n) continue;
-    const uint32_t d = dig[it];
-    const uint32_t pos = offsets[(size_t)d * tiles + blockIdx.x] + (uint32_t)mine[d] + rk[it];
-    vals_out[pos] = vals_in[j];
-    if (keys_out) keys_out[pos] = keys_in[j];
-  }
+}
+
+// What the sort leaves for the gathers of the state into cell order.
+struct CellSort {
+  const uint2* arrivals;  // (reference index, slot), every bin's in its range
+  const uint32_t *key, *cell_start, *place;
+};
+
+// The sorted slot of arrival j (reference index o, bin key k).
+__device__ __forceinline__ uint32_t sorted_slot(const CellSort& S, uint32_t j, uint32_t o, uint32_t k) {
+  const uint32_t s = S.cell_start[k], e = S.cell_start[k + 1];
+  if (e - s > kCountBin) return S.place[j];
+  uint32_t at = s;
+#pragma unroll 4
+  for (uint32_t i = s; i < e; ++i) at += S.arrivals[i].x < o ? 1u : 0u;
+  return at;
 }
 
 // Gather the state into sorted order.  FULL = also scratch and lambda (the
 // per-stage path, where every reference array must follow its particle); the
 // fused step passes the learned warm start's lambda sums as lamH/lamS.
 template <bool FULL>
-__global__ void k_reorder(int n, const unsigned long long* __restrict__ pairs, const uint32_t* __restrict__ key,
-                          const float4* __restrict__ posH, const float4* __restrict__ pstH,
+__global__ void k_reorder(int n, CellSort S, const float4* __restrict__ posH, const float4* __restrict__ pstH,
                           const float4* __restrict__ velH, const float4* __restrict__ scrH,
                           const float* __restrict__ lamH, float4* posS, float4* pstS, float4* velS,
                           float4* scrS, float* lamS, uint32_t* origS, uint32_t* keyH) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  const unsigned long long pr = pairs[b];
-  const uint32_t a = (uint32_t)(pr & 0xffffffffull);
-  origS[b] = (uint32_t)(pr >> 32);
-  keyH[b] = key[a];
-  posS[b] = posH[a];
-  pstS[b] = pstH[a];
-  velS[b] = velH[a];
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const uint2 arrival = S.arrivals[j];
+  const uint32_t a = arrival.y, k = S.key[a];
+  const float4 pos = posH[a], pst = pstH[a], vel = velH[a];
+  const uint32_t b = sorted_slot(S, (uint32_t)j, arrival.x, k);
+  origS[b] = arrival.x;
+  keyH[b] = k;
+  posS[b] = pos;
+  pstS[b] = pst;
+  velS[b] = vel;
   if (FULL) scrS[b] = scrH[a];
   if (lamS) lamS[b] = lamH[a];  // FULL: lambda; fused step: last step's lambda sum, when kept
 }
@@ -2691,15 +2660,11 @@ struct pbf_ctx {
   float *lamH = nullptr, *lamS = nullptr;
   uint32_t *origH = nullptr, *origS = nullptr, *key = nullptr, *keyH = nullptr;
   uint32_t* run_end = nullptr;  // per sorted slot: end of its run of bit-identical x* (k_runs)
-  // radix sort: keys at the reference index and their ping-pong twin, digit
-  // histograms, their scan, scan partials; `sorted` = the pair buffer holding
-  // the sorted pairs after the last pass
-  uint32_t *key_ref = nullptr, *key_alt = nullptr, *radix_hist = nullptr, *radix_off = nullptr,
-           *radix_parts = nullptr;
-  int radix_passes = 0;
-  unsigned long long* sorted = nullptr;
+  // cell sort: arrival numbers, (reference index, slot) at cell start + arrival
+  // number, the places k_order_crowded finds, the crowded bins
+  uint32_t *rank = nullptr, *place = nullptr, *crowded = nullptr;
+  uint2* arrivals = nullptr;
   uint32_t *cell_count = nullptr, *cell_start = nullptr, *scan_part = nullptr, *err = nullptr, *nudge = nullptr;
-  unsigned long long *pairs = nullptr, *pairs_sorted = nullptr;
   int32_t *nbr = nullptr, *cnt = nullptr;
   __half* wvis = nullptr;  // XSPH weights per list entry (the list's layout, half precision), in stage_i's memory
   float* stage = nullptr;  // 6*C floats: two AoS float3 staging areas
@@ -3155,8 +3120,20 @@ int harvest_times(pbf_ctx* ctx) {
 }
 
 // ---- neighbor build ----
-// Hash + histogram must already have produced key/rank/cell_count.
-void launch_sort_to_pairs(pbf_ctx* ctx) {
+CellSort cell_sort(const pbf_ctx* ctx) { return CellSort{ctx->arrivals, ctx->key, ctx->cell_start, ctx->place}; }
+
+// Words of a bitmap of n indices, and the blocks k_order_crowded gets: as many
+// as have room for a bitmap and its prefix sums in `room` words, at most two
+// per SM (six words a particle leave 96).
+int bitmap_words(size_t n) { return (int)((n + 31) / 32); }
+int order_grid(size_t n, size_t room, int sms) {
+  return (int)std::max<size_t>(1, std::min<size_t>(room / (2 * (size_t)bitmap_words(n)), 2 * (size_t)sms));
+}
+
+// Bin bounds and the arrivals of every bin; the hash must already have
+// produced key, rank, cell_count and the crowded bins.  k_order_crowded's
+// bitmaps lie in the host staging area, which no step uses.
+void launch_cell_sort(pbf_ctx* ctx) {
   const int n = (int)ctx->n;
   const int m = ctx->nbins;  // scan m entries -> m+1 outputs
   cudaStream_t s = ctx->stream;
@@ -3165,49 +3142,17 @@ void launch_sort_to_pairs(pbf_ctx* ctx) {
     k_scan_reduce<<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part);
   }
   {
-    Launch L(ctx, "scan_partials");
-    k_scan_partials<<<1, kScanThreads, 0, s>>>(ctx->scan_part, ctx->nscan_parts);
-  }
-  {
     Launch L(ctx, "scan_apply");
     k_scan_apply<<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
   }
-  // stable LSD radix sort of (key, pair), input in reference-index order
-  const int tiles = (int)(((size_t)n + kRadixTile - 1) / kRadixTile);
-  const int hm = kRadixDigits * tiles;
-  const int hp = (int)(((size_t)hm + 1 + kScanTile - 1) / kScanTile);
-  uint32_t* kin = ctx->key_ref;
-  uint32_t* kout = ctx->key_alt;
-  unsigned long long* vin = ctx->pairs;
-  unsigned long long* vout = ctx->pairs_sorted;
-  for (int p = 0; p < ctx->radix_passes; ++p) {
-    const int shift = p * kRadixBits;
-    const bool last = p == ctx->radix_passes - 1;
-    {
-      Launch L(ctx, "radix_hist");
-      k_radix_hist<<<tiles, kRadixThreads, 0, s>>>(kin, n, shift, tiles, ctx->radix_hist);
-    }
-    {
-      Launch L(ctx, "radix_scan");
-      k_scan_reduce<<<hp, kScanThreads, 0, s>>>(ctx->radix_hist, hm, ctx->radix_parts);
-    }
-    {
-      Launch L(ctx, "radix_scan");
-      k_scan_partials<<<1, kScanThreads, 0, s>>>(ctx->radix_parts, hp);
-    }
-    {
-      Launch L(ctx, "radix_scan");
-      k_scan_apply<<<hp, kScanThreads, 0, s>>>(ctx->radix_hist, hm, ctx->radix_parts, ctx->radix_off);
-    }
-    {
-      Launch L(ctx, "radix_scatter");
-      k_radix_scatter<<<tiles, kRadixThreads, 0, s>>>(kin, vin, n, shift, tiles, ctx->radix_off,
-                                                     last ? nullptr : kout, vout);
-    }
-    std::swap(kin, kout);
-    std::swap(vin, vout);
+  {
+    Launch L(ctx, "arrivals");
+    k_arrivals<<<blocks_for(n), kBlock, 0, s>>>(n, ctx->key, ctx->rank, ctx->origH, ctx->cell_start, ctx->arrivals);
   }
-  ctx->sorted = vin;  // the last pass's output (the input itself when no pass is needed)
+  Launch L(ctx, "order_crowded");
+  k_order_crowded<<<order_grid(ctx->n, 6 * ctx->capacity, ctx->sms), kOrderThreads, 0, s>>>(
+      bitmap_words(ctx->n), ctx->cell_count + m + kCrowdedBins, ctx->crowded, ctx->cell_start, ctx->arrivals,
+      reinterpret_cast<uint32_t*>(ctx->stage), ctx->place);
 }
 
 void launch_fill(pbf_ctx* ctx, const float4* pst) {
@@ -3216,7 +3161,7 @@ void launch_fill(pbf_ctx* ctx, const float4* pst) {
   {
     Launch L(ctx, "runs");
     k_runs<<<blocks_for(ctx->n, kRunBlock), kRunBlock, 0, ctx->stream>>>((int)ctx->n, pst, ctx->run_end,
-                                                                         ctx->cell_count + ctx->nbins, fw);
+                                                                         ctx->cell_count + ctx->nbins + kCrowdedRuns, fw);
   }
   // fast math: lists in slot order (the gathers' sums in any order are within
   // the fast path's tolerance); exact math and the staged gathers' 16-bit
@@ -3508,17 +3453,17 @@ void launch_step_t(pbf_ctx* ctx) {
   const Dev& P = ctx->dev;
   cudaStream_t s = ctx->stream;
   const int g = blocks_for(n);
-  cudaMemsetAsync(ctx->cell_count, 0, sizeof(uint32_t) * ((size_t)ctx->nbins + 1), s);  // + the crowded flag
+  cudaMemsetAsync(ctx->cell_count, 0, sizeof(uint32_t) * ((size_t)ctx->nbins + kCrowdedWords), s);  // + the crowded words
   {
     Launch L(ctx, "ext_predict_hash");
-    k_ext_predict_hash<<<g, kBlock, 0, s>>>(P, n, ctx->posH, ctx->velH, ctx->pstH, ctx->origH, ctx->key,
-                                            ctx->cell_count, ctx->key_ref, ctx->pairs, ctx->err);
+    k_ext_predict_hash<<<g, kBlock, 0, s>>>(P, n, ctx->posH, ctx->velH, ctx->pstH, ctx->key, ctx->rank,
+                                            ctx->cell_count, ctx->crowded, ctx->err);
   }
-  launch_sort_to_pairs(ctx);
+  launch_cell_sort(ctx);
   {
     Launch L(ctx, "reorder");
     const bool keep = !X && (ctx->recording || ctx->params.solver == 1);
-    k_reorder<false><<<g, kBlock, 0, s>>>(n, ctx->sorted, ctx->key, ctx->posH, ctx->pstH, ctx->velH, nullptr,
+    k_reorder<false><<<g, kBlock, 0, s>>>(n, cell_sort(ctx), ctx->posH, ctx->pstH, ctx->velH, nullptr,
                                           keep ? ctx->lamsumH : nullptr, ctx->posS, ctx->pstS, ctx->velS, nullptr,
                                           keep ? ctx->lamprevS : nullptr, ctx->origS, ctx->keyH);
   }
@@ -3698,30 +3643,29 @@ void launch_step(pbf_ctx* ctx) {
 int launches_per_step(const pbf_ctx* ctx) {
   // kernels only (the memsets are not), as launched eagerly (a captured
   // learned step runs its plain iterations in a conditional graph node and
-  // launches fewer once converged): ext/predict/hash + 3 scan + radix
-  // passes x (histogram, 3 scan, scatter) + reorder + runs + fill + [fast math: rest] +
+  // launches fewer once converged): ext/predict/hash + sort + reorder + runs + fill + [fast math: rest] +
   // K x (density/lambda, [exact: lambda fix-up], delta-p)
   // + (K==0: velocity) + 2 if gamma + 4 (visc, vort, apply, visc)
-  const int sort = 5 * ctx->radix_passes;
+  const int sort = 4;  // 2 scan, arrivals, crowded bins
   const int fill = ctx->params.exact_math || any_staged(ctx) ? 2 : 3;  // runs, fill, [rest]
-  if (persist_on(ctx)) return 1 + 3 + sort + 1 + fill + 1;  // ... reorder, runs, fill, rest, the persistent step
+  if (persist_on(ctx)) return 1 + sort + 1 + fill + 1;  // ... reorder, runs, fill, rest, the persistent step
   const int K = ctx->params.solve_steps;
   const int tail = (ctx->params.gamma != 0.0f ? 2 : 0) + 4;
   if (ctx->params.solver == 1 && !ctx->params.exact_math && !(ctx->params.residual_tol > 0.0f)) {
     // learned, a fixed count: warm iteration (features, network, delta-p) + (iters-1) x (density, delta-p)
     // + velocity
     const int it = ctx->params.max_iterations > 0 ? ctx->params.max_iterations : 1;
-    return 1 + 3 + sort + 1 + fill + 3 + 2 * (it - 1) + 1 + tail;
+    return 1 + sort + 1 + fill + 3 + 2 * (it - 1) + 1 + tail;
   }
   if (ctx->params.solver == 1 && !ctx->params.exact_math) {
     // learned: warm iteration (features, network, delta-p) + (iters-1) x (check, [sampled checks:
     // density/lambda,] delta-p) + final check + velocity
     const int it = ctx->params.max_iterations > 0 ? ctx->params.max_iterations : 1;
     const bool sampled = ctx->params.residual_sample > 1 && !ctx->tune.staged[PBF_TUNE_DENSITY];
-    return 1 + 3 + sort + 1 + fill + 3 + (sampled ? 3 : 2) * (it - 1) + 1 + 1 + tail;
+    return 1 + sort + 1 + fill + 3 + (sampled ? 3 : 2) * (it - 1) + 1 + 1 + tail;
   }
   const int per_iter = ctx->params.exact_math ? 3 : 2;
-  return 1 + 3 + sort + 1 + fill + per_iter * K + (K == 0 ? 1 : 0) + tail;
+  return 1 + sort + 1 + fill + per_iter * K + (K == 0 ? 1 : 0) + tail;
 }
 
 }  // namespace
@@ -3754,7 +3698,6 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
   ctx->capacity = capacity;
   ctx->nbins = ctx->dev.nbins;
   ctx->nbins_cap = ctx->nbins;
-  ctx->radix_passes = radix_passes_for(ctx->nbins);
   ctx->nscan_parts = (int)(((size_t)ctx->nbins + 1 + kScanTile - 1) / kScanTile);
   auto bail = [&](int code) {
     g_create_error = ctx->error;
@@ -3789,16 +3732,14 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
       (rc = dalloc(ctx, &ctx->velS, C + 1)) || (rc = dalloc(ctx, &ctx->scrS, C)) || (rc = dalloc(ctx, &ctx->xl, C + 1)) ||
       (rc = dalloc(ctx, &ctx->velT, C + 1)) || (rc = dalloc(ctx, &ctx->lamH, C)) || (rc = dalloc(ctx, &ctx->lamS, C)) ||
       (rc = dalloc(ctx, &ctx->origH, C)) || (rc = dalloc(ctx, &ctx->origS, C)) || (rc = dalloc(ctx, &ctx->key, C)) ||
-      (rc = dalloc(ctx, &ctx->key_ref, C)) || (rc = dalloc(ctx, &ctx->key_alt, C)) ||
+      (rc = dalloc(ctx, &ctx->rank, C)) || (rc = dalloc(ctx, &ctx->place, C)) ||
+      (rc = dalloc(ctx, &ctx->crowded, C / kCountBin + 1)) || (rc = dalloc(ctx, &ctx->arrivals, C)) ||
       (rc = dalloc(ctx, &ctx->keyH, C)) || (rc = dalloc(ctx, &ctx->run_end, C)) ||
-      (rc = dalloc(ctx, &ctx->radix_hist, radix_entries(C))) ||
-      (rc = dalloc(ctx, &ctx->radix_off, radix_entries(C) + 1)) ||
-      (rc = dalloc(ctx, &ctx->radix_parts, (radix_entries(C) + 1 + kScanTile - 1) / kScanTile)) ||
-      (rc = dalloc(ctx, &ctx->cell_count, (size_t)ctx->nbins + 1)) ||
+      (rc = dalloc(ctx, &ctx->cell_count, (size_t)ctx->nbins + kCrowdedWords)) ||
       (rc = dalloc(ctx, &ctx->cell_start, (size_t)ctx->nbins + 1)) ||
       (rc = dalloc(ctx, &ctx->scan_part, (size_t)ctx->nscan_parts)) || (rc = dalloc(ctx, &ctx->err, 1)) ||
       (rc = dalloc(ctx, &ctx->nudge, 1)) ||
-      (rc = dalloc(ctx, &ctx->pairs, C)) || (rc = dalloc(ctx, &ctx->pairs_sorted, C)) || (rc = dalloc(ctx, &ctx->nbr, pbf::list_entries(C, cap))) ||
+      (rc = dalloc(ctx, &ctx->nbr, pbf::list_entries(C, cap))) ||
       (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->walk, (C + 15) / 16 * 16)) || (rc = dalloc(ctx, &ctx->rest, (C + 31) / 32)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
       (rc = dalloc(ctx, &ctx->cnt, C)) || (rc = dalloc(ctx, &ctx->stage, 6 * C)) ||
       (rc = dalloc(ctx, &ctx->stage_i, std::max(C * cap + C, pbf::list_entries(C, cap)))) ||
@@ -3885,7 +3826,6 @@ int pbf_set_params(pbf_ctx* ctx, const pbf_params* p) {
   ctx->lstride = lstride;
   std::memcpy(ctx->dims, dims, sizeof(dims));
   ctx->nbins = d.nbins;
-  ctx->radix_passes = radix_passes_for(ctx->nbins);
   ctx->nscan_parts = (int)(((size_t)ctx->nbins + 1 + kScanTile - 1) / kScanTile);
   if (batch) {
     ctx->regions = regions;
@@ -4213,11 +4153,10 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
   }
   const int n = (int)ctx->n, g = blocks_for(ctx->n);
   cudaStream_t s = ctx->stream;
-  CK(cudaMemsetAsync(ctx->cell_count, 0, sizeof(uint32_t) * ((size_t)ctx->nbins + 1), s));  // + the crowded flag
-  k_hash<<<g, kBlock, 0, s>>>(ctx->dev, n, ctx->pstH, ctx->origH, ctx->key, ctx->cell_count, ctx->key_ref,
-                              ctx->pairs, ctx->err);
-  launch_sort_to_pairs(ctx);
-  k_reorder<true><<<g, kBlock, 0, s>>>(n, ctx->sorted, ctx->key, ctx->posH, ctx->pstH, ctx->velH, ctx->scrH,
+  CK(cudaMemsetAsync(ctx->cell_count, 0, sizeof(uint32_t) * ((size_t)ctx->nbins + kCrowdedWords), s));  // + the crowded words
+  k_hash<<<g, kBlock, 0, s>>>(ctx->dev, n, ctx->pstH, ctx->key, ctx->rank, ctx->cell_count, ctx->crowded, ctx->err);
+  launch_cell_sort(ctx);
+  k_reorder<true><<<g, kBlock, 0, s>>>(n, cell_sort(ctx), ctx->posH, ctx->pstH, ctx->velH, ctx->scrH,
                                        ctx->lamH, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS,
                                        ctx->keyH);
   const size_t f4 = sizeof(float4) * ctx->n;
@@ -5115,10 +5054,9 @@ int pbf_launches_per_step(pbf_ctx* ctx, int64_t* out) {
 //             the bin histogram (calculate_bins, neighbors.h:120-125)
 //   bounds    exclusive scan of the histogram = begin/end of every bin
 //             (find_bin_bounds, neighbors.h:137-148)
-//   sort      the stable LSD radix passes of the regular path, ping-ponging
-//             between two key/pair buffers of the array: O(n) per pass however
-//             particles crowd into bins (sort_bins, neighbors.h:130-132)
-//   gather    positions into sorted order, with their reference indices
+//   sort      the regular path's: arrivals at their bins' starts, crowded
+//             bins ordered by a bitmap, the others by counting while the
+//             positions are gathered (sort_bins, neighbors.h:130-132)
 //   runs      runs of bit-identical positions among consecutive sorted slots
 //   fill      the lists in reference index space (fill_neighbors,
 //             neighbors.h:197-230); a bin of more than kRunBin particles is
@@ -5132,26 +5070,23 @@ constexpr size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign;
 constexpr size_t kNaN = PBF_NOALLOC_MAX_PARTICLES;
 constexpr size_t kNaB = PBF_NOALLOC_MAX_BINS;
 constexpr size_t kNaParts = (kNaB + 1 + kScanTile - 1) / kScanTile;
-constexpr size_t kNaTiles = (kNaN + kRadixTile - 1) / kRadixTile;
-constexpr size_t kNaHist = (size_t)kRadixDigits * kNaTiles;
-constexpr size_t kNaHistParts = (kNaHist + 1 + kScanTile - 1) / kScanTile;
+constexpr size_t kNaWords = kNaN / 32, kNaOrderBlocks = 16;  // k_order_crowded's bitmap of the indices, its blocks
 // layout of the scratch array (byte offsets)
 constexpr size_t kOffCount = 0;
-constexpr size_t kOffStart = align_up(kOffCount + 4 * kNaB);
+constexpr size_t kOffStart = align_up(kOffCount + 4 * (kNaB + kCrowdedWords));
 constexpr size_t kOffParts = align_up(kOffStart + 4 * (kNaB + 1));
-constexpr size_t kOffKeyA = align_up(kOffParts + 4 * kNaParts);
-constexpr size_t kOffKeyB = align_up(kOffKeyA + 4 * kNaN);
-constexpr size_t kOffPairA = align_up(kOffKeyB + 4 * kNaN);
-constexpr size_t kOffPairB = align_up(kOffPairA + 8 * kNaN);
-constexpr size_t kOffHist = align_up(kOffPairB + 8 * kNaN);
-constexpr size_t kOffHistOff = align_up(kOffHist + 4 * kNaHist);
-constexpr size_t kOffHistParts = align_up(kOffHistOff + 4 * (kNaHist + 1));
-constexpr size_t kOffRunEnd = align_up(kOffHistParts + 4 * kNaHistParts);
+constexpr size_t kOffKey = align_up(kOffParts + 4 * kNaParts);
+constexpr size_t kOffRank = align_up(kOffKey + 4 * kNaN);
+constexpr size_t kOffArrivals = align_up(kOffRank + 4 * kNaN);
+constexpr size_t kOffPlace = align_up(kOffArrivals + 8 * kNaN);
+constexpr size_t kOffCrowded = align_up(kOffPlace + 4 * kNaN);
+constexpr size_t kOffBits = align_up(kOffCrowded + 4 * (kNaN / kCountBin + 1));
+constexpr size_t kOffRunEnd = align_up(kOffBits + 4 * 2 * kNaWords * kNaOrderBlocks);
 constexpr size_t kOffSortedX = align_up(kOffRunEnd + 4 * kNaN);
-constexpr size_t kOffSortedId = align_up(kOffSortedX + 16 * kNaN);
+constexpr size_t kOffSortedId = align_up(kOffSortedX + 16 * (kNaN + kMaskOver));
 constexpr size_t kOffErr = align_up(kOffSortedId + 4 * kNaN);
-constexpr size_t kNoallocBytes = align_up(kOffErr + 4);
-static_assert(kNoallocBytes == PBF_NOALLOC_SCRATCH_BYTES, "PBF_NOALLOC_SCRATCH_BYTES in pbf.h is stale");
+constexpr size_t kNoallocBytes = PBF_NOALLOC_SCRATCH_BYTES;
+static_assert(kOffErr + 4 <= kNoallocBytes, "PBF_NOALLOC_SCRATCH_BYTES in pbf.h is too small");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 
@@ -5160,30 +5095,26 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 std::mutex g_noalloc_mu;
 void* g_noalloc_addr[128] = {nullptr};
 
-// calculate_bins over caller AoS positions (neighbors.h:120-125), the sort's
-// input at the caller's index and the bin histogram (one atomic per distinct
-// bin of a warp).
-__global__ void k_noalloc_hash(Dev P, int n, const float* __restrict__ x, uint32_t* key, unsigned long long* pair,
-                               uint32_t* cell_count, uint32_t* err) {
+// calculate_bins over caller AoS positions (neighbors.h:120-125), the bin
+// histogram and the arrival numbers (hash_out).
+__global__ void k_noalloc_hash(Dev P, int n, const float* __restrict__ x, uint32_t* key, uint32_t* rank,
+                               uint32_t* cell_count, uint32_t* crowded, uint32_t* err) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   uint32_t k;
   if (!pbf::bin_of(P, pbf::region_of(P, 0), x[3 * (size_t)a], x[3 * (size_t)a + 1], x[3 * (size_t)a + 2], k))
     atomicOr(err, PBF_FLAG_KEY_RANGE);
-  key[a] = k;
-  pair[a] = ((unsigned long long)a << 32) | (unsigned long long)a;
-  const unsigned peers = __match_any_sync(__activemask(), k);
-  if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0u) atomicAdd(&cell_count[k], (uint32_t)__popc(peers));
+  hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
-__global__ void k_noalloc_gather(int n, const unsigned long long* __restrict__ pairs, const float* __restrict__ x,
-                                 float4* sorted_x, uint32_t* sorted_id) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  const unsigned long long pr = pairs[b];
-  const size_t a = (size_t)(pr & 0xffffffffull);
+__global__ void k_noalloc_gather(int n, CellSort S, const float* __restrict__ x, float4* sorted_x,
+                                 uint32_t* sorted_id) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const size_t a = S.arrivals[j].y;  // its slot is its index
+  const uint32_t b = sorted_slot(S, (uint32_t)j, (uint32_t)a, S.key[a]);
   sorted_x[b] = make_float4(x[3 * a], x[3 * a + 1], x[3 * a + 2], 0.0f);
-  sorted_id[b] = (uint32_t)(pr >> 32);
+  sorted_id[b] = (uint32_t)a;
 }
 
 // A crowded bin [q0, q1) run by run (runs of bit-identical positions from
@@ -5241,14 +5172,10 @@ __global__ void __launch_bounds__(kBlock) k_noalloc_fill(Dev P, int n, const flo
                                     row, count);
           continue;
         }
-        for (uint32_t q = q0; q < q1; ++q) {
-          if (q == (uint32_t)b) continue;
-          const float4 xq = pst[q];
-          const float d2 = pbf::mag2<true>(pbf::xsub(xp.x, xq.x), pbf::xsub(xp.y, xq.y), pbf::xsub(xp.z, xq.z));
-          if (d2 < P.s2) {
-            row[count] = (int32_t)sorted_id[q];
-            if (++count >= cap) break;
-          }
+        for (uint32_t q = q0; q < q1 && count < cap; q += 32) {
+          uint32_t m = test_chunk(pst + q, (int)min(q1 - q, 32u), xp.x, xp.y, xp.z, P.s2);
+          if ((uint32_t)b - q < 32u) m &= ~(1u << ((uint32_t)b - q));  // the particle itself
+          for (; m && count < cap; m &= m - 1u) row[count++] = (int32_t)sorted_id[q + (uint32_t)__ffs(m) - 1u];
         }
       }
     }
@@ -5297,13 +5224,12 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
   auto* cell_count = reinterpret_cast<uint32_t*>(base + kOffCount);
   auto* cell_start = reinterpret_cast<uint32_t*>(base + kOffStart);
   auto* parts = reinterpret_cast<uint32_t*>(base + kOffParts);
-  uint32_t* kin = reinterpret_cast<uint32_t*>(base + kOffKeyA);
-  uint32_t* kout = reinterpret_cast<uint32_t*>(base + kOffKeyB);
-  auto* vin = reinterpret_cast<unsigned long long*>(base + kOffPairA);
-  auto* vout = reinterpret_cast<unsigned long long*>(base + kOffPairB);
-  auto* hist = reinterpret_cast<uint32_t*>(base + kOffHist);
-  auto* hist_off = reinterpret_cast<uint32_t*>(base + kOffHistOff);
-  auto* hist_parts = reinterpret_cast<uint32_t*>(base + kOffHistParts);
+  auto* key = reinterpret_cast<uint32_t*>(base + kOffKey);
+  auto* rank = reinterpret_cast<uint32_t*>(base + kOffRank);
+  auto* arrivals = reinterpret_cast<uint2*>(base + kOffArrivals);
+  auto* place = reinterpret_cast<uint32_t*>(base + kOffPlace);
+  auto* crowded = reinterpret_cast<uint32_t*>(base + kOffCrowded);
+  auto* bits = reinterpret_cast<uint32_t*>(base + kOffBits);
   auto* run_end = reinterpret_cast<uint32_t*>(base + kOffRunEnd);
   auto* sorted_x = reinterpret_cast<float4*>(base + kOffSortedX);
   auto* sorted_id = reinterpret_cast<uint32_t*>(base + kOffSortedId);
@@ -5311,33 +5237,21 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
   // The array keeps the previous call's contents: clear what must start at
   // zero (the histogram and the error word; every other buffer is written in
   // full before it is read).
-  e = cudaMemsetAsync(cell_count, 0, 4 * (size_t)d.nbins, s);
+  e = cudaMemsetAsync(cell_count, 0, 4 * ((size_t)d.nbins + kCrowdedWords), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, 4, s);
   if (e != cudaSuccess) return fail(nullptr, PBF_ERR_CUDA, "cudaMemsetAsync failed: %s", cudaGetErrorString(e));
   const int nn = (int)n, g = blocks_for(n);
   const int nparts = (int)(((size_t)d.nbins + 1 + kScanTile - 1) / kScanTile);
-  k_noalloc_hash<<<g, kBlock, 0, s>>>(d, nn, d_x, kin, vin, cell_count, err);
+  const CellSort sort{arrivals, key, cell_start, place};
+  k_noalloc_hash<<<g, kBlock, 0, s>>>(d, nn, d_x, key, rank, cell_count, crowded, err);
   k_scan_reduce<<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts);
-  k_scan_partials<<<1, kScanThreads, 0, s>>>(parts, nparts);
   k_scan_apply<<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts, cell_start);
-  const int tiles = (int)(((size_t)n + kRadixTile - 1) / kRadixTile);
-  const int hm = kRadixDigits * tiles;
-  const int hp = (int)(((size_t)hm + 1 + kScanTile - 1) / kScanTile);
-  const int passes = radix_passes_for(d.nbins);
-  for (int pass = 0; pass < passes; ++pass) {
-    const int shift = pass * kRadixBits;
-    const bool last = pass == passes - 1;
-    k_radix_hist<<<tiles, kRadixThreads, 0, s>>>(kin, nn, shift, tiles, hist);
-    k_scan_reduce<<<hp, kScanThreads, 0, s>>>(hist, hm, hist_parts);
-    k_scan_partials<<<1, kScanThreads, 0, s>>>(hist_parts, hp);
-    k_scan_apply<<<hp, kScanThreads, 0, s>>>(hist, hm, hist_parts, hist_off);
-    k_radix_scatter<<<tiles, kRadixThreads, 0, s>>>(kin, vin, nn, shift, tiles, hist_off, last ? nullptr : kout,
-                                                   vout);
-    std::swap(kin, kout);
-    std::swap(vin, vout);
-  }
-  k_noalloc_gather<<<g, kBlock, 0, s>>>(nn, vin, d_x, sorted_x, sorted_id);
-  k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end, nullptr, nullptr);
+  k_arrivals<<<g, kBlock, 0, s>>>(nn, key, rank, nullptr, cell_start, arrivals);
+  k_order_crowded<<<(int)kNaOrderBlocks, kOrderThreads, 0, s>>>(bitmap_words(n), cell_count + d.nbins + kCrowdedBins,
+                                                               crowded, cell_start, arrivals, bits, place);
+  k_noalloc_gather<<<g, kBlock, 0, s>>>(nn, sort, d_x, sorted_x, sorted_id);
+  k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end,
+                                                        cell_count + d.nbins + kCrowdedRuns, nullptr);
   k_noalloc_fill<<<g, kBlock, 0, s>>>(d, nn, sorted_x, sorted_id, cell_start, run_end, d_nbr, d_cnt, err);
   if (d_flags) e = cudaMemcpyAsync(d_flags, err, 4, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaGetLastError();
