@@ -425,6 +425,29 @@ __global__ void k_reorder(int n, CellSort S, const float4* __restrict__ posH, co
   if (lamS) lamS[b] = lamH[a];  // FULL: lambda; fused step: last step's lambda sum, when kept
 }
 
+// The per-stage path keeps the sorted arrays as the home arrays (the paths
+// start at zero), and slot n as the record that adds nothing (k_upload).
+__global__ void k_adopt(int n, const float4* __restrict__ posS, const float4* __restrict__ pstS,
+                        const float4* __restrict__ velS, const float4* __restrict__ scrS,
+                        const float* __restrict__ lamS, const uint32_t* __restrict__ origS, float4* posH, float4* pstH,
+                        float4* velH, float4* scrH, float* lamH, uint32_t* origH) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b == 0) {
+    pstH[n] = make_float4(kFar, kFar, kFar, 0.0f);
+    velH[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    scrH[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    lamH[n] = 0.0f;
+  }
+  if (b >= n) return;
+  posH[b] = posS[b];
+  const float4 x = pstS[b];
+  pstH[b] = make_float4(x.x, x.y, x.z, 0.0f);
+  velH[b] = velS[b];
+  scrH[b] = scrS[b];
+  lamH[b] = lamS[b];
+  origH[b] = origS[b];
+}
+
 // Device words of the fast path's fill (FillWord): the lists that reached the
 // cap in the last fill, its particle count, whether at most 1 in
 // kSlotCappedShare lists had reached the cap in the fill before it (1 after an
@@ -1142,6 +1165,42 @@ __device__ __forceinline__ float moved(const Dev& P, float4 old, float3 s, bool&
   return path;
 }
 
+// ---- sequential walks: one lane a particle, entries in list order ----
+// The exact path's sums follow the list; four index and record loads are in
+// flight before the four bodies (one at a time, the walk was a chain of two
+// dependent loads an entry).  Entries past the count name the particle itself
+// and are left out.  Bound by the rounded divisions and square roots of the
+// reference's expressions; exact math at 98k particles, one entry at a time
+// and four: density/lambda 36 -> 29 us, delta-p 31 -> 24, vorticity 36 -> 29.
+template <class Body>
+__device__ __forceinline__ void seq1(const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+                                     const float4* __restrict__ a, Body&& body) {
+  const int4* r4 = reinterpret_cast<const int4*>(nbr + pbf::list_base(b, stride));
+  for (int j = 0; j < c; j += 4) {
+    const int4 q = pbf::tail4(__ldg(r4 + pbf::vec4_at(j >> 2)), j >> 2, c, b);
+    const float4 v0 = a[q.x], v1 = a[q.y], v2 = a[q.z], v3 = a[q.w];
+    body(q.x, v0);
+    if (j + 1 < c) body(q.y, v1);
+    if (j + 2 < c) body(q.z, v2);
+    if (j + 3 < c) body(q.w, v3);
+  }
+}
+
+template <class Body>
+__device__ __forceinline__ void seq2(const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+                                     const float4* __restrict__ a, const float4* __restrict__ a2, Body&& body) {
+  const int4* r4 = reinterpret_cast<const int4*>(nbr + pbf::list_base(b, stride));
+  for (int j = 0; j < c; j += 4) {
+    const int4 q = pbf::tail4(__ldg(r4 + pbf::vec4_at(j >> 2)), j >> 2, c, b);
+    const float4 v0 = a[q.x], v1 = a[q.y], v2 = a[q.z], v3 = a[q.w];
+    const float4 w0 = a2[q.x], w1 = a2[q.y], w2 = a2[q.z], w3 = a2[q.w];
+    body(q.x, v0, w0);
+    if (j + 1 < c) body(q.y, v1, w1);
+    if (j + 2 < c) body(q.z, v2, w2);
+    if (j + 3 < c) body(q.w, v3, w3);
+  }
+}
+
 // ---- density (particles.h:292-313) ----
 // Per-stage form: writes rho into vel.w.  A particle sitting on a neighbour is
 // nudged (particles.h:303-305); the reference writes position_stars_[p] in
@@ -1149,22 +1208,11 @@ __device__ __forceinline__ float moved(const Dev& P, float4 old, float3 s, bool&
 // nudged position and every position goes to pst_out, copied back after the
 // pass (deterministic: neighbours see nudges from the next stage on).
 template <bool X>
-__global__ void __launch_bounds__(kBlock) k_density(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
-                                                    const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
-                                                    float4* vel, float4* pst_out) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  float4 xp = pst[b];
-  if (!pbf::in_span(P, b)) {  // outside the span: x* and rho stay
-    pst_out[b] = xp;
-    return;
-  }
-  const int c = cnt[b];
+__device__ __forceinline__ bool density_one(const Dev& P, int b, size_t stride, const int32_t* __restrict__ nbr, int c,
+                                            const float4* __restrict__ pst, float4* vel, float4& xp) {
   float rho = pbf::M<X>(P.m, P.W0);
   bool nudged = false;
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q];
+  seq1(nbr, b, stride, c, pst, [&](int, float4 xq) {
     float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     float rm = pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz));
     if ((double)rm < 0.00000001) {
@@ -1177,10 +1225,19 @@ __global__ void __launch_bounds__(kBlock) k_density(Dev P, int n, size_t stride,
       rm = pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz));
     }
     rho = pbf::A<X>(rho, pbf::M<X>(P.m, pbf::poly6<X>(P, rm)));
-  }
+  });
   vel[b].w = rho;
+  return nudged;
+}
+
+__global__ void __launch_bounds__(kBlock) k_density(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
+                                                    const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
+                                                    float4* vel, float4* pst_out) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n) return;
+  float4 xp = pst[b];
+  if (pbf::in_span(P, b)) density_one<true>(P, b, stride, nbr, cnt[b], pst, vel, xp);  // outside: x* and rho stay
   pst_out[b] = xp;
-  (void)nudged;
 }
 
 // compute_pressure_lambdas (particles.h:318-342), per-stage form.
@@ -1204,21 +1261,20 @@ __device__ __forceinline__ float lambda_of(const Dev& P, float rho, float3 sg, f
   return pbf::D<X>(-Cp, pbf::A<X>(sumC, P.lambda_eps));
 }
 
-template <bool X>
 __global__ void __launch_bounds__(kBlock) k_lambda(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                    const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                    const float4* __restrict__ vel, float* lam) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n || !pbf::in_span(P, b)) return;
   const float4 xp = pst[b];
   const int c = cnt[b];
   float3 sg = make_float3(0.f, 0.f, 0.f);
   float sumC = 0.0f;
-  for (int k = 0; k < c; ++k) {
-    const float4 xq = pst[nbr[pbf::list_at(b, stride, k)]];
+  seq1(nbr, b, stride, c, pst, [&](int, float4 xq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     lambda_terms<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), sg, sumC);
-  }
+  });
   lam[b] = lambda_of<X>(P, vel[b].w, sg, sumC);
 }
 
@@ -1239,8 +1295,7 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
   float3 sg = make_float3(0.f, 0.f, 0.f);
   float sumC = 0.0f;
   bool nudged = false;
-  for (int k = 0; k < c; ++k) {
-    const float4 xq = pst[nbr[pbf::list_at(b, stride, k)]];
+  seq1(nbr, b, stride, c, pst, [&](int, float4 xq) {
     float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     float rm = pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz));
     if ((double)rm < 0.00000001) {
@@ -1254,7 +1309,7 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
     }
     rho = pbf::A<X>(rho, pbf::M<X>(P.m, pbf::poly6<X>(P, rm)));
     lambda_terms<X>(P, rx, ry, rz, rm, sg, sumC);
-  }
+  });
   if (nudged) *nudge = 1u;
   const float l = lambda_of<X>(P, rho, sg, sumC);
   xl[b] = make_float4(xp.x, xp.y, xp.z, l);
@@ -1263,12 +1318,12 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
   return nudged;
 }
 
-template <bool X>
 __global__ void __launch_bounds__(kBlock) k_density_lambda(Dev P, int n, size_t stride,
                                                            const int32_t* __restrict__ nbr,
                                                            const int32_t* __restrict__ cnt,
                                                            const float4* __restrict__ pst, float4* xl,
                                                            float4* vel, float* lam, uint32_t* nudge) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   density_lambda_one<X>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
@@ -1763,11 +1818,11 @@ __global__ void __launch_bounds__(pbf::tc::kThreads, 6) kl_mlp_tc(pbf::MlpDev M,
 // Lambda recomputed from the (nudged) positions in xl, only when the
 // preceding density_lambda launch nudged a particle; otherwise every block
 // returns at once.
-template <bool X>
 __global__ void __launch_bounds__(kBlock) k_lambda_fixup(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                          const int32_t* __restrict__ cnt,
                                                          const float4* __restrict__ xl, const float4* __restrict__ vel,
                                                          float* lam, const uint32_t* __restrict__ nudge) {
+  constexpr bool X = true;
   if (*nudge == 0u) return;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
@@ -1775,11 +1830,10 @@ __global__ void __launch_bounds__(kBlock) k_lambda_fixup(Dev P, int n, size_t st
   const int c = cnt[b];
   float3 sg = make_float3(0.f, 0.f, 0.f);
   float sumC = 0.0f;
-  for (int k = 0; k < c; ++k) {
-    const float4 xq = xl[nbr[pbf::list_at(b, stride, k)]];
+  seq1(nbr, b, stride, c, xl, [&](int, float4 xq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     lambda_terms<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), sg, sumC);
-  }
+  });
   lam[b] = lambda_of<X>(P, vel[b].w, sg, sumC);
 }
 
@@ -1799,33 +1853,36 @@ __device__ __forceinline__ void dp_term(const Dev& P, float lp, float lq, float 
 }
 
 // Per-stage delta-p -> scratch.
-template <bool X, bool SCORR>
+template <bool SCORR>
 __global__ void __launch_bounds__(kBlock) k_dp(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                const float* __restrict__ lam, float4* scr) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n || !pbf::in_span(P, b)) return;
   const float4 xp = pst[b];
   const float lp = lam[b];
   const int c = cnt[b];
   float3 dp = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q];
+  seq1(nbr, b, stride, c, pst, [&](int q, float4 xq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     dp_term<X, SCORR>(P, lp, lam[q], rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
-  }
+  });
   scr[b] = make_float4(pbf::M<X>(P.inv_rho0, dp.x), pbf::M<X>(P.inv_rho0, dp.y), pbf::M<X>(P.inv_rho0, dp.z), 0.0f);
 }
 
-// update_position_stars (particles.h:363-370), per-stage.
+// update_position_stars (particles.h:363-370), per-stage; P.walk given: the
+// moves are followed for the near lists.
 __global__ void k_update_xs(Dev P, int n, float4* pst, const float4* __restrict__ scr) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n || !pbf::in_span(P, b)) return;
-  const float4 x = pst[b], d = scr[b];
-  const float3 s = pbf::boundary(P, pbf::region_of(P, b),
-                                 make_float3(pbf::xadd(x.x, d.x), pbf::xadd(x.y, d.y), pbf::xadd(x.z, d.z)));
-  pst[b] = make_float4(s.x, s.y, s.z, 0.0f);
+  bool mark = false;
+  if (b < n && pbf::in_span(P, b)) {
+    const float4 x = pst[b], d = scr[b];
+    const float3 s = pbf::boundary(P, pbf::region_of(P, b),
+                                   make_float3(pbf::xadd(x.x, d.x), pbf::xadd(x.y, d.y), pbf::xadd(x.z, d.z)));
+    pst[b] = make_float4(s.x, s.y, s.z, P.walk ? moved(P, x, s, mark) : 0.0f);
+  }
+  if (P.walk) mark_neighbourhoods(P, b, mark);
 }
 
 // update_velocities (particles.h:375-385), always exact (per-particle).
@@ -1860,31 +1917,29 @@ __global__ void k_clear_outside_span(int n, const uint32_t* __restrict__ orig, u
 // Fused delta-p + x* update (+ velocity update on the last iteration): reads
 // (x*, lambda) of neighbours from xl, writes the new x* (Jacobi: nobody reads
 // pst in this kernel).
-template <bool X, bool SCORR, bool LAST>
+template <bool SCORR, bool LAST>
 __global__ void __launch_bounds__(kBlock) k_dp_update(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                       const int32_t* __restrict__ cnt, const float4* __restrict__ xl,
                                                       float4* pst, const float4* __restrict__ pos, float4* vel,
                                                       const float* __restrict__ lam,
                                                       const uint32_t* __restrict__ nudge) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   const float4 xp = xl[b];
   const int c = cnt[b];
   float3 dp = make_float3(0.f, 0.f, 0.f);
   if (*nudge == 0u) {
-    for (int k = 0; k < c; ++k) {
-      const float4 xq = xl[nbr[pbf::list_at(b, stride, k)]];
+    seq1(nbr, b, stride, c, xl, [&](int, float4 xq) {
       const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
       dp_term<X, SCORR>(P, xp.w, xq.w, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
-    }
+    });
   } else {  // lambdas were recomputed by k_lambda_fixup
     const float lp = lam[b];
-    for (int k = 0; k < c; ++k) {
-      const int q = nbr[pbf::list_at(b, stride, k)];
-      const float4 xq = xl[q];
+    seq1(nbr, b, stride, c, xl, [&](int q, float4 xq) {
       const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
       dp_term<X, SCORR>(P, lp, lam[q], rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
-    }
+    });
   }
   const float dx = pbf::M<X>(P.inv_rho0, dp.x), dy = pbf::M<X>(P.inv_rho0, dp.y), dz = pbf::M<X>(P.inv_rho0, dp.z);
   const float3 s = pbf::boundary(P, pbf::region_of(P, b),
@@ -1898,25 +1953,23 @@ __global__ void __launch_bounds__(kBlock) k_dp_update(Dev P, int n, size_t strid
 }
 
 // apply_surface_tension (particles.h:400-431): colour-field pass ...
-template <bool X>
 __global__ void __launch_bounds__(kBlock) k_color(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                   const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                   const float4* __restrict__ vel, float4* scr) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n || !pbf::in_span(P, b)) return;
   const float4 xp = pst[b];
   const int c = cnt[b];
   float3 col = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q];
+  seq1(nbr, b, stride, c, pst, [&](int q, float4 xq) {
     const float rq = vel[q].w;
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float3 dw = pbf::del_spikey<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     col.x = pbf::A<X>(col.x, pbf::D<X>(dw.x, rq));
     col.y = pbf::A<X>(col.y, pbf::D<X>(dw.y, rq));
     col.z = pbf::A<X>(col.z, pbf::D<X>(dw.z, rq));
-  }
+  });
   scr[b] = make_float4(pbf::M<X>(P.h, col.x), pbf::M<X>(P.h, col.y), pbf::M<X>(P.h, col.z), 0.0f);
 }
 
@@ -1931,9 +1984,7 @@ __global__ void __launch_bounds__(kBlock) k_surface(Dev P, int n, size_t stride,
   const int c = cnt[b];
   const float ng = -P.gamma;
   float3 f = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q], sq = scr[q];
+  seq2(nbr, b, stride, c, pst, scr, [&](int q, float4 xq, float4 sq) {
     const float rq = vel[q].w;
     const float rx = pbf::xsub(xp.x, xq.x), ry = pbf::xsub(xp.y, xq.y), rz = pbf::xsub(xp.z, xq.z);
     float rm = __fsqrt_rn(pbf::mag2<true>(rx, ry, rz));
@@ -1943,7 +1994,7 @@ __global__ void __launch_bounds__(kBlock) k_surface(Dev P, int n, size_t stride,
     f.x = pbf::xadd(f.x, pbf::xmul(K, pbf::xadd(pbf::xdiv(pbf::xmul(cs, rx), rm), pbf::xmul(ng, pbf::xsub(sp.x, sq.x)))));
     f.y = pbf::xadd(f.y, pbf::xmul(K, pbf::xadd(pbf::xdiv(pbf::xmul(cs, ry), rm), pbf::xmul(ng, pbf::xsub(sp.y, sq.y)))));
     f.z = pbf::xadd(f.z, pbf::xmul(K, pbf::xadd(pbf::xdiv(pbf::xmul(cs, rz), rm), pbf::xmul(ng, pbf::xsub(sp.z, sq.z)))));
-  }
+  });
   float4 v = vel[b];
   v.x = pbf::xadd(v.x, pbf::xmul(pbf::xdiv(f.x, rp), P.dt));
   v.y = pbf::xadd(v.y, pbf::xmul(pbf::xdiv(f.y, rp), P.dt));
@@ -1954,12 +2005,13 @@ __global__ void __launch_bounds__(kBlock) k_surface(Dev P, int n, size_t stride,
 // XSPH viscosity (particles.h:436-447), Jacobi: reads vin, writes vout.
 // FINAL also performs update_positions (particles.h:390-394) and writes the
 // step's results into the home buffers.
-template <bool X, bool FINAL>
+template <bool FINAL>
 __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                       const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                       const float4* __restrict__ vin, float4* vout, float4* posH,
                                                       float4* pstH, const uint32_t* __restrict__ origS,
                                                       uint32_t* origH) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   const float4 xp = pst[b], vp = vin[b];
@@ -1969,9 +2021,7 @@ __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t strid
   }
   const int c = cnt[b];
   float3 dv = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q], vq = vin[q];
+  seq2(nbr, b, stride, c, pst, vin, [&](int q, float4 xq, float4 vq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float w = pbf::poly6<X>(P, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     if (X) {
@@ -1984,7 +2034,7 @@ __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t strid
       dv.y = fmaf(vq.y - vp.y, wr, dv.y);
       dv.z = fmaf(vq.z - vp.z, wr, dv.z);
     }
-  }
+  });
   vout[b] = make_float4(pbf::A<X>(vp.x, pbf::M<X>(P.visc_c, dv.x)), pbf::A<X>(vp.y, pbf::M<X>(P.visc_c, dv.y)),
                         pbf::A<X>(vp.z, pbf::M<X>(P.visc_c, dv.z)), vp.w);
   if (FINAL) {
@@ -1996,18 +2046,16 @@ __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t strid
 
 // compute_vorticity (particles.h:452-466): omega into scratch (w = |omega|,
 // computed as magnitude() would) and (x*, |omega|) into xl for the apply pass.
-template <bool X>
 __global__ void __launch_bounds__(kBlock) k_vorticity(Dev P, int n, size_t stride, const int32_t* __restrict__ nbr,
                                                       const int32_t* __restrict__ cnt, const float4* __restrict__ pst,
                                                       const float4* __restrict__ vel, float4* scr, float4* xl) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n || !pbf::in_span(P, b)) return;
   const float4 xp = pst[b], vp = vel[b];
   const int c = cnt[b];
   float3 w = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    const float4 xq = pst[q], vq = vel[q];
+  seq2(nbr, b, stride, c, pst, vel, [&](int q, float4 xq, float4 vq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float3 d = pbf::del_spikey<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     const float ax = pbf::S<X>(vq.x, vp.x), ay = pbf::S<X>(vq.y, vp.y), az = pbf::S<X>(vq.z, vp.z);
@@ -2015,7 +2063,7 @@ __global__ void __launch_bounds__(kBlock) k_vorticity(Dev P, int n, size_t strid
     w.x = pbf::A<X>(w.x, pbf::S<X>(pbf::M<X>(ay, d.z), pbf::M<X>(az, d.y)));
     w.y = pbf::A<X>(w.y, pbf::S<X>(pbf::M<X>(az, d.x), pbf::M<X>(ax, d.z)));
     w.z = pbf::A<X>(w.z, pbf::S<X>(pbf::M<X>(ax, d.y), pbf::M<X>(ay, d.x)));
-  }
+  });
   const float wm = __fsqrt_rn(pbf::mag2<true>(w.x, w.y, w.z));
   scr[b] = make_float4(w.x, w.y, w.z, wm);
   if (xl) xl[b] = make_float4(xp.x, xp.y, xp.z, wm);
@@ -2023,36 +2071,32 @@ __global__ void __launch_bounds__(kBlock) k_vorticity(Dev P, int n, size_t strid
 
 // apply_vorticity (particles.h:471-487).  PACKED reads (x*, |omega|) of
 // neighbours from xl (one 16-byte load); otherwise from pst and scratch.
-template <bool X, bool PACKED>
+template <bool PACKED>
 __global__ void __launch_bounds__(kBlock) k_apply_vorticity(Dev P, int n, size_t stride,
                                                             const int32_t* __restrict__ nbr,
                                                             const int32_t* __restrict__ cnt,
                                                             const float4* __restrict__ xl,
                                                             const float4* __restrict__ pst,
                                                             const float4* __restrict__ scr, float4* vel) {
+  constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n || !pbf::in_span(P, b)) return;
   const float4 xp = PACKED ? xl[b] : pst[b];
   const int c = cnt[b];
   float3 eta = make_float3(0.f, 0.f, 0.f);
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    float4 xq;
-    float vm;
-    if (PACKED) {
-      xq = xl[q];
-      vm = xq.w;
-    } else {
-      xq = pst[q];
-      const float4 sq = scr[q];
-      vm = __fsqrt_rn(pbf::mag2<true>(sq.x, sq.y, sq.z));
-    }
+  auto add = [&](float4 xq, float vm) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float3 d = pbf::del_spikey<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     eta.x = pbf::A<X>(eta.x, pbf::M<X>(vm, d.x));
     eta.y = pbf::A<X>(eta.y, pbf::M<X>(vm, d.y));
     eta.z = pbf::A<X>(eta.z, pbf::M<X>(vm, d.z));
-  }
+  };
+  if (PACKED)
+    seq1(nbr, b, stride, c, xl, [&](int, float4 xq) { add(xq, xq.w); });
+  else
+    seq2(nbr, b, stride, c, pst, scr, [&](int, float4 xq, float4 sq) {
+      add(xq, __fsqrt_rn(pbf::mag2<true>(sq.x, sq.y, sq.z)));
+    });
   const float den = pbf::A<X>(pbf::SQ<X>(pbf::mag2<X>(eta.x, eta.y, eta.z)), FLT_EPSILON);
   const float Nx = pbf::D<X>(eta.x, den), Ny = pbf::D<X>(eta.y, den), Nz = pbf::D<X>(eta.z, den);
   const float4 wp = scr[b];
@@ -2353,6 +2397,262 @@ __global__ void __launch_bounds__(kStageThreads) ks_apply_vorticity(Dev P, Fast 
     apply_vorticity_tile<4>(tile, P, F, n, stride, nbr, cnt, xl, scr, vel);
 }
 
+// ---- fast per-stage gathers (exact_math = 0) ----
+// The reference's stages one by one, for callers that drive them themselves:
+// the fused step's walks (kStageGL lanes a particle) over the home arrays, which
+// keep every reference array apart.  One lane a particle walked 262k particles'
+// lists in 45-80 us a stage, a chain of dependent loads an entry; these take
+// 17-30 us (the surface force, over the whole list, 91 instead of 153, the
+// colour field 41 instead of 54), bound as the fused gathers by the L1 path.
+// Positions can change in any way between two stage calls, so a list is walked
+// whole unless the context knows that x* only moved by update_position_stars
+// since the fill (P.walk given: walk_count).  Slots past a count are read at
+// slot n, the dummy record (k_adopt).
+constexpr int kStageGL = 2, kStageBlock = 128;
+
+__device__ __forceinline__ int stage_count(const Dev& P, const pbf::Group& G, const int32_t* __restrict__ cnt) {
+  if (!G.live) return 0;
+  return P.walk ? walk_count(P, G.b, cnt) : cnt[G.b];
+}
+
+// The group of this thread; not live outside the stage's span.
+__device__ __forceinline__ pbf::Group stage_group(const Dev& P, int n) {
+  pbf::Group G = pbf::group_of<kStageGL>(n);
+  G.live = G.live && pbf::in_span(P, G.b);
+  return G;
+}
+
+// compute_densities (particles.h:292-313).  A particle on a neighbour takes
+// the reference-ordered path (density_one), which nudges it.
+__global__ void __launch_bounds__(kStageBlock) kt_density(Dev P, Fast F, int n, size_t stride,
+                                                          const int32_t* __restrict__ nbr,
+                                                          const int32_t* __restrict__ cnt,
+                                                          const float4* __restrict__ pst, float4* vel,
+                                                          float4* pst_out) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b];
+  const int c = stage_count(P, G, cnt);
+  float sw = 0.f, dmin = FLT_MAX;
+  pbf::gwalk1<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, [&](int, float4 xq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    dmin = fminf(dmin, d2);
+    const float a = fmaxf(F.h2 - d2, 0.0f);
+    sw = fmaf(a * a, a, sw);
+  });
+  sw = pbf::gsum<kStageGL>(sw);
+  dmin = pbf::gmin<kStageGL>(dmin);
+  bool mark = false;
+  const int gid = blockIdx.x * blockDim.x + threadIdx.x, own = gid / kStageGL;
+  if (G.lane == 0 && own < n) {
+    float4 x = G.live ? xp : pst[own];  // outside the span: x* and rho stay
+    if (G.live && dmin < 4e-16f)
+      mark = density_one<false>(P, b, stride, nbr, cnt[b], pst, vel, x);
+    else if (G.live)
+      vel[b].w = fmaf(F.m_poly, sw, F.m_w0);
+    pst_out[own] = x;
+  }
+  if (P.walk) mark_neighbourhoods(P, b, mark);
+}
+
+// compute_pressure_lambdas (particles.h:318-342)
+__global__ void __launch_bounds__(kStageBlock) kt_lambda(Dev P, Fast F, int n, size_t stride,
+                                                         const int32_t* __restrict__ nbr,
+                                                         const int32_t* __restrict__ cnt,
+                                                         const float4* __restrict__ pst,
+                                                         const float4* __restrict__ vel, float* lam) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b];
+  const int c = stage_count(P, G, cnt);
+  const DensitySums S = density_sums<kStageGL, false>(F, G, nbr + pbf::list_base(b, stride), nullptr, c, n, pst, xp);
+  if (!G.live || G.lane != 0) return;
+  const float L2 = F.lam_grad * F.lam_grad;
+  const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));
+  const float C = fmaxf(fmaf(vel[b].w, F.inv_rho0, -1.0f), 0.0f);
+  lam[b] = -C / (L2 * S.s2 + g2 + F.lambda_eps);
+}
+
+// compute_pressure_dps (particles.h:348-358) -> scratch
+template <bool SCORR>
+__global__ void __launch_bounds__(kStageBlock) kt_dp(Dev P, Fast F, int n, size_t stride,
+                                                     const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
+                                                     const float4* __restrict__ pst, const float* __restrict__ lam,
+                                                     float4* scr) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b];
+  const float lp = lam[b];
+  const int c = stage_count(P, G, cnt);
+  float ax = 0.f, ay = 0.f, az = 0.f;
+  pbf::gwalk1<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, [&](int q, float4 xq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    float l = lp + __ldg(lam + q);
+    if (SCORR) l -= P.scorr_k * __powf(F.visc_poly * pbf::poly_cube(F, d2) * P.inv_wdq, P.scorr_n);
+    const float t = l * pbf::spikey_over_r(F, d2);
+    ax = fmaf(t, dx, ax);
+    ay = fmaf(t, dy, ay);
+    az = fmaf(t, dz, az);
+  });
+  ax = pbf::gsum<kStageGL>(ax);
+  ay = pbf::gsum<kStageGL>(ay);
+  az = pbf::gsum<kStageGL>(az);
+  if (!G.live || G.lane != 0) return;
+  scr[b] = make_float4(F.dp_scale * ax, F.dp_scale * ay, F.dp_scale * az, 0.0f);
+}
+
+// apply_surface_tension (particles.h:400-431): the colour field -> scratch
+// (whole: over the whole list, where a density not computed yet, 0, has to
+// show as in the reference) ...
+__global__ void __launch_bounds__(kStageBlock) kt_color(Dev P, Fast F, int n, size_t stride,
+                                                        const int32_t* __restrict__ nbr,
+                                                        const int32_t* __restrict__ cnt,
+                                                        const float4* __restrict__ pst,
+                                                        const float4* __restrict__ vel, float4* scr, bool whole) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b];
+  const int c = !G.live ? 0 : (whole ? cnt[b] : stage_count(P, G, cnt));
+  float ax = 0.f, ay = 0.f, az = 0.f;
+  pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, vel, [&](int, float4 xq, float4 vq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float t = __fdividef(pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx))), vq.w);
+    ax = fmaf(t, dx, ax);
+    ay = fmaf(t, dy, ay);
+    az = fmaf(t, dz, az);
+  });
+  const float k = F.h * F.spikey;
+  ax = pbf::gsum<kStageGL>(ax) * k;
+  ay = pbf::gsum<kStageGL>(ay) * k;
+  az = pbf::gsum<kStageGL>(az) * k;
+  if (!G.live || G.lane != 0) return;
+  scr[b] = make_float4(ax, ay, az, 0.0f);
+}
+
+// ... then the cohesion + curvature force: the reference's expressions, its
+// double ones in double, over the whole list (the curvature term does not
+// vanish beyond h).  Bound by the walk's three records a neighbour.
+__global__ void __launch_bounds__(kStageBlock) kt_surface(Dev P, Fast F, int n, size_t stride,
+                                                          const int32_t* __restrict__ nbr,
+                                                          const int32_t* __restrict__ cnt,
+                                                          const float4* __restrict__ pst,
+                                                          const float4* __restrict__ scr, float4* vel) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b], sp = scr[b];
+  const float rp = vel[b].w, ng = -P.gamma, h_eps = (float)P.h_eps;
+  const int c = G.live ? cnt[b] : 0;
+  float fx = 0.f, fy = 0.f, fz = 0.f;
+  pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, b, G.lane, pst, scr, [&](int q, float4 xq, float4 sq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    const float rm = fmaxf(__fsqrt_rn(d2), h_eps);
+    const float cs = __fdiv_rn(ng * pbf::c_spline<true>(P, rm), rm);
+    const float K = __fdiv_rn(2.0f * P.rho0, rp + vel[q].w);  // entries past the count: the particle itself, no force
+    fx = fmaf(K, fmaf(cs, dx, ng * (sp.x - sq.x)), fx);
+    fy = fmaf(K, fmaf(cs, dy, ng * (sp.y - sq.y)), fy);
+    fz = fmaf(K, fmaf(cs, dz, ng * (sp.z - sq.z)), fz);
+  });
+  fx = pbf::gsum<kStageGL>(fx);
+  fy = pbf::gsum<kStageGL>(fy);
+  fz = pbf::gsum<kStageGL>(fz);
+  if (!G.live || G.lane != 0) return;
+  const float k = __fdiv_rn(P.dt, rp);
+  // v.w (the density, read by other blocks) stays as it is
+  vel[b].x = fmaf(fx, k, vel[b].x);
+  vel[b].y = fmaf(fy, k, vel[b].y);
+  vel[b].z = fmaf(fz, k, vel[b].z);
+}
+
+// apply_viscosity (particles.h:436-447), Jacobi
+__global__ void __launch_bounds__(kStageBlock) kt_viscosity(Dev P, Fast F, int n, size_t stride,
+                                                            const int32_t* __restrict__ nbr,
+                                                            const int32_t* __restrict__ cnt,
+                                                            const float4* __restrict__ pst,
+                                                            const float4* __restrict__ vin, float4* vout) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b], vp = vin[b];
+  const int c = stage_count(P, G, cnt);
+  float ax = 0.f, ay = 0.f, az = 0.f;
+  pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, vin, [&](int, float4 xq, float4 vq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float wr = __fdividef(pbf::poly_cube(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx))), vq.w);
+    ax = fmaf(vq.x - vp.x, wr, ax);
+    ay = fmaf(vq.y - vp.y, wr, ay);
+    az = fmaf(vq.z - vp.z, wr, az);
+  });
+  ax = pbf::gsum<kStageGL>(ax);
+  ay = pbf::gsum<kStageGL>(ay);
+  az = pbf::gsum<kStageGL>(az);
+  const int own = (blockIdx.x * blockDim.x + threadIdx.x) / kStageGL;
+  if (G.lane != 0 || own >= n) return;
+  const float k = F.visc_c * F.visc_poly;
+  vout[own] = G.live ? make_float4(fmaf(k, ax, vp.x), fmaf(k, ay, vp.y), fmaf(k, az, vp.z), vp.w) : vin[own];
+}
+
+// compute_vorticity (particles.h:452-466) -> scratch
+__global__ void __launch_bounds__(kStageBlock) kt_vorticity(Dev P, Fast F, int n, size_t stride,
+                                                            const int32_t* __restrict__ nbr,
+                                                            const int32_t* __restrict__ cnt,
+                                                            const float4* __restrict__ pst,
+                                                            const float4* __restrict__ vel, float4* scr) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b], vp = vel[b];
+  const int c = stage_count(P, G, cnt);
+  float wx = 0.f, wy = 0.f, wz = 0.f;
+  pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, vel, [&](int, float4 xq, float4 vq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float t = pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+    const float ux = vq.x - vp.x, uy = vq.y - vp.y, uz = vq.z - vp.z;
+    wx = fmaf(t, fmaf(uy, dz, -uz * dy), wx);
+    wy = fmaf(t, fmaf(uz, dx, -ux * dz), wy);
+    wz = fmaf(t, fmaf(ux, dy, -uy * dx), wz);
+  });
+  wx = pbf::gsum<kStageGL>(wx) * F.spikey;
+  wy = pbf::gsum<kStageGL>(wy) * F.spikey;
+  wz = pbf::gsum<kStageGL>(wz) * F.spikey;
+  if (!G.live || G.lane != 0) return;
+  scr[b] = make_float4(wx, wy, wz, sqrtf(fmaf(wz, wz, fmaf(wy, wy, wx * wx))));
+}
+
+// apply_vorticity (particles.h:471-487); |omega| of a neighbour from its
+// scratch vector, which the caller may have set
+__global__ void __launch_bounds__(kStageBlock) kt_apply_vorticity(Dev P, Fast F, int n, size_t stride,
+                                                                  const int32_t* __restrict__ nbr,
+                                                                  const int32_t* __restrict__ cnt,
+                                                                  const float4* __restrict__ pst,
+                                                                  const float4* __restrict__ scr, float4* vel) {
+  const pbf::Group G = stage_group(P, n);
+  const int b = G.b;
+  const float4 xp = pst[b];
+  const int c = stage_count(P, G, cnt);
+  float ex = 0.f, ey = 0.f, ez = 0.f;
+  pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, scr, [&](int, float4 xq, float4 sq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float vm = __fsqrt_rn(fmaf(sq.z, sq.z, fmaf(sq.y, sq.y, sq.x * sq.x)));
+    const float t = vm * pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+    ex = fmaf(t, dx, ex);
+    ey = fmaf(t, dy, ey);
+    ez = fmaf(t, dz, ez);
+  });
+  ex = pbf::gsum<kStageGL>(ex) * F.spikey;
+  ey = pbf::gsum<kStageGL>(ey) * F.spikey;
+  ez = pbf::gsum<kStageGL>(ez) * F.spikey;
+  if (!G.live || G.lane != 0) return;
+  const float inv = __fdividef(1.0f, sqrtf(fmaf(ez, ez, fmaf(ey, ey, ex * ex))) + FLT_EPSILON);
+  const float Nx = ex * inv, Ny = ey * inv, Nz = ez * inv;
+  const float4 wp = scr[b];
+  float4 v = vel[b];
+  v.x = fmaf(fmaf(Ny, wp.z, -Nz * wp.y), F.vort_dt, v.x);
+  v.y = fmaf(fmaf(Nz, wp.x, -Nx * wp.z), F.vort_dt, v.y);
+  v.z = fmaf(fmaf(Nx, wp.y, -Ny * wp.x), F.vort_dt, v.z);
+  vel[b] = v;
+}
+
 // ---- the persistent step (batches of scenes) ----
 // Every gather pass of a fast-math plain step (K Jacobi iterations of
 // density/lambda and delta-p, both XSPH passes, vorticity and its
@@ -2566,11 +2866,10 @@ __global__ void __launch_bounds__(kBlock) k_stats(Dev P, int b0, int b1, size_t 
     const float4 xp = pst[b];
     const int c = cnt[b];
     float d = pbf::xmul(P.m, P.W0);
-    for (int k = 0; k < c; ++k) {
-      const float4 xq = pst[nbr[pbf::list_at(b, stride, k)]];
+    seq1(nbr, b, stride, c, pst, [&](int, float4 xq) {
       const float rx = pbf::xsub(xp.x, xq.x), ry = pbf::xsub(xp.y, xq.y), rz = pbf::xsub(xp.z, xq.z);
       d = pbf::xadd(d, pbf::xmul(P.m, pbf::poly6<true>(P, __fsqrt_rn(pbf::mag2<true>(rx, ry, rz)))));
-    }
+    });
     e = (double)d / (double)P.rho0 - 1.0;
     if (e < 0.0) e = 0.0;
     atomicMax(maxerr, (unsigned long long)__double_as_longlong(e));
@@ -2649,6 +2948,7 @@ struct pbf_ctx {
   cudaStream_t side = nullptr;  // captures the body of the learned solver's conditional loop
   bool capture_failed = false;  // a step's conditional loop could not be captured whole
   bool lists_valid = false;
+  bool near_stages = false;  // since find_neighbors x* has only moved by the stages that follow it (Dev::walk)
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
   uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order, near entries first
@@ -2996,6 +3296,7 @@ int check_span(pbf_ctx* ctx, size_t b, size_t e) {
 // The constant block of a per-stage call over the span [0, e).
 Dev span_dev(const pbf_ctx* ctx, size_t e) {
   Dev d = ctx->dev;
+  if (!ctx->near_stages) d.walk = nullptr;
   if (e < ctx->n) {
     d.span_orig = ctx->origH;
     d.span_end = (uint32_t)e;
@@ -3485,7 +3786,7 @@ void launch_step_t(pbf_ctx* ctx) {
     {
       Launch L(ctx, "density_lambda");
       if (X)
-        k_density_lambda<X><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->xl, ctx->velS,
+        k_density_lambda<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->xl, ctx->velS,
                                                  ctx->lamH, ctx->nudge);
       else if (T.staged[PBF_TUNE_DENSITY]) {
         const int gd = grid_of(ctx, PBF_TUNE_DENSITY);
@@ -3511,17 +3812,17 @@ void launch_step_t(pbf_ctx* ctx) {
     }
     if (X) {
       Launch L(ctx, "lambda_fixup");
-      k_lambda_fixup<X><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->velS, ctx->lamH,
+      k_lambda_fixup<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->velS, ctx->lamH,
                                              ctx->nudge);
     }
     Launch L(ctx, "dp_update");
     const bool last = it == K - 1;
     if (X) {
       if (last)
-        k_dp_update<X, SCORR, true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS,
+        k_dp_update<SCORR, true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS,
                                                          ctx->posS, ctx->velS, ctx->lamH, ctx->nudge);
       else
-        k_dp_update<X, SCORR, false><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS,
+        k_dp_update<SCORR, false><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS,
                                                           ctx->posS, ctx->velS, ctx->lamH, ctx->nudge);
     } else if (T.staged[PBF_TUNE_DELTA_P]) {
       const int gd = grid_of(ctx, PBF_TUNE_DELTA_P);
@@ -3552,30 +3853,37 @@ void launch_step_t(pbf_ctx* ctx) {
     k_update_v<<<g, kBlock, 0, s>>>(P, n, ctx->pstS, ctx->posS, ctx->velS);
   }
   if (ctx->params.gamma != 0.0f) {
+    const int gt = blocks_for((size_t)n * kStageGL, kStageBlock);
     {
       Launch L(ctx, "color_field");
-      k_color<X><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velS, ctx->scrH);
+      if (X)
+        k_color<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velS, ctx->scrH);
+      else
+        kt_color<<<gt, kStageBlock, 0, s>>>(P, F, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velS, ctx->scrH, false);
     }
     Launch L(ctx, "surface_tension");
-    k_surface<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
+    if (X)
+      k_surface<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
+    else
+      kt_surface<<<gt, kStageBlock, 0, s>>>(P, F, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
   }
   if (X) {
     {
       Launch L(ctx, "viscosity");
-      k_viscosity<X, false><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velS, ctx->velT,
+      k_viscosity<false><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velS, ctx->velT,
                                                  nullptr, nullptr, nullptr, nullptr);
     }
     {
       Launch L(ctx, "vorticity");
-      k_vorticity<X><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velT, ctx->scrH, ctx->xl);
+      k_vorticity<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velT, ctx->scrH, ctx->xl);
     }
     {
       Launch L(ctx, "apply_vorticity");
-      k_apply_vorticity<X, true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, nullptr, ctx->scrH,
+      k_apply_vorticity<true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->xl, nullptr, ctx->scrH,
                                                       ctx->velT);
     }
     Launch L(ctx, "viscosity_final");
-    k_viscosity<X, true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velT, ctx->velH,
+    k_viscosity<true><<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->velT, ctx->velH,
                                               ctx->posH, ctx->pstH, ctx->origS, ctx->origH);
   } else {
     const TileIO tio = tile_io(ctx);
@@ -3727,10 +4035,10 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
   ctx->lstride = list_stride(p->neighbor_cap);
   ctx->lstride_cap = ctx->lstride;
   const size_t cap = ctx->lstride;
-  if ((rc = dalloc(ctx, &ctx->posH, C)) || (rc = dalloc(ctx, &ctx->pstH, C + kMaskOver)) || (rc = dalloc(ctx, &ctx->velH, C)) ||
-      (rc = dalloc(ctx, &ctx->scrH, C)) || (rc = dalloc(ctx, &ctx->posS, C)) || (rc = dalloc(ctx, &ctx->pstS, C + 1 + kMaskOver)) ||
+  if ((rc = dalloc(ctx, &ctx->posH, C)) || (rc = dalloc(ctx, &ctx->pstH, C + kMaskOver)) || (rc = dalloc(ctx, &ctx->velH, C + 1)) ||
+      (rc = dalloc(ctx, &ctx->scrH, C + 1)) || (rc = dalloc(ctx, &ctx->posS, C)) || (rc = dalloc(ctx, &ctx->pstS, C + 1 + kMaskOver)) ||
       (rc = dalloc(ctx, &ctx->velS, C + 1)) || (rc = dalloc(ctx, &ctx->scrS, C)) || (rc = dalloc(ctx, &ctx->xl, C + 1)) ||
-      (rc = dalloc(ctx, &ctx->velT, C + 1)) || (rc = dalloc(ctx, &ctx->lamH, C)) || (rc = dalloc(ctx, &ctx->lamS, C)) ||
+      (rc = dalloc(ctx, &ctx->velT, C + 1)) || (rc = dalloc(ctx, &ctx->lamH, C + 1)) || (rc = dalloc(ctx, &ctx->lamS, C)) ||
       (rc = dalloc(ctx, &ctx->origH, C)) || (rc = dalloc(ctx, &ctx->origS, C)) || (rc = dalloc(ctx, &ctx->key, C)) ||
       (rc = dalloc(ctx, &ctx->rank, C)) || (rc = dalloc(ctx, &ctx->place, C)) ||
       (rc = dalloc(ctx, &ctx->crowded, C / kCountBin + 1)) || (rc = dalloc(ctx, &ctx->arrivals, C)) ||
@@ -3821,6 +4129,7 @@ int pbf_set_params(pbf_ctx* ctx, const pbf_params* p) {
     ctx->lists_valid = false;
   ctx->params = *p;
   ctx->dev = d;
+  ctx->near_stages = false;
   bind_lists(ctx);
   ctx->fast = pbf::make_fast(d);
   ctx->lstride = lstride;
@@ -3899,6 +4208,7 @@ int pbf_set_array(pbf_ctx* ctx, int which, const float* host_in) {
   if (ctx->n == 0) return PBF_OK;
   const int n = (int)ctx->n, g = blocks_for(n);
   const bool vec = which <= PBF_ARRAY_SCRATCH;
+  if (which == PBF_ARRAY_POSITION_STARS) ctx->near_stages = false;
   CK(cudaMemcpyAsync(ctx->stage, host_in, ctx->n * (vec ? 3 : 1) * sizeof(float), cudaMemcpyHostToDevice,
                      ctx->stream));
   switch (which) {
@@ -4135,6 +4445,7 @@ int pbf_apply_external_forces(pbf_ctx* ctx, size_t b, size_t e) {
 
 int pbf_predict_positions(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
+  ctx->near_stages = false;
   k_predict<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->posH, ctx->velH, ctx->pstH);
   return check_launch(ctx, "predict_positions");
 }
@@ -4159,27 +4470,25 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
   k_reorder<true><<<g, kBlock, 0, s>>>(n, cell_sort(ctx), ctx->posH, ctx->pstH, ctx->velH, ctx->scrH,
                                        ctx->lamH, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS,
                                        ctx->keyH);
-  const size_t f4 = sizeof(float4) * ctx->n;
-  CK(cudaMemcpyAsync(ctx->posH, ctx->posS, f4, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(ctx->pstH, ctx->pstS, f4, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(ctx->velH, ctx->velS, f4, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(ctx->scrH, ctx->scrS, f4, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(ctx->lamH, ctx->lamS, sizeof(float) * ctx->n, cudaMemcpyDeviceToDevice, s));
-  CK(cudaMemcpyAsync(ctx->origH, ctx->origS, sizeof(uint32_t) * ctx->n, cudaMemcpyDeviceToDevice, s));
+  k_adopt<<<g, kBlock, 0, s>>>(n, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS, ctx->posH,
+                               ctx->pstH, ctx->velH, ctx->scrH, ctx->lamH, ctx->origH);
   launch_fill(ctx, ctx->pstH);
   if (fill_e < ctx->n)  // particles outside the fill span (halo particles) get empty lists
     k_clear_outside_span<<<g, kBlock, 0, s>>>(n, ctx->origH, (uint32_t)fill_e, ctx->cnt);
   rc = check_launch(ctx, "find_neighbors");
   if (rc) return rc;
   ctx->lists_valid = true;
+  ctx->near_stages = ctx->lists_slot_order;
   return PBF_OK;
 }
 
 int pbf_compute_densities(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_density<true><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
-  else k_density<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
+  if (X)
+    k_density<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
+  else
+    kt_density<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
   CK(cudaMemcpyAsync(ctx->pstH, ctx->pstS, sizeof(float4) * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
   return check_launch(ctx, "compute_densities");
 }
@@ -4187,8 +4496,10 @@ int pbf_compute_densities(pbf_ctx* ctx, size_t b, size_t e) {
 int pbf_compute_pressure_lambdas(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_lambda<true><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->lamH);
-  else k_lambda<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->lamH);
+  if (X)
+    k_lambda<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->lamH);
+  else
+    kt_lambda<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->lamH);
   return check_launch(ctx, "compute_pressure_lambdas");
 }
 
@@ -4197,11 +4508,14 @@ int pbf_compute_pressure_dps(pbf_ctx* ctx, size_t b, size_t e, int substep) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
   const bool SC = ctx->params.scorr_k > 0.0f;
-  const Dev& P = SP;
-  if (X && SC) k_dp<true, true><<<g, kBlock, 0, ctx->stream>>>(P, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
-  else if (X) k_dp<true, false><<<g, kBlock, 0, ctx->stream>>>(P, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
-  else if (SC) k_dp<false, true><<<g, kBlock, 0, ctx->stream>>>(P, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
-  else k_dp<false, false><<<g, kBlock, 0, ctx->stream>>>(P, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
+  if (X && SC)
+    k_dp<true><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
+  else if (X)
+    k_dp<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
+  else if (SC)
+    kt_dp<true><<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
+  else
+    kt_dp<false><<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->lamH, ctx->scrH);
   return check_launch(ctx, "compute_pressure_dps");
 }
 
@@ -4222,17 +4536,24 @@ int pbf_apply_surface_tension(pbf_ctx* ctx, size_t cb, size_t ce, size_t sb, siz
   if (int rc = check_span(ctx, sb, se)) return rc;
   STAGE_PROLOGUE(cb, ce);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_color<true><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
-  else k_color<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
-  k_surface<<<g, kBlock, 0, ctx->stream>>>(span_dev(ctx, se), n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+  if (X) {
+    k_color<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
+    k_surface<<<g, kBlock, 0, ctx->stream>>>(span_dev(ctx, se), n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+  } else {
+    kt_color<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, true);
+    kt_surface<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(span_dev(ctx, se), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+  }
   return check_launch(ctx, "apply_surface_tension");
 }
 
 int pbf_apply_viscosity(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_viscosity<true, false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT, nullptr, nullptr, nullptr, nullptr);
-  else k_viscosity<false, false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT, nullptr, nullptr, nullptr, nullptr);
+  if (X)
+    k_viscosity<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT, nullptr, nullptr,
+                                                      nullptr, nullptr);
+  else
+    kt_viscosity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT);
   CK(cudaMemcpyAsync(ctx->velH, ctx->velT, sizeof(float4) * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
   return check_launch(ctx, "apply_viscosity");
 }
@@ -4240,16 +4561,20 @@ int pbf_apply_viscosity(pbf_ctx* ctx, size_t b, size_t e) {
 int pbf_compute_vorticity(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_vorticity<true><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, nullptr);
-  else k_vorticity<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, nullptr);
+  if (X)
+    k_vorticity<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, nullptr);
+  else
+    kt_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
   return check_launch(ctx, "compute_vorticity");
 }
 
 int pbf_apply_vorticity(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (X) k_apply_vorticity<true, false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, nullptr, ctx->pstH, ctx->scrH, ctx->velH);
-  else k_apply_vorticity<false, false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, nullptr, ctx->pstH, ctx->scrH, ctx->velH);
+  if (X)
+    k_apply_vorticity<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, nullptr, ctx->pstH, ctx->scrH, ctx->velH);
+  else
+    kt_apply_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
   return check_launch(ctx, "apply_vorticity");
 }
 
@@ -4293,6 +4618,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
     return PBF_OK;
   }
   ctx->steps_done += (uint64_t)nsteps;
+  ctx->near_stages = false;
   if (ctx->timing) {
     for (int i = 0; i < nsteps; ++i) launch_step(ctx);
     int rc = check_launch(ctx, "step");
@@ -4449,6 +4775,7 @@ int pbf_group_step(pbf_group* g, int nsteps) {
   for (pbf_ctx* c : g->ctxs) {
     if (c->n == 0) continue;
     c->steps_done += (uint64_t)nsteps;
+    c->near_stages = false;
     c->lists_valid = true;
   }
   return PBF_OK;
