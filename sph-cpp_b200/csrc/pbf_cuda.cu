@@ -467,10 +467,10 @@ constexpr uint8_t kWalkAll = 0xFF;
 // crowded (may be null): the histogram's flag; zero means no bin is large
 // enough for the fill to read the runs, and the launch returns at once.
 constexpr int kRunBlock = 1024;
-// fw (fast math, may be null): the fill words, moved on to the fill that follows.
+// fw: the fill words, moved on to the fill that follows.
 __global__ void __launch_bounds__(kRunBlock) k_runs(int n, const float4* __restrict__ pst, uint32_t* run_end,
                                                     const uint32_t* __restrict__ crowded, uint32_t* fw) {
-  if (fw && blockIdx.x == 0 && threadIdx.x == 0) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     fw[kFillFewCapped] = (uint64_t)fw[kFillCapped] * kSlotCappedShare <= (uint64_t)fw[kFillCount] ? 1u : 0u;
     fw[kFillCapped] = 0u;
     fw[kFillCount] = (uint32_t)n;
@@ -535,6 +535,33 @@ __device__ __forceinline__ uint32_t test_chunk(const float4* __restrict__ p, int
   }
   m = __brev(m << (32 - c));
   return many < 32 ? m & ((1u << many) - 1u) : m;
+}
+
+// The same against two radii: x within s2, y within near2.
+__device__ __forceinline__ uint2 test_chunk2(const float4* __restrict__ p, int many, float px, float py, float pz,
+                                             float s2, float near2) {
+  uint32_t m = 0, mn = 0;
+  int c = 0;
+#pragma unroll 1
+  for (; c < many; c += 4) {
+    const float4 q0 = __ldg(p + c), q1 = __ldg(p + c + 1), q2 = __ldg(p + c + 2), q3 = __ldg(p + c + 3);
+    auto test = [&](const float4& q) {
+      const float d2 = pbf::mag2<true>(pbf::xsub(px, q.x), pbf::xsub(py, q.y), pbf::xsub(pz, q.z));
+      m = __funnelshift_l(__float_as_uint(pbf::xsub(d2, s2)), m, 1);
+      mn = __funnelshift_l(__float_as_uint(pbf::xsub(d2, near2)), mn, 1);
+    };
+    test(q0);
+    test(q1);
+    test(q2);
+    test(q3);
+  }
+  const uint32_t valid = many < 32 ? (1u << many) - 1u : 0xffffffffu;
+  return make_uint2(__brev(m << (32 - c)) & valid, __brev(mn << (32 - c)) & valid);
+}
+
+// Bits 0 .. k-1 (none below 1, all from 32 on).
+__device__ __forceinline__ uint32_t low_bits(int k) {
+  return k >= 32 ? 0xffffffffu : (k <= 0 ? 0u : (1u << k) - 1u);
 }
 
 // One crowded bin [q0, q1) of the list fill, run by run: one distance test per
@@ -696,7 +723,7 @@ __device__ __forceinline__ void count_capped(uint32_t* fw, bool capped) {
 
 // The list of slot b in the reference's order (a thread's share of k_fill2).
 // fw (fast math): the lists at the cap are counted.
-template <bool STAGE>
+template <bool STAGE = true>
 __device__ __forceinline__ void fill_thread(int b, const Dev& P, int n, size_t stride, const float4* __restrict__ pst,
                                             const uint32_t* __restrict__ cell_start,
                                             const uint32_t* __restrict__ run_end, int32_t* nbr, int32_t* cnt,
@@ -775,12 +802,11 @@ __device__ __forceinline__ void fill_thread(int b, const Dev& P, int n, size_t s
   if (STAGE && stray) T.nruns[tile] = 0;
 }
 
-template <bool STAGE>
 __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t stride, const float4* __restrict__ pst,
                                                       const uint32_t* __restrict__ cell_start,
                                                       const uint32_t* __restrict__ run_end, int32_t* nbr,
                                                       int32_t* cnt, uint32_t* err, TileIO T, uint32_t* fw) {
-  fill_thread<STAGE>(blockIdx.x * kFillBlock + threadIdx.x, P, n, stride, pst, cell_start, run_end, nbr, cnt, err, T,
+  fill_thread(blockIdx.x * kFillBlock + threadIdx.x, P, n, stride, pst, cell_start, run_end, nbr, cnt, err, T,
                      fw);
 }
 
@@ -815,8 +841,9 @@ constexpr int kMaskUnits = 9 * kMaskWords;                 // mask words of a pa
 
 // Keep the first `cap` candidates of the reference's order (x offset outer, z
 // inner; within a bin ascending slots), clear the others' bits.
-__device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t key0, uint32_t (*m)[kMaskBlock],
-                                         uint32_t (*near)[kMaskBlock], const uint32_t* __restrict__ cell_start) {
+template <int PITCH>
+__device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t key0, uint32_t (*m)[PITCH],
+                                         uint32_t (*near)[PITCH], int col, const uint32_t* __restrict__ cell_start) {
   int rem = cap;
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
@@ -828,15 +855,15 @@ __device__ __noinline__ void keep_capped(int cap, const pbf::Region& R, uint32_t
         for (int w = lo >> 5; w < kMaskWords && 32 * w < hi; ++w) {
           const int l = max(lo - 32 * w, 0), e = min(hi - 32 * w, 32);
           const uint32_t range = (e == 32 ? 0xffffffffu : (1u << e) - 1u) & ~((1u << l) - 1u);
-          const uint32_t all = m[r * kMaskWords + w][threadIdx.x];
+          const uint32_t all = m[r * kMaskWords + w][col];
           uint32_t keep = all & range;
           int extra = __popc(keep) - rem;
           rem = max(-extra, 0);
           if (extra > 0) {
             for (; extra > 0; --extra) keep &= ~(0x80000000u >> __clz(keep));
             keep |= all & ~range;
-            m[r * kMaskWords + w][threadIdx.x] = keep;
-            near[r * kMaskWords + w][threadIdx.x] &= keep;
+            m[r * kMaskWords + w][col] = keep;
+            near[r * kMaskWords + w][col] &= keep;
           }
         }
       }
@@ -904,28 +931,13 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
       const float4* p = pst + a0;
 #pragma unroll 1
       for (int w = 0; w < kMaskWords; ++w, p += 32) {
-        const int rest = min(len - 32 * w, 32);
+        const int many = min(len - 32 * w, 32);
         uint32_t m = 0, mn = 0;
-        if (rest > 0) {
-          int c = 0;
-#pragma unroll 1
-          for (; c < rest; c += 4) {
-            const float4 q0 = __ldg(p + c), q1 = __ldg(p + c + 1), q2 = __ldg(p + c + 2), q3 = __ldg(p + c + 3);
-            auto test = [&](const float4& q) {  // the sign bits of d^2 - s^2 and d^2 - near^2 (a NaN's are clear)
-              const float d2 = pbf::mag2<true>(pbf::xsub(xp.x, q.x), pbf::xsub(xp.y, q.y), pbf::xsub(xp.z, q.z));
-              m = __funnelshift_l(__float_as_uint(pbf::xsub(d2, s2)), m, 1);
-              mn = __funnelshift_l(__float_as_uint(pbf::xsub(d2, near2)), mn, 1);
-            };
-            test(q0);
-            test(q1);
-            test(q2);
-            test(q3);
-          }
-          m = __brev(m << (32 - c));  // candidate t at bit t
-          if (rest < 32) m &= (1u << rest) - 1u;
+        if (many > 0) {
+          const uint2 mm = test_chunk2(p, many, xp.x, xp.y, xp.z, s2, near2);
           const uint32_t self = (uint32_t)b - a0 - 32u * (uint32_t)w;
-          if (r == 4 && self < 32u) m &= ~(1u << self);
-          mn = __brev(mn << (32 - c)) & m;
+          m = r == 4 && self < 32u ? mm.x & ~(1u << self) : mm.x;
+          mn = mm.y & m;
         }
         const int u = r * kMaskWords + w;
         mask[u][tid] = m;
@@ -940,7 +952,7 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
   int32_t* row = nbr + pbf::list_base(b, stride);
   const int cap = P.cap;
   if (count > cap) {
-    keep_capped(cap, R, key0, mask, near, cell_start);
+    keep_capped<kMaskBlock>(cap, R, key0, mask, near, tid, cell_start);
     count = cap;
     walk = 0;
     near_units = far_units = 0;
@@ -1092,6 +1104,234 @@ __global__ void __launch_bounds__(kFillBlock) k_fill_rest(Dev P, int n, size_t s
     if (lane == 0 && capped) atomicAdd(&fw[kFillCapped], (uint32_t)__popc(capped));
   }
 }
+// ---- the fill of a few particles: T warps a tile of 32 ----
+// k_fill_masks gives a particle one thread, whose nine rows are a chain of
+// about a hundred groups of loads; with few particles that chain is the launch's
+// time (37 us at 2k particles).  Here the 32 particles of a tile get T = 3 or 9
+// warps, each with rows of its own (three or one of the nine); counts in
+// shared memory then give every warp the places of its entries, stored one by
+// one.  The setup is repeated in every warp and the stores are scattered, so
+// k_fill_masks is faster for many particles (kSplit9Most, kSplit3Most).
+// REF: the lists in the reference's order for exact math and the search on
+// device arrays (T = 1 there for many particles): the entries' places follow
+// from the counts of the 27 visits, those past the cap are dropped.
+template <int T, bool REF>
+struct SplitShared {
+  uint32_t mask[kMaskUnits][32];                // within s
+  uint32_t near[REF ? 1 : kMaskUnits][32];      // ... and within the near radius
+  uint32_t first[9][32];                        // the rows' first slots
+  uint8_t length[9][32];                        // ... and candidates
+  uint8_t cut[REF ? 9 : 1][2][32];              // REF: where the row's second and third bin start
+  uint8_t count[REF ? 27 : 2 * T][32];          // REF: per visit; else per warp, all and near
+  uint32_t bad, over;                           // lanes left to the walk; some list is over the cap
+};
+
+// Where the lists go: the context's warp-tiled lists, or rows of caller
+// indices (the search on device arrays).
+struct ListOut {
+  int32_t* nbr;
+  size_t stride;
+  __device__ __forceinline__ void put(int b, int at, uint32_t q) const {
+    nbr[pbf::list_base(b, stride) + pbf::list_off(at)] = (int32_t)q;
+  }
+  __device__ __forceinline__ void end(int, int, int, int, int) const {}
+  __device__ __forceinline__ size_t index(int b) const { return (size_t)b; }
+};
+struct IndexOut {
+  int32_t* out;
+  const uint32_t* id;
+  int cap;
+  __device__ __forceinline__ void put(int b, int at, uint32_t q) const {
+    out[(size_t)id[b] * cap + at] = (int32_t)id[q];
+  }
+  // -1 past the count, by warp t of the tile's
+  __device__ __forceinline__ void end(int b, int count, int t, int warps, int) const {
+    for (int k = count + t; k < cap; k += warps) out[(size_t)id[b] * cap + k] = -1;
+  }
+  __device__ __forceinline__ size_t index(int b) const { return (size_t)id[b]; }
+};
+
+template <int T, bool REF, class Out>
+__global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float4* __restrict__ pst,
+                                                       const uint32_t* __restrict__ cell_start, Out out, int32_t* cnt,
+                                                       uint8_t* ref_order, uint32_t* fw, uint2* rest) {
+  constexpr int kRows = 9 / T;
+  __shared__ SplitShared<T, REF> S;
+  const int lane = threadIdx.x & 31, t = threadIdx.x >> 5;
+  const int b = blockIdx.x * 32 + lane;
+  const bool live = b < n;
+  const int bb = live ? b : n - 1;
+  const float4 xp = pst[bb];
+  const float s = P.s, s2 = P.s2, near2 = P.near2;
+  const int cap = P.cap;
+  const pbf::Region R = pbf::region_of(P, bb);
+  int bx[3], by[3], bz[3];
+  axis_bins(xp.x, s, bx);
+  axis_bins(xp.y, s, by);
+  axis_bins(xp.z, s, bz);
+  const bool finite = isfinite(xp.x) && isfinite(xp.y) && isfinite(xp.z);
+  bool masks = finite && bx[1] - bx[0] == 1 && bx[2] - bx[1] == 1 && by[1] - by[0] == 1 && by[2] - by[1] == 1 &&
+               bz[1] - bz[0] == 1 && bz[2] - bz[1] == 1 && bx[0] >= 0 && by[0] >= 0 && bz[0] >= 0 &&
+               bx[2] < R.dimx && by[2] < R.dimy && bz[2] < R.dimz;
+  const uint32_t key0 =
+      R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)bz[0] + ((uint32_t)by[0] * (uint32_t)R.dimx + (uint32_t)bx[0]);
+  if (threadIdx.x == 0) S.bad = S.over = 0u;
+  __syncthreads();
+  if (masks) {
+    const float ylo = fmaxf(xp.y - ((float)by[1] * s - s) - P.skip_eps, 0.f);
+    const float yhi = fmaxf(((float)(by[1] + 1) * s - s) - xp.y - P.skip_eps, 0.f);
+    const float zlo = fmaxf(xp.z - ((float)bz[1] * s - s) - P.skip_eps, 0.f);
+    const float zhi = fmaxf(((float)(bz[1] + 1) * s - s) - xp.z - P.skip_eps, 0.f);
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+      const int r = t * kRows + i, k = r / 3, j = r - 3 * k;
+      const float ey = j == 0 ? ylo : (j == 2 ? yhi : 0.f), ez = k == 0 ? zlo : (k == 2 ? zhi : 0.f);
+      const uint32_t rk = key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)k + (uint32_t)(j * R.dimx);
+      uint32_t a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+      if (!(ey * ey + ez * ez > s2)) {
+        a0 = cell_start[rk];
+        a3 = cell_start[rk + 3];
+        if (REF) {
+          a1 = cell_start[rk + 1];
+          a2 = cell_start[rk + 2];
+        }
+      }
+      S.first[r][lane] = a0;
+      S.length[r][lane] = (uint8_t)min(a3 - a0, 255u);
+      if (REF) {
+        S.cut[r][0][lane] = (uint8_t)min(a1 - a0, 255u);
+        S.cut[r][1][lane] = (uint8_t)min(a2 - a0, 255u);
+      }
+      masks = masks && a3 - a0 <= (uint32_t)kMaskRow;
+    }
+  }
+  const unsigned left = __ballot_sync(0xffffffffu, live && !masks);
+  if (lane == 0 && left) atomicOr(&S.bad, left);
+  __syncthreads();
+  const bool mine = live && !(S.bad >> lane & 1u);
+  if (t == 0 && lane == 0 && S.bad) rest[atomicAdd(&fw[kFillRest], 1u)] = make_uint2(blockIdx.x, S.bad);
+  int all = 0, walk = 0;  // this warp's rows
+  if (mine) {
+    for (int i = 0; i < kRows; ++i) {
+      const int r = t * kRows + i;
+      const uint32_t a0 = S.first[r][lane];
+      const int len = S.length[r][lane];
+      for (int w = 0; w < kMaskWords; ++w) {
+        const int many = min(len - 32 * w, 32);
+        uint32_t m = 0, mn = 0;
+        if (many > 0) {
+          const float4* p = pst + a0 + 32 * w;
+          if (REF) {
+            m = test_chunk(p, many, xp.x, xp.y, xp.z, s2);
+          } else {
+            const uint2 mm = test_chunk2(p, many, xp.x, xp.y, xp.z, s2, near2);
+            m = mm.x;
+            mn = mm.y;
+          }
+          const uint32_t self = (uint32_t)b - a0 - 32u * (uint32_t)w;
+          if (r == 4 && self < 32u) m &= ~(1u << self);
+          mn &= m;
+        }
+        const int u = r * kMaskWords + w;
+        S.mask[u][lane] = m;
+        if (!REF) S.near[u][lane] = mn;
+        all += __popc(m);
+        walk += __popc(mn);
+      }
+      if (REF) {
+        const int k = r / 3, j = r - 3 * k;
+        const int c1 = S.cut[r][0][lane], c2 = S.cut[r][1][lane];
+        int n0 = 0, n1 = 0, n2 = 0;
+        for (int w = 0; w < kMaskWords; ++w) {
+          const uint32_t m = S.mask[r * kMaskWords + w][lane];
+          const uint32_t below1 = low_bits(c1 - 32 * w), below2 = low_bits(c2 - 32 * w);
+          n0 += __popc(m & below1);
+          n1 += __popc(m & below2 & ~below1);
+          n2 += __popc(m & ~below2);
+        }
+        S.count[j * 3 + k][lane] = (uint8_t)n0;
+        S.count[9 + j * 3 + k][lane] = (uint8_t)n1;
+        S.count[18 + j * 3 + k][lane] = (uint8_t)n2;
+      }
+    }
+  }
+  if (REF) {
+    __syncthreads();
+    if (!mine) return;
+    // every visit's first place, in the reference's order; this warp's visits' entries
+    int at = 0;
+    for (int v = 0; v < 27; ++v) {
+      const int i = v / 9, j = v / 3 % 3, k = v % 3, r = k * 3 + j;
+      if (r / kRows == t && at < cap) {
+        const int lo = i == 0 ? 0 : S.cut[r][i - 1][lane], hi = i == 2 ? kMaskRow : S.cut[r][i][lane];
+        int e = at;
+        for (int w = lo >> 5; w < kMaskWords && 32 * w < hi; ++w) {
+          uint32_t m = S.mask[r * kMaskWords + w][lane] & low_bits(hi - 32 * w) & ~low_bits(lo - 32 * w);
+          for (; m && e < cap; m &= m - 1u) out.put(b, e++, S.first[r][lane] + 32u * (uint32_t)w + (uint32_t)__ffs(m) - 1u);
+        }
+      }
+      at += S.count[v][lane];
+    }
+    at = min(at, cap);
+    out.end(b, at, t, T, cap);
+    if (t == 0) {
+      cnt[out.index(b)] = at;
+      count_capped(fw, at >= cap);
+    }
+    return;
+  }
+  S.count[REF ? 0 : t][lane] = (uint8_t)min(all, 255);
+  S.count[REF ? 0 : T + t][lane] = (uint8_t)walk;
+  int total = 0;
+  __syncthreads();
+  for (int w = 0; w < T; ++w) total += S.count[REF ? 0 : w][lane];
+  if (mine && total > cap) S.over = 1u;
+  __syncthreads();
+  if (S.over) {  // uniform: the lists over the cap lose bits, then every warp counts again
+    if (t == 0 && mine && total > cap) keep_capped<32>(cap, R, key0, S.mask, S.near, lane, cell_start);
+    __syncthreads();
+    if (mine && total > cap) {
+      all = walk = 0;
+      for (int u = t * kRows * kMaskWords; u < (t + 1) * kRows * kMaskWords; ++u) {
+        all += __popc(S.mask[u][lane]);
+        walk += __popc(S.near[REF ? 0 : u][lane]);
+      }
+      S.count[REF ? 0 : t][lane] = (uint8_t)all;
+      S.count[REF ? 0 : T + t][lane] = (uint8_t)walk;
+    }
+    __syncthreads();
+    total = min(total, cap);
+  }
+  if (!mine) return;
+  // places: the near entries of the warps before, then all near and the other entries of the warps before
+  int near_at = 0, far_at = 0, near_all = 0;
+  for (int w = 0; w < T; ++w) {
+    const int a = S.count[REF ? 0 : w][lane], c = S.count[REF ? 0 : T + w][lane];
+    near_all += c;
+    if (w < t) {
+      near_at += c;
+      far_at += a - c;
+    }
+  }
+  far_at += near_all;
+  for (int u = t * kRows * kMaskWords; u < (t + 1) * kRows * kMaskWords; ++u) {
+    uint32_t m = S.mask[u][lane];
+    if (m == 0u) continue;
+    const uint32_t mn = S.near[REF ? 0 : u][lane];
+    const uint32_t q = S.first[u / kMaskWords][lane] + 32u * (uint32_t)(u % kMaskWords);
+    for (; m; m &= m - 1u) {
+      const int bit = __ffs(m) - 1;
+      out.put(b, mn >> bit & 1u ? near_at++ : far_at++, q + (uint32_t)bit);
+    }
+  }
+  if (t == 0) {
+    cnt[b] = total;
+    P.walk[b] = (uint8_t)near_all;
+    ref_order[b] = 0;
+    count_capped(fw, total >= cap);
+  }
+}
+
 static_assert(kMaskWords == 3 && kMaskUnits <= 32, "the words' division by 3 and their bit set");
 // ---- near entries ----
 // The lists reach to s (1.2 h in the reference) because x* moves during the
@@ -3456,42 +3696,60 @@ void launch_cell_sort(pbf_ctx* ctx) {
       reinterpret_cast<uint32_t*>(ctx->stage), ctx->place);
 }
 
+// Particles up to which the fill takes nine and three warps a tile.  Measured,
+// us, fast math: 2k 15.6 with nine warps, 27.4 with three, 36.5 k_fill_masks;
+// 16k 17.6 / 23.8 / 34.0; 33k 24.6 / 25.7 / 34.0; 48k 30.8 / 32.7 / 37.6; 66k
+// 40.6 / 41.4 / 40.4; 1M 525 / 429 / 388.  Exact math and the search on device
+// arrays (one warp a tile in k_fill_masks's place): 2k 12.5 / 25.7 / 38.8, 33k
+// 29.4 / 31.6 / 44.3, 48k 42.5 / 38.4 / 47.0, 98k 78.6 / 65.7 / 64.9.
+constexpr size_t kSplit9Most = 40960, kSplit3Most = 61440;
+
 void launch_fill(pbf_ctx* ctx, const float4* pst) {
-  const bool fast = ctx->params.exact_math == 0;
-  uint32_t* fw = fast ? ctx->fill_words : nullptr;
+  const bool fast = ctx->params.exact_math == 0, staged = any_staged(ctx);
+  const int n = (int)ctx->n, tiles = blocks_for(ctx->n, 32);
+  const Dev& P = ctx->dev;
+  cudaStream_t s = ctx->stream;
+  uint32_t* fw = ctx->fill_words;
   {
     Launch L(ctx, "runs");
-    k_runs<<<blocks_for(ctx->n, kRunBlock), kRunBlock, 0, ctx->stream>>>((int)ctx->n, pst, ctx->run_end,
-                                                                         ctx->cell_count + ctx->nbins + kCrowdedRuns, fw);
+    k_runs<<<blocks_for(ctx->n, kRunBlock), kRunBlock, 0, s>>>(n, pst, ctx->run_end,
+                                                               ctx->cell_count + ctx->nbins + kCrowdedRuns, fw);
   }
   // fast math: lists in slot order (the gathers' sums in any order are within
   // the fast path's tolerance); exact math and the staged gathers' 16-bit
   // lists: the reference's order
-  const bool staged = any_staged(ctx);
   ctx->lists_slot_order = fast && !staged;
-  const int n = (int)ctx->n;
-  cudaStream_t s = ctx->stream;
-  if (!ctx->lists_slot_order) {
-    Launch L(ctx, "fill_neighbors");
-    const int grid = blocks_for(ctx->n, kFillBlock);
-    if (staged)
-      k_fill2<true><<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr,
-                                                ctx->cnt, ctx->err, tile_io(ctx), fw);
-    else
-      k_fill2<false><<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end,
-                                                 ctx->nbr, ctx->cnt, ctx->err, tile_io(ctx), fw);
-    return;
-  }
   {
     Launch L(ctx, "fill_neighbors");
-    k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start,
-                                                                      ctx->nbr, ctx->cnt, ctx->ref_order, fw,
-                                                                      ctx->rest);
+    const ListOut out{ctx->nbr, ctx->lstride};
+    auto split = [&](auto warps, auto ref) {
+      constexpr int T = decltype(warps)::value;
+      k_fill_split<T, decltype(ref)::value, ListOut><<<tiles, 32 * T, 0, s>>>(P, n, pst, ctx->cell_start, out, ctx->cnt,
+                                                                            ctx->ref_order, fw, ctx->rest);
+    };
+    using W1 = std::integral_constant<int, 1>;
+    using W3 = std::integral_constant<int, 3>;
+    using W9 = std::integral_constant<int, 9>;
+    if (staged)
+      k_fill2<<<blocks_for(ctx->n, kFillBlock), kFillBlock, 0, s>>>(P, n, ctx->lstride, pst, ctx->cell_start,
+                                                                    ctx->run_end, ctx->nbr, ctx->cnt, ctx->err,
+                                                                    tile_io(ctx), fw);
+    else if (ctx->n <= kSplit9Most)
+      fast ? split(W9{}, std::false_type{}) : split(W9{}, std::true_type{});
+    else if (ctx->n <= kSplit3Most)
+      fast ? split(W3{}, std::false_type{}) : split(W3{}, std::true_type{});
+    else if (!fast)
+      split(W1{}, std::true_type{});
+    else
+      k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, s>>>(P, n, ctx->lstride, pst, ctx->cell_start,
+                                                                        ctx->nbr, ctx->cnt, ctx->ref_order, fw,
+                                                                        ctx->rest);
   }
+  if (staged) return;
   Launch L(ctx, "fill_rest");
   const int grid = std::min(blocks_for(ctx->n, kFillBlock), 16 * ctx->sms);  // a warp or more for every queued one
-  k_fill_rest<<<grid, kFillBlock, 0, s>>>(ctx->dev, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr,
-                                          ctx->cnt, ctx->err, ctx->ref_order, fw, ctx->rest);
+  k_fill_rest<<<grid, kFillBlock, 0, s>>>(P, n, ctx->lstride, pst, ctx->cell_start, ctx->run_end, ctx->nbr, ctx->cnt,
+                                          ctx->err, ctx->ref_order, fw, ctx->rest);
 }
 
 // An upload forgets the fills before it: no lists counted at the cap.
@@ -3951,11 +4209,11 @@ void launch_step(pbf_ctx* ctx) {
 int launches_per_step(const pbf_ctx* ctx) {
   // kernels only (the memsets are not), as launched eagerly (a captured
   // learned step runs its plain iterations in a conditional graph node and
-  // launches fewer once converged): ext/predict/hash + sort + reorder + runs + fill + [fast math: rest] +
+  // launches fewer once converged): ext/predict/hash + sort + reorder + runs + fill + [not staged: rest] +
   // K x (density/lambda, [exact: lambda fix-up], delta-p)
   // + (K==0: velocity) + 2 if gamma + 4 (visc, vort, apply, visc)
   const int sort = 4;  // 2 scan, arrivals, crowded bins
-  const int fill = ctx->params.exact_math || any_staged(ctx) ? 2 : 3;  // runs, fill, [rest]
+  const int fill = any_staged(ctx) ? 2 : 3;  // runs, fill, [rest]
   if (persist_on(ctx)) return 1 + sort + 1 + fill + 1;  // ... reorder, runs, fill, rest, the persistent step
   const int K = ctx->params.solve_steps;
   const int tail = (ctx->params.gamma != 0.0f ? 2 : 0) + 4;
@@ -5412,8 +5670,10 @@ constexpr size_t kOffRunEnd = align_up(kOffBits + 4 * 2 * kNaWords * kNaOrderBlo
 constexpr size_t kOffSortedX = align_up(kOffRunEnd + 4 * kNaN);
 constexpr size_t kOffSortedId = align_up(kOffSortedX + 16 * (kNaN + kMaskOver));
 constexpr size_t kOffErr = align_up(kOffSortedId + 4 * kNaN);
+constexpr size_t kOffFillWords = align_up(kOffErr + 4);
+constexpr size_t kOffRest = align_up(kOffFillWords + 4 * kFillWords);
 constexpr size_t kNoallocBytes = PBF_NOALLOC_SCRATCH_BYTES;
-static_assert(kOffErr + 4 <= kNoallocBytes, "PBF_NOALLOC_SCRATCH_BYTES in pbf.h is too small");
+static_assert(kOffRest + 8 * kNaWords <= kNoallocBytes, "PBF_NOALLOC_SCRATCH_BYTES in pbf.h is too small");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 
@@ -5469,15 +5729,20 @@ __device__ __noinline__ int noalloc_fill_runs(float px, float py, float pz, floa
   return count;
 }
 
-// The list fill writing straight into the caller's output in reference index
-// space: out[id][k], -1 past the count.
-__global__ void __launch_bounds__(kBlock) k_noalloc_fill(Dev P, int n, const float4* __restrict__ pst,
+// The particles k_fill_split left, by the warp it queued, into the caller's
+// output in reference index space: out[id][k], -1 past the count.
+__global__ void __launch_bounds__(kBlock) k_noalloc_rest(Dev P, const uint32_t* __restrict__ fw,
+                                                         const uint2* __restrict__ rest,
+                                                         const float4* __restrict__ pst,
                                                          const uint32_t* __restrict__ sorted_id,
                                                          const uint32_t* __restrict__ cell_start,
                                                          const uint32_t* __restrict__ run_end, int32_t* out,
                                                          int32_t* out_cnt, uint32_t* err) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
+  const uint32_t t = (blockIdx.x * kBlock + threadIdx.x) >> 5;
+  if (t >= fw[kFillRest]) return;
+  const uint2 w = rest[t];
+  if (!(w.y >> (threadIdx.x & 31) & 1u)) return;
+  const int b = (int)(w.x * 32u + (threadIdx.x & 31u));
   const float4 xp = pst[b];
   const int cap = P.cap;
   int32_t* row = out + (size_t)sorted_id[b] * cap;
@@ -5561,6 +5826,8 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
   auto* sorted_x = reinterpret_cast<float4*>(base + kOffSortedX);
   auto* sorted_id = reinterpret_cast<uint32_t*>(base + kOffSortedId);
   auto* err = reinterpret_cast<uint32_t*>(base + kOffErr);
+  auto* fw = reinterpret_cast<uint32_t*>(base + kOffFillWords);
+  auto* rest = reinterpret_cast<uint2*>(base + kOffRest);
   // The array keeps the previous call's contents: clear what must start at
   // zero (the histogram and the error word; every other buffer is written in
   // full before it is read).
@@ -5578,8 +5845,14 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
                                                                crowded, cell_start, arrivals, bits, place);
   k_noalloc_gather<<<g, kBlock, 0, s>>>(nn, sort, d_x, sorted_x, sorted_id);
   k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end,
-                                                        cell_count + d.nbins + kCrowdedRuns, nullptr);
-  k_noalloc_fill<<<g, kBlock, 0, s>>>(d, nn, sorted_x, sorted_id, cell_start, run_end, d_nbr, d_cnt, err);
+                                                        cell_count + d.nbins + kCrowdedRuns, fw);
+  const IndexOut out{d_nbr, sorted_id, d.cap};
+  const int fill_tiles = blocks_for(n, 32);
+  if (n <= kSplit9Most)
+    k_fill_split<9, true, IndexOut><<<fill_tiles, 288, 0, s>>>(d, nn, sorted_x, cell_start, out, d_cnt, nullptr, fw, rest);
+  else
+    k_fill_split<3, true, IndexOut><<<fill_tiles, 96, 0, s>>>(d, nn, sorted_x, cell_start, out, d_cnt, nullptr, fw, rest);
+  k_noalloc_rest<<<g, kBlock, 0, s>>>(d, fw, rest, sorted_x, sorted_id, cell_start, run_end, d_nbr, d_cnt, err);
   if (d_flags) e = cudaMemcpyAsync(d_flags, err, 4, cudaMemcpyDeviceToDevice, s);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return fail(nullptr, PBF_ERR_CUDA, "noalloc neighbor search launch: %s", cudaGetErrorString(e));

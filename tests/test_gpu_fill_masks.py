@@ -1,11 +1,12 @@
-"""The fast path's list fill (k_fill_masks) against the reference-order walk.
+"""The list fill from mask words against the oracle's lists.
 
-It tests a row of three bins into 32-bit mask words, at most 96 candidates a
-row, and clears the candidates past the cap before it writes a list; other
-particles (longer rows, positions whose float re-hash leaves the integer
-neighbour bins) are walked in the reference's order.  Exact math always walks
-in the reference's order, so the two must export the same lists, bit for bit;
-the oracle's are the third.
+The fill tests a row of three bins into 32-bit mask words, at most 96
+candidates a row; other particles (longer rows, positions whose float re-hash
+leaves the integer neighbour bins) are walked in the reference's order.  Fast
+math writes its lists in slot order and drops the candidates past the cap by
+the reference's order, exact math writes the reference's order, and both take
+more or fewer warps a tile of 32 particles by the particle count; all must
+export the same lists, bit for bit.
 """
 from __future__ import annotations
 
@@ -80,3 +81,21 @@ def test_batch_lists(squeeze):
             got.append(g.neighbors(60))
             assert g.stats()["error_flags"] == 0
     assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][0], got[1][0])
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 40960, 40961, 61440, 61441, 70003])
+@pytest.mark.parametrize("squeeze,cap", [(1.0, 60), (0.8, 60), (0.8, 33)])
+def test_particle_counts_at_the_dispatch_edges(n, squeeze, cap):
+    sc = make_scene("dam_65k", neighbor_cap=cap)
+    p = sc.params()
+    i = np.arange(n)
+    rng = np.random.default_rng(n)
+    x = np.stack([i % 41, i // 41 % 41, i // 1681], 1) * 0.5 * squeeze + 1.0 + rng.uniform(-0.1, 0.1, (n, 3))
+    x = x.astype(np.float32)
+    o = OracleSim(p, n)
+    o.set_state(x)
+    o.stage(2)
+    want = o.neighbors()
+    for exact in (0, 1):
+        got = _lists(p, n, x, exact)
+        assert np.array_equal(got[1], want[1]) and np.array_equal(got[0], want[0])
