@@ -5305,7 +5305,7 @@ int pbf_mlp_train(pbf_ctx* ctx, int adam_steps, int batch, float lr, uint64_t se
   for (int it = 0; it < adam_steps; ++it) {
     CK(cudaMemsetAsync(ctx->mlp_grad, 0, sizeof(float) * pbf::kMlpParams, ctx->stream));
     CK(cudaMemsetAsync(ctx->mlp_loss, 0, sizeof(float), ctx->stream));
-    pbf::k_mlp_grad_tc<true, true><<<grad_tc_grid(ctx, batch), pbf::tc::kThreads, pbf::tt::kSmemBytes,
+    pbf::k_mlp_grad_tc<true, true><<<grad_tc_grid(ctx, batch), pbf::tt::kThreads, pbf::tt::kSmemBytes,
                                       ctx->stream>>>(M, ctx->feats, ctx->lamsumH, (int)ctx->n, batch,
                                                      seed + 0x632BE59BD9B4E019ull * (uint64_t)it,
                                                      1.0f / ctx->label_scale, ctx->mlp_grad, ctx->mlp_loss,
@@ -5336,7 +5336,7 @@ int pbf_mlp_gradients(pbf_ctx* ctx, const float* features, const float* targets,
   CK(cudaMemsetAsync(ctx->mlp_grad, 0, sizeof(float) * pbf::kMlpParams, ctx->stream));
   CK(cudaMemsetAsync(ctx->mlp_loss, 0, sizeof(float), ctx->stream));
   if (int rc = grad_tc_setup(ctx)) return rc;
-  pbf::k_mlp_grad_tc<false, false><<<grad_tc_grid(ctx, (int)n), pbf::tc::kThreads, pbf::tt::kSmemBytes,
+  pbf::k_mlp_grad_tc<false, false><<<grad_tc_grid(ctx, (int)n), pbf::tt::kThreads, pbf::tt::kSmemBytes,
                                      ctx->stream>>>(mlp_dev(ctx), df, dt, (int)n, (int)n, 0, 1.0f, ctx->mlp_grad,
                                                     ctx->mlp_loss, ctx->err);
   if (int rc = check_launch(ctx, "mlp_gradients")) return rc;

@@ -43,14 +43,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-// GELU(x) = x/2 (1 + erf(x/sqrt 2)) and its derivative.
-__device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-__device__ __forceinline__ float gelu_grad(float x) {
-  const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
-  const float pdf = 0.3989422804014327f * __expf(-0.5f * x * x);
-  return cdf + x * pdf;
-}
-
 // GELU of two values at once for the tensor-core network's epilogues:
 // x/2 (1 + erf(u)), u = x/sqrt 2 clamped to [-3, 3], erf(u) = u q(u^2) with q a
 // degree-8 polynomial fitted to erf on [0, 3] (iteratively reweighted least

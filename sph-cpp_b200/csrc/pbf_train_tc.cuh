@@ -11,13 +11,22 @@
 //   MMA2  Z2[s][n]  = H1[s][k] . W2[n][k]         M128 N64 K64    (A sH1,  B sW2)
 //   epilogue 2: y = GELU(Z2 + b2) . w3 + b3, dy = 2 (y - t) / B,
 //               dZ2 = dy w3 GELU'(Z2 + b2)  -> sD2 [s][n] and sD2T [n][s];
-//               dw3, db2, db3 and the loss summed per CTA
+//               dw3, db2, db3 and the loss summed per thread
 //   MMA3  dH1[s][k] = dZ2[s][n] . W2T[k][n]       M128 N64 K64    (A sD2,  B sW2T)
 //   MMA4  dW2[n][k] += dZ2T[n][s] . H1T[k][s]     M128 N64 K128   (A sD2T, B sH1T; rows 64..127 of A zero)
-//   epilogue 3: dZ1 = dH1 GELU'(Z1 + b1)  -> sD1T [n][s]; db1 summed
+//   epilogue 3: dZ1 = dH1 GELU'(Z1 + b1)  -> sD1T [n][s]; db1 summed per thread
 //   MMA5  dW1[n][f] += dZ1T[n][s] . XT[f][s]      M128 N16 K128   (A sD1T, B sXT;  rows 64..127 of A zero)
 // TMEM columns: Z1 0..63, Z2 64..127, dH1 128..191, dW2 192..255, dW1 256..271
 // (512 allocated; the kernel's shared memory keeps it to one CTA per SM).
+// Four threads share a sample row, 16 columns each: with one CTA per SM the
+// epilogues are what its warps have to hide each other's latency with.  The
+// column sums (b1, b2, w3) stay in registers over all of a CTA's tiles and are
+// reduced over the lanes once, with one shuffle a column; every erf is
+// evaluated once a hidden unit and tile.  MMA5 is not waited for: the next
+// tile's first commit covers it (XT is double-buffered).  Bound by the
+// epilogues' arithmetic (two erff a hidden unit and sample) and the four waits
+// a tile; 65,536 samples: 97 us with two threads a row, three warp sums a
+// column and tile and four erff a unit, 42 us so.
 // Operand layouts and descriptors are those of pbf_mlp_tc.cuh (K-major, no
 // swizzle, core matrices 128 B apart along K, K/8 * 128 B along M/N).  Every
 // wait on the MMAs' mbarrier is bounded; a wait that gives up raises
@@ -30,13 +39,15 @@
 namespace pbf {
 namespace tt {
 
-constexpr int kCols = 512;  // TMEM columns allocated
+constexpr int kCols = 512;     // TMEM columns allocated
+constexpr int kThreads = 512;  // four threads per row, each for a quarter of the columns
+constexpr int kMine = kMlpH / 4;
 constexpr uint32_t kIdescM128N16 = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
 
 // Shared-memory operand offsets (bytes, 1024-aligned) of the dynamic buffer.
 constexpr uint32_t kX = 0;                                  // [128][16]
 constexpr uint32_t kXT = kX + 128 * 16 * 2;                 // [16][128]
-constexpr uint32_t kW1 = kXT + 16 * 128 * 2;                // [64][16]
+constexpr uint32_t kW1 = kXT + 2 * 16 * 128 * 2;            // [64][16] (XT twice: by tile parity)
 constexpr uint32_t kW2 = kW1 + 64 * 16 * 2;                 // [64][64]
 constexpr uint32_t kW2T = kW2 + 64 * 64 * 2;                // [64][64]
 constexpr uint32_t kH1 = kW2T + 64 * 64 * 2;                // [128][64]
@@ -44,7 +55,7 @@ constexpr uint32_t kH1T = kH1 + 128 * 64 * 2;               // [64][128]
 constexpr uint32_t kD2 = kH1T + 64 * 128 * 2;               // [128][64]
 constexpr uint32_t kD2T = kD2 + 128 * 64 * 2;               // [128][128], rows 64..127 zero
 constexpr uint32_t kD1T = kD2T + 128 * 128 * 2;             // [128][128], rows 64..127 zero
-constexpr uint32_t kSmemBytes = kD1T + 128 * 128 * 2;       // 141,312
+constexpr uint32_t kSmemBytes = kD1T + 128 * 128 * 2;       // 145,408
 static_assert(kX % 1024 == 0 && kXT % 1024 == 0 && kW1 % 1024 == 0 && kW2 % 1024 == 0 && kW2T % 1024 == 0 &&
                   kH1 % 1024 == 0 && kH1T % 1024 == 0 && kD2 % 1024 == 0 && kD2T % 1024 == 0 && kD1T % 1024 == 0,
               "operand alignment");
@@ -69,6 +80,29 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// Column sums of 16 values a lane over the 32 lanes: 16 shuffles (each step
+// halves the columns a lane keeps).  Lane l ends with column column_of(l),
+// lanes 2i and 2i + 1 with the same.
+__device__ __forceinline__ float column_sums(float (&v)[16], int lane) {
+#pragma unroll
+  for (int o = 16, k = 8; k > 0; o >>= 1, k >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < k; ++i) {
+      const float keep = up ? v[i + k] : v[i], give = up ? v[i] : v[i + k];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+__device__ __forceinline__ int column_of(int lane) {
+  return (lane >> 4 & 1) * 8 + (lane >> 3 & 1) * 4 + (lane >> 2 & 1) * 2 + (lane >> 1 & 1);
+}
+
+// GELU(x) = x cdf(x), GELU'(x) = cdf(x) + x pdf(x).
+__device__ __forceinline__ float normal_cdf(float x) { return 0.5f * (1.0f + erff(x * 0.70710678118654752f)); }
+__device__ __forceinline__ float normal_pdf(float x) { return 0.3989422804014327f * __expf(-0.5f * x * x); }
+
 }  // namespace tt
 
 // Gradient of L = mean over the batch of (y - target)^2, added into grad
@@ -76,38 +110,39 @@ __device__ __forceinline__ float warp_sum(float v) {
 // normalised here (else already normalised); SAMPLE: rows drawn from the
 // n_data recorded rows by the counter-based hash sample_row (else rows
 // 0..batch-1); targets = labels * inv_label_scale.  A persistent grid, one
-// 256-thread CTA per SM: two threads per sample row, each for half the
-// columns.
+// 512-thread CTA per SM.
 template <bool NORMALIZE, bool SAMPLE, bool NO_ARRIVE = false>
-__global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const float* __restrict__ feats,
+__global__ void __launch_bounds__(tt::kThreads, 1) k_mlp_grad_tc(MlpDev M, const float* __restrict__ feats,
                                                                 const float* __restrict__ labels, int n_data,
                                                                 int batch, uint64_t seed, float inv_label_scale,
                                                                 float* grad, float* loss, uint32_t* err) {
   extern __shared__ __align__(1024) uint8_t sm[];
   __shared__ float sb1[kMlpH], sb2[kMlpH], sw3[kMlpH];
-  __shared__ float gb1[kMlpH], gb2[kMlpH], gw3[kMlpH], half2[2][tc::kRows];
+  __shared__ float gb1[kMlpH], gb2[kMlpH], gw3[kMlpH], part4[4][tc::kRows];
   __shared__ float gloss, gb3;
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tslot;
   __shared__ int fail;
   namespace T = tc;
+  constexpr int kMine = tt::kMine;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = tid & (T::kRows - 1), h = tid >> 7;
+  const int row = tid & (T::kRows - 1), h = tid >> 7;  // row of the tile, quarter of the columns
+  const int c0 = kMine * h;
   const int tiles = (batch + T::kRows - 1) / T::kRows;
   // weights (BF16 operand copies), biases, zeroed sums and padding rows
-  for (int i = tid; i < kMlpH * 2; i += T::kThreads) {
+  for (int i = tid; i < kMlpH * 2; i += tt::kThreads) {
     const int r = i >> 1, kc = (i & 1) * 8;
     *reinterpret_cast<uint4*>(sm + tt::kW1 + T::core_off(r, kc, kMlpInPad)) =
         *reinterpret_cast<const uint4*>(M.w1 + r * kMlpInPad + kc);
   }
-  for (int i = tid; i < kMlpH * 8; i += T::kThreads) {
+  for (int i = tid; i < kMlpH * 8; i += tt::kThreads) {
     const int r = i >> 3, kc = (i & 7) * 8;
     *reinterpret_cast<uint4*>(sm + tt::kW2 + T::core_off(r, kc, kMlpH)) =
         *reinterpret_cast<const uint4*>(M.w2 + r * kMlpH + kc);
     *reinterpret_cast<uint4*>(sm + tt::kW2T + T::core_off(r, kc, kMlpH)) =
         *reinterpret_cast<const uint4*>(M.w2t + r * kMlpH + kc);
   }
-  for (int i = tid; i < 64 * 128 / 8; i += T::kThreads) {  // rows 64..127 of the transposed A operands
+  for (int i = tid; i < 64 * 128 / 8; i += tt::kThreads) {  // rows 64..127 of the transposed A operands
     const int r = 64 + i / 16, kc = (i % 16) * 8;
     *reinterpret_cast<uint4*>(sm + tt::kD2T + T::core_off(r, kc, 128)) = make_uint4(0u, 0u, 0u, 0u);
     *reinterpret_cast<uint4*>(sm + tt::kD1T + T::core_off(r, kc, 128)) = make_uint4(0u, 0u, 0u, 0u);
@@ -129,7 +164,7 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
   __syncthreads();
   T::fence_after_sync();
   const uint32_t tmem = tslot;
-  const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(32 * h);
+  const uint32_t lanes = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
   const uint32_t s0 = T::smem_u32(sm);
   const float b3 = M.b3[0];
   const float inv_b = 1.0f / (float)batch;
@@ -140,28 +175,42 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
     phase ^= 1u;
     __syncthreads();
   };
-  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+  // this thread's sums over its rows: columns c0 .. c0 + 15, the loss and b3 (h = 0)
+  float aw3[kMine], ab2[kMine], ab1[kMine], aloss = 0.0f, ab3 = 0.0f;
+#pragma unroll
+  for (int q = 0; q < kMine; ++q) aw3[q] = ab2[q] = ab1[q] = 0.0f;
+  // a row's features 4h .. 4h + 3 (12..15 are zero) and target, loaded a tile ahead
+  float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+  float target = 0.0f;
+  auto load = [&](int tile) {
     const int s = tile * T::kRows + row;
-    const bool ok = s < batch;
-    const int src = ok ? sample_row<SAMPLE>(seed, s, n_data) : 0;
-    // features: half h holds columns 8h..8h+7 (12..15 are zero)
-    float f[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int k = 8 * h + j;
-      float x = 0.0f;
-      if (ok && k < kMlpIn) {
-        x = feats[(size_t)src * kMlpIn + k];
-        if (NORMALIZE) x = (x - M.feat_mean[k]) * M.feat_inv_std[k];
+    f = make_float4(0.f, 0.f, 0.f, 0.f);
+    target = 0.0f;
+    if (tile < tiles && s < batch) {
+      const int src = sample_row<SAMPLE>(seed, s, n_data);
+      if (h < 3) {
+        f = *reinterpret_cast<const float4*>(feats + (size_t)src * kMlpIn + 4 * h);
+        if (NORMALIZE) {
+          f.x = (f.x - M.feat_mean[4 * h]) * M.feat_inv_std[4 * h];
+          f.y = (f.y - M.feat_mean[4 * h + 1]) * M.feat_inv_std[4 * h + 1];
+          f.z = (f.z - M.feat_mean[4 * h + 2]) * M.feat_inv_std[4 * h + 2];
+          f.w = (f.w - M.feat_mean[4 * h + 3]) * M.feat_inv_std[4 * h + 3];
+        }
       }
-      f[j] = x;
+      target = labels[src] * inv_label_scale;
     }
-    *reinterpret_cast<uint4*>(sm + tt::kX + T::core_off(row, 8 * h, kMlpInPad)) =
-        make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                   pack_bf16x2(f[6], f[7]));
-#pragma unroll
-    for (int j = 0; j < 8; ++j) tt::st_bf16(sm, tt::kXT + T::core_off(8 * h + j, row, 128), f[j]);
-    const float target = ok ? labels[src] * inv_label_scale : 0.0f;
+  };
+  load(blockIdx.x);
+  uint32_t xt = tt::kXT;  // this tile's transposed features
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const bool ok = tile * T::kRows + row < batch;
+    const float t = target;
+    *reinterpret_cast<uint2*>(sm + tt::kX + T::core_off(row, 4 * h, kMlpInPad)) =
+        make_uint2(pack_bf16x2(f.x, f.y), pack_bf16x2(f.z, f.w));
+    tt::st_bf16(sm, xt + T::core_off(4 * h, row, 128), f.x);
+    tt::st_bf16(sm, xt + T::core_off(4 * h + 1, row, 128), f.y);
+    tt::st_bf16(sm, xt + T::core_off(4 * h + 2, row, 128), f.z);
+    tt::st_bf16(sm, xt + T::core_off(4 * h + 3, row, 128), f.w);
     T::fence_proxy_async();
     T::fence_before_sync();
     __syncthreads();
@@ -173,26 +222,27 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
         T::mma_commit(bar);
       }
     }
+    load(tile + gridDim.x);
     wait();
     if (fail) break;
     T::fence_after_sync();
     // epilogue 1: H1 = GELU(Z1 + b1)
+    float cdf1[kMine];
+    {
+      float v[kMine];
+      T::tmem_ld16(lanes, v);
 #pragma unroll
-    for (int c = 0; c < 32; c += 16) {
-      float v[16];
-      T::tmem_ld16(lanes + (uint32_t)c, v);
-      const int c0 = 32 * h + c;
-#pragma unroll
-      for (int j = 0; j < 16; j += 8) {
-        float g[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) g[q] = gelu(v[j + q] + sb1[c0 + j + q]);
-        *reinterpret_cast<uint4*>(sm + tt::kH1 + T::core_off(row, c0 + j, kMlpH)) =
-            make_uint4(pack_bf16x2(g[0], g[1]), pack_bf16x2(g[2], g[3]), pack_bf16x2(g[4], g[5]),
-                       pack_bf16x2(g[6], g[7]));
-#pragma unroll
-        for (int q = 0; q < 8; ++q) tt::st_bf16(sm, tt::kH1T + T::core_off(c0 + j + q, row, 128), g[q]);
+      for (int q = 0; q < kMine; ++q) {
+        const float z = v[q] + sb1[c0 + q];
+        cdf1[q] = tt::normal_cdf(z);
+        v[q] = z * cdf1[q];
+        tt::st_bf16(sm, tt::kH1T + T::core_off(c0 + q, row, 128), v[q]);
       }
+#pragma unroll
+      for (int q = 0; q < kMine; q += 8)
+        *reinterpret_cast<uint4*>(sm + tt::kH1 + T::core_off(row, c0 + q, kMlpH)) =
+            make_uint4(pack_bf16x2(v[q], v[q + 1]), pack_bf16x2(v[q + 2], v[q + 3]), pack_bf16x2(v[q + 4], v[q + 5]),
+                       pack_bf16x2(v[q + 6], v[q + 7]));
     }
     T::fence_proxy_async();
     T::fence_before_sync();
@@ -211,47 +261,36 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
     if (fail) break;
     T::fence_after_sync();
     // epilogue 2: the output, its error, dZ2 and the layer-3 / bias-2 sums
-    float z2[32];
-    float part = 0.0f;
+    {
+      float z2[kMine], cdf2[kMine];
+      T::tmem_ld16(lanes + 64u, z2);
+      float part = 0.0f;
 #pragma unroll
-    for (int c = 0; c < 32; c += 16) {
-      T::tmem_ld16(lanes + 64u + (uint32_t)c, z2 + c);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        z2[c + q] += sb2[32 * h + c + q];
-        part = fmaf(gelu(z2[c + q]), sw3[32 * h + c + q], part);
+      for (int q = 0; q < kMine; ++q) {
+        z2[q] += sb2[c0 + q];
+        cdf2[q] = tt::normal_cdf(z2[q]);
+        part = fmaf(z2[q] * cdf2[q], sw3[c0 + q], part);
       }
-    }
-    half2[h][row] = part;
-    __syncthreads();
-    const float y = half2[0][row] + half2[1][row] + b3;
-    const float e = ok ? y - target : 0.0f;
-    const float dy = 2.0f * e * inv_b;
-    if (h == 0) {
-      const float l = tt::warp_sum(e * e * inv_b), d3 = tt::warp_sum(dy);
-      if (lane == 0) {
-        atomicAdd(&gloss, l);
-        atomicAdd(&gb3, d3);
-      }
-    }
+      part4[h][row] = part;
+      __syncthreads();
+      const float y = ((part4[0][row] + part4[1][row]) + (part4[2][row] + part4[3][row])) + b3;
+      const float e = ok ? y - t : 0.0f;
+      const float dy = 2.0f * e * inv_b;
+      aloss = fmaf(e * inv_b, e, aloss);
+      ab3 += dy;
 #pragma unroll
-    for (int c = 0; c < 32; c += 8) {
-      float d[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int n = 32 * h + c + q;
-        const float gw = tt::warp_sum(gelu(z2[c + q]) * dy);
-        d[q] = dy * sw3[n] * gelu_grad(z2[c + q]);
-        const float gb = tt::warp_sum(d[q]);
-        if (lane == 0) {
-          atomicAdd(&gw3[n], gw);
-          atomicAdd(&gb2[n], gb);
-        }
-        tt::st_bf16(sm, tt::kD2T + T::core_off(n, row, 128), d[q]);
+      for (int q = 0; q < kMine; ++q) {
+        aw3[q] = fmaf(z2[q] * cdf2[q], dy, aw3[q]);
+        const float d = dy * sw3[c0 + q] * fmaf(z2[q], tt::normal_pdf(z2[q]), cdf2[q]);
+        ab2[q] += d;
+        z2[q] = d;
+        tt::st_bf16(sm, tt::kD2T + T::core_off(c0 + q, row, 128), d);
       }
-      *reinterpret_cast<uint4*>(sm + tt::kD2 + T::core_off(row, 32 * h + c, kMlpH)) =
-          make_uint4(pack_bf16x2(d[0], d[1]), pack_bf16x2(d[2], d[3]), pack_bf16x2(d[4], d[5]),
-                     pack_bf16x2(d[6], d[7]));
+#pragma unroll
+      for (int q = 0; q < kMine; q += 8)
+        *reinterpret_cast<uint4*>(sm + tt::kD2 + T::core_off(row, c0 + q, kMlpH)) =
+            make_uint4(pack_bf16x2(z2[q], z2[q + 1]), pack_bf16x2(z2[q + 2], z2[q + 3]),
+                       pack_bf16x2(z2[q + 4], z2[q + 5]), pack_bf16x2(z2[q + 6], z2[q + 7]));
     }
     T::fence_proxy_async();
     T::fence_before_sync();
@@ -275,18 +314,16 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
     if (fail) break;
     T::fence_after_sync();
     // epilogue 3: dZ1 = dH1 GELU'(Z1 + b1) and the bias-1 sums
+    {
+      float dh[kMine], z1[kMine];
+      T::tmem_ld16(lanes + 128u, dh);
+      T::tmem_ld16(lanes, z1);
 #pragma unroll
-    for (int c = 0; c < 32; c += 16) {
-      float dh[16], z1[16];
-      T::tmem_ld16(lanes + 128u + (uint32_t)c, dh);
-      T::tmem_ld16(lanes + (uint32_t)c, z1);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int n = 32 * h + c + q;
-        const float d = dh[q] * gelu_grad(z1[q] + sb1[n]);
-        const float gb = tt::warp_sum(d);
-        if (lane == 0) atomicAdd(&gb1[n], gb);
-        tt::st_bf16(sm, tt::kD1T + T::core_off(n, row, 128), d);
+      for (int q = 0; q < kMine; ++q) {
+        const float z = z1[q] + sb1[c0 + q];
+        const float d = dh[q] * fmaf(z, tt::normal_pdf(z), cdf1[q]);
+        ab1[q] += d;
+        tt::st_bf16(sm, tt::kD1T + T::core_off(c0 + q, row, 128), d);
       }
     }
     T::fence_proxy_async();
@@ -296,36 +333,49 @@ __global__ void __launch_bounds__(tc::kThreads, 1) k_mlp_grad_tc(MlpDev M, const
       T::fence_after_sync();
       if (!NO_ARRIVE) {
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)  // dW1 += dZ1^T X
+        for (int ks = 0; ks < 8; ++ks)  // dW1 += dZ1^T X; done before the next commit arrives
           T::mma_bf16(tmem + 256, T::smem_desc(s0 + tt::kD1T + 256u * ks, 128, 2048),
-                      T::smem_desc(s0 + tt::kXT + 256u * ks, 128, 2048), tt::kIdescM128N16,
+                      T::smem_desc(s0 + xt + 256u * ks, 128, 2048), tt::kIdescM128N16,
                       (first && ks == 0) ? 0u : 1u);
-        T::mma_commit(bar);
       }
     }
-    wait();  // the next tile's features overwrite this MMA's B operand
-    if (fail) break;
-    T::fence_after_sync();
+    xt = tt::kXT + (tt::kXT + 16 * 128 * 2 - xt);
     first = false;
+  }
+  if (!fail && !first) {  // the last tile's MMA5
+    if (tid == 0 && !NO_ARRIVE) T::mma_commit(bar);
+    wait();
+    T::fence_after_sync();
   }
   // the CTA's sums to global memory: weight gradients from TMEM (rows 0..63)
   if (!fail && !first) {
     if ((warp & 3) < 2) {  // TMEM lanes 0..63: the rows of dW2 and dW1
       const int n = row;
+      float v[kMine];
+      T::tmem_ld16(lanes + 192u, v);
 #pragma unroll
-      for (int c = 0; c < 32; c += 16) {
-        float v[16];
-        T::tmem_ld16(lanes + 192u + (uint32_t)c, v);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) atomicAdd(grad + kOffW2 + n * kMlpH + 32 * h + c + q, v[q]);
-      }
+      for (int q = 0; q < kMine; ++q) atomicAdd(grad + kOffW2 + n * kMlpH + c0 + q, v[q]);
       if (h == 0) {
-        float v[16];
         T::tmem_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + 256u, v);
 #pragma unroll
         for (int k = 0; k < kMlpIn; ++k) atomicAdd(grad + kOffW1 + n * kMlpIn + k, v[k]);
       }
     }
+    const int n = c0 + tt::column_of(lane);
+    const float w3 = tt::column_sums(aw3, lane), g2 = tt::column_sums(ab2, lane), g1 = tt::column_sums(ab1, lane);
+    if (!(lane & 1)) {
+      atomicAdd(&gw3[n], w3);
+      atomicAdd(&gb2[n], g2);
+      atomicAdd(&gb1[n], g1);
+    }
+    if (h == 0) {
+      const float l = tt::warp_sum(aloss), d3 = tt::warp_sum(ab3);
+      if (lane == 0) {
+        atomicAdd(&gloss, l);
+        atomicAdd(&gb3, d3);
+      }
+    }
+    __syncthreads();
     if (tid < kMlpH) {
       atomicAdd(grad + kOffB1 + tid, gb1[tid]);
       atomicAdd(grad + kOffB2 + tid, gb2[tid]);
