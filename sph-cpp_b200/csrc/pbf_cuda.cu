@@ -3218,6 +3218,13 @@ struct pbf_ctx {
   cudaStream_t side = nullptr;  // captures the body of the learned solver's conditional loop
   bool capture_failed = false;  // a step's conditional loop could not be captured whole
   bool lists_valid = false;
+  // The positions of a step are final before its viscosity and vorticity
+  // passes: the step's graph records x_ready there, and a download that
+  // follows the step copies them out on its own stream meanwhile (x_early:
+  // the last call that changed the state was such a step).
+  cudaStream_t copy = nullptr;
+  cudaEvent_t x_ready = nullptr;
+  bool record_x = false, x_early = false;
   bool near_stages = false;  // since find_neighbors x* has only moved by the stages that follow it (Dev::walk)
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
@@ -4134,6 +4141,7 @@ void launch_step_t(pbf_ctx* ctx) {
     Launch L(ctx, "update_velocities");
     k_update_v<<<g, kBlock, 0, s>>>(P, n, ctx->pstS, ctx->posS, ctx->velS);
   }
+  if (ctx->record_x) cudaEventRecordWithFlags(ctx->x_ready, s, cudaEventRecordExternal);
   if (ctx->params.gamma != 0.0f) {
     const int gt = blocks_for((size_t)n * kStageGL, kStageBlock);
     {
@@ -4309,7 +4317,9 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
     if ((rc = update_shapes(ctx))) return bail(rc);
   }
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&ctx->copy, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->x_ready, cudaEventDisableTiming) != cudaSuccess) {
     fail(ctx, PBF_ERR_CUDA, "cudaStreamCreate failed");
     return bail(PBF_ERR_CUDA);
   }
@@ -4390,6 +4400,8 @@ void pbf_destroy(pbf_ctx* ctx) {
     cudaEventDestroy(m.stop);
   }
   for (void* p : ctx->allocations) cudaFree(p);
+  if (ctx->x_ready) cudaEventDestroy(ctx->x_ready);
+  if (ctx->copy) cudaStreamDestroy(ctx->copy);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -4446,6 +4458,7 @@ int pbf_upload(pbf_ctx* ctx, const float* x, const float* v, size_t n) {
   if (n != ctx->n) drop_graphs(ctx);
   ctx->n = n;
   ctx->lists_valid = false;
+  ctx->x_early = false;
   if (n == 0) {
     CK(cudaMemsetAsync(ctx->fill_words, 0, kFillWords * sizeof(uint32_t), ctx->stream));
     return PBF_OK;
@@ -4492,6 +4505,7 @@ int pbf_set_array(pbf_ctx* ctx, int which, const float* host_in) {
   const int n = (int)ctx->n, g = blocks_for(n);
   const bool vec = which <= PBF_ARRAY_SCRATCH;
   if (which == PBF_ARRAY_POSITION_STARS) ctx->near_stages = false;
+  ctx->x_early = false;
   CK(cudaMemcpyAsync(ctx->stage, host_in, ctx->n * (vec ? 3 : 1) * sizeof(float), cudaMemcpyHostToDevice,
                      ctx->stream));
   switch (which) {
@@ -4514,6 +4528,7 @@ int pbf_add_particles(pbf_ctx* ctx, const float* x, const float* v, size_t k) {
   if (!ctx || (!x && k)) return ctx ? fail(ctx, PBF_ERR_ARG, "null positions") : PBF_ERR_ARG;
   if (!ctx->scenes.empty()) return fail(ctx, PBF_ERR_STATE, "the scenes of a batch have fixed particle counts");
   if (k == 0) return PBF_OK;
+  ctx->x_early = false;
   if (ctx->n + k > ctx->capacity)
     return fail(ctx, PBF_ERR_CAPACITY, "Not enough capacity: %zu particles > capacity %zu", ctx->n + k,
                 ctx->capacity);
@@ -4683,14 +4698,23 @@ int pbf_download(pbf_ctx* ctx, float* x, float* v, float* rho, float* lambda) {
   // the sort's arrival numbers and places are used up: staging of the scalars
   float* sr = reinterpret_cast<float*>(ctx->rank);
   float* sl = reinterpret_cast<float*>(ctx->place);
-  k_unpermute_state<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, ctx->posH, ctx->velH, ctx->lamH, ctx->origH,
-                                                               x ? sx : nullptr, v ? sv : nullptr,
-                                                               rho ? sr : nullptr, lambda ? sl : nullptr);
+  const bool early = x && ctx->x_early;
+  if (early) {  // the positions, as the sorted slots' x*, while the step's last passes run
+    CK(cudaStreamWaitEvent(ctx->copy, ctx->x_ready, 0));
+    k_unpermute_vec<<<blocks_for(n), kBlock, 0, ctx->copy>>>((int)n, ctx->pstS, ctx->origS, sx);
+    if (int rc = check_launch(ctx, "unpermute")) return rc;
+    CK(cudaMemcpyAsync(x, sx, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, ctx->copy));
+  }
+  if ((x && !early) || v || rho || lambda)
+    k_unpermute_state<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, ctx->posH, ctx->velH, ctx->lamH, ctx->origH,
+                                                                 x && !early ? sx : nullptr, v ? sv : nullptr,
+                                                                 rho ? sr : nullptr, lambda ? sl : nullptr);
   if (int rc = check_launch(ctx, "unpermute")) return rc;
-  if (x) CK(cudaMemcpyAsync(x, sx, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  if (x && !early) CK(cudaMemcpyAsync(x, sx, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   if (v) CK(cudaMemcpyAsync(v, sv, n * 3 * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   if (rho) CK(cudaMemcpyAsync(rho, sr, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   if (lambda) CK(cudaMemcpyAsync(lambda, sl, n * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
+  if (early) CK(cudaStreamSynchronize(ctx->copy));
   CK(cudaStreamSynchronize(ctx->stream));
   return PBF_OK;
 }
@@ -4709,7 +4733,8 @@ int pbf_download(pbf_ctx* ctx, float* x, float* v, float* rho, float* lambda) {
   const bool X = ctx->params.exact_math != 0; \
   (void)X;                                \
   const Dev SP = span_dev(ctx, e);        \
-  (void)SP;
+  (void)SP;                               \
+  ctx->x_early = false;
 
 int pbf_apply_external_forces(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
@@ -4732,6 +4757,7 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
   if (bin_e != ctx->n)
     return fail(ctx, PBF_ERR_SPAN, "find_neighbors bins every held particle: bin span [0, %zu) given, [0, %zu) held",
                 bin_e, ctx->n);
+  ctx->x_early = false;
   if (ctx->n == 0) {
     ctx->lists_valid = true;
     return PBF_OK;
@@ -4864,11 +4890,19 @@ int pbf_update_positions(pbf_ctx* ctx, size_t b, size_t e) {
 
 // nsteps fused steps captured from the context's stream into a graph (not
 // instantiated; the caller owns it).
-static int capture_steps(pbf_ctx* ctx, int nsteps, cudaGraph_t* out) {
+// Particles from which a download overlaps the step's last passes (below, the
+// second stream costs more than the copy).
+constexpr size_t kEarlyLeast = 32768;
+
+static int capture_steps(pbf_ctx* ctx, int nsteps, bool early, cudaGraph_t* out) {
   cudaGraph_t graph = nullptr;
   ctx->capture_failed = false;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  for (int i = 0; i < nsteps; ++i) launch_step(ctx);
+  for (int i = 0; i < nsteps; ++i) {
+    ctx->record_x = early && i == nsteps - 1;
+    launch_step(ctx);
+  }
+  ctx->record_x = false;
   cudaError_t le = cudaGetLastError();
   cudaError_t ce = cudaStreamEndCapture(ctx->stream, &graph);
   if (le != cudaSuccess || ce != cudaSuccess || ctx->capture_failed) {
@@ -4893,6 +4927,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
   }
   ctx->steps_done += (uint64_t)nsteps;
   ctx->near_stages = false;
+  ctx->x_early = false;
   if (ctx->timing) {
     for (int i = 0; i < nsteps; ++i) launch_step(ctx);
     int rc = check_launch(ctx, "step");
@@ -4900,10 +4935,11 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
     ctx->lists_valid = true;
     return harvest_times(ctx);
   }
+  const bool early = ctx->n >= kEarlyLeast && !persist_on(ctx);
   auto it = ctx->graphs.find(nsteps);
   if (it == ctx->graphs.end()) {
     cudaGraph_t graph = nullptr;
-    if (int rc = capture_steps(ctx, nsteps, &graph)) return rc;
+    if (int rc = capture_steps(ctx, nsteps, early, &graph)) return rc;
     cudaGraphExec_t exec = nullptr;
     cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -4912,6 +4948,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
   }
   CK(cudaGraphLaunch(it->second, ctx->stream));
   ctx->lists_valid = true;
+  ctx->x_early = early;
   return PBF_OK;
 }
 
@@ -5000,7 +5037,7 @@ int pbf_group_step(pbf_group* g, int nsteps) {
       pbf_ctx* c = order[rank];
       if (c->n == 0) continue;
       cudaGraph_t child = nullptr;
-      if (int rc = capture_steps(c, nsteps, &child)) {
+      if (int rc = capture_steps(c, nsteps, false, &child)) {
         cudaGraphDestroy(parent);
         return fail(nullptr, rc, "pbf_group_step: capture of a member failed: %s", pbf_last_error(c));
       }
@@ -5050,6 +5087,7 @@ int pbf_group_step(pbf_group* g, int nsteps) {
     if (c->n == 0) continue;
     c->steps_done += (uint64_t)nsteps;
     c->near_stages = false;
+    c->x_early = false;
     c->lists_valid = true;
   }
   return PBF_OK;
@@ -5539,6 +5577,7 @@ struct StateSnapshot {
 
 int pbf_autotune(pbf_ctx* ctx, int steps, pbf_tuning* chosen, double* ms) {
   if (!ctx) return PBF_ERR_ARG;
+  ctx->x_early = false;
   if (steps < 1) return fail(ctx, PBF_ERR_ARG, "autotune needs steps >= 1");
   if (ms) std::fill(ms, ms + PBF_TUNE_CANDIDATES * PBF_TUNE_FAMILIES, 0.0);
   if (ctx->params.solver == 1 && !ctx->mlp_ready)
