@@ -56,6 +56,10 @@ constexpr int kBlock = 256;
 // 12 of the autotuned 128, per SM): measured faster than at their natural
 // 44-48; the other gathers are faster as the compiler leaves them.
 constexpr int kGatherMinBlocks = 6;
+// ... density/lambda in the one-thread form to 64: its two sets of sums spill
+// at 42 (1M 72 us a pass, 68 at 64; delta-p 63 and 67, with s_corr 69, 63 at
+// the 51 it gets there).
+constexpr int kOneLaneMinBlocks = 4;
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
@@ -1638,8 +1642,7 @@ template <int GL, bool NH, bool STAGED = false, bool COH = false>
 __device__ __forceinline__ DensitySums density_sums(const Fast& F, const pbf::Group& G, const int32_t* row,
                                                     const uint16_t* row16, int c, int dummy, const float4* src,
                                                     float4 xp) {
-  DensitySums S{0.f, 0.f, 0.f, 0.f, 0.f, FLT_MAX, 0.f};
-  auto body = [&](int, float4 xq) {
+  auto add = [&](DensitySums& S, float4 xq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
     S.dmin = fminf(S.dmin, d2);
@@ -1652,10 +1655,25 @@ __device__ __forceinline__ DensitySums density_sums(const Fast& F, const pbf::Gr
     S.s1z = fmaf(t, dz, S.s1z);
     S.s2 = fmaf(t * t, d2, S.s2);
   };
-  if (STAGED)
-    pbf::swalk1<GL>(row16, c, dummy, G.lane, src, body);
-  else
-    pbf::gwalk1<GL, false, COH>(row, c, dummy, G.lane, src, body);
+  DensitySums S{0.f, 0.f, 0.f, 0.f, 0.f, FLT_MAX, 0.f};
+  if constexpr (GL == 1) {  // the two lanes' sums in one thread
+    DensitySums B = S;
+    pbf::gwalk_pair(row, c, dummy, src, [&](float4 xq) { add(S, xq); }, [&](float4 xq) { add(B, xq); });
+    S.sw += B.sw;
+    S.s1x += B.s1x;
+    S.s1y += B.s1y;
+    S.s1z += B.s1z;
+    S.s2 += B.s2;
+    if (NH) S.nh += B.nh;
+    S.dmin = fminf(S.dmin, B.dmin);
+    return S;
+  } else {
+    auto body = [&](int, float4 xq) { add(S, xq); };
+    if (STAGED)
+      pbf::swalk1<GL>(row16, c, dummy, G.lane, src, body);
+    else
+      pbf::gwalk1<GL, false, COH>(row, c, dummy, G.lane, src, body);
+  }
   S.sw = pbf::gsum<GL>(S.sw);
   S.s1x = pbf::gsum<GL>(S.s1x);
   S.s1y = pbf::gsum<GL>(S.s1y);
@@ -1685,15 +1703,16 @@ __device__ __forceinline__ void density_lambda_tile(int tile, const Dev& P, cons
   bool mark = false;  // nudged: a move the delta-p pass already sees
   if (G.live && G.lane == 0) {
     const float L2 = F.lam_grad * F.lam_grad;
-    const float sc = L2 * S.s2;  // sum |grad_q C|^2
-    const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));  // |grad_p C|^2
+    // rounded one by one: every form of the pass has the same bits
+    const float sc = pbf::xmul(L2, S.s2);  // sum |grad_q C|^2
+    const float g2 = pbf::xmul(L2, fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x)));  // |grad_p C|^2
     const bool close = S.dmin < 4e-16f;
     const float nh = S.nh;
     if (close) {  // a neighbour (almost) on top: the reference-ordered path decides the nudge
       mark = density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
     } else {
       const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
-      const float l = -C / (sc + g2 + F.lambda_eps);
+      const float l = -C / pbf::xadd(pbf::xadd(sc, g2), F.lambda_eps);
       xl[b] = make_float4(xp.x, xp.y, xp.z, l);
       vel[b].w = rho;
       lam[b] = l;
@@ -1719,7 +1738,7 @@ __device__ __forceinline__ void density_lambda_tile(int tile, const Dev& P, cons
 // COND: a plain pass of the learned solver's sampled checks, skipped once the
 // step has converged.
 template <int MODE, int GL, bool LOOP = false, bool COND = false>
-__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kf_density_lambda(Dev P, Fast F, int n, size_t stride,
+__global__ void __launch_bounds__(kBlock, GL == 1 ? kOneLaneMinBlocks : kGatherMinBlocks) kf_density_lambda(Dev P, Fast F, int n, size_t stride,
                                                             const int32_t* __restrict__ nbr,
                                                             const int32_t* __restrict__ cnt,
                                                             const float4* __restrict__ pst, float4* xl, float4* vel,
@@ -1867,7 +1886,7 @@ __global__ void __launch_bounds__(kStageThreads) ks_density_lambda(Dev P, Fast F
 constexpr float kWarmMaxGain = 5.0f;
 
 template <int GL>
-__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kl_features(Dev P, Fast F, pbf::MlpDev M, int n,
+__global__ void __launch_bounds__(kBlock, GL == 1 ? kOneLaneMinBlocks : kGatherMinBlocks) kl_features(Dev P, Fast F, pbf::MlpDev M, int n,
                                                                         size_t stride,
                                                       const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
                                                       const float4* __restrict__ pst, float4* xl, float4* vel,
@@ -1882,8 +1901,8 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kl_features(Dev P, F
   if (G.live && G.lane == 0) {
     const float rho = fmaf(F.m_poly, S.sw, F.m_w0);
     const float L2 = F.lam_grad * F.lam_grad;
-    const float sc = L2 * S.s2;
-    const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));
+    const float sc = pbf::xmul(L2, S.s2);
+    const float g2 = pbf::xmul(L2, fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x)));
     const bool close = S.dmin < 4e-16f;
     const float nh = S.nh;
     const float4 v = vel[b];
@@ -1903,7 +1922,7 @@ __global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kl_features(Dev P, F
       mark = density_lambda_one<false>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
     } else {
       const float C = fmaxf(fmaf(rho, F.inv_rho0, -1.0f), 0.0f);
-      const float l1 = -C / (sc + g2 + F.lambda_eps);
+      const float l1 = -C / pbf::xadd(pbf::xadd(sc, g2), F.lambda_eps);
       xl[b] = make_float4(xp.x, xp.y, xp.z, l1);
       vel[b] = make_float4(v.x, v.y, v.z, rho);
       lam[b] = l1;
@@ -2402,23 +2421,31 @@ __device__ __forceinline__ void dp_update_tile(int tile, const Dev& P, const Fas
   const int b = G.b;
   const float4 xp = xl[b];
   const int c = G.live ? walk_count(P, b, cnt) : 0;
-  float ax = 0.f, ay = 0.f, az = 0.f;
   const float lp = xp.w;
-  pbf::walk1<GL, STAGED, false, COH>(nbr + pbf::list_base(b, stride),
-                                     STAGED ? src.nbr16 + (size_t)b * stride : nullptr, c, STAGED ? src.dummy : n,
-                                     G.lane, STAGED ? src.a : xl, [&](int, float4 xq) {
+  auto add = [&](float3& s, float4 xq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
     float l = lp + xq.w;
     if (SCORR) l -= P.scorr_k * __powf(F.visc_poly * pbf::poly_cube(F, d2) * P.inv_wdq, P.scorr_n);
     const float t = l * pbf::spikey_over_r(F, d2);
-    ax = fmaf(t, dx, ax);
-    ay = fmaf(t, dy, ay);
-    az = fmaf(t, dz, az);
-  });
-  ax = pbf::gsum<GL>(ax);
-  ay = pbf::gsum<GL>(ay);
-  az = pbf::gsum<GL>(az);
+    s.x = fmaf(t, dx, s.x);
+    s.y = fmaf(t, dy, s.y);
+    s.z = fmaf(t, dz, s.z);
+  };
+  const int32_t* row = nbr + pbf::list_base(b, stride);
+  float3 sum = make_float3(0.f, 0.f, 0.f);
+  if constexpr (GL == 1) {  // the two lanes' sums in one thread
+    float3 odd = sum;
+    pbf::gwalk_pair(row, c, n, xl, [&](float4 xq) { add(sum, xq); }, [&](float4 xq) { add(odd, xq); });
+    sum.x += odd.x;
+    sum.y += odd.y;
+    sum.z += odd.z;
+  } else {
+    pbf::walk1<GL, STAGED, false, COH>(row, STAGED ? src.nbr16 + (size_t)b * stride : nullptr, c,
+                                       STAGED ? src.dummy : n, G.lane, STAGED ? src.a : xl,
+                                       [&](int, float4 xq) { add(sum, xq); });
+  }
+  const float ax = pbf::gsum<GL>(sum.x), ay = pbf::gsum<GL>(sum.y), az = pbf::gsum<GL>(sum.z);
   bool mark = false;
   if (G.live && G.lane == 0) {
     if (lamsum) lamsum[b] += xp.w;
@@ -2438,7 +2465,7 @@ __device__ __forceinline__ void dp_update_tile(int tile, const Dev& P, const Fas
 // COND launches (the learned solver's extra iterations) use a persistent grid
 // and skip the whole launch once the step has converged.
 template <bool SCORR, bool LAST, bool COND, int GL>
-__global__ void __launch_bounds__(kBlock, kGatherMinBlocks) kf_dp_update(Dev P, Fast F, int n, size_t stride,
+__global__ void __launch_bounds__(kBlock, GL == 1 && SCORR ? 5 : kGatherMinBlocks) kf_dp_update(Dev P, Fast F, int n, size_t stride,
                                                        const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
                                                        const float4* __restrict__ xl, float4* pst,
                                                        const float4* __restrict__ pos, float4* vel,
@@ -2739,9 +2766,9 @@ __global__ void __launch_bounds__(kStageBlock) kt_lambda(Dev P, Fast F, int n, s
   const DensitySums S = density_sums<kStageGL, false>(F, G, nbr + pbf::list_base(b, stride), nullptr, c, n, pst, xp);
   if (!G.live || G.lane != 0) return;
   const float L2 = F.lam_grad * F.lam_grad;
-  const float g2 = L2 * fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x));
+  const float g2 = pbf::xmul(L2, fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x)));
   const float C = fmaxf(fmaf(vel[b].w, F.inv_rho0, -1.0f), 0.0f);
-  lam[b] = -C / (L2 * S.s2 + g2 + F.lambda_eps);
+  lam[b] = -C / (fmaf(L2, S.s2, g2) + F.lambda_eps);
 }
 
 // compute_pressure_dps (particles.h:348-358) -> scratch
@@ -3587,6 +3614,14 @@ int need_lists(pbf_ctx* ctx) {
 }
 
 // ---- launch shapes of the fast gather kernels ----
+// Particles from which the two-lane shapes of density/lambda and delta-p run
+// both lanes' work in one thread (GL = 1 below, the same bits).  Two lanes and
+// one, us a pass in the step: density/lambda 212k particles 16.2 and 17.0, 500k
+// (whole lists) 64.6 and 61.0, 1M 75.6 and 67.5, 16.8M 1,144 and 996; delta-p
+// 66k 6.9 and 7.3, 212k 16.1 and 14.7, 1M 67.3 and 62.7, 16.8M 955 and 871.  The
+// two-record walks of viscosity and vorticity lose with one lane at every size.
+constexpr size_t kOneLaneDensity = 262144, kOneLaneDeltaP = 196608;
+
 // fn(std::integral_constant<int, GL>) for the lanes-per-particle of a shape.
 template <class Fn>
 void with_lanes(int lanes, Fn&& fn) {
@@ -3596,6 +3631,22 @@ void with_lanes(int lanes, Fn&& fn) {
     fn(std::integral_constant<int, 2>{});
   else
     fn(std::integral_constant<int, 8>{});
+}
+
+// The same for the families that have a one-thread form.
+template <class Fn>
+void with_lanes1(int lanes, Fn&& fn) {
+  if (lanes == 1)
+    fn(std::integral_constant<int, 1>{});
+  else
+    with_lanes(lanes, fn);
+}
+
+// The lanes the density/lambda and delta-p passes launch with.
+int lanes_of(const pbf_ctx* ctx, int family) {
+  const int lanes = ctx->tune.lanes[family];
+  const size_t least = family == PBF_TUNE_DENSITY ? kOneLaneDensity : kOneLaneDeltaP;
+  return lanes == 2 && !ctx->tune.staged[family] && ctx->n >= least ? 1 : lanes;
 }
 
 bool shape_ok(int lanes, int block, int staged) {
@@ -3623,7 +3674,8 @@ int mlp_tc_grid(const pbf_ctx* ctx, int n) {
 
 int grid_of(const pbf_ctx* ctx, int family) {
   if (ctx->tune.staged[family]) return (int)((ctx->n + kTile - 1) / kTile);
-  return blocks_for(ctx->n * (size_t)ctx->tune.lanes[family], ctx->tune.block[family]);
+  const bool one = family == PBF_TUNE_DENSITY || family == PBF_TUNE_DELTA_P;
+  return blocks_for(ctx->n * (size_t)(one ? lanes_of(ctx, family) : ctx->tune.lanes[family]), ctx->tune.block[family]);
 }
 
 // Persistent grids of the residual check and the conditional delta-p pass for
@@ -3852,7 +3904,10 @@ void launch_learned_solve(pbf_ctx* ctx) {
   const pbf_tuning& T = ctx->tune;
   const int g = blocks_for(n);
   // skippable launches: persistent grids
-  const int gpc = std::min(grid_of(ctx, PBF_TUNE_DENSITY), ctx->pgrid_check);
+  const int gpc =
+      T.staged[PBF_TUNE_DENSITY]
+          ? std::min(grid_of(ctx, PBF_TUNE_DENSITY), ctx->pgrid_check)
+          : std::min(blocks_for((size_t)n * T.lanes[PBF_TUNE_DENSITY], T.block[PBF_TUNE_DENSITY]), ctx->pgrid_check);
   const int gpd = std::min(grid_of(ctx, PBF_TUNE_DELTA_P), ctx->pgrid_dp);
   const int bd = T.block[PBF_TUNE_DENSITY], bp = T.block[PBF_TUNE_DELTA_P];
   const float tol = ctx->params.residual_tol;
@@ -3862,9 +3917,9 @@ void launch_learned_solve(pbf_ctx* ctx) {
   const pbf::MlpDev M = mlp_dev(ctx);
   {
     // the density family's shape (4 lanes x 128 threads when that family is staged)
-    const int fl = T.staged[PBF_TUNE_DENSITY] ? 4 : T.lanes[PBF_TUNE_DENSITY];
+    const int fl = T.staged[PBF_TUNE_DENSITY] ? 4 : lanes_of(ctx, PBF_TUNE_DENSITY);
     const int fb = T.staged[PBF_TUNE_DENSITY] ? kStageThreads : T.block[PBF_TUNE_DENSITY];
-    with_lanes(fl, [&](auto gl) {
+    with_lanes1(fl, [&](auto gl) {
       Launch L(ctx, "warm_features");
       kl_features<decltype(gl)::value><<<blocks_for((size_t)n * fl, fb), fb, 0, s>>>(
           P, F, M, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->xl, ctx->velS, ctx->lamH, ctx->nudge, ctx->lamprevS,
@@ -3882,7 +3937,7 @@ void launch_learned_solve(pbf_ctx* ctx) {
     ks_dp_update<SCORR, false, false><<<grid_of(ctx, PBF_TUNE_DELTA_P), kStageThreads, 0, s>>>(
         P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, nullptr, tio);
   } else {
-    with_lanes(T.lanes[PBF_TUNE_DELTA_P], [&](auto gl) {
+    with_lanes1(lanes_of(ctx, PBF_TUNE_DELTA_P), [&](auto gl) {
       Launch L(ctx, "dp_update");
       kf_dp_update<SCORR, false, false, decltype(gl)::value><<<grid_of(ctx, PBF_TUNE_DELTA_P), bp, 0, s>>>(
           P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, nullptr);
@@ -3899,7 +3954,7 @@ void launch_learned_solve(pbf_ctx* ctx) {
         ks_density_lambda<kDlPlain><<<grid_of(ctx, PBF_TUNE_DENSITY), kStageThreads, 0, s>>>(
             P, F, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->xl, ctx->velS, ctx->lamH, ctx->nudge, io, tio);
       } else {
-        with_lanes(T.lanes[PBF_TUNE_DENSITY], [&](auto gl) {
+        with_lanes1(lanes_of(ctx, PBF_TUNE_DENSITY), [&](auto gl) {
           Launch L(ctx, "density_lambda");
           kf_density_lambda<kDlPlain, decltype(gl)::value><<<grid_of(ctx, PBF_TUNE_DENSITY), bd, 0, s>>>(
               P, F, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->xl, ctx->velS, ctx->lamH, ctx->nudge, io);
@@ -3911,7 +3966,7 @@ void launch_learned_solve(pbf_ctx* ctx) {
             P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, ctx->lamsumH,
             tio);
       } else {
-        with_lanes(T.lanes[PBF_TUNE_DELTA_P], [&](auto gl) {
+        with_lanes1(lanes_of(ctx, PBF_TUNE_DELTA_P), [&](auto gl) {
           Launch L(ctx, "dp_update");
           kf_dp_update<SCORR, false, false, decltype(gl)::value><<<grid_of(ctx, PBF_TUNE_DELTA_P), bp, 0, s>>>(
               P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, ctx->lamsumH);
@@ -3975,7 +4030,7 @@ void launch_learned_solve(pbf_ctx* ctx) {
       ks_dp_update<SCORR, false, true><<<gpd, kStageThreads, 0, cs>>>(
           P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, ctx->lamsumH, tio);
     } else {
-      with_lanes(T.lanes[PBF_TUNE_DELTA_P], [&](auto gl) {
+      with_lanes1(lanes_of(ctx, PBF_TUNE_DELTA_P), [&](auto gl) {
         Launch L(ctx, "dp_update");
         kf_dp_update<SCORR, false, true, decltype(gl)::value><<<gpd, bp, 0, cs>>>(
             P, F, n, st, ctx->nbr, ctx->cnt, ctx->xl, ctx->pstS, ctx->posS, ctx->velS, ctx->state, ctx->lamsumH);
@@ -4088,7 +4143,7 @@ void launch_step_t(pbf_ctx* ctx) {
                                                                    ctx->xl, ctx->velS, ctx->lamH, ctx->nudge, io,
                                                                    tile_io(ctx));
       } else
-        with_lanes(T.lanes[PBF_TUNE_DENSITY], [&](auto gl) {
+        with_lanes1(lanes_of(ctx, PBF_TUNE_DENSITY), [&](auto gl) {
           constexpr int GL = decltype(gl)::value;
           const int gd = grid_of(ctx, PBF_TUNE_DENSITY), bd = T.block[PBF_TUNE_DENSITY];
           if (ctx->recording)
@@ -4124,7 +4179,7 @@ void launch_step_t(pbf_ctx* ctx) {
                                                                        ctx->pstS, ctx->posS, ctx->velS, ctx->state,
                                                                        nullptr, tile_io(ctx));
     } else {
-      with_lanes(T.lanes[PBF_TUNE_DELTA_P], [&](auto gl) {
+      with_lanes1(lanes_of(ctx, PBF_TUNE_DELTA_P), [&](auto gl) {
         constexpr int GL = decltype(gl)::value;
         const int gd = grid_of(ctx, PBF_TUNE_DELTA_P), bd = T.block[PBF_TUNE_DELTA_P];
         if (last)

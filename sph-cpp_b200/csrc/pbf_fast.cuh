@@ -206,6 +206,35 @@ __device__ __forceinline__ void gwalk1(const int32_t* __restrict__ row, int c, i
   }
 }
 
+// The two-lane walk in one thread: `even` takes the entries of lane 0, `odd`
+// those of lane 1, so that two sets of sums, added at the end, have the bits
+// of the two lanes' shuffled ones.  One thread a particle halves the warps'
+// setup, epilogues and shuffles and reads twice as many particles' records in
+// one instruction; it needs enough particles to fill the GPU.
+template <class Even, class Odd>
+__device__ __forceinline__ void gwalk_pair(const int32_t* __restrict__ row, int c, int dummy,
+                                           const float4* __restrict__ a, Even&& even, Odd&& odd) {
+  const int4* r4 = reinterpret_cast<const int4*>(row);
+  auto four = [&](int4 q, auto&& body) {
+    const float4 v0 = __ldg(a + q.x), v1 = __ldg(a + q.y), v2 = __ldg(a + q.z), v3 = __ldg(a + q.w);
+    body(v0);
+    body(v1);
+    body(v2);
+    body(v3);
+  };
+  const int full = c / 8;
+  int t = 0;
+  for (; t < full; ++t) {
+    const int4 qe = __ldg(r4 + vec4_at(2 * t)), qo = __ldg(r4 + vec4_at(2 * t + 1));
+    four(qe, even);
+    four(qo, odd);
+  }
+  if (t * 8 < c) {
+    four(tail4(__ldg(r4 + vec4_at(2 * t)), 2 * t, c, dummy), even);
+    four(tail4(__ldg(r4 + vec4_at(2 * t + 1)), 2 * t + 1, c, dummy), odd);
+  }
+}
+
 // Two records per neighbour: entries 2l, 2l+1 of every 2*GL-entry batch (an
 // 8-byte index load), so that four records are in flight per lane, as in the
 // one-record walk; PF as there.

@@ -17,8 +17,8 @@ pytestmark = pytest.mark.gpu
 
 def _check(g):
     d = g.download()
-    assert np.array_equal(d["x"], g.positions())
-    assert np.array_equal(d["v"], g.velocities(), equal_nan=True)  # no iteration: densities of 0, velocities NaN
+    assert np.array_equal(d["x"], g.positions(), equal_nan=True)
+    assert np.array_equal(d["v"], g.velocities(), equal_nan=True)  # (no iteration: densities of 0, NaN)
     assert np.array_equal(d["rho"], g.densities())
     assert np.array_equal(d["lambda"], g.lambdas())
     return d["x"]
