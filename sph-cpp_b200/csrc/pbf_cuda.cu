@@ -1032,10 +1032,11 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
 }
 
 // One particle's list in the reference's order, by a whole warp: lane v looks
-// up visit v's bin, then the bins' candidates are tested 32 at a time and the
-// hits appended in order.  k_fill_rest takes it for a few particles of a warp:
-// a single lane's walk is a chain of dependent loads, 27 bins long (about
-// 60 us, the whole launch where one particle of a million sits on a bin face).
+// up visit v's bin, then the bins' candidates, end to end, are tested 32 at a
+// time and the hits appended in order.  k_fill_rest takes it for a few
+// particles of a warp: a single lane's walk is a chain of dependent loads, 27
+// bins long (about 60 us, the whole launch where one particle of a million sits
+// on a bin face; bin after bin with a whole warp 15 us, end to end 10).
 // -1: a bin holds more than kCooperativeBin particles, where 32 tests a step
 // with nothing in flight behind them are slower than the lane's walk.
 constexpr uint32_t kCooperativeBin = 512;
@@ -1059,22 +1060,35 @@ __device__ __forceinline__ int fill_cooperative(const Dev& P, int b, size_t stri
     }
   }
   if (__any_sync(0xffffffffu, q1 - q0 > kCooperativeBin)) return -1;
+  // candidate i of the 27 bins end to end is slot q0[v] + i - before[v] of the last visit v with before[v] <= i
+  const int mine = (int)(q1 - q0);
+  int upto = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int below = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += below;
+  }
+  const int before = upto - mine, total = __shfl_sync(0xffffffffu, upto, 31);
   int32_t* row = nbr + pbf::list_base(b, stride);
   int count = 0;
-  for (int v = 0; v < 27 && count < P.cap; ++v) {
-    const uint32_t e = __shfl_sync(0xffffffffu, q1, v);
-    for (uint32_t q = __shfl_sync(0xffffffffu, q0, v); q < e && count < P.cap; q += 32) {
-      const uint32_t c = q + (uint32_t)lane;
-      bool hit = false;
-      if (c < e && c != (uint32_t)b) {
-        const float4 xq = pst[c];
-        hit = pbf::mag2<true>(pbf::xsub(xp.x, xq.x), pbf::xsub(xp.y, xq.y), pbf::xsub(xp.z, xq.z)) < P.s2;
-      }
-      const unsigned hits = __ballot_sync(0xffffffffu, hit);
-      const int at = count + __popc(hits & ((1u << lane) - 1u));
-      if (hit && at < P.cap) row[pbf::list_off(at)] = (int32_t)c;
-      count += __popc(hits);
+  for (int i0 = 0; i0 < total && count < P.cap; i0 += 32) {
+    const int i = i0 + lane;
+    int v = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const int first = __shfl_sync(0xffffffffu, before, v + o);
+      if (v + o < 27 && first <= i) v += o;
     }
+    const uint32_t c = __shfl_sync(0xffffffffu, q0, v) + (uint32_t)(i - __shfl_sync(0xffffffffu, before, v));
+    bool hit = false;
+    if (i < total && c != (uint32_t)b) {
+      const float4 xq = pst[c];
+      hit = pbf::mag2<true>(pbf::xsub(xp.x, xq.x), pbf::xsub(xp.y, xq.y), pbf::xsub(xp.z, xq.z)) < P.s2;
+    }
+    const unsigned hits = __ballot_sync(0xffffffffu, hit);
+    const int at = count + __popc(hits & ((1u << lane) - 1u));
+    if (hit && at < P.cap) row[pbf::list_off(at)] = (int32_t)c;
+    count += __popc(hits);
   }
   return min(count, P.cap);
 }
@@ -3252,6 +3266,7 @@ struct pbf_ctx {
   cudaStream_t copy = nullptr;
   cudaEvent_t x_ready = nullptr;
   bool record_x = false, x_early = false;
+  bool rho_whole = false;    // every density is one of compute_densities' (never zero) since the last upload
   bool near_stages = false;  // since find_neighbors x* has only moved by the stages that follow it (Dev::walk)
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
@@ -4514,6 +4529,7 @@ int pbf_upload(pbf_ctx* ctx, const float* x, const float* v, size_t n) {
   ctx->n = n;
   ctx->lists_valid = false;
   ctx->x_early = false;
+  ctx->rho_whole = false;
   if (n == 0) {
     CK(cudaMemsetAsync(ctx->fill_words, 0, kFillWords * sizeof(uint32_t), ctx->stream));
     return PBF_OK;
@@ -4561,6 +4577,7 @@ int pbf_set_array(pbf_ctx* ctx, int which, const float* host_in) {
   const bool vec = which <= PBF_ARRAY_SCRATCH;
   if (which == PBF_ARRAY_POSITION_STARS) ctx->near_stages = false;
   ctx->x_early = false;
+  if (which == PBF_ARRAY_DENSITIES) ctx->rho_whole = false;
   CK(cudaMemcpyAsync(ctx->stage, host_in, ctx->n * (vec ? 3 : 1) * sizeof(float), cudaMemcpyHostToDevice,
                      ctx->stream));
   switch (which) {
@@ -4584,6 +4601,7 @@ int pbf_add_particles(pbf_ctx* ctx, const float* x, const float* v, size_t k) {
   if (!ctx->scenes.empty()) return fail(ctx, PBF_ERR_STATE, "the scenes of a batch have fixed particle counts");
   if (k == 0) return PBF_OK;
   ctx->x_early = false;
+  ctx->rho_whole = false;
   if (ctx->n + k > ctx->capacity)
     return fail(ctx, PBF_ERR_CAPACITY, "Not enough capacity: %zu particles > capacity %zu", ctx->n + k,
                 ctx->capacity);
@@ -4840,6 +4858,7 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
 int pbf_compute_densities(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
+  if (e == ctx->n) ctx->rho_whole = true;
   if (X)
     k_density<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
   else
@@ -4896,7 +4915,10 @@ int pbf_apply_surface_tension(pbf_ctx* ctx, size_t cb, size_t ce, size_t sb, siz
     k_surface<<<g, kBlock, 0, ctx->stream>>>(span_dev(ctx, se), n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
   } else {
     kt_color<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, true);
-    kt_surface<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(span_dev(ctx, se), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+    // without surface tension the force is exactly zero, but where a density
+    // not computed yet makes it NaN
+    if (ctx->params.gamma != 0.0f || !ctx->rho_whole)
+      kt_surface<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(span_dev(ctx, se), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
   }
   return check_launch(ctx, "apply_surface_tension");
 }

@@ -98,3 +98,28 @@ def test_positions_set_between_stages_are_seen():
             g.compute_pressure_lambdas()
         _close(f.densities(), e.densities(), 1e-5, 0.0)
         _close(f.lambdas(), e.lambdas(), 1e-4, 1e-12)
+
+
+@pytest.mark.parametrize("densities", ["computed", "missing", "zeroed"])
+def test_no_surface_tension_changes_no_velocity(densities):
+    """gamma = 0 adds exactly zero, except where a density is still 0: NaN there, as in exact math."""
+    sc = make_scene("dam_2k")
+    n = 1000
+    x, v = _state(n, 5)
+    got = []
+    for exact in (0, 1):
+        with Particles(sc.with_(exact_math=exact).params(), n) as g:
+            g.upload(x, v)
+            g.find_neighbors()
+            if densities != "missing":
+                g.compute_densities()
+            if densities == "zeroed":
+                rho = g.densities()
+                rho[:200] = 0.0
+                g.set_array(_abi.ARRAY_DENSITIES, rho)
+            g.apply_surface_tension()
+            got.append(g.velocities())
+    assert np.array_equal(np.isnan(got[0]), np.isnan(got[1]))
+    fine = ~np.isnan(got[1])
+    assert np.array_equal(got[0][fine], v[fine])
+    assert fine.all() == (densities == "computed") and not (densities == "missing" and fine.any())
