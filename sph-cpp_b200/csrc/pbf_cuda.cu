@@ -1166,17 +1166,19 @@ __global__ void __launch_bounds__(kFillBlock) k_fill_rest(Dev P, int n, size_t s
 template <int T, bool REF>
 struct SplitShared {
   uint32_t mask[kMaskUnits][32];                // within s
-  uint32_t near[REF ? 1 : kMaskUnits][32];      // ... and within the near radius
+  uint32_t near[kMaskUnits][32];                // ... and within the near radius
   uint32_t first[9][32];                        // the rows' first slots
   uint8_t length[9][32];                        // ... and candidates
   uint8_t cut[REF ? 9 : 1][2][32];              // REF: where the row's second and third bin start
   uint8_t count[REF ? 27 : 2 * T][32];          // REF: per visit; else per warp, all and near
+  uint32_t near_bits[REF ? 2 : 1][32];          // REF: the near entries by their places in the list
   uint32_t bad, over;                           // lanes left to the walk; some list is over the cap
 };
 
 // Where the lists go: the context's warp-tiled lists, or rows of caller
 // indices (the search on device arrays).
 struct ListOut {
+  static constexpr bool kNear = true;
   int32_t* nbr;
   size_t stride;
   __device__ __forceinline__ void put(int b, int at, uint32_t q) const {
@@ -1186,6 +1188,7 @@ struct ListOut {
   __device__ __forceinline__ size_t index(int b) const { return (size_t)b; }
 };
 struct IndexOut {
+  static constexpr bool kNear = false;
   int32_t* out;
   const uint32_t* id;
   int cap;
@@ -1224,6 +1227,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
   const uint32_t key0 =
       R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)bz[0] + ((uint32_t)by[0] * (uint32_t)R.dimx + (uint32_t)bx[0]);
   if (threadIdx.x == 0) S.bad = S.over = 0u;
+  if (REF && t == 0) S.near_bits[0][lane] = S.near_bits[REF ? 1 : 0][lane] = 0u;
   __syncthreads();
   if (masks) {
     const float ylo = fmaxf(xp.y - ((float)by[1] * s - s) - P.skip_eps, 0.f);
@@ -1269,7 +1273,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
         uint32_t m = 0, mn = 0;
         if (many > 0) {
           const float4* p = pst + a0 + 32 * w;
-          if (REF) {
+          if (REF && !Out::kNear) {
             m = test_chunk(p, many, xp.x, xp.y, xp.z, s2);
           } else {
             const uint2 mm = test_chunk2(p, many, xp.x, xp.y, xp.z, s2, near2);
@@ -1282,7 +1286,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
         }
         const int u = r * kMaskWords + w;
         S.mask[u][lane] = m;
-        if (!REF) S.near[u][lane] = mn;
+        if (!REF || Out::kNear) S.near[u][lane] = mn;
         all += __popc(m);
         walk += __popc(mn);
       }
@@ -1305,22 +1309,40 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
   }
   if (REF) {
     __syncthreads();
-    if (!mine) return;
     // every visit's first place, in the reference's order; this warp's visits' entries
     int at = 0;
-    for (int v = 0; v < 27; ++v) {
+    uint64_t near = 0;
+    for (int v = 0; mine && v < 27; ++v) {
       const int i = v / 9, j = v / 3 % 3, k = v % 3, r = k * 3 + j;
       if (r / kRows == t && at < cap) {
         const int lo = i == 0 ? 0 : S.cut[r][i - 1][lane], hi = i == 2 ? kMaskRow : S.cut[r][i][lane];
         int e = at;
         for (int w = lo >> 5; w < kMaskWords && 32 * w < hi; ++w) {
           uint32_t m = S.mask[r * kMaskWords + w][lane] & low_bits(hi - 32 * w) & ~low_bits(lo - 32 * w);
-          for (; m && e < cap; m &= m - 1u) out.put(b, e++, S.first[r][lane] + 32u * (uint32_t)w + (uint32_t)__ffs(m) - 1u);
+          const uint32_t mn = Out::kNear ? S.near[r * kMaskWords + w][lane] : 0u;
+          for (; m && e < cap; m &= m - 1u, ++e) {
+            const int bit = __ffs(m) - 1;
+            out.put(b, e, S.first[r][lane] + 32u * (uint32_t)w + (uint32_t)bit);
+            if (Out::kNear) near |= (uint64_t)(mn >> bit & 1u) << e;
+          }
         }
       }
       at += S.count[v][lane];
     }
     at = min(at, cap);
+    if (Out::kNear) {
+      if (T > 1) {
+        if (mine && (uint32_t)near) atomicOr(&S.near_bits[0][lane], (uint32_t)near);
+        if (mine && near >> 32) atomicOr(&S.near_bits[REF ? 1 : 0][lane], (uint32_t)(near >> 32));
+        __syncthreads();
+        near = (uint64_t)S.near_bits[REF ? 1 : 0][lane] << 32 | S.near_bits[0][lane];
+      }
+      if (mine && t == 0) {
+        P.near_bits[b] = make_uint2((uint32_t)near, (uint32_t)(near >> 32));
+        P.walk[b] = 0;  // the near bits, until marked
+      }
+    }
+    if (!mine) return;
     out.end(b, at, t, T, cap);
     if (t == 0) {
       cnt[out.index(b)] = at;
@@ -1342,7 +1364,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
       all = walk = 0;
       for (int u = t * kRows * kMaskWords; u < (t + 1) * kRows * kMaskWords; ++u) {
         all += __popc(S.mask[u][lane]);
-        walk += __popc(S.near[REF ? 0 : u][lane]);
+        walk += __popc(S.near[u][lane]);
       }
       S.count[REF ? 0 : t][lane] = (uint8_t)all;
       S.count[REF ? 0 : T + t][lane] = (uint8_t)walk;
@@ -1365,7 +1387,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
   for (int u = t * kRows * kMaskWords; u < (t + 1) * kRows * kMaskWords; ++u) {
     uint32_t m = S.mask[u][lane];
     if (m == 0u) continue;
-    const uint32_t mn = S.near[REF ? 0 : u][lane];
+    const uint32_t mn = S.near[u][lane];
     const uint32_t q = S.first[u / kMaskWords][lane] + 32u * (uint32_t)(u % kMaskWords);
     for (; m; m &= m - 1u) {
       const int bit = __ffs(m) - 1;
@@ -1472,6 +1494,67 @@ __device__ __forceinline__ void seq1(const int32_t* __restrict__ nbr, int b, siz
     if (j + 2 < c) body(q.z, v2);
     if (j + 3 < c) body(q.w, v3);
   }
+}
+
+// The entries the exact path's fused kernels walk: all, or the near ones in
+// their places in the list.  The lists keep the reference's order, so the near
+// entries are not first in them: k_fill_split leaves one bit an entry.  The
+// others lie past h and add exact zeros, which leave every sum's bits as they
+// are (near_move in make_dev says when they may not).  These kernels wait on
+// divides and square roots of correctly rounded pairs, half of them past h; at
+// 97,336 particles, us, all entries and the near ones: density 29.4 and 22.0,
+// delta-p 23.7 and 18.7, viscosity 54.5 and 21.2, vorticity 28.9 and 21.4,
+// confinement 23.7 and 18.0, for 17 more in the fill.
+__device__ __forceinline__ uint2 walk_bits(const Dev& P, int b, int c) {
+  if (P.walk == nullptr || P.walk[b] == kWalkAll) return make_uint2(low_bits(c), low_bits(c - 32));
+  return P.near_bits[b];
+}
+
+// seq1 and seq2 over the entries of `bits` (at least one bit below the count
+// each), again four at a time.
+template <class Body>
+__device__ __forceinline__ void near_fours(const int32_t* __restrict__ row, uint2 bits, Body&& body) {
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half, row += pbf::list_off(32)) {
+    uint32_t m = half ? bits.y : bits.x;
+    while (m) {
+      int at[4];
+      bool has[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        has[k] = m != 0u;
+        at[k] = has[k] ? __ffs(m) - 1 : at[0];
+        m &= m - 1u;
+      }
+      body(make_int4(__ldg(row + pbf::list_off(at[0])), __ldg(row + pbf::list_off(at[1])),
+                     __ldg(row + pbf::list_off(at[2])), __ldg(row + pbf::list_off(at[3]))), has);
+    }
+  }
+}
+
+template <class Body>
+__device__ __forceinline__ void near1(const Dev& P, const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+                                      const float4* __restrict__ a, Body&& body) {
+  near_fours(nbr + pbf::list_base(b, stride), walk_bits(P, b, c), [&](int4 q, const bool (&has)[4]) {
+    const float4 v0 = a[q.x], v1 = a[q.y], v2 = a[q.z], v3 = a[q.w];
+    body(q.x, v0);
+    if (has[1]) body(q.y, v1);
+    if (has[2]) body(q.z, v2);
+    if (has[3]) body(q.w, v3);
+  });
+}
+
+template <class Body>
+__device__ __forceinline__ void near2(const Dev& P, const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+                                      const float4* __restrict__ a, const float4* __restrict__ a2, Body&& body) {
+  near_fours(nbr + pbf::list_base(b, stride), walk_bits(P, b, c), [&](int4 q, const bool (&has)[4]) {
+    const float4 v0 = a[q.x], v1 = a[q.y], v2 = a[q.z], v3 = a[q.w];
+    const float4 w0 = a2[q.x], w1 = a2[q.y], w2 = a2[q.z], w3 = a2[q.w];
+    body(q.x, v0, w0);
+    if (has[1]) body(q.y, v1, w1);
+    if (has[2]) body(q.z, v2, w2);
+    if (has[3]) body(q.w, v3, w3);
+  });
 }
 
 template <class Body>
@@ -1583,7 +1666,7 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
   float3 sg = make_float3(0.f, 0.f, 0.f);
   float sumC = 0.0f;
   bool nudged = false;
-  seq1(nbr, b, stride, c, pst, [&](int, float4 xq) {
+  auto add = [&](int, float4 xq) {
     float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     float rm = pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz));
     if ((double)rm < 0.00000001) {
@@ -1597,7 +1680,16 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
     }
     rho = pbf::A<X>(rho, pbf::M<X>(P.m, pbf::poly6<X>(P, rm)));
     lambda_terms<X>(P, rx, ry, rz, rm, sg, sumC);
-  });
+  };
+  if (X) near1(P, nbr, b, stride, c, pst, add);
+  if (!X || nudged) {  // a nudge may bring any entry within h: the whole list, from the start
+    xp = pst[b];
+    rho = pbf::M<X>(P.m, P.W0);
+    sg = make_float3(0.f, 0.f, 0.f);
+    sumC = 0.0f;
+    nudged = false;
+    seq1(nbr, b, stride, c, pst, add);
+  }
   if (nudged) *nudge = 1u;
   const float l = lambda_of<X>(P, rho, sg, sumC);
   xl[b] = make_float4(xp.x, xp.y, xp.z, l);
@@ -1613,8 +1705,8 @@ __global__ void __launch_bounds__(kBlock) k_density_lambda(Dev P, int n, size_t 
                                                            float4* vel, float* lam, uint32_t* nudge) {
   constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  density_lambda_one<X>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
+  const bool mark = b < n && density_lambda_one<X>(P, b, stride, nbr, cnt, pst, xl, vel, lam, nudge);
+  mark_neighbourhoods(P, b, mark);
 }
 
 // Fast density + lambda (see pbf_fast.cuh), kGL lanes per particle.  A
@@ -2133,7 +2225,7 @@ __global__ void __launch_bounds__(kBlock) k_lambda_fixup(Dev P, int n, size_t st
   const int c = cnt[b];
   float3 sg = make_float3(0.f, 0.f, 0.f);
   float sumC = 0.0f;
-  seq1(nbr, b, stride, c, xl, [&](int, float4 xq) {
+  near1(P, nbr, b, stride, c, xl, [&](int, float4 xq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     lambda_terms<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), sg, sumC);
   });
@@ -2228,31 +2320,34 @@ __global__ void __launch_bounds__(kBlock) k_dp_update(Dev P, int n, size_t strid
                                                       const uint32_t* __restrict__ nudge) {
   constexpr bool X = true;
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  const float4 xp = xl[b];
-  const int c = cnt[b];
-  float3 dp = make_float3(0.f, 0.f, 0.f);
-  if (*nudge == 0u) {
-    seq1(nbr, b, stride, c, xl, [&](int, float4 xq) {
-      const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
-      dp_term<X, SCORR>(P, xp.w, xq.w, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
-    });
-  } else {  // lambdas were recomputed by k_lambda_fixup
-    const float lp = lam[b];
-    seq1(nbr, b, stride, c, xl, [&](int q, float4 xq) {
-      const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
-      dp_term<X, SCORR>(P, lp, lam[q], rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
-    });
+  bool mark = false;
+  if (b < n) {
+    const float4 xp = xl[b];
+    const int c = cnt[b];
+    float3 dp = make_float3(0.f, 0.f, 0.f);
+    if (*nudge == 0u) {
+      near1(P, nbr, b, stride, c, xl, [&](int, float4 xq) {
+        const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
+        dp_term<X, SCORR>(P, xp.w, xq.w, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
+      });
+    } else {  // lambdas were recomputed by k_lambda_fixup
+      const float lp = lam[b];
+      near1(P, nbr, b, stride, c, xl, [&](int q, float4 xq) {
+        const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
+        dp_term<X, SCORR>(P, lp, lam[q], rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)), dp);
+      });
+    }
+    const float dx = pbf::M<X>(P.inv_rho0, dp.x), dy = pbf::M<X>(P.inv_rho0, dp.y), dz = pbf::M<X>(P.inv_rho0, dp.z);
+    const float3 s = pbf::boundary(P, pbf::region_of(P, b),
+                                   make_float3(pbf::xadd(xp.x, dx), pbf::xadd(xp.y, dy), pbf::xadd(xp.z, dz)));
+    const float4 ns = make_float4(s.x, s.y, s.z, moved(P, pst[b], s, mark));
+    pst[b] = ns;
+    if (LAST) {
+      const float3 v = velocity_of(P, ns, pos[b]);
+      vel[b] = make_float4(v.x, v.y, v.z, vel[b].w);
+    }
   }
-  const float dx = pbf::M<X>(P.inv_rho0, dp.x), dy = pbf::M<X>(P.inv_rho0, dp.y), dz = pbf::M<X>(P.inv_rho0, dp.z);
-  const float3 s = pbf::boundary(P, pbf::region_of(P, b),
-                                 make_float3(pbf::xadd(xp.x, dx), pbf::xadd(xp.y, dy), pbf::xadd(xp.z, dz)));
-  const float4 ns = make_float4(s.x, s.y, s.z, 0.0f);
-  pst[b] = ns;
-  if (LAST) {
-    const float3 v = velocity_of(P, ns, pos[b]);
-    vel[b] = make_float4(v.x, v.y, v.z, vel[b].w);
-  }
+  mark_neighbourhoods(P, b, mark);
 }
 
 // apply_surface_tension (particles.h:400-431): colour-field pass ...
@@ -2265,7 +2360,7 @@ __global__ void __launch_bounds__(kBlock) k_color(Dev P, int n, size_t stride, c
   const float4 xp = pst[b];
   const int c = cnt[b];
   float3 col = make_float3(0.f, 0.f, 0.f);
-  seq1(nbr, b, stride, c, pst, [&](int q, float4 xq) {
+  near1(P, nbr, b, stride, c, pst, [&](int q, float4 xq) {
     const float rq = vel[q].w;
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float3 dw = pbf::del_spikey<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
@@ -2324,7 +2419,7 @@ __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t strid
   }
   const int c = cnt[b];
   float3 dv = make_float3(0.f, 0.f, 0.f);
-  seq2(nbr, b, stride, c, pst, vin, [&](int q, float4 xq, float4 vq) {
+  near2(P, nbr, b, stride, c, pst, vin, [&](int q, float4 xq, float4 vq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float w = pbf::poly6<X>(P, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     if (X) {
@@ -2358,7 +2453,7 @@ __global__ void __launch_bounds__(kBlock) k_vorticity(Dev P, int n, size_t strid
   const float4 xp = pst[b], vp = vel[b];
   const int c = cnt[b];
   float3 w = make_float3(0.f, 0.f, 0.f);
-  seq2(nbr, b, stride, c, pst, vel, [&](int q, float4 xq, float4 vq) {
+  near2(P, nbr, b, stride, c, pst, vel, [&](int q, float4 xq, float4 vq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float3 d = pbf::del_spikey<X>(P, rx, ry, rz, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
     const float ax = pbf::S<X>(vq.x, vp.x), ay = pbf::S<X>(vq.y, vp.y), az = pbf::S<X>(vq.z, vp.z);
@@ -2395,7 +2490,7 @@ __global__ void __launch_bounds__(kBlock) k_apply_vorticity(Dev P, int n, size_t
     eta.z = pbf::A<X>(eta.z, pbf::M<X>(vm, d.z));
   };
   if (PACKED)
-    seq1(nbr, b, stride, c, xl, [&](int, float4 xq) { add(xq, xq.w); });
+    near1(P, nbr, b, stride, c, xl, [&](int, float4 xq) { add(xq, xq.w); });
   else
     seq2(nbr, b, stride, c, pst, scr, [&](int, float4 xq, float4 sq) {
       add(xq, __fsqrt_rn(pbf::mag2<true>(sq.x, sq.y, sq.z)));
@@ -3272,6 +3367,7 @@ struct pbf_ctx {
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
   uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order, near entries first
   uint2* rest = nullptr;           // [C / 32] warps of particles k_fill_masks leaves to k_fill_rest: number, lanes
+  uint2* near_bits = nullptr;      // [C] Dev::near_bits
   uint8_t* walk = nullptr;         // [C, rounded up to whole 16-byte words] Dev::walk
 
   float4 *posH = nullptr, *pstH = nullptr, *velH = nullptr, *scrH = nullptr;
@@ -3461,10 +3557,13 @@ int make_dev(pbf_ctx* ctx, const pbf_params& p, Dev& d, int64_t dims[3]) {
     d.skip_eps = 64.0f * std::ldexp(1.0f, std::ilogb(mx) - 23);
   }
   {
-    // near entries (walk_count): within h + kNearMargin * h at the fill, when that is short of s
+    // near entries (walk_count): within h + kNearMargin * h at the fill, when that is short of s and the
+    // other entries' terms are zeros: a lambda of -0 / 0 (no relaxation), densities never computed (no
+    // iteration) or a power of s_corr that does not rise make them NaN or more
     const float near = h + kNearMargin * h;
-    d.near2 = near < s ? near * near : d.s2;
-    d.near_move = near < s ? (0.5f * kNearMargin - kNearSlack) * h : FLT_MAX;
+    const bool zeros = p.lambda_epsilon > 0.0f && p.solve_steps > 0 && !(p.scorr_k > 0.0f && !(p.scorr_n > 0.0f));
+    d.near2 = near < s && zeros ? near * near : d.s2;
+    d.near_move = near < s && zeros ? (0.5f * kNearMargin - kNearSlack) * h : FLT_MAX;
   }
   d.dimx = (int)dims[0];
   d.dimy = (int)dims[1];
@@ -3537,6 +3636,7 @@ int upload_scenes(pbf_ctx* ctx) {
 // The list arrays Dev carries.
 void bind_lists(pbf_ctx* ctx) {
   ctx->dev.walk = ctx->walk;
+  ctx->dev.near_bits = ctx->near_bits;
   ctx->dev.slot_key = ctx->keyH;
   ctx->dev.cell_start = ctx->cell_start;
   ctx->dev.cell_mark = ctx->cell_count;
@@ -3803,9 +3903,10 @@ void launch_cell_sort(pbf_ctx* ctx) {
 // Particles up to which the fill takes nine and three warps a tile.  Measured,
 // us, fast math: 2k 15.6 with nine warps, 27.4 with three, 36.5 k_fill_masks;
 // 16k 17.6 / 23.8 / 34.0; 33k 24.6 / 25.7 / 34.0; 48k 30.8 / 32.7 / 37.6; 66k
-// 40.6 / 41.4 / 40.4; 1M 525 / 429 / 388.  Exact math and the search on device
-// arrays (one warp a tile in k_fill_masks's place): 2k 12.5 / 25.7 / 38.8, 33k
-// 29.4 / 31.6 / 44.3, 48k 42.5 / 38.4 / 47.0, 98k 78.6 / 65.7 / 64.9.
+// 40.6 / 41.4 / 40.4; 1M 525 / 429 / 388.  The search on device arrays (one warp
+// a tile in k_fill_masks's place): 2k 12.5 / 25.7 / 38.8, 33k 29.4 / 31.6 / 44.3,
+// 48k 42.5 / 38.4 / 47.0.  Exact math, with the near bits: 64k 59.9 / 55.9 /
+// 55.8, 97k 86.9 / 79.0 / 80.7, 262k 217 / 172 / 169, 1M 806 / 605 / 589.
 constexpr size_t kSplit9Most = 40960, kSplit3Most = 61440;
 
 void launch_fill(pbf_ctx* ctx, const float4* pst) {
@@ -4410,7 +4511,9 @@ static int create_ctx(const pbf_params* p, size_t capacity, const pbf_scene* sce
       (rc = dalloc(ctx, &ctx->scan_part, (size_t)ctx->nscan_parts)) || (rc = dalloc(ctx, &ctx->err, 1)) ||
       (rc = dalloc(ctx, &ctx->nudge, 1)) ||
       (rc = dalloc(ctx, &ctx->nbr, pbf::list_entries(C, cap))) ||
-      (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->walk, (C + 15) / 16 * 16)) || (rc = dalloc(ctx, &ctx->rest, (C + 31) / 32)) || (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
+      (rc = dalloc(ctx, &ctx->ref_order, C)) || (rc = dalloc(ctx, &ctx->walk, (C + 15) / 16 * 16)) ||
+      (rc = dalloc(ctx, &ctx->rest, (C + 31) / 32)) || (rc = dalloc(ctx, &ctx->near_bits, C)) ||
+      (rc = dalloc(ctx, &ctx->fill_words, kFillWords)) ||
       (rc = dalloc(ctx, &ctx->cnt, C)) || (rc = dalloc(ctx, &ctx->stage, 6 * C)) ||
       (rc = dalloc(ctx, &ctx->stage_i, std::max(C * cap + C, pbf::list_entries(C, cap)))) ||
       (rc = dalloc(ctx, &ctx->acc, 8)) ||

@@ -80,6 +80,7 @@ struct Dev {
   // sorted slot, the bins' first slots and the bins' marks
   float near2, near_move;
   uint8_t* walk;
+  uint2* near_bits;  // exact math: the near entries of every list, one bit an entry (the lists keep their order)
   const uint32_t* slot_key;
   const uint32_t* cell_start;
   uint32_t* cell_mark;
