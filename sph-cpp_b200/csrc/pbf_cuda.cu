@@ -3909,6 +3909,31 @@ void launch_cell_sort(pbf_ctx* ctx) {
 // 55.8, 97k 86.9 / 79.0 / 80.7, 262k 217 / 172 / 169, 1M 806 / 605 / 589.
 constexpr size_t kSplit9Most = 40960, kSplit3Most = 61440;
 
+// Particles up to which the fill asks for 60% of the SM's memory as shared
+// memory (164 KB) instead of all that its residency can use (228 KB).  Small
+// contexts run side by side, on streams of their own or in a scene group, and
+// the gathers of one then find the L1 that another one's fill left: 92 KB
+// instead of 28.  64 scenes of 4,480 to 230,958 particles, ms a step over 200
+// steps: a scene group 9.6 all, 8.1 with 60% (50% 8.0, 85% 9.7), single
+// contexts on 64 streams 10.9 and 9.8.  Alone a fill has 18 warps an SM
+// instead of 24: 65k 42.2 and 40.4 us, 212k 93 and 104, 1M 388 and 438, so
+// large contexts keep all.
+constexpr size_t kSideBySideMost = 262144;
+
+template <class... Args>
+void launch_beside(const pbf_ctx* ctx, void (*kernel)(Args...), int grid, int block, std::common_type_t<Args>... args) {
+  cudaLaunchAttribute carve{};
+  carve.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  carve.val.sharedMemCarveout = 60;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3((unsigned)grid);
+  config.blockDim = dim3((unsigned)block);
+  config.stream = ctx->stream;
+  config.attrs = &carve;
+  config.numAttrs = ctx->n <= kSideBySideMost ? 1 : 0;
+  cudaLaunchKernelEx(&config, kernel, args...);
+}
+
 void launch_fill(pbf_ctx* ctx, const float4* pst) {
   const bool fast = ctx->params.exact_math == 0, staged = any_staged(ctx);
   const int n = (int)ctx->n, tiles = blocks_for(ctx->n, 32);
@@ -3929,8 +3954,8 @@ void launch_fill(pbf_ctx* ctx, const float4* pst) {
     const ListOut out{ctx->nbr, ctx->lstride};
     auto split = [&](auto warps, auto ref) {
       constexpr int T = decltype(warps)::value;
-      k_fill_split<T, decltype(ref)::value, ListOut><<<tiles, 32 * T, 0, s>>>(P, n, pst, ctx->cell_start, out, ctx->cnt,
-                                                                            ctx->ref_order, fw, ctx->rest);
+      launch_beside(ctx, k_fill_split<T, decltype(ref)::value, ListOut>, tiles, 32 * T, P, n, pst, ctx->cell_start, out,
+                    ctx->cnt, ctx->ref_order, fw, ctx->rest);
     };
     using W1 = std::integral_constant<int, 1>;
     using W3 = std::integral_constant<int, 3>;
@@ -3946,9 +3971,8 @@ void launch_fill(pbf_ctx* ctx, const float4* pst) {
     else if (!fast)
       split(W1{}, std::true_type{});
     else
-      k_fill_masks<<<blocks_for(ctx->n, kMaskBlock), kMaskBlock, 0, s>>>(P, n, ctx->lstride, pst, ctx->cell_start,
-                                                                        ctx->nbr, ctx->cnt, ctx->ref_order, fw,
-                                                                        ctx->rest);
+      launch_beside(ctx, k_fill_masks, blocks_for(ctx->n, kMaskBlock), kMaskBlock, P, n, ctx->lstride, pst,
+                    ctx->cell_start, ctx->nbr, ctx->cnt, ctx->ref_order, fw, ctx->rest);
   }
   if (staged) return;
   Launch L(ctx, "fill_rest");
