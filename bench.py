@@ -178,8 +178,11 @@ def kernel_bytes(name: str, n: int, nbar: float, K: int, nbins: int) -> float:
     """Compulsory DRAM bytes per launch of each kernel: each per-particle input
     read once, each output written once, int32 neighbor-list entries read once;
     gathered neighbour values counted as cache hits (they are re-reads of
-    arrays already streamed by the same launch)."""
-    L = 4.0 + 4.0 * nbar   # count + list
+    arrays already streamed by the same launch).  A fast gather reads a list's
+    near entries (within h + 5% of the 1.2 h wide list) and a byte that says so:
+    (1.05 / 1.2)^3 of the list at an even density; more once particles moved."""
+    near = nbar * (1.05 / 1.2) ** 3
+    L = 4.0 + 4.0 * near + 1.0  # count, near entries, walk byte
     per = {
         "ext_predict_hash": 16 + 16 + 16 + 16 + 4 + 4,           # x, v in; v, x*, key, rank out (+ histogram in L2)
         "scan_reduce": 4.0 * nbins / n,
@@ -191,19 +194,19 @@ def kernel_bytes(name: str, n: int, nbar: float, K: int, nbins: int) -> float:
         "residual_check": 16 + L + 16 + 4 + 4,                  # as density_lambda
         "reorder": 8 + 4 + 3 * 16 + 3 * 16 + 4 + 4,             # arrival, key, (x, x*, v) in and out, orig, key
         "runs": 16 + 4,                                         # x* in (the previous slot's is a cache hit); run end out
-        "fill_neighbors": 16 + 4 * nbar + 4 + 8.0 * nbins / n + 2,  # own x*, list + counts out, bin starts, order byte
+        "fill_neighbors": 16 + 4 * nbar + 4 + 8.0 * nbins / n + 2,  # own x*, list + counts out, bin starts, order and walk bytes
         "fill_rest": 4.0 / n,                                   # the count of particles the mask fill left
         "density_lambda": 16 + L + 16 + 4 + 4,                  # x* in; list; (x*, lambda), rho, lambda out
         "lambda_fixup": 16 + L + 16 + 4,                        # exact math after a nudge: x* in, list; (x*, lambda), lambda out
         "dp_update": 16 + L + 16 + (32.0 / K),                  # (x*, lambda) in; list; x* out; last: x in, v out
-        "viscosity": 16 + 16 + L + 16 + 2 * nbar,                # ...; v out and the weight of every entry (half)
+        "viscosity": 16 + 16 + L + 16 + 2 * near,                # ...; v out and the weight of every entry (half)
         "vorticity": 16 + 16 + L + 16 + 16,
         "apply_vorticity": 16 + 16 + 16 + L + 16,
-        "viscosity_final": 16 + 16 + L + 2 * nbar + 16 + 16 + 16 + 4 + 4,  # ...; the entries' weights in (half)
+        "viscosity_final": 16 + 16 + L + 2 * near + 16 + 16 + 16 + 4 + 4,  # ...; the entries' weights in (half)
         "update_velocities": 16 + 16 + 16,
         # every gather pass of the step in one launch (pbf_set_persistent)
-        "persistent_step": K * ((40 + L) + (32 + L)) + 32 + (48 + L + 2 * nbar) + (64 + L) + (64 + L)
-                           + (96 + L + 2 * nbar),
+        "persistent_step": K * ((40 + L) + (32 + L)) + 32 + (48 + L + 2 * near) + (64 + L) + (64 + L)
+                           + (96 + L + 2 * near),
         "color_field": 16 + 16 + L + 16,
         "surface_tension": 16 + 16 + 16 + L + 16,
     }
