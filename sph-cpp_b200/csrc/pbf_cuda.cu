@@ -5094,9 +5094,12 @@ int pbf_update_positions(pbf_ctx* ctx, size_t b, size_t e) {
 
 // nsteps fused steps captured from the context's stream into a graph (not
 // instantiated; the caller owns it).
-// Particles from which a download overlaps the step's last passes (below, the
-// second stream costs more than the copy).
-constexpr size_t kEarlyLeast = 32768;
+// Particles from which a download overlaps the step's last passes.  The event
+// record node this takes holds back contexts that run side by side: 64 of
+// 4,480 to 230,958 particles on 64 streams, ms a step, recorded from 32,768
+// particles 9.8, from 131,072 8.1, from 262,145 8.2.  Alone, a frame of 65k
+// takes 387 us without the overlap and 377 with it, of 212k 734 and 686.
+constexpr size_t kEarlyLeast = 131072;
 
 static int capture_steps(pbf_ctx* ctx, int nsteps, bool early, cudaGraph_t* out) {
   cudaGraph_t graph = nullptr;

@@ -1,6 +1,6 @@
 """Downloads that overlap the step before them return the state after it.
 
-From 32,768 particles on, a download right after a step copies the positions
+From 131,072 particles on, a download right after a step copies the positions
 out while the step's last passes run.  It must return what the per-array
 access returns once everything is done, after steps, repeated steps, and steps
 followed by other calls.
@@ -24,10 +24,10 @@ def _check(g):
     return d["x"]
 
 
-@pytest.mark.parametrize("nz", [31, 32, 33, 64])  # 31,744 to 65,536 particles
+@pytest.mark.parametrize("lattice", [(32, 32, 31), (32, 32, 64), (64, 32, 63), (64, 32, 64), (64, 32, 65)])
 @pytest.mark.parametrize("options", [{}, {"exact_math": 1}, {"gamma": 1.0}, {"solve_steps": 0}])
-def test_download_after_a_step(nz, options):
-    sc = make_scene("dam_65k", lattice=(32, 32, nz), **options)
+def test_download_after_a_step(lattice, options):
+    sc = make_scene("dam_65k", lattice=lattice, **options)
     x = sc.positions()
     with Particles(sc.params(), sc.n) as g:
         g.upload(x)
@@ -46,14 +46,14 @@ def test_download_after_a_step(nz, options):
 
 def test_download_after_a_learned_step_and_a_batch():
     params, norm, _ = learn.load_model()
-    sc = make_scene("dam_65k", lambda_epsilon=1.0, solver=1, max_iterations=4)
+    sc = make_scene("dam_65k", lattice=(64, 32, 66), lambda_epsilon=1.0, solver=1, max_iterations=4)
     with Particles(sc.params(), sc.n) as g:
         g.mlp_set(params, norm)
         g.upload(sc.positions())
         for _ in range(3):
             g.step(1)
             _check(g)
-    b = make_batch(6, seed=2, n_min=4096, n_max=16384)
+    b = make_batch(12, seed=2, n_min=8192, n_max=32768)
     with Particles.batch(b) as g:
         g.upload(b.positions())
         g.step(2)
