@@ -951,11 +951,11 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
       masks = masks && a1 - a0 <= (uint32_t)kMaskRow;
     }
   }
-  // a warp with particles left to k_fill_rest is queued: its number and their lanes
+  // a warp with particles left to k_fill_rest is queued, once (the queue has one entry a warp): its number and
+  // their lanes.  The ballot waits for all of the warp's particles, however they come out of the branch above.
   {
-    const unsigned act = __activemask();
-    const unsigned left = __ballot_sync(act, !masks);
-    if (left && (int)(tid & 31) == __ffs(act) - 1) rest[atomicAdd(&fw[kFillRest], 1u)] = make_uint2((uint32_t)b >> 5, left);
+    const unsigned left = __ballot_sync(low_bits(n - (b & ~31)), !masks);
+    if (left && (tid & 31) == 0) rest[atomicAdd(&fw[kFillRest], 1u)] = make_uint2((uint32_t)b >> 5, left);
   }
   if (!masks) return;
   {
