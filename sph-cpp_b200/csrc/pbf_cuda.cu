@@ -80,21 +80,33 @@ inline size_t list_stride(int cap) { return ((size_t)cap + kListAlign - 1) / kLi
 // Upload: AoS float3 host layout -> float4 home buffers, identity order.
 // The dummy slot n the list padding points at: far from every particle (all
 // kernel terms vanish: Poly6 and Spiky are 0 beyond h, lambda and |w| are 0),
-// unit density (XSPH divides by it).  Kernels only write slots < n.
+// unit density (XSPH divides by it).  Whatever sets the particle count writes
+// it in every array a gather reads, of the fused step and of the stage calls
+// alike; all other kernels only write slots < n.
 constexpr float kFar = 1e15f;
+struct DummySlots {
+  float4 *pstS, *xl, *velS, *velT;  // the fused step's
+  float4 *pstH, *velH, *scrH;       // the stage calls'
+  float* lamH;
+  __device__ __forceinline__ void put(int n) const {
+    const float4 far = make_float4(kFar, kFar, kFar, 0.0f), still = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+    pstS[n] = far;
+    xl[n] = far;
+    velS[n] = still;
+    velT[n] = still;
+    pstH[n] = far;
+    velH[n] = still;
+    scrH[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    lamH[n] = 0.0f;
+  }
+};
 
 __global__ void k_upload(int n, const float* __restrict__ x, const float* __restrict__ v,
                          float4* posH, float4* pstH, float4* velH, float4* scrH, float* lamH, float* lamsumH,
-                         uint32_t* origH, float4* pstS, float4* xl, float4* velS, float4* velT, uint32_t* fill_words,
-                         int nwords) {
+                         uint32_t* origH, DummySlots dummies, uint32_t* fill_words, int nwords) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nwords) fill_words[i] = 0u;  // no fill before: no lists at the cap
-  if (i == 0) {
-    pstS[n] = make_float4(kFar, kFar, kFar, 0.0f);
-    xl[n] = make_float4(kFar, kFar, kFar, 0.0f);
-    velS[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-    velT[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-  }
+  if (i == 0) dummies.put(n);
   if (i >= n) return;
   const float4 p = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], 0.0f);
   posH[i] = p;
@@ -111,15 +123,9 @@ __global__ void k_upload(int n, const float* __restrict__ x, const float* __rest
 // moves to the new end.
 __global__ void k_append(int n0, int k, const float* __restrict__ x, const float* __restrict__ v, float4* posH,
                          float4* pstH, float4* velH, float4* scrH, float* lamH, float* lamsumH, uint32_t* origH,
-                         float4* pstS, float4* xl, float4* velS, float4* velT) {
+                         DummySlots dummies) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n = n0 + k;
-  if (i == 0) {
-    pstS[n] = make_float4(kFar, kFar, kFar, 0.0f);
-    xl[n] = make_float4(kFar, kFar, kFar, 0.0f);
-    velS[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-    velT[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-  }
+  if (i == 0) dummies.put(n0 + k);
   if (i >= k) return;
   const int a = n0 + i;
   const float4 p = make_float4(x[3 * i], x[3 * i + 1], x[3 * i + 2], 0.0f);
@@ -460,18 +466,12 @@ __global__ void k_reorder(int n, CellSort S, const float4* __restrict__ posH, co
 }
 
 // The per-stage path keeps the sorted arrays as the home arrays (the paths
-// start at zero), and slot n as the record that adds nothing (k_upload).
+// start at zero).
 __global__ void k_adopt(int n, const float4* __restrict__ posS, const float4* __restrict__ pstS,
                         const float4* __restrict__ velS, const float4* __restrict__ scrS,
                         const float* __restrict__ lamS, const uint32_t* __restrict__ origS, float4* posH, float4* pstH,
                         float4* velH, float4* scrH, float* lamH, uint32_t* origH) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b == 0) {
-    pstH[n] = make_float4(kFar, kFar, kFar, 0.0f);
-    velH[n] = make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-    scrH[n] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    lamH[n] = 0.0f;
-  }
   if (b >= n) return;
   posH[b] = posS[b];
   const float4 x = pstS[b];
@@ -2813,7 +2813,7 @@ __global__ void __launch_bounds__(kStageThreads) ks_apply_vorticity(Dev P, Fast 
 // Positions can change in any way between two stage calls, so a list is walked
 // whole unless the context knows that x* only moved by update_position_stars
 // since the fill (P.walk given: walk_count).  Slots past a count are read at
-// slot n, the dummy record (k_adopt).
+// slot n, the dummy record (DummySlots).
 constexpr int kStageGL = 2, kStageBlock = 128;
 
 __device__ __forceinline__ int stage_count(const Dev& P, const pbf::Group& G, const int32_t* __restrict__ cnt) {
@@ -3631,6 +3631,10 @@ int upload_scenes(pbf_ctx* ctx) {
   ctx->dev.scene_first = ctx->d_scene_first;
   ctx->dev.nscenes = (int)ctx->scenes.size();
   return PBF_OK;
+}
+
+DummySlots dummy_slots(const pbf_ctx* ctx) {
+  return DummySlots{ctx->pstS, ctx->xl, ctx->velS, ctx->velT, ctx->pstH, ctx->velH, ctx->scrH, ctx->lamH};
 }
 
 // The list arrays Dev carries.
@@ -4666,8 +4670,8 @@ int pbf_upload(pbf_ctx* ctx, const float* x, const float* v, size_t n) {
   CK(cudaMemcpyAsync(dx, x, n * 3 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   if (v) CK(cudaMemcpyAsync(dv, v, n * 3 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   k_upload<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, dx, v ? dv : nullptr, ctx->posH, ctx->pstH, ctx->velH,
-                                                      ctx->scrH, ctx->lamH, ctx->lamsumH, ctx->origH, ctx->pstS,
-                                                      ctx->xl, ctx->velS, ctx->velT, ctx->fill_words, kFillWords);
+                                                      ctx->scrH, ctx->lamH, ctx->lamsumH, ctx->origH,
+                                                      dummy_slots(ctx), ctx->fill_words, kFillWords);
   return check_launch(ctx, "upload");
 }
 
@@ -4738,7 +4742,7 @@ int pbf_add_particles(pbf_ctx* ctx, const float* x, const float* v, size_t k) {
   if (v) CK(cudaMemcpyAsync(dv, v, k * 3 * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   k_append<<<blocks_for(k), kBlock, 0, ctx->stream>>>((int)ctx->n, (int)k, dx, v ? dv : nullptr, ctx->posH,
                                                       ctx->pstH, ctx->velH, ctx->scrH, ctx->lamH, ctx->lamsumH,
-                                                      ctx->origH, ctx->pstS, ctx->xl, ctx->velS, ctx->velT);
+                                                      ctx->origH, dummy_slots(ctx));
   if (int rc = check_launch(ctx, "add_particles")) return rc;
   CK(cudaStreamSynchronize(ctx->stream));  // the host buffers may go once this returns
   ctx->n += k;
