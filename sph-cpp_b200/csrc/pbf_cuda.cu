@@ -3716,10 +3716,19 @@ int check_span(pbf_ctx* ctx, size_t b, size_t e) {
   return PBF_OK;
 }
 
-// The constant block of a per-stage call over the span [0, e).
+// The lists do not fit the state any more, nor do the keys and walk bytes the
+// stage calls' marks go by.
+void drop_lists(pbf_ctx* ctx) {
+  ctx->lists_valid = false;
+  ctx->near_stages = false;
+}
+
+// The constant block of a per-stage call over the span [0, e).  Without valid
+// lists nothing may be marked (update_position_stars needs none): the slots'
+// keys are of another set, or of none.
 Dev span_dev(const pbf_ctx* ctx, size_t e) {
   Dev d = ctx->dev;
-  if (!ctx->near_stages) d.walk = nullptr;
+  if (!ctx->near_stages || !ctx->lists_valid) d.walk = nullptr;
   if (e < ctx->n) {
     d.span_orig = ctx->origH;
     d.span_end = (uint32_t)e;
@@ -4621,7 +4630,7 @@ int pbf_set_params(pbf_ctx* ctx, const pbf_params* p) {
   if (d.nbins > ctx->nbins_cap || lstride > ctx->lstride_cap)
     return fail(ctx, PBF_ERR_PARAMS, "new parameters need a larger grid or neighbor cap than allocated");
   if (d.nbins != ctx->nbins || p->neighbor_cap != ctx->params.neighbor_cap || d.s != ctx->dev.s)
-    ctx->lists_valid = false;
+    drop_lists(ctx);
   ctx->params = *p;
   ctx->dev = d;
   ctx->near_stages = false;
@@ -4658,7 +4667,7 @@ int pbf_upload(pbf_ctx* ctx, const float* x, const float* v, size_t n) {
                 ctx->scenes.size(), ctx->scene_first.back(), n);
   if (n != ctx->n) drop_graphs(ctx);
   ctx->n = n;
-  ctx->lists_valid = false;
+  drop_lists(ctx);
   ctx->x_early = false;
   ctx->rho_whole = false;
   if (n == 0) {
@@ -4746,7 +4755,7 @@ int pbf_add_particles(pbf_ctx* ctx, const float* x, const float* v, size_t k) {
   if (int rc = check_launch(ctx, "add_particles")) return rc;
   CK(cudaStreamSynchronize(ctx->stream));  // the host buffers may go once this returns
   ctx->n += k;
-  ctx->lists_valid = false;
+  drop_lists(ctx);
   drop_graphs(ctx);
   return PBF_OK;
 }
@@ -5816,7 +5825,7 @@ int pbf_autotune(pbf_ctx* ctx, int steps, pbf_tuning* chosen, double* ms) {
     ctx->times.clear();
     ctx->time_order.clear();
     ctx->marks_used = 0;
-    ctx->lists_valid = false;
+    drop_lists(ctx);
     drop_graphs(ctx);
     return code;
   };
