@@ -3364,6 +3364,7 @@ struct pbf_ctx {
   bool rho_whole = false;    // every density is one of compute_densities' (never zero) since the last upload
   bool near_stages = false;  // since find_neighbors x* has only moved by the stages that follow it (Dev::walk)
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
+  Dev list_dev{};                 // the grid the lists and the slots' bin keys are of (set_params may keep them valid)
   uint32_t* fill_words = nullptr;  // [kFillWords] the fast fill's counts (FillWord)
   uint8_t* ref_order = nullptr;    // [C] 1: the list is in the reference's order, 0: in slot order, near entries first
   uint2* rest = nullptr;           // [C / 32] warps of particles k_fill_masks leaves to k_fill_rest: number, lanes
@@ -3789,6 +3790,13 @@ bool any_staged(const pbf_ctx* ctx) {
   return false;
 }
 
+// The lists of the present positions and parameters are there, or on their way.
+void have_lists(pbf_ctx* ctx) {
+  ctx->lists_valid = true;
+  ctx->lists_slot_order = ctx->params.exact_math == 0 && !any_staged(ctx);
+  ctx->list_dev = ctx->dev;
+}
+
 TileIO tile_io(const pbf_ctx* ctx) { return TileIO{ctx->tile_nruns, ctx->tile_total, ctx->tile_runs, ctx->nbr16}; }
 
 
@@ -3960,8 +3968,7 @@ void launch_fill(pbf_ctx* ctx, const float4* pst) {
   }
   // fast math: lists in slot order (the gathers' sums in any order are within
   // the fast path's tolerance); exact math and the staged gathers' 16-bit
-  // lists: the reference's order
-  ctx->lists_slot_order = fast && !staged;
+  // lists: the reference's order (have_lists)
   {
     Launch L(ctx, "fill_neighbors");
     const ListOut out{ctx->nbr, ctx->lstride};
@@ -4990,7 +4997,7 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
     k_clear_outside_span<<<g, kBlock, 0, s>>>(n, ctx->origH, (uint32_t)fill_e, ctx->cnt);
   rc = check_launch(ctx, "find_neighbors");
   if (rc) return rc;
-  ctx->lists_valid = true;
+  have_lists(ctx);
   ctx->near_stages = ctx->lists_slot_order;
   return PBF_OK;
 }
@@ -5152,7 +5159,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
     for (int i = 0; i < nsteps; ++i) launch_step(ctx);
     int rc = check_launch(ctx, "step");
     if (rc) return rc;
-    ctx->lists_valid = true;
+    have_lists(ctx);
     return harvest_times(ctx);
   }
   const bool early = ctx->n >= kEarlyLeast && !persist_on(ctx);
@@ -5167,7 +5174,7 @@ int pbf_step(pbf_ctx* ctx, int nsteps) {
     it = ctx->graphs.emplace(nsteps, exec).first;
   }
   CK(cudaGraphLaunch(it->second, ctx->stream));
-  ctx->lists_valid = true;
+  have_lists(ctx);
   ctx->x_early = early;
   return PBF_OK;
 }
@@ -5308,7 +5315,7 @@ int pbf_group_step(pbf_group* g, int nsteps) {
     c->steps_done += (uint64_t)nsteps;
     c->near_stages = false;
     c->x_early = false;
-    c->lists_valid = true;
+    have_lists(c);
   }
   return PBF_OK;
 }
@@ -5358,7 +5365,7 @@ int pbf_get_neighbors(pbf_ctx* ctx, int32_t* idx, int32_t* count) {
   k_export_neighbors<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, ctx->lstride, (int)cap, ctx->nbr, ctx->cnt,
                                                                  ctx->origH, di, dc,
                                                                  ctx->lists_slot_order ? ctx->ref_order : nullptr,
-                                                                 ctx->keyH, ctx->dev);
+                                                                 ctx->keyH, ctx->list_dev);
   if (int rc = check_launch(ctx, "export_neighbors")) return rc;
   if (idx) CK(cudaMemcpyAsync(idx, di, n * cap * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   if (count) CK(cudaMemcpyAsync(count, dc, n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
