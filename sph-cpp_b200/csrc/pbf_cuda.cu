@@ -3293,45 +3293,111 @@ __global__ void __launch_bounds__(kBlock) k_stats(Dev P, int b0, int b1, size_t 
   }
 }
 
-// Neighbour lists in reference index space, [N][cap], -1 past count.
+// Neighbour lists in reference index space, [N][cap], -1 past count; a warp a
+// list, an entry or two a lane (lists hold at most 64).
 // ref_order (may be null: every list is in the reference's order): a list
-// whose byte is 0 holds its entries in another order.  Its bins are the 27 at
-// integer offsets of the particle's own, so an entry's visit follows from the
-// two bin keys (key, per slot), and its place in the reference's list is the
-// number of entries of an earlier visit, or of the same visit and a lower slot.
-__global__ void k_export_neighbors(int n, size_t stride, int cap, const int32_t* __restrict__ nbr,
-                                   const int32_t* __restrict__ cnt, const uint32_t* __restrict__ orig,
-                                   int32_t* idx_out, int32_t* cnt_out, const uint8_t* __restrict__ ref_order,
-                                   const uint32_t* __restrict__ key, Dev P) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
+// whose byte is 0 holds its entries near ones first, in ascending slots
+// within the near ones and within the others.  Its bins are the 27 at integer
+// offsets of the particle's own, so an entry's visit follows from the two bin
+// keys (key, per slot; P: the grid they are of), and a visit's entries are two
+// segments of the list, one in each part.  An entry's place in the reference's
+// list is the number of entries of earlier visits, plus its place in its own
+// segment, plus the lower slots in the other one.
+// Bound by the latency of the two gathers (keys, indices).  1M particles, 54
+// entries a list, us a call without the copy to the host: 476; a thread a list,
+// which reads the list and the keys again for every entry and writes 4 bytes
+// into 32 rows a store, 7,006; every entry compared with all that go round the
+// warp 728.  2k particles 19, 463 and 20.
+struct ExportSegments {
+  uint32_t slot[64];
+  int start[2][27], end[2][27], before[27];  // of every visit: its segment in either part, the earlier visits' entries
+};
+__global__ void __launch_bounds__(kBlock) k_export_neighbors(int n, size_t stride, int cap,
+                                                             const int32_t* __restrict__ nbr,
+                                                             const int32_t* __restrict__ cnt,
+                                                             const uint32_t* __restrict__ orig, int32_t* idx_out,
+                                                             int32_t* cnt_out, const uint8_t* __restrict__ ref_order,
+                                                             const uint32_t* __restrict__ key, Dev P) {
+  __shared__ ExportSegments shared[kBlock / 32];
+  const int lane = threadIdx.x & 31;
+  const int b = (int)(blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5));
+  if (b >= n) return;  // the whole warp
   const size_t o = orig[b];
   const int c = cnt[b];
-  if (cnt_out) cnt_out[o] = c;
-  if (!idx_out) return;
-  for (int k = c; k < cap; ++k) idx_out[o * cap + k] = -1;
-  if (ref_order == nullptr || ref_order[b]) {
-    for (int k = 0; k < c; ++k) idx_out[o * cap + k] = (int32_t)orig[nbr[pbf::list_at(b, stride, k)]];
-    return;
+  int32_t* row = idx_out + o * cap;
+  if (lane == 0) cnt_out[o] = c;
+  const int k[2] = {lane, lane + 32};
+  uint32_t q[2];
+  int at[2] = {k[0], k[1]};
+#pragma unroll
+  for (int e = 0; e < 2; ++e) q[e] = k[e] < c ? (uint32_t)nbr[pbf::list_at(b, stride, k[e])] : 0u;
+  if (ref_order != nullptr && !ref_order[b]) {
+    ExportSegments& S = shared[threadIdx.x >> 5];
+    const pbf::Region R = pbf::region_of(P, b);
+    const int plane = R.dimx * R.dimy, half = (plane - 1) / 2;  // |dy * dimx + dx| <= half: at least 3 bins per axis
+    const int own = (int)key[b];
+    int v[2];  // visits
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int d = k[e] < c ? (int)key[q[e]] - own : 0;
+      const int dz = d > half ? 1 : (d < -half ? -1 : 0);
+      const int r = d - dz * plane;
+      const int dy = r > 1 ? 1 : (r < -1 ? -1 : 0);
+      v[e] = (r - dy * R.dimx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
+      S.slot[k[e]] = q[e];
+    }
+    if (lane < 27) S.start[0][lane] = S.start[1][lane] = S.end[0][lane] = S.end[1][lane] = 0;
+    // the entries before: their slots and visits; the first descent begins the second part
+    const uint32_t q31 = __shfl_sync(0xffffffffu, q[0], 31);
+    const int v31 = __shfl_sync(0xffffffffu, v[0], 31);
+    uint32_t pq[2];
+    int pv[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      pq[e] = __shfl_up_sync(0xffffffffu, q[e], 1);
+      pv[e] = __shfl_up_sync(0xffffffffu, v[e], 1);
+    }
+    if (lane == 0) {
+      pq[0] = 0u;
+      pq[1] = q31;
+      pv[1] = v31;
+    }
+    const unsigned d0 = __ballot_sync(0xffffffffu, k[0] < c && q[0] < pq[0]);
+    const unsigned d1 = __ballot_sync(0xffffffffu, k[1] < c && q[1] < pq[1]);
+    const int split = d0 ? __ffs(d0) - 1 : (d1 ? 31 + __ffs(d1) : c);
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (k[e] < c) {
+        const int part = k[e] >= split ? 1 : 0;
+        if (k[e] == 0 || v[e] != pv[e] || k[e] == split) {
+          S.start[part][v[e]] = k[e];
+          if (k[e] > 0) S.end[k[e] - 1 >= split ? 1 : 0][pv[e]] = k[e];
+        }
+        if (k[e] == c - 1) S.end[part][v[e]] = c;
+      }
+    __syncwarp();
+    const int mine = lane < 27 ? S.end[0][lane] - S.start[0][lane] + S.end[1][lane] - S.start[1][lane] : 0;
+    int upto = mine;
+#pragma unroll
+    for (int t = 1; t < 32; t <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, upto, t);
+      if (lane >= t) upto += below;
+    }
+    if (lane < 27) S.before[lane] = upto - mine;
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+      if (k[e] < c) {
+        const int part = k[e] >= split ? 1 : 0;
+        at[e] = S.before[v[e]] + k[e] - S.start[part][v[e]];
+        for (int t = S.start[1 - part][v[e]]; t < S.end[1 - part][v[e]]; ++t) at[e] += S.slot[t] < q[e];
+      }
   }
-  const pbf::Region R = pbf::region_of(P, b);
-  const int plane = R.dimx * R.dimy, half = (plane - 1) / 2;  // |dy * dimx + dx| <= half: at least 3 bins per axis
-  const int own = (int)key[b];
-  int place[64];  // the visit of every entry (c <= 64)
-  for (int k = 0; k < c; ++k) {
-    const int d = (int)key[nbr[pbf::list_at(b, stride, k)]] - own;
-    const int dz = d > half ? 1 : (d < -half ? -1 : 0);
-    const int r = d - dz * plane;
-    const int dy = r > 1 ? 1 : (r < -1 ? -1 : 0);
-    place[k] = (r - dy * R.dimx + 1) * 9 + (dy + 1) * 3 + (dz + 1);
-  }
-  for (int k = 0; k < c; ++k) {
-    const int q = nbr[pbf::list_at(b, stride, k)];
-    int rank = 0;
-    for (int t = 0; t < c; ++t)
-      rank += place[t] < place[k] || (place[t] == place[k] && nbr[pbf::list_at(b, stride, t)] < q) ? 1 : 0;
-    idx_out[o * cap + rank] = (int32_t)orig[q];
-  }
+#pragma unroll
+  for (int e = 0; e < 2; ++e)
+    if (k[e] < c) row[at[e]] = (int32_t)orig[q[e]];
+  for (int t = c + lane; t < cap; t += 32) row[t] = -1;
 }
 
 }  // namespace
@@ -5362,10 +5428,9 @@ int pbf_get_neighbors(pbf_ctx* ctx, int32_t* idx, int32_t* count) {
   const size_t n = ctx->n, cap = (size_t)ctx->params.neighbor_cap;
   int32_t* di = ctx->stage_i;
   int32_t* dc = ctx->stage_i + n * cap;
-  k_export_neighbors<<<blocks_for(n), kBlock, 0, ctx->stream>>>((int)n, ctx->lstride, (int)cap, ctx->nbr, ctx->cnt,
-                                                                 ctx->origH, di, dc,
-                                                                 ctx->lists_slot_order ? ctx->ref_order : nullptr,
-                                                                 ctx->keyH, ctx->list_dev);
+  k_export_neighbors<<<blocks_for(n, kBlock / 32), kBlock, 0, ctx->stream>>>(
+      (int)n, ctx->lstride, (int)cap, ctx->nbr, ctx->cnt, ctx->origH, di, dc,
+      ctx->lists_slot_order ? ctx->ref_order : nullptr, ctx->keyH, ctx->list_dev);
   if (int rc = check_launch(ctx, "export_neighbors")) return rc;
   if (idx) CK(cudaMemcpyAsync(idx, di, n * cap * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
   if (count) CK(cudaMemcpyAsync(count, dc, n * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
