@@ -335,9 +335,26 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t* __
   if (threadIdx.x == 0) partial[blockIdx.x] = total;
 }
 
+// The tiles' sums -> the sums of the tiles before (one block), for grids of
+// more than kScanOwnMost tiles.
+__global__ void __launch_bounds__(kScanThreads) k_scan_partials(uint32_t* partial, int np) {
+  __shared__ uint32_t ws[32];
+  uint32_t before = 0;
+  for (int i0 = 0; i0 < np; i0 += kScanThreads) {
+    const int i = i0 + (int)threadIdx.x;
+    const uint32_t v = i < np ? partial[i] : 0u;
+    uint32_t total;
+    const uint32_t ex = block_exclusive_scan(v, ws, total);
+    if (i < np) partial[i] = before + ex;
+    before += total;
+    __syncthreads();  // ws is written again
+  }
+}
+
 // out[0..m] (m+1 entries): exclusive prefix of in[0..m-1], out[m] = total.
-// Every block adds up the tiles' sums before its own (310 at 1M particles): a
-// launch that scanned them took 2 us of every step.
+// SCANNED: partial is k_scan_partials's; else every block adds up the sums of
+// the tiles before its own itself.
+template <bool SCANNED>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in, int m,
                                                              const uint32_t* __restrict__ partial,
                                                              uint32_t* out) {
@@ -350,12 +367,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
     v[i] = base + i < (size_t)m ? in[base + i] : 0u;
     s += v[i];
   }
-  uint32_t before = 0;
-  for (int i = threadIdx.x; i < (int)blockIdx.x; i += kScanThreads) before += partial[i];
-  uint32_t total;
-  block_exclusive_scan(before, ws, total);
-  before = total;
-  __syncthreads();  // ws is written again
+  uint32_t before = 0, total;
+  if (SCANNED) {
+    before = partial[blockIdx.x];
+  } else {
+    for (int i = threadIdx.x; i < (int)blockIdx.x; i += kScanThreads) before += partial[i];
+    block_exclusive_scan(before, ws, total);
+    before = total;
+    __syncthreads();  // ws is written again
+  }
   uint32_t run = block_exclusive_scan(s, ws, total) + before;
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
@@ -3962,6 +3982,14 @@ int order_grid(size_t n, size_t room, int sms) {
   return (int)std::max<size_t>(1, std::min<size_t>(room / (2 * (size_t)bitmap_words(n)), 2 * (size_t)sms));
 }
 
+// Tiles of 4,096 bins up to which every block of the scan adds up the tiles'
+// sums before its own, instead of a launch between that scans them: the
+// sums are quadratic in the tiles, the launch takes 6 us of a chain of small
+// ones.  Both forms, us for the whole scan, with the launch between and
+// without: 267 tiles 21.3 and 15.0, 1,058 33.9 and 31.4, 2,043 46.6 and 45.9,
+// 4,145 83.2 and 84.7, 15,980 288 and 316, 126,412 2,134 and 3,246.
+constexpr int kScanOwnMost = 2048;
+
 // Bin bounds and the arrivals of every bin; the hash must already have
 // produced key, rank, cell_count and the crowded bins.  k_order_crowded's
 // bitmaps lie in the host staging area, which no step uses.
@@ -3973,9 +4001,16 @@ void launch_cell_sort(pbf_ctx* ctx) {
     Launch L(ctx, "scan_reduce");
     k_scan_reduce<<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part);
   }
-  {
+  if (ctx->nscan_parts > kScanOwnMost) {
+    {
+      Launch L(ctx, "scan_partials");
+      k_scan_partials<<<1, kScanThreads, 0, s>>>(ctx->scan_part, ctx->nscan_parts);
+    }
     Launch L(ctx, "scan_apply");
-    k_scan_apply<<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
+    k_scan_apply<true><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
+  } else {
+    Launch L(ctx, "scan_apply");
+    k_scan_apply<false><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
   }
   {
     Launch L(ctx, "arrivals");
@@ -4525,7 +4560,7 @@ int launches_per_step(const pbf_ctx* ctx) {
   // launches fewer once converged): ext/predict/hash + sort + reorder + runs + fill + [not staged: rest] +
   // K x (density/lambda, [exact: lambda fix-up], delta-p)
   // + (K==0: velocity) + 2 if gamma + 4 (visc, vort, apply, visc)
-  const int sort = 4;  // 2 scan, arrivals, crowded bins
+  const int sort = ctx->nscan_parts > kScanOwnMost ? 5 : 4;  // 2 or 3 scan, arrivals, crowded bins
   const int fill = any_staged(ctx) ? 2 : 3;  // runs, fill, [rest]
   if (persist_on(ctx)) return 1 + sort + 1 + fill + 1;  // ... reorder, runs, fill, rest, the persistent step
   const int K = ctx->params.solve_steps;
@@ -6002,6 +6037,7 @@ constexpr size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign;
 constexpr size_t kNaN = PBF_NOALLOC_MAX_PARTICLES;
 constexpr size_t kNaB = PBF_NOALLOC_MAX_BINS;
 constexpr size_t kNaParts = (kNaB + 1 + kScanTile - 1) / kScanTile;
+static_assert(kNaParts <= (size_t)kScanOwnMost, "the scan here is two launches");
 constexpr size_t kNaWords = kNaN / 32, kNaOrderBlocks = 16;  // k_order_crowded's bitmap of the indices, its blocks
 // layout of the scratch array (byte offsets)
 constexpr size_t kOffCount = 0;
@@ -6186,7 +6222,7 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
   const CellSort sort{arrivals, key, cell_start, place};
   k_noalloc_hash<<<g, kBlock, 0, s>>>(d, nn, d_x, key, rank, cell_count, crowded, err);
   k_scan_reduce<<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts);
-  k_scan_apply<<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts, cell_start);
+  k_scan_apply<false><<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts, cell_start);
   k_arrivals<<<g, kBlock, 0, s>>>(nn, key, rank, nullptr, cell_start, arrivals);
   k_order_crowded<<<(int)kNaOrderBlocks, kOrderThreads, 0, s>>>(bitmap_words(n), cell_count + d.nbins + kCrowdedBins,
                                                                crowded, cell_start, arrivals, bits, place);
