@@ -391,8 +391,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
 // rest): k_arrivals writes every particle's reference index and slot at its
 // bin's start plus its arrival number, and k_reorder counts the smaller
 // indices in the bin.  Bins of more than kCountBin particles, where that
-// count would be quadratic, are ordered by k_order_crowded: linear in the bin
-// plus a bitmap of all indices.  A stable radix sort of (key, index) and its
+// count would be quadratic, are ordered by k_order_crowded.  A stable radix sort of (key, index) and its
 // scans took 10 launches, 51 us a step at 65k particles and 73 us at 1M; what
 // takes their place (k_arrivals, k_order_crowded's launch, the count) 5 and
 // 10 us.  Bound by the scattered 8-byte stores of k_arrivals and, in
@@ -405,42 +404,84 @@ __global__ void k_arrivals(int n, const uint32_t* __restrict__ key, const uint32
   arrivals[cell_start[key[a]] + rank[a]] = make_uint2(orig ? orig[a] : (uint32_t)a, (uint32_t)a);
 }
 
-// Crowded bins, a block each: the bin's reference indices as bits, the bits'
-// prefix sums, and every particle's place from the two.  bits: `regions`
-// regions of 2 * words words (words = the bitmap of n indices), one per block.
-constexpr int kOrderThreads = 1024;
+// Crowded bins, a block each.  By the bitmap: the bin's reference indices as
+// bits, the bits' prefix sums, and every particle's place from the two, which
+// costs a pass over all n indices' bits whatever the bin holds.  So bins of at
+// most kOrderSort particles are sorted in shared memory instead (bitonic, then
+// every index is looked up) where the bitmap is longer than kOrderBits words.
+// Bitmap and sort, us a launch: 65,536 particles, one bin of 2,000 10 and 23,
+// of 8,000 17 and 62; 1M, 40 bins of 2,000 21 and 21, of 8,000 31 and 66; 16.8M,
+// one bin of 8,000 193 and 58, 4,000 bins of 2,000 10,116 and 629.  With more
+// particles a bin the bitmap's pass weighs little (16.8M, 40 bins of 60,000:
+// 318 us).  Bound by the block-wide synchronisations of the sort and the scan.
+// bits: a region of 2 * words words a block (words = the bitmap of n indices,
+// a multiple of 4).
+constexpr int kOrderThreads = 1024, kOrderSort = 8192, kOrderBits = 32768;
 __global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, const uint32_t* __restrict__ crowded_bins,
                                                                  const uint32_t* __restrict__ crowded,
                                                                  const uint32_t* __restrict__ cell_start,
                                                                  const uint2* __restrict__ arrivals, uint32_t* bits,
                                                                  uint32_t* place) {
   __shared__ uint32_t ws[32];
+  __shared__ uint32_t sorted[kOrderSort];
   const uint32_t bins = *crowded_bins;
-  uint32_t* mine = bits + 2 * (size_t)words * blockIdx.x;
-  uint32_t* before = mine + words;
+  const int tid = threadIdx.x;
+  uint4* mine = reinterpret_cast<uint4*>(bits + 2 * (size_t)words * blockIdx.x);
+  uint32_t* mine1 = reinterpret_cast<uint32_t*>(mine);
+  uint4* before = mine + words / 4;
+  const uint32_t* before1 = reinterpret_cast<const uint32_t*>(before);
   for (uint32_t i = blockIdx.x; i < bins; i += gridDim.x) {
     const uint32_t s = cell_start[crowded[i]], e = cell_start[crowded[i] + 1];
-    for (int w = threadIdx.x; w < words; w += kOrderThreads) __stcg(mine + w, 0u);
+    const int m = (int)(e - s);
+    if (words > kOrderBits && m <= kOrderSort) {
+      int size = 2;
+      while (size < m) size <<= 1;
+      for (int t = tid; t < size; t += kOrderThreads) sorted[t] = t < m ? __ldg(&arrivals[s + t].x) : 0xffffffffu;
+      __syncthreads();
+      for (int k = 2; k <= size; k <<= 1)
+        for (int d = k >> 1; d > 0; d >>= 1) {
+          for (int t = tid; t < size / 2; t += kOrderThreads) {
+            const int a = 2 * t - (t & (d - 1)), b = a + d;
+            const uint32_t x = sorted[a], y = sorted[b];
+            if ((x > y) == ((a & k) == 0)) {
+              sorted[a] = y;
+              sorted[b] = x;
+            }
+          }
+          __syncthreads();
+        }
+      for (int t = tid; t < m; t += kOrderThreads) {
+        const uint32_t o = __ldg(&arrivals[s + t].x);
+        int at = 0;
+        for (int d = size / 2; d > 0; d >>= 1) at += sorted[at + d - 1] < o ? d : 0;
+        place[s + t] = s + (uint32_t)at;
+      }
+      __syncthreads();
+      continue;
+    }
+    for (int w = tid; w < words / 4; w += kOrderThreads) __stcg(mine + w, make_uint4(0u, 0u, 0u, 0u));
     __syncthreads();
 #pragma unroll 8
-    for (uint32_t j = s + threadIdx.x; j < e; j += kOrderThreads) {
+    for (uint32_t j = s + tid; j < e; j += kOrderThreads) {
       const uint32_t o = __ldg(&arrivals[j].x);
-      atomicOr(mine + (o >> 5), 1u << (o & 31u));
+      atomicOr(mine1 + (o >> 5), 1u << (o & 31u));
     }
     __syncthreads();
     uint32_t run = 0;
-    for (int w0 = 0; w0 < words; w0 += kOrderThreads) {
-      const int w = w0 + (int)threadIdx.x;
+    for (int w0 = 0; w0 < words / 4; w0 += kOrderThreads) {
+      const int w = w0 + tid;
+      const uint4 b = w < words / 4 ? __ldcg(mine + w) : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t n0 = __popc(b.x), n1 = n0 + __popc(b.y), n2 = n1 + __popc(b.z);
       uint32_t total;
-      const uint32_t ex = block_exclusive_scan(w < words ? (uint32_t)__popc(__ldcg(mine + w)) : 0u, ws, total);
-      if (w < words) before[w] = run + ex;
+      const uint32_t ex = run + block_exclusive_scan(n2 + __popc(b.w), ws, total);
+      if (w < words / 4) before[w] = make_uint4(ex, ex + n0, ex + n1, ex + n2);
       run += total;
       __syncthreads();  // ws is written again
     }
 #pragma unroll 8
-    for (uint32_t j = s + threadIdx.x; j < e; j += kOrderThreads) {
+    for (uint32_t j = s + tid; j < e; j += kOrderThreads) {
       const uint32_t o = __ldg(&arrivals[j].x);
-      place[j] = s + before[o >> 5] + (uint32_t)__popc(__ldcg(mine + (o >> 5)) & ((1u << (o & 31u)) - 1u));
+      place[j] = s + before1[o >> 5] + (uint32_t)__popc(__ldcg(mine1 + (o >> 5)) & ((1u << (o & 31u)) - 1u));
     }
     __syncthreads();
   }
@@ -3974,10 +4015,11 @@ int harvest_times(pbf_ctx* ctx) {
 // ---- neighbor build ----
 CellSort cell_sort(const pbf_ctx* ctx) { return CellSort{ctx->arrivals, ctx->key, ctx->cell_start, ctx->place}; }
 
-// Words of a bitmap of n indices, and the blocks k_order_crowded gets: as many
-// as have room for a bitmap and its prefix sums in `room` words, at most two
-// per SM (six words a particle leave 96).
-int bitmap_words(size_t n) { return (int)((n + 31) / 32); }
+// Words of a bitmap of n indices (whole 16-byte groups), and the blocks
+// k_order_crowded gets: as many as have room for a bitmap and its prefix sums
+// in `room` words, at most two per SM (six words a particle leave 96; one block
+// has room from 22 particles on, and no bin is crowded below 1,025).
+int bitmap_words(size_t n) { return (int)((n + 127) / 128 * 4); }
 int order_grid(size_t n, size_t room, int sms) {
   return (int)std::max<size_t>(1, std::min<size_t>(room / (2 * (size_t)bitmap_words(n)), 2 * (size_t)sms));
 }
