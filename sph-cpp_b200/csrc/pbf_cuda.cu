@@ -230,12 +230,9 @@ __global__ void k_predict(Dev P, int n, const float4* __restrict__ pos, const fl
   pst[a] = make_float4(s.x, s.y, s.z, 0.0f);
 }
 
-// Bins holding more particles than this walk their candidates run by run.  A
-// run waits for the load before it, so short runs lose to the tests' four
-// loads in flight: the fill of the 1M dam at steps 150 / 200 / 250 / 290 takes
-// 0.72 / 1.27 / 2.83 / 2.81 ms at 512, 0.56 / 1.26 / 2.63 / 2.78 at 1,024,
-// 0.56 / 1.07 / 2.25 / 2.14 at 4,096.
-constexpr uint32_t kRunBin = 4096;
+// Bins holding more particles than this are walked run by run where they are
+// mostly long runs of bit-identical x* (long_runs).
+constexpr uint32_t kRunBin = 512;
 
 // Bins of more than this many particles are ordered by k_order_crowded, the
 // others by counting within the bin (k_reorder).
@@ -659,6 +656,29 @@ __device__ __forceinline__ uint32_t low_bits(int k) {
   return k >= 32 ? 0xffffffffu : (k <= 0 ? 0u : (1u << k) - 1u);
 }
 
+// Whether the bin [q0, q1) of more than kRunBin particles is mostly long runs,
+// from four of its slots: the slots their runs still hold, added up.  A run
+// ends at the last slot of a block of k_runs (kRunBlock), so the four lie at
+// different places of those blocks whatever the bin's length.
+// A run waits for the load before it, so short runs lose to the tests' four
+// loads in flight; a pile of particles on one point loses by its size without
+// them.  1M particles, us a step, bins of 1,100 / 2,000 identical points (400 / 40
+// bins): tests up to 4,096 a bin 3,960 / 3,174, runs 1,548 / 1,870, so 1,547 /
+// 1,873.  The fill of the 1M dam's state at step 200 / 250 / 290 / 320, few of
+// whose points coincide, ms: tests up to 4,096 1.15 / 2.57 / 2.37 / 7.36, runs
+// 1.34 / 3.09 / 3.02 / 7.84, so 1.12 / 2.51 / 2.31 / 6.28.
+__device__ __forceinline__ bool long_runs(uint32_t q0, uint32_t q1, const uint32_t* __restrict__ run_end) {
+  constexpr uint32_t kLong = 64, kPlace[4] = {3, 10, 19, 30};
+  const uint32_t spread = (q1 - q0 - kRunBin) / 32;
+  uint32_t sum = 0;
+#pragma unroll
+  for (uint32_t i = 0; i < 4; ++i) {
+    const uint32_t q = q0 + kPlace[i] * spread + 128u * i;
+    sum += run_end[q] - q;
+  }
+  return sum >= kLong;
+}
+
 // One crowded bin [q0, q1) of the list fill, run by run: one distance test per
 // run of bit-identical x*; on a hit the run's slots are appended in order, the
 // particle's own slot left out, while the list has room.  Returns the new
@@ -694,7 +714,7 @@ __device__ __noinline__ int fill_runs(float px, float py, float pz, float s2, in
 // (P.skip_eps), squared and summed, exceeds s^2.  Only bins equal to the
 // integer offset of the particle's own bin are skipped, so the reference's
 // float re-hash still decides which bins are visited.  A bin of more than
-// kRunBin particles is walked run by run (k_runs): a run of bit-identical x*
+// kRunBin particles is walked run by run (k_runs) where its runs are long: a run of bit-identical x*
 // is one distance test, and on a hit its slots are appended in order (the
 // particle's own slot left out), the list the one-by-one walk gives.
 constexpr int kFillBlock = 128;
@@ -749,7 +769,7 @@ __device__ __forceinline__ int fill_visit(int cx, int cy, int cz, bool at_offset
     else off = soff[(threadIdx.x & ~31) + rz * S.ny + ry];
   }
   const uint32_t q0 = cell_start[nb], q1 = cell_start[nb + 1];
-  if (q1 - q0 > kRunBin) {
+  if (q1 - q0 > kRunBin && long_runs(q0, q1, run_end)) {
     count = fill_runs(px, py, pz, s2, cap, self, q0, q1, pst, run_end, row, staged ? S.row16 : nullptr, off, count);
   } else {
     for (uint32_t q = q0; q < q1 && count < cap; q += 32) {
@@ -6184,7 +6204,7 @@ __global__ void __launch_bounds__(kBlock) k_noalloc_rest(Dev P, const uint32_t* 
           continue;
         }
         const uint32_t q0 = cell_start[nb], q1 = cell_start[nb + 1];
-        if (q1 - q0 > kRunBin) {
+        if (q1 - q0 > kRunBin && long_runs(q0, q1, run_end)) {
           count = noalloc_fill_runs(xp.x, xp.y, xp.z, P.s2, cap, (uint32_t)b, q0, q1, pst, run_end, sorted_id,
                                     row, count);
           continue;
