@@ -1127,12 +1127,13 @@ __device__ __forceinline__ int fill_cooperative(const Dev& P, int b, size_t stri
   const float4 xp = pst[b];
   const pbf::Region R = pbf::region_of(P, b);
   uint32_t q0 = 0, q1 = 0;
+  bool outside = false;
   if (lane < 27) {
     auto bin = [&](float c, int o) { return pbf::dev_axis_bin(pbf::xadd(c, pbf::xmul((float)(o - 1), P.s)), P.s); };
     const int cx = bin(xp.x, lane / 9), cy = bin(xp.y, lane / 3 % 3), cz = bin(xp.z, lane % 3);
     if (!isfinite(xp.x) || !isfinite(xp.y) || !isfinite(xp.z) || cx < 0 || cy < 0 || cz < 0 || cx >= R.dimx ||
         cy >= R.dimy || cz >= R.dimz) {
-      atomicOr(err, PBF_FLAG_KEY_RANGE);
+      outside = true;
     } else {
       const uint32_t key =
           R.key0 + (uint32_t)(R.dimx * R.dimy) * (uint32_t)cz + ((uint32_t)cy * (uint32_t)R.dimx + (uint32_t)cx);
@@ -1151,7 +1152,7 @@ __device__ __forceinline__ int fill_cooperative(const Dev& P, int b, size_t stri
   }
   const int before = upto - mine, total = __shfl_sync(0xffffffffu, upto, 31);
   int32_t* row = nbr + pbf::list_base(b, stride);
-  int count = 0;
+  int count = 0, last = total;  // last: the candidate that fills the list
   for (int i0 = 0; i0 < total && count < P.cap; i0 += 32) {
     const int i = i0 + lane;
     int v = 0;
@@ -1169,8 +1170,11 @@ __device__ __forceinline__ int fill_cooperative(const Dev& P, int b, size_t stri
     const unsigned hits = __ballot_sync(0xffffffffu, hit);
     const int at = count + __popc(hits & ((1u << lane) - 1u));
     if (hit && at < P.cap) row[pbf::list_off(at)] = (int32_t)c;
+    const unsigned fills = __ballot_sync(0xffffffffu, hit && at == P.cap - 1);
+    if (fills) last = i0 + __ffs(fills) - 1;
     count += __popc(hits);
   }
+  if (outside && before <= last) atomicOr(err, PBF_FLAG_KEY_RANGE);  // a visit after the list is full is none
   return min(count, P.cap);
 }
 
