@@ -1590,9 +1590,9 @@ __device__ __forceinline__ void seq1(const int32_t* __restrict__ nbr, int b, siz
 // 97,336 particles, us, all entries and the near ones: density 29.4 and 22.0,
 // delta-p 23.7 and 18.7, viscosity 54.5 and 21.2, vorticity 28.9 and 21.4,
 // confinement 23.7 and 18.0, for 17 more in the fill.
+__device__ __forceinline__ uint2 all_bits(int c) { return make_uint2(low_bits(c), low_bits(c - 32)); }
 __device__ __forceinline__ uint2 walk_bits(const Dev& P, int b, int c) {
-  if (P.walk == nullptr || P.walk[b] == kWalkAll) return make_uint2(low_bits(c), low_bits(c - 32));
-  return P.near_bits[b];
+  return P.walk == nullptr || P.walk[b] == kWalkAll ? all_bits(c) : P.near_bits[b];
 }
 
 // seq1 and seq2 over the entries of `bits` (at least one bit below the count
@@ -1618,15 +1618,21 @@ __device__ __forceinline__ void near_fours(const int32_t* __restrict__ row, uint
 }
 
 template <class Body>
-__device__ __forceinline__ void near1(const Dev& P, const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+__device__ __forceinline__ void near1(const int32_t* __restrict__ nbr, int b, size_t stride, uint2 bits,
                                       const float4* __restrict__ a, Body&& body) {
-  near_fours(nbr + pbf::list_base(b, stride), walk_bits(P, b, c), [&](int4 q, const bool (&has)[4]) {
+  near_fours(nbr + pbf::list_base(b, stride), bits, [&](int4 q, const bool (&has)[4]) {
     const float4 v0 = a[q.x], v1 = a[q.y], v2 = a[q.z], v3 = a[q.w];
     body(q.x, v0);
     if (has[1]) body(q.y, v1);
     if (has[2]) body(q.z, v2);
     if (has[3]) body(q.w, v3);
   });
+}
+
+template <class Body>
+__device__ __forceinline__ void near1(const Dev& P, const int32_t* __restrict__ nbr, int b, size_t stride, int c,
+                                      const float4* __restrict__ a, Body&& body) {
+  near1(nbr, b, stride, walk_bits(P, b, c), a, body);
 }
 
 template <class Body>
@@ -1766,8 +1772,16 @@ __device__ __forceinline__ bool density_lambda_one(const Dev& P, int b, size_t s
     rho = pbf::A<X>(rho, pbf::M<X>(P.m, pbf::poly6<X>(P, rm)));
     lambda_terms<X>(P, rx, ry, rz, rm, sg, sumC);
   };
-  if (X) near1(P, nbr, b, stride, c, pst, add);
-  if (!X || nudged) {  // a nudge may bring any entry within h: the whole list, from the start
+  // A nudge may bring any entry within h: the whole list, from the start, unless it was the whole list.  (A
+  // collapsed 65k dam, where most particles are nudged and walk their whole lists, us for three passes: walked
+  // again 258, so 162, without near entries 158.)
+  bool again = !X;
+  if (X) {
+    const uint2 bits = walk_bits(P, b, c), all = all_bits(c);
+    near1(nbr, b, stride, bits, pst, add);
+    again = nudged && (bits.x != all.x || bits.y != all.y);
+  }
+  if (again) {
     xp = pst[b];
     rho = pbf::M<X>(P.m, P.W0);
     sg = make_float3(0.f, 0.f, 0.f);
