@@ -291,6 +291,24 @@ __global__ void k_ext_predict_hash(Dev P, int n, const float4* __restrict__ pos,
   hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
+// Bins that hold a sixteenth of all particles or more (a collapsed dam piles
+// almost everything into one).  Their order within the bin is found by all
+// blocks of the sort's launches instead of one (k_order_crowded): k_scan_apply
+// clears a bitmap of the reference indices, k_arrivals sets the bin's bits,
+// k_order_crowded leaves the words' prefix sums and k_reorder looks up.  The
+// bitmap and its sums lie in the bin's own part of the place array.
+constexpr int kGiantMost = 16;
+struct GiantBins {
+  uint32_t* place;
+  uint32_t least;  // particles of such a bin
+  int words;       // the bitmap of n indices, a multiple of 4
+  __host__ __device__ __forceinline__ uint32_t* bits(uint32_t start) const { return place + ((start + 3u) & ~3u); }
+  __device__ __forceinline__ uint32_t slot(uint32_t start, uint32_t o) const {
+    const uint32_t* b = bits(start) + (o >> 5);
+    return start + b[words] + (uint32_t)__popc(b[0] & ((1u << (o & 31u)) - 1u));
+  }
+};
+
 // ---- exclusive scan of cell_count[0..m-1] (+ total at [m]) -> cell_start ----
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* warp_sums,
                                                          uint32_t& total) {
@@ -350,12 +368,14 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_partials(uint32_t* partia
 
 // out[0..m] (m+1 entries): exclusive prefix of in[0..m-1], out[m] = total.
 // SCANNED: partial is k_scan_partials's; else every block adds up the sums of
-// the tiles before its own itself.
+// the tiles before its own itself.  The bitmaps of giant bins (GiantBins) are
+// cleared on the way.
 template <bool SCANNED>
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __restrict__ in, int m,
                                                              const uint32_t* __restrict__ partial,
-                                                             uint32_t* out) {
+                                                             uint32_t* out, GiantBins G) {
   __shared__ uint32_t ws[32];
+  __shared__ uint32_t giant_start[kGiantMost], giants;
   const size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t v[kScanItems];
   uint32_t s = 0;
@@ -379,6 +399,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
     if (base + i <= (size_t)m) out[base + i] = run;
     run += v[i];
   }
+  if (!__syncthreads_or(v[0] >= G.least || v[1] >= G.least || v[2] >= G.least || v[3] >= G.least)) return;
+  if (threadIdx.x == 0) giants = 0u;
+  __syncthreads();
+  static_assert(kScanItems == 4, "the items above");
+  for (int i = kScanItems - 1; i >= 0; --i) {
+    run -= v[i];
+    if (v[i] >= G.least) giant_start[atomicAdd(&giants, 1u)] = run;
+  }
+  __syncthreads();
+  for (uint32_t g = 0; g < giants; ++g) {
+    uint4* bits = reinterpret_cast<uint4*>(G.bits(giant_start[g]));
+    for (int w = threadIdx.x; w < G.words / 4; w += kScanThreads) bits[w] = make_uint4(0u, 0u, 0u, 0u);
+  }
 }
 
 // ---- the cell sort ----
@@ -395,10 +428,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(const uint32_t* __r
 // k_reorder, by the state's bytes.
 __global__ void k_arrivals(int n, const uint32_t* __restrict__ key, const uint32_t* __restrict__ rank,
                            const uint32_t* __restrict__ orig, const uint32_t* __restrict__ cell_start,
-                           uint2* arrivals) {
+                           const uint32_t* __restrict__ crowded_bins, uint2* arrivals, GiantBins G) {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
-  arrivals[cell_start[key[a]] + rank[a]] = make_uint2(orig ? orig[a] : (uint32_t)a, (uint32_t)a);
+  const uint32_t k = key[a], s = cell_start[k], o = orig ? orig[a] : (uint32_t)a;
+  arrivals[s + rank[a]] = make_uint2(o, (uint32_t)a);
+  if (*crowded_bins != 0u && cell_start[k + 1] - s >= G.least) atomicOr(G.bits(s) + (o >> 5), 1u << (o & 31u));
 }
 
 // Crowded bins, a block each.  By the bitmap: the bin's reference indices as
@@ -410,27 +445,30 @@ __global__ void k_arrivals(int n, const uint32_t* __restrict__ key, const uint32
 // of 8,000 17 and 62; 1M, 40 bins of 2,000 21 and 21, of 8,000 31 and 66; 16.8M,
 // one bin of 8,000 193 and 58, 4,000 bins of 2,000 10,116 and 629.  With more
 // particles a bin the bitmap's pass weighs little (16.8M, 40 bins of 60,000:
-// 318 us).  Bound by the block-wide synchronisations of the sort and the scan.
+// 318 us).  Of a giant bin only the prefix sums are left to find: by one block
+// alone, the whole sort of a bin of 1M took 872 us, of 52,000 among 65,536 67,
+// so 67 and 25 (a cluster of eight blocks a bin 163 and 36, but its blocks
+// wait for eight SMs of a kind at once, also where there is nothing to do: 16
+// contexts of 13,824 in a group 3.4 instead of 2.4 ms a five steps).
+// Bound by the block-wide synchronisations of the sort and the scan.
 // bits: a region of 2 * words words a block (words = the bitmap of n indices,
 // a multiple of 4).
 constexpr int kOrderThreads = 1024, kOrderSort = 8192, kOrderBits = 32768;
-__global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, const uint32_t* __restrict__ crowded_bins,
+__global__ void __launch_bounds__(kOrderThreads) k_order_crowded(const uint32_t* __restrict__ crowded_bins,
                                                                  const uint32_t* __restrict__ crowded,
                                                                  const uint32_t* __restrict__ cell_start,
                                                                  const uint2* __restrict__ arrivals, uint32_t* bits,
-                                                                 uint32_t* place) {
+                                                                 GiantBins G) {
   __shared__ uint32_t ws[32];
   __shared__ uint32_t sorted[kOrderSort];
   const uint32_t bins = *crowded_bins;
-  const int tid = threadIdx.x;
-  uint4* mine = reinterpret_cast<uint4*>(bits + 2 * (size_t)words * blockIdx.x);
-  uint32_t* mine1 = reinterpret_cast<uint32_t*>(mine);
-  uint4* before = mine + words / 4;
-  const uint32_t* before1 = reinterpret_cast<const uint32_t*>(before);
+  const int tid = threadIdx.x, words = G.words;
+  uint32_t* place = G.place;
   for (uint32_t i = blockIdx.x; i < bins; i += gridDim.x) {
     const uint32_t s = cell_start[crowded[i]], e = cell_start[crowded[i] + 1];
     const int m = (int)(e - s);
-    if (words > kOrderBits && m <= kOrderSort) {
+    const bool giant = e - s >= G.least;
+    if (words > kOrderBits && m <= kOrderSort && !giant) {
       int size = 2;
       while (size < m) size <<= 1;
       for (int t = tid; t < size; t += kOrderThreads) sorted[t] = t < m ? __ldg(&arrivals[s + t].x) : 0xffffffffu;
@@ -456,14 +494,20 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, cons
       __syncthreads();
       continue;
     }
-    for (int w = tid; w < words / 4; w += kOrderThreads) __stcg(mine + w, make_uint4(0u, 0u, 0u, 0u));
-    __syncthreads();
+    uint4* mine = reinterpret_cast<uint4*>(giant ? G.bits(s) : bits + 2 * (size_t)words * blockIdx.x);
+    uint32_t* mine1 = reinterpret_cast<uint32_t*>(mine);
+    uint4* before = mine + words / 4;
+    const uint32_t* before1 = reinterpret_cast<const uint32_t*>(before);
+    if (!giant) {
+      for (int w = tid; w < words / 4; w += kOrderThreads) __stcg(mine + w, make_uint4(0u, 0u, 0u, 0u));
+      __syncthreads();
 #pragma unroll 8
-    for (uint32_t j = s + tid; j < e; j += kOrderThreads) {
-      const uint32_t o = __ldg(&arrivals[j].x);
-      atomicOr(mine1 + (o >> 5), 1u << (o & 31u));
+      for (uint32_t j = s + tid; j < e; j += kOrderThreads) {
+        const uint32_t o = __ldg(&arrivals[j].x);
+        atomicOr(mine1 + (o >> 5), 1u << (o & 31u));
+      }
+      __syncthreads();
     }
-    __syncthreads();
     uint32_t run = 0;
     for (int w0 = 0; w0 < words / 4; w0 += kOrderThreads) {
       const int w = w0 + tid;
@@ -475,6 +519,7 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, cons
       run += total;
       __syncthreads();  // ws is written again
     }
+    if (giant) continue;
 #pragma unroll 8
     for (uint32_t j = s + tid; j < e; j += kOrderThreads) {
       const uint32_t o = __ldg(&arrivals[j].x);
@@ -487,13 +532,15 @@ __global__ void __launch_bounds__(kOrderThreads) k_order_crowded(int words, cons
 // What the sort leaves for the gathers of the state into cell order.
 struct CellSort {
   const uint2* arrivals;  // (reference index, slot), every bin's in its range
-  const uint32_t *key, *cell_start, *place;
+  const uint32_t *key, *cell_start;
+  GiantBins giants;  // and every crowded bin's places
 };
 
 // The sorted slot of arrival j (reference index o, bin key k).
 __device__ __forceinline__ uint32_t sorted_slot(const CellSort& S, uint32_t j, uint32_t o, uint32_t k) {
   const uint32_t s = S.cell_start[k], e = S.cell_start[k + 1];
-  if (e - s > kCountBin) return S.place[j];
+  if (e - s >= S.giants.least) return S.giants.slot(s, o);
+  if (e - s > kCountBin) return S.giants.place[j];
   uint32_t at = s;
 #pragma unroll 4
   for (uint32_t i = s; i < e; ++i) at += S.arrivals[i].x < o ? 1u : 0u;
@@ -4051,15 +4098,23 @@ int harvest_times(pbf_ctx* ctx) {
 }
 
 // ---- neighbor build ----
-CellSort cell_sort(const pbf_ctx* ctx) { return CellSort{ctx->arrivals, ctx->key, ctx->cell_start, ctx->place}; }
-
 // Words of a bitmap of n indices (whole 16-byte groups), and the blocks
-// k_order_crowded gets: as many as have room for a bitmap and its prefix sums
-// in `room` words, at most two per SM (six words a particle leave 96; one block
-// has room from 22 particles on, and no bin is crowded below 1,025).
+// k_order_crowded gets: one for every bin that may be crowded, as many as have
+// room for a bitmap and its prefix sums in `room` words, at most two per SM
+// (six words a particle leave 96).
 int bitmap_words(size_t n) { return (int)((n + 127) / 128 * 4); }
 int order_grid(size_t n, size_t room, int sms) {
-  return (int)std::max<size_t>(1, std::min<size_t>(room / (2 * (size_t)bitmap_words(n)), 2 * (size_t)sms));
+  const size_t most = std::min<size_t>(n / (kCountBin + 1), 2 * (size_t)sms);
+  return (int)std::max<size_t>(1, std::min<size_t>(room / (2 * (size_t)bitmap_words(n)), most));
+}
+
+GiantBins giant_bins(size_t n, uint32_t* place) {
+  const int words = bitmap_words(n);
+  return GiantBins{place, std::max(2u * (uint32_t)words + 4u, kCountBin + 1u), words};
+}
+
+CellSort cell_sort(const pbf_ctx* ctx) {
+  return CellSort{ctx->arrivals, ctx->key, ctx->cell_start, giant_bins(ctx->n, ctx->place)};
 }
 
 // Tiles of 4,096 bins up to which every block of the scan adds up the tiles'
@@ -4076,6 +4131,8 @@ constexpr int kScanOwnMost = 2048;
 void launch_cell_sort(pbf_ctx* ctx) {
   const int n = (int)ctx->n;
   const int m = ctx->nbins;  // scan m entries -> m+1 outputs
+  const GiantBins giants = giant_bins(ctx->n, ctx->place);
+  const uint32_t* crowded_bins = ctx->cell_count + m + kCrowdedBins;
   cudaStream_t s = ctx->stream;
   {
     Launch L(ctx, "scan_reduce");
@@ -4087,19 +4144,21 @@ void launch_cell_sort(pbf_ctx* ctx) {
       k_scan_partials<<<1, kScanThreads, 0, s>>>(ctx->scan_part, ctx->nscan_parts);
     }
     Launch L(ctx, "scan_apply");
-    k_scan_apply<true><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
+    k_scan_apply<true><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start,
+                                                                    giants);
   } else {
     Launch L(ctx, "scan_apply");
-    k_scan_apply<false><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start);
+    k_scan_apply<false><<<ctx->nscan_parts, kScanThreads, 0, s>>>(ctx->cell_count, m, ctx->scan_part, ctx->cell_start,
+                                                                    giants);
   }
   {
     Launch L(ctx, "arrivals");
-    k_arrivals<<<blocks_for(n), kBlock, 0, s>>>(n, ctx->key, ctx->rank, ctx->origH, ctx->cell_start, ctx->arrivals);
+    k_arrivals<<<blocks_for(n), kBlock, 0, s>>>(n, ctx->key, ctx->rank, ctx->origH, ctx->cell_start, crowded_bins,
+                                                ctx->arrivals, giants);
   }
   Launch L(ctx, "order_crowded");
   k_order_crowded<<<order_grid(ctx->n, 6 * ctx->capacity, ctx->sms), kOrderThreads, 0, s>>>(
-      bitmap_words(ctx->n), ctx->cell_count + m + kCrowdedBins, ctx->crowded, ctx->cell_start, ctx->arrivals,
-      reinterpret_cast<uint32_t*>(ctx->stage), ctx->place);
+      crowded_bins, ctx->crowded, ctx->cell_start, ctx->arrivals, reinterpret_cast<uint32_t*>(ctx->stage), giants);
 }
 
 // Particles up to which the fill takes nine and three warps a tile.  Measured,
@@ -6299,13 +6358,15 @@ extern "C" int pbf_find_neighbors_noalloc(const pbf_params* p, const float* d_x,
   if (e != cudaSuccess) return fail(nullptr, PBF_ERR_CUDA, "cudaMemsetAsync failed: %s", cudaGetErrorString(e));
   const int nn = (int)n, g = blocks_for(n);
   const int nparts = (int)(((size_t)d.nbins + 1 + kScanTile - 1) / kScanTile);
-  const CellSort sort{arrivals, key, cell_start, place};
+  const GiantBins giants = giant_bins(n, place);
+  const uint32_t* crowded_bins = cell_count + d.nbins + kCrowdedBins;
+  const CellSort sort{arrivals, key, cell_start, giants};
   k_noalloc_hash<<<g, kBlock, 0, s>>>(d, nn, d_x, key, rank, cell_count, crowded, err);
   k_scan_reduce<<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts);
-  k_scan_apply<false><<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts, cell_start);
-  k_arrivals<<<g, kBlock, 0, s>>>(nn, key, rank, nullptr, cell_start, arrivals);
-  k_order_crowded<<<(int)kNaOrderBlocks, kOrderThreads, 0, s>>>(bitmap_words(n), cell_count + d.nbins + kCrowdedBins,
-                                                               crowded, cell_start, arrivals, bits, place);
+  k_scan_apply<false><<<nparts, kScanThreads, 0, s>>>(cell_count, d.nbins, parts, cell_start, giants);
+  k_arrivals<<<g, kBlock, 0, s>>>(nn, key, rank, nullptr, cell_start, crowded_bins, arrivals, giants);
+  k_order_crowded<<<(int)kNaOrderBlocks, kOrderThreads, 0, s>>>(crowded_bins, crowded, cell_start, arrivals, bits,
+                                                               giants);
   k_noalloc_gather<<<g, kBlock, 0, s>>>(nn, sort, d_x, sorted_x, sorted_id);
   k_runs<<<blocks_for(n, kRunBlock), kRunBlock, 0, s>>>(nn, sorted_x, run_end,
                                                         cell_count + d.nbins + kCrowdedRuns, fw);
