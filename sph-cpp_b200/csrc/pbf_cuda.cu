@@ -240,8 +240,17 @@ constexpr uint32_t kCountBin = 1024;
 
 // The words after the bin histogram (cleared with it): kCrowdedRuns is raised
 // when a bin passes kRunBin particles (only then does the list fill need the
-// runs, k_runs), kCrowdedBins counts the bins past kCountBin.
-enum CrowdedWord { kCrowdedRuns = 0, kCrowdedBins = 1, kCrowdedWords = 2 };
+// runs, k_runs), kCrowdedBins counts the bins past kCountBin, kWildValues is
+// raised when some value is so large, or none, that zero times it may not be
+// zero: the lists of that search are walked whole (near entries, below).
+enum CrowdedWord { kCrowdedRuns = 0, kCrowdedBins = 1, kWildValues = 2, kCrowdedWords = 3 };
+
+constexpr float kTame = 1e12f;
+__device__ __forceinline__ bool tame(float v) { return fabsf(v) <= kTame; }
+// Of the velocity that the move from x to x* comes to.
+__device__ __forceinline__ float move_size(float4 xs, float4 x) {
+  return fabsf(xs.x - x.x) + fabsf(xs.y - x.y) + fabsf(xs.z - x.z);
+}
 
 // calculate_bins (neighbors.h:120-125) + bin histogram; rank = the particle's
 // arrival number in its bin (any order).  The lanes of a warp with the same
@@ -288,6 +297,8 @@ __global__ void k_ext_predict_hash(Dev P, int n, const float4* __restrict__ pos,
   pst[a] = make_float4(s.x, s.y, s.z, 0.0f);
   uint32_t k;
   if (!pbf::bin_of(P, R, s.x, s.y, s.z, k)) atomicOr(err, PBF_FLAG_KEY_RANGE);
+  // (of a NaN x* there are no lists)
+  if (move_size(make_float4(s.x, s.y, s.z, 0.0f), pos[a]) > kTame * P.dt) cell_count[P.nbins + kWildValues] = 1u;
   hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
@@ -570,21 +581,47 @@ __global__ void k_reorder(int n, CellSort S, const float4* __restrict__ posH, co
   if (lamS) lamS[b] = lamH[a];  // FULL: lambda; fused step: last step's lambda sum, when kept
 }
 
+// Whether the stages that follow a search may meet a value for which zero
+// times it is no zero; rho: densities count too (else they are computed first,
+// or the lists walked whole).
+__device__ __forceinline__ bool wild(const Dev& P, float4 xs, float4 x, float4 v, float4 scr, float lam, bool rho) {
+  const float at = xs.x + xs.y + xs.z;
+  if (at != at) return false;  // no list holds it
+  const bool r = !rho || (fabsf(v.w) >= 1e-30f && fabsf(v.w) <= 1e30f);
+  return !(r && move_size(xs, x) <= kTame * P.dt && tame(v.x) && tame(v.y) && tame(v.z) && tame(scr.x) &&
+           tame(scr.y) && tame(scr.z) && tame(lam));
+}
+
+__global__ void k_wild(Dev P, int n, const float4* __restrict__ pstH, const float4* __restrict__ posH,
+                       const float4* __restrict__ velH, const float4* __restrict__ scrH,
+                       const float* __restrict__ lamH, bool rho, uint32_t* word) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b < n && wild(P, pstH[b], posH[b], velH[b], scrH[b], lamH[b], rho)) *word = 1u;
+}
+
+// All lists are walked whole from here on when the word is raised.
+__global__ void k_walk_whole(int n, const uint32_t* __restrict__ word, uint8_t* walk) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (*word != 0u && 16 * i < n) reinterpret_cast<uint4*>(walk)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+}
+
 // The per-stage path keeps the sorted arrays as the home arrays (the paths
 // start at zero).
-__global__ void k_adopt(int n, const float4* __restrict__ posS, const float4* __restrict__ pstS,
+__global__ void k_adopt(Dev P, int n, const float4* __restrict__ posS, const float4* __restrict__ pstS,
                         const float4* __restrict__ velS, const float4* __restrict__ scrS,
                         const float* __restrict__ lamS, const uint32_t* __restrict__ origS, float4* posH, float4* pstH,
-                        float4* velH, float4* scrH, float* lamH, uint32_t* origH) {
+                        float4* velH, float4* scrH, float* lamH, uint32_t* origH, bool rho, uint32_t* word) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
-  posH[b] = posS[b];
-  const float4 x = pstS[b];
-  pstH[b] = make_float4(x.x, x.y, x.z, 0.0f);
-  velH[b] = velS[b];
-  scrH[b] = scrS[b];
-  lamH[b] = lamS[b];
+  const float4 x = posS[b], xs = pstS[b], v = velS[b], scr = scrS[b];
+  const float lam = lamS[b];
+  posH[b] = x;
+  pstH[b] = make_float4(xs.x, xs.y, xs.z, 0.0f);
+  velH[b] = v;
+  scrH[b] = scr;
+  lamH[b] = lam;
   origH[b] = origS[b];
+  if (wild(P, xs, x, v, scr, lam, rho)) *word = 1u;
 }
 
 // Device words of the fast path's fill (FillWord): the lists that reached the
@@ -1154,7 +1191,7 @@ __global__ void __launch_bounds__(kMaskBlock) k_fill_masks(Dev P, int n, size_t 
     dst[1] = make_int4(e[4], e[5], e[6], e[7]);
   }
   cnt[b] = count;
-  P.walk[b] = (uint8_t)walk;
+  P.walk[b] = P.cell_mark[P.nbins + kWildValues] ? kWalkAll : (uint8_t)walk;
   ref_order[b] = 0;
   count_capped(fw, count >= cap);
 }
@@ -1471,7 +1508,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
       }
       if (mine && t == 0) {
         P.near_bits[b] = make_uint2((uint32_t)near, (uint32_t)(near >> 32));
-        P.walk[b] = 0;  // the near bits, until marked
+        P.walk[b] = P.cell_mark[P.nbins + kWildValues] ? kWalkAll : (uint8_t)0;  // 0: the near bits, until marked
       }
     }
     if (!mine) return;
@@ -1528,7 +1565,7 @@ __global__ void __launch_bounds__(32 * T) k_fill_split(Dev P, int n, const float
   }
   if (t == 0) {
     cnt[b] = total;
-    P.walk[b] = (uint8_t)near_all;
+    P.walk[b] = P.cell_mark[P.nbins + kWildValues] ? kWalkAll : (uint8_t)near_all;
     ref_order[b] = 0;
     count_capped(fw, total >= cap);
   }
@@ -1546,6 +1583,10 @@ static_assert(kMaskWords == 3 && kMaskUnits <= 32, "the words' division by 3 and
 // half the margin marks the 27 bins around its own, and the lists there are
 // walked whole from the next launch on.  (An unmarked list's entries past the
 // near ones would add zeros, so a mark more or less changes no bit.)
+// Zero times infinity or NaN is no zero: where a search or what is set after
+// it finds such a value (kWildValues: a position far from its x*, a velocity,
+// scratch vector, lambda or density given by the caller), every list is walked
+// whole, so that it reaches as far as in the reference.
 // kNearSlack is left out of the path's bound for rounding: the squared
 // distances' (3e-7 of h^2), the path's sum and rsqrt's.
 // A margin of 0.05 h keeps 0.67 of a disordered list.  1M dam, all 54 entries
@@ -3574,6 +3615,7 @@ struct pbf_ctx {
   cudaEvent_t x_ready = nullptr;
   bool record_x = false, x_early = false;
   bool rho_whole = false;    // every density is one of compute_densities' (never zero) since the last upload
+  bool rho_known = false;    // every density was computed or set since the last upload (k_adopt and k_wild look at it)
   bool near_stages = false;  // since find_neighbors x* has only moved by the stages that follow it (Dev::walk)
   bool lists_slot_order = false;  // the lists are k_fill_masks's: ref_order says, per list, which order it is in
   Dev list_dev{};                 // the grid the lists and the slots' bin keys are of (set_params may keep them valid)
@@ -3946,6 +3988,14 @@ Dev span_dev(const pbf_ctx* ctx, size_t e) {
     d.span_orig = ctx->origH;
     d.span_end = (uint32_t)e;
   }
+  return d;
+}
+
+// For the stages that divide by a neighbour's density or follow one that does:
+// while densities are missing (0, so that zero times their inverse is NaN) the
+// lists are walked whole.
+Dev density_dev(const pbf_ctx* ctx, Dev d) {
+  if (!ctx->rho_known) d.walk = nullptr;
   return d;
 }
 
@@ -4916,7 +4966,7 @@ int pbf_upload(pbf_ctx* ctx, const float* x, const float* v, size_t n) {
   ctx->n = n;
   drop_lists(ctx);
   ctx->x_early = false;
-  ctx->rho_whole = false;
+  ctx->rho_whole = ctx->rho_known = false;
   if (n == 0) {
     CK(cudaMemsetAsync(ctx->fill_words, 0, kFillWords * sizeof(uint32_t), ctx->stream));
     return PBF_OK;
@@ -4964,7 +5014,10 @@ int pbf_set_array(pbf_ctx* ctx, int which, const float* host_in) {
   const bool vec = which <= PBF_ARRAY_SCRATCH;
   if (which == PBF_ARRAY_POSITION_STARS) ctx->near_stages = false;
   ctx->x_early = false;
-  if (which == PBF_ARRAY_DENSITIES) ctx->rho_whole = false;
+  if (which == PBF_ARRAY_DENSITIES) {
+    ctx->rho_whole = false;
+    ctx->rho_known = true;
+  }
   CK(cudaMemcpyAsync(ctx->stage, host_in, ctx->n * (vec ? 3 : 1) * sizeof(float), cudaMemcpyHostToDevice,
                      ctx->stream));
   switch (which) {
@@ -4975,6 +5028,12 @@ int pbf_set_array(pbf_ctx* ctx, int which, const float* host_in) {
     case PBF_ARRAY_DENSITIES: k_permute_w_in<<<g, kBlock, 0, ctx->stream>>>(n, ctx->stage, ctx->origH, ctx->velH, nullptr); break;
     case PBF_ARRAY_LAMBDAS: k_permute_w_in<<<g, kBlock, 0, ctx->stream>>>(n, ctx->stage, ctx->origH, nullptr, ctx->lamH); break;
     default: return fail(ctx, PBF_ERR_ARG, "unknown array %d", which);
+  }
+  if (ctx->near_stages && ctx->lists_valid) {
+    uint32_t* word = ctx->cell_count + ctx->nbins + kWildValues;
+    k_wild<<<g, kBlock, 0, ctx->stream>>>(ctx->dev, n, ctx->pstH, ctx->posH, ctx->velH, ctx->scrH, ctx->lamH,
+                                          ctx->rho_known, word);
+    k_walk_whole<<<blocks_for((ctx->n + 15) / 16), kBlock, 0, ctx->stream>>>(n, word, ctx->walk);
   }
   int rc = check_launch(ctx, "set_array");
   if (rc) return rc;
@@ -4988,7 +5047,7 @@ int pbf_add_particles(pbf_ctx* ctx, const float* x, const float* v, size_t k) {
   if (!ctx->scenes.empty()) return fail(ctx, PBF_ERR_STATE, "the scenes of a batch have fixed particle counts");
   if (k == 0) return PBF_OK;
   ctx->x_early = false;
-  ctx->rho_whole = false;
+  ctx->rho_whole = ctx->rho_known = false;
   if (ctx->n + k > ctx->capacity)
     return fail(ctx, PBF_ERR_CAPACITY, "Not enough capacity: %zu particles > capacity %zu", ctx->n + k,
                 ctx->capacity);
@@ -5230,8 +5289,9 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
   k_reorder<true><<<g, kBlock, 0, s>>>(n, cell_sort(ctx), ctx->posH, ctx->pstH, ctx->velH, ctx->scrH,
                                        ctx->lamH, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS,
                                        ctx->keyH);
-  k_adopt<<<g, kBlock, 0, s>>>(n, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS, ctx->posH,
-                               ctx->pstH, ctx->velH, ctx->scrH, ctx->lamH, ctx->origH);
+  k_adopt<<<g, kBlock, 0, s>>>(ctx->dev, n, ctx->posS, ctx->pstS, ctx->velS, ctx->scrS, ctx->lamS, ctx->origS,
+                               ctx->posH, ctx->pstH, ctx->velH, ctx->scrH, ctx->lamH, ctx->origH, ctx->rho_known,
+                               ctx->cell_count + ctx->nbins + kWildValues);
   launch_fill(ctx, ctx->pstH);
   if (fill_e < ctx->n)  // particles outside the fill span (halo particles) get empty lists
     k_clear_outside_span<<<g, kBlock, 0, s>>>(n, ctx->origH, (uint32_t)fill_e, ctx->cnt);
@@ -5245,7 +5305,7 @@ int pbf_find_neighbors(pbf_ctx* ctx, size_t bin_b, size_t bin_e, size_t fill_b, 
 int pbf_compute_densities(pbf_ctx* ctx, size_t b, size_t e) {
   STAGE_PROLOGUE(b, e);
   if (int rc = need_lists(ctx)) return rc;
-  if (e == ctx->n) ctx->rho_whole = true;
+  if (e == ctx->n) ctx->rho_whole = ctx->rho_known = true;
   if (X)
     k_density<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->pstS);
   else
@@ -5317,7 +5377,7 @@ int pbf_apply_viscosity(pbf_ctx* ctx, size_t b, size_t e) {
     k_viscosity<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT, nullptr, nullptr,
                                                       nullptr, nullptr);
   else
-    kt_viscosity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT);
+    kt_viscosity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(density_dev(ctx, SP), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->velT);
   CK(cudaMemcpyAsync(ctx->velH, ctx->velT, sizeof(float4) * ctx->n, cudaMemcpyDeviceToDevice, ctx->stream));
   return check_launch(ctx, "apply_viscosity");
 }
@@ -5328,7 +5388,7 @@ int pbf_compute_vorticity(pbf_ctx* ctx, size_t b, size_t e) {
   if (X)
     k_vorticity<<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, nullptr);
   else
-    kt_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
+    kt_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(density_dev(ctx, SP), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH);
   return check_launch(ctx, "compute_vorticity");
 }
 
@@ -5338,7 +5398,7 @@ int pbf_apply_vorticity(pbf_ctx* ctx, size_t b, size_t e) {
   if (X)
     k_apply_vorticity<false><<<g, kBlock, 0, ctx->stream>>>(SP, n, ctx->lstride, ctx->nbr, ctx->cnt, nullptr, ctx->pstH, ctx->scrH, ctx->velH);
   else
-    kt_apply_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+    kt_apply_vorticity<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(density_dev(ctx, SP), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
   return check_launch(ctx, "apply_vorticity");
 }
 
