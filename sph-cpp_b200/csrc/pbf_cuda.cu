@@ -1606,8 +1606,12 @@ __device__ __forceinline__ int walk_count(const Dev& P, int b, const int32_t* __
 // it; one lane a bin).  A bin's particles share the 27, so the first of them
 // marks for all: the word of the bin's histogram, used up by the scan, carries
 // the flag until the next step clears it.  16 slots a store; the slots beside
-// a bin's own are marked too.  A bin of more than kMaskRow particles needs no
-// mark: its particles' own rows are longer, their lists walked whole anyway.
+// a bin's own are marked too, but for OWN: in the persistent step those may be
+// of another scene that is between its two viscosity passes, where a longer
+// walk would read weights (wvis) that the first of them did not write.  A bin
+// of more than kMaskRow particles needs no mark: its particles' own rows are
+// longer, their lists walked whole anyway.
+template <bool OWN = false>
 __device__ __forceinline__ void mark_neighbourhoods(const Dev& P, int b, bool mark) {
   constexpr uint32_t kMarked = 0x80000000u;
   if (__any_sync(0xffffffffu, mark)) {
@@ -1629,10 +1633,14 @@ __device__ __forceinline__ void mark_neighbourhoods(const Dev& P, int b, bool ma
         if (cx >= 0 && cy >= 0 && cz >= 0 && cx < R.dimx && cy < R.dimy && cz < R.dimz) {
           const uint32_t c = R.key0 + (uint32_t)plane * (uint32_t)cz + (uint32_t)(cy * R.dimx + cx);
           const uint32_t q0 = P.cell_start[c], q1 = P.cell_start[c + 1];
-          if (q1 - q0 <= (uint32_t)kMaskRow)
+          if (q1 - q0 > (uint32_t)kMaskRow) {
+          } else if (OWN) {
+            for (uint32_t q = q0; q < q1; ++q) P.walk[q] = kWalkAll;
+          } else {
             for (uint32_t q = q0 & ~15u; q < q1; q += 16)
               *reinterpret_cast<uint4*>(P.walk + q) =
                   make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+          }
         }
       }
     }
@@ -2022,7 +2030,7 @@ __device__ __forceinline__ void density_lambda_tile(int tile, const Dev& P, cons
       }
     }
   }
-  mark_neighbourhoods(P, b, mark);
+  mark_neighbourhoods<COH>(P, b, mark);
 }
 
 // The residual check runs on a persistent grid walking the tiles, so that
@@ -2755,7 +2763,7 @@ __device__ __forceinline__ void dp_update_tile(int tile, const Dev& P, const Fas
       vel[b] = make_float4(v.x, v.y, v.z, vel[b].w);
     }
   }
-  mark_neighbourhoods(P, b, mark);
+  mark_neighbourhoods<COH>(P, b, mark);
 }
 
 // COND launches (the learned solver's extra iterations) use a persistent grid
