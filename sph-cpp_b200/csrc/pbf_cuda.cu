@@ -452,8 +452,8 @@ __global__ void k_arrivals(int n, const uint32_t* __restrict__ key, const uint32
 // costs a pass over all n indices' bits whatever the bin holds.  So bins of at
 // most kOrderSort particles are sorted in shared memory instead (bitonic, then
 // every index is looked up) where the bitmap is longer than kOrderBits words.
-// Bitmap and sort, us a launch: 65,536 particles, one bin of 2,000 10 and 23,
-// of 8,000 17 and 62; 1M, 40 bins of 2,000 21 and 21, of 8,000 31 and 66; 16.8M,
+// Bitmap and sort, us a launch: 65,536 particles, one bin of 2,000 10 and 23;
+// 1M, 40 bins of 2,000 21 and 21, of 8,000 31 and 66; 16.8M,
 // one bin of 8,000 193 and 58, 4,000 bins of 2,000 10,116 and 629.  With more
 // particles a bin the bitmap's pass weighs little (16.8M, 40 bins of 60,000:
 // 318 us).  Of a giant bin only the prefix sums are left to find: by one block
@@ -2617,16 +2617,9 @@ __global__ void __launch_bounds__(kBlock) k_viscosity(Dev P, int n, size_t strid
   near2(P, nbr, b, stride, c, pst, vin, [&](int q, float4 xq, float4 vq) {
     const float rx = pbf::S<X>(xp.x, xq.x), ry = pbf::S<X>(xp.y, xq.y), rz = pbf::S<X>(xp.z, xq.z);
     const float w = pbf::poly6<X>(P, pbf::SQ<X>(pbf::mag2<X>(rx, ry, rz)));
-    if (X) {
-      dv.x = pbf::xadd(dv.x, pbf::xdiv(pbf::xmul(pbf::xsub(vq.x, vp.x), w), vq.w));
-      dv.y = pbf::xadd(dv.y, pbf::xdiv(pbf::xmul(pbf::xsub(vq.y, vp.y), w), vq.w));
-      dv.z = pbf::xadd(dv.z, pbf::xdiv(pbf::xmul(pbf::xsub(vq.z, vp.z), w), vq.w));
-    } else {
-      const float wr = __fdividef(w, vq.w);
-      dv.x = fmaf(vq.x - vp.x, wr, dv.x);
-      dv.y = fmaf(vq.y - vp.y, wr, dv.y);
-      dv.z = fmaf(vq.z - vp.z, wr, dv.z);
-    }
+    dv.x = pbf::xadd(dv.x, pbf::xdiv(pbf::xmul(pbf::xsub(vq.x, vp.x), w), vq.w));
+    dv.y = pbf::xadd(dv.y, pbf::xdiv(pbf::xmul(pbf::xsub(vq.y, vp.y), w), vq.w));
+    dv.z = pbf::xadd(dv.z, pbf::xdiv(pbf::xmul(pbf::xsub(vq.z, vp.z), w), vq.w));
   });
   vout[b] = make_float4(pbf::A<X>(vp.x, pbf::M<X>(P.visc_c, dv.x)), pbf::A<X>(vp.y, pbf::M<X>(P.visc_c, dv.y)),
                         pbf::A<X>(vp.z, pbf::M<X>(P.visc_c, dv.z)), vp.w);
@@ -3310,8 +3303,8 @@ struct PersistArrays {
   float4 *pst, *xl, *vel, *velT, *pos, *scr, *velH, *posH, *pstH;
   float* lam;
   __half* wvis;
-  uint32_t *nudge, *err, *origH;
-  const uint32_t *cell_start, *run_end, *origS;
+  uint32_t *nudge, *origH;
+  const uint32_t* origS;
   int32_t *nbr, *cnt;
 };
 
@@ -4320,10 +4313,7 @@ void launch_persistent(pbf_ctx* ctx) {
   A.lam = ctx->lamH;
   A.wvis = ctx->wvis;
   A.nudge = ctx->nudge;
-  A.err = ctx->err;
   A.origH = ctx->origH;
-  A.cell_start = ctx->cell_start;
-  A.run_end = ctx->run_end;
   A.origS = ctx->origS;
   A.nbr = ctx->nbr;
   A.cnt = ctx->cnt;
@@ -6224,17 +6214,19 @@ int pbf_launches_per_step(pbf_ctx* ctx, int64_t* out) {
 // (PBF_NOALLOC_SCRATCH_BYTES, held on every GPU that loads the library until
 // the process exits); the caller passes only its inputs and outputs.
 // The steps are the regular neighbor search's:
-//   hash      bin key and (index << 32 | index) at the caller's index, plus
-//             the bin histogram (calculate_bins, neighbors.h:120-125)
+//   hash      bin key and arrival number in the bin at the caller's index, the
+//             bin histogram and the list of crowded bins (calculate_bins,
+//             neighbors.h:120-125)
 //   bounds    exclusive scan of the histogram = begin/end of every bin
 //             (find_bin_bounds, neighbors.h:137-148)
 //   sort      the regular path's: arrivals at their bins' starts, crowded
-//             bins ordered by a bitmap, the others by counting while the
-//             positions are gathered (sort_bins, neighbors.h:130-132)
+//             bins ordered by a bitmap or in shared memory, the others by
+//             counting while the positions are gathered (sort_bins, neighbors.h:130-132)
 //   runs      runs of bit-identical positions among consecutive sorted slots
 //   fill      the lists in reference index space (fill_neighbors,
-//             neighbors.h:197-230); a bin of more than kRunBin particles is
-//             walked run by run, one distance test per run
+//             neighbors.h:197-230): the split fill's masks, the particles it
+//             leaves by the walk; a bin of more than kRunBin particles is
+//             walked run by run where its runs are long, one distance test a run
 //   flags     the error word (out-of-grid or non-finite positions) copied to
 //             the caller's flag word.
 namespace {
