@@ -3000,7 +3000,9 @@ __global__ void __launch_bounds__(kStageThreads) ks_apply_vorticity(Dev P, Fast 
 // colour field 41 instead of 54), bound as the fused gathers by the L1 path.
 // Positions can change in any way between two stage calls, so a list is walked
 // whole unless the context knows that x* only moved by update_position_stars
-// since the fill (P.walk given: walk_count).  Slots past a count are read at
+// since the fill (P.walk given: walk_count).  Del_Spikey keeps the reference's
+// r + eps (spikey_over_r_eps): particles that compute_densities has nudged off
+// one another are that close.  Slots past a count are read at
 // slot n, the dummy record (DummySlots).
 constexpr int kStageGL = 2, kStageBlock = 128;
 
@@ -3060,12 +3062,25 @@ __global__ void __launch_bounds__(kStageBlock) kt_lambda(Dev P, Fast F, int n, s
   const int b = G.b;
   const float4 xp = pst[b];
   const int c = stage_count(P, G, cnt);
-  const DensitySums S = density_sums<kStageGL, false>(F, G, nbr + pbf::list_base(b, stride), nullptr, c, n, pst, xp);
+  float sx = 0.f, sy = 0.f, sz = 0.f, s2 = 0.f;
+  pbf::gwalk1<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, [&](int, float4 xq) {
+    const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    const float t = pbf::spikey_over_r_eps(F, d2);
+    sx = fmaf(t, dx, sx);
+    sy = fmaf(t, dy, sy);
+    sz = fmaf(t, dz, sz);
+    s2 = fmaf(t * t, d2, s2);
+  });
+  sx = pbf::gsum<kStageGL>(sx);
+  sy = pbf::gsum<kStageGL>(sy);
+  sz = pbf::gsum<kStageGL>(sz);
+  s2 = pbf::gsum<kStageGL>(s2);
   if (!G.live || G.lane != 0) return;
   const float L2 = F.lam_grad * F.lam_grad;
-  const float g2 = pbf::xmul(L2, fmaf(S.s1z, S.s1z, fmaf(S.s1y, S.s1y, S.s1x * S.s1x)));
+  const float g2 = pbf::xmul(L2, fmaf(sz, sz, fmaf(sy, sy, sx * sx)));
   const float C = fmaxf(fmaf(vel[b].w, F.inv_rho0, -1.0f), 0.0f);
-  lam[b] = -C / (fmaf(L2, S.s2, g2) + F.lambda_eps);
+  lam[b] = -C / (fmaf(L2, s2, g2) + F.lambda_eps);
 }
 
 // compute_pressure_dps (particles.h:348-358) -> scratch
@@ -3084,8 +3099,8 @@ __global__ void __launch_bounds__(kStageBlock) kt_dp(Dev P, Fast F, int n, size_
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
     const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
     float l = lp + __ldg(lam + q);
-    if (SCORR) l -= P.scorr_k * __powf(F.visc_poly * pbf::poly_cube(F, d2) * P.inv_wdq, P.scorr_n);
-    const float t = l * pbf::spikey_over_r(F, d2);
+    if (SCORR) l -= P.scorr_k * powf(F.visc_poly * pbf::poly_cube(F, d2) * P.inv_wdq, P.scorr_n);
+    const float t = l * pbf::spikey_over_r_eps(F, d2);
     ax = fmaf(t, dx, ax);
     ay = fmaf(t, dy, ay);
     az = fmaf(t, dz, az);
@@ -3112,7 +3127,7 @@ __global__ void __launch_bounds__(kStageBlock) kt_color(Dev P, Fast F, int n, si
   float ax = 0.f, ay = 0.f, az = 0.f;
   pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, vel, [&](int, float4 xq, float4 vq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
-    const float t = __fdividef(pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx))), vq.w);
+    const float t = __fdividef(pbf::spikey_over_r_eps(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx))), vq.w);
     ax = fmaf(t, dx, ax);
     ay = fmaf(t, dy, ay);
     az = fmaf(t, dz, az);
@@ -3200,7 +3215,7 @@ __global__ void __launch_bounds__(kStageBlock) kt_vorticity(Dev P, Fast F, int n
   float wx = 0.f, wy = 0.f, wz = 0.f;
   pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, vel, [&](int, float4 xq, float4 vq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
-    const float t = pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+    const float t = pbf::spikey_over_r_eps(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
     const float ux = vq.x - vp.x, uy = vq.y - vp.y, uz = vq.z - vp.z;
     wx = fmaf(t, fmaf(uy, dz, -uz * dy), wx);
     wy = fmaf(t, fmaf(uz, dx, -ux * dz), wy);
@@ -3228,7 +3243,7 @@ __global__ void __launch_bounds__(kStageBlock) kt_apply_vorticity(Dev P, Fast F,
   pbf::gwalk2<kStageGL>(nbr + pbf::list_base(b, stride), c, n, G.lane, pst, scr, [&](int, float4 xq, float4 sq) {
     const float dx = xp.x - xq.x, dy = xp.y - xq.y, dz = xp.z - xq.z;
     const float vm = __fsqrt_rn(fmaf(sq.z, sq.z, fmaf(sq.y, sq.y, sq.x * sq.x)));
-    const float t = vm * pbf::spikey_over_r(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+    const float t = vm * pbf::spikey_over_r_eps(F, fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
     ex = fmaf(t, dx, ex);
     ey = fmaf(t, dy, ey);
     ez = fmaf(t, dz, ez);

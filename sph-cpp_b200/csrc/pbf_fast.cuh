@@ -444,6 +444,14 @@ __device__ __forceinline__ float spikey_over_r(const Fast& F, float d2) {
   return hr * hr * rinv;
 }
 
+// The same over r + FLT_EPSILON, as in the reference (kernels.h:155-178): a
+// pair closer than 1e-4 differs in more than the third digit.
+__device__ __forceinline__ float spikey_over_r_eps(const Fast& F, float d2) {
+  const float r = d2 * rsqrtf(fmaxf(d2, 1e-30f));
+  const float hr = fmaxf(F.h - r, 0.0f);
+  return hr * hr * __fdividef(1.0f, r + FLT_EPSILON);
+}
+
 __device__ __forceinline__ float poly_cube(const Fast& F, float d2) {
   const float a = fmaxf(F.h2 - d2, 0.0f);
   return a * a * a;
