@@ -297,8 +297,10 @@ __global__ void k_ext_predict_hash(Dev P, int n, const float4* __restrict__ pos,
   pst[a] = make_float4(s.x, s.y, s.z, 0.0f);
   uint32_t k;
   if (!pbf::bin_of(P, R, s.x, s.y, s.z, k)) atomicOr(err, PBF_FLAG_KEY_RANGE);
-  // (of a NaN x* there are no lists)
-  if (move_size(make_float4(s.x, s.y, s.z, 0.0f), pos[a]) > kTame * P.dt) cell_count[P.nbins + kWildValues] = 1u;
+  // the velocity nudges a particle off a neighbour, the move becomes the velocity (of a NaN x* there are no lists)
+  if (move_size(make_float4(s.x, s.y, s.z, 0.0f), pos[a]) > kTame * P.dt ||
+      fabsf(v.x) + fabsf(v.y) + fabsf(v.z) > kTame)
+    cell_count[P.nbins + kWildValues] = 1u;
   hash_out(P.nbins, a, k, key, rank, cell_count, crowded);
 }
 
