@@ -186,6 +186,7 @@ def kernel_bytes(name: str, n: int, nbar: float, K: int, nbins: int) -> float:
     per = {
         "ext_predict_hash": 16 + 16 + 16 + 16 + 4 + 4,           # x, v in; v, x*, key, rank out (+ histogram in L2)
         "scan_reduce": 4.0 * nbins / n,
+        "scan_partials": 8.0 * nbins / n / 4096,                # one sum per scan tile of 4096 bins, read and written
         "scan_apply": 8.0 * nbins / n,
         "arrivals": 4 + 4 + 4 + 8,                              # key, arrival number, orig in; (orig, slot) out
         "order_crowded": 4.0 / n,                               # the count of crowded bins
