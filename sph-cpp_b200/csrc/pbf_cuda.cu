@@ -1029,13 +1029,13 @@ __global__ void __launch_bounds__(kFillBlock) k_fill2(Dev P, int n, size_t strid
 // grid, no row longer than kMaskRow candidates.  The others are left to
 // k_fill_rest, which walks them in the reference's order and stops at the cap:
 // in a crowded region that is early.
-// Bound by instruction issue (70% of the slots; 27 of 32 lanes active) with
-// the L1 data path at 62% (a 16-byte load moves 512 bytes to the registers
+// Bound by instruction issue (72% of the slots; 27 of 32 lanes active) with
+// the L1 data path at 65% (a 16-byte load moves 512 bytes to the registers
 // even where the lanes read one record).  Measured against the walk that
 // appended in its test loop and its second launch for the capped lists: 1M dam
-// 0.497 + 0.092 -> 0.378 ms, 65k 0.062 + 0.060 -> 0.042 ms, 500k squeezed to
+// 0.497 + 0.092 -> 0.384 ms, 65k 0.062 + 0.060 -> 0.042 ms, 500k squeezed to
 // 92% of the lists at the cap 0.295 + 0.515 -> 0.311 ms; warp instructions at
-// 1M 446M -> 269M.
+// 1M 446M -> 306M.
 constexpr int kMaskBlock = 64;
 constexpr int kMaskWords = 3, kMaskRow = 32 * kMaskWords;  // mask words and candidates of a row
 constexpr int kMaskUnits = 9 * kMaskWords;                 // mask words of a particle; at most 32
@@ -4235,7 +4235,9 @@ void launch_cell_sort(pbf_ctx* ctx) {
 // 40.6 / 41.4 / 40.4; 1M 525 / 429 / 388.  The search on device arrays (one warp
 // a tile in k_fill_masks's place): 2k 12.5 / 25.7 / 38.8, 33k 29.4 / 31.6 / 44.3,
 // 48k 42.5 / 38.4 / 47.0.  Exact math, with the near bits: 64k 59.9 / 55.9 /
-// 55.8, 97k 86.9 / 79.0 / 80.7, 262k 217 / 172 / 169, 1M 806 / 605 / 589.
+// 55.8, 97k 86.9 / 79.0 / 80.7, 262k 217 / 172 / 169, 1M 806 / 605 / 589.  Frames
+// of five steps in fast math, all of it: 24k 611 / 638 / 682, 33k 682 / 663 / 695,
+// 48k 764 / 749 / 767, 64k 902 / 862 / 846.
 constexpr size_t kSplit9Most = 40960, kSplit3Most = 61440;
 
 // Particles up to which the fill asks for 60% of the SM's memory as shared
