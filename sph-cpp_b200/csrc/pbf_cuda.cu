@@ -594,17 +594,17 @@ __device__ __forceinline__ bool wild(const Dev& P, float4 xs, float4 x, float4 v
            tame(scr.y) && tame(scr.z) && tame(lam));
 }
 
+// All lists are walked whole from here on when the word is raised.
+__global__ void k_walk_whole(int n, const uint32_t* __restrict__ word, uint8_t* walk) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (*word != 0u && 16 * i < n) reinterpret_cast<uint4*>(walk)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+}
+
 __global__ void k_wild(Dev P, int n, const float4* __restrict__ pstH, const float4* __restrict__ posH,
                        const float4* __restrict__ velH, const float4* __restrict__ scrH,
                        const float* __restrict__ lamH, bool rho, uint32_t* word) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < n && wild(P, pstH[b], posH[b], velH[b], scrH[b], lamH[b], rho)) *word = 1u;
-}
-
-// All lists are walked whole from here on when the word is raised.
-__global__ void k_walk_whole(int n, const uint32_t* __restrict__ word, uint8_t* walk) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (*word != 0u && 16 * i < n) reinterpret_cast<uint4*>(walk)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
 }
 
 // The per-stage path keeps the sorted arrays as the home arrays (the paths
@@ -2468,13 +2468,26 @@ __global__ void __launch_bounds__(kBlock) k_dp(Dev P, int n, size_t stride, cons
 __global__ void k_update_xs(Dev P, int n, float4* pst, const float4* __restrict__ scr) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   bool mark = false;
+  float path = 0.0f;
   if (b < n && pbf::in_span(P, b)) {
     const float4 x = pst[b], d = scr[b];
     const float3 s = pbf::boundary(P, pbf::region_of(P, b),
                                    make_float3(pbf::xadd(x.x, d.x), pbf::xadd(x.y, d.y), pbf::xadd(x.z, d.z)));
-    pst[b] = make_float4(s.x, s.y, s.z, P.walk ? moved(P, x, s, mark) : 0.0f);
+    path = P.walk ? moved(P, x, s, mark) : 0.0f;
+    pst[b] = make_float4(s.x, s.y, s.z, path);
   }
-  if (P.walk) mark_neighbourhoods(P, b, mark);
+  // an x* that is none: what follows from it spreads from stage to stage, so the first warp to find one has all
+  // lists walked whole
+  if (P.walk && __any_sync(0xffffffffu, !(path <= FLT_MAX))) {
+    const int lane = threadIdx.x & 31;
+    uint32_t before = 0;
+    if (lane == 0) before = atomicExch(P.cell_mark + P.nbins + kWildValues, 1u);
+    if (__shfl_sync(0xffffffffu, before, 0) == 0u)
+      for (int q = 16 * lane; q < n; q += 16 * 32)
+        *reinterpret_cast<uint4*>(P.walk + q) = make_uint4(~0u, ~0u, ~0u, ~0u);
+  } else if (P.walk) {
+    mark_neighbourhoods(P, b, mark);
+  }
 }
 
 // update_velocities (particles.h:375-385), always exact (per-particle).
@@ -3014,8 +3027,8 @@ __device__ __forceinline__ int stage_count(const Dev& P, const pbf::Group& G, co
 }
 
 // The group of this thread; not live outside the stage's span.
-__device__ __forceinline__ pbf::Group stage_group(const Dev& P, int n) {
-  pbf::Group G = pbf::group_of<kStageGL>(n);
+__device__ __forceinline__ pbf::Group stage_group(const Dev& P, int n, int tile = blockIdx.x) {
+  pbf::Group G = pbf::group_at<kStageGL>(n, tile);
   G.live = G.live && pbf::in_span(P, G.b);
   return G;
 }
@@ -3145,12 +3158,10 @@ __global__ void __launch_bounds__(kStageBlock) kt_color(Dev P, Fast F, int n, si
 // ... then the cohesion + curvature force: the reference's expressions, its
 // double ones in double, over the whole list (the curvature term does not
 // vanish beyond h).  Bound by the walk's three records a neighbour.
-__global__ void __launch_bounds__(kStageBlock) kt_surface(Dev P, Fast F, int n, size_t stride,
-                                                          const int32_t* __restrict__ nbr,
-                                                          const int32_t* __restrict__ cnt,
-                                                          const float4* __restrict__ pst,
-                                                          const float4* __restrict__ scr, float4* vel) {
-  const pbf::Group G = stage_group(P, n);
+__device__ __forceinline__ void surface_of(const pbf::Group& G, const Dev& P, size_t stride,
+                                           const int32_t* __restrict__ nbr, const int32_t* __restrict__ cnt,
+                                           const float4* __restrict__ pst, const float4* __restrict__ scr,
+                                           float4* vel) {
   const int b = G.b;
   const float4 xp = pst[b], sp = scr[b];
   const float rp = vel[b].w, ng = -P.gamma, h_eps = (float)P.h_eps;
@@ -3175,6 +3186,27 @@ __global__ void __launch_bounds__(kStageBlock) kt_surface(Dev P, Fast F, int n, 
   vel[b].x = fmaf(fx, k, vel[b].x);
   vel[b].y = fmaf(fy, k, vel[b].y);
   vel[b].z = fmaf(fz, k, vel[b].z);
+}
+
+__global__ void __launch_bounds__(kStageBlock) kt_surface(Dev P, int n, size_t stride,
+                                                          const int32_t* __restrict__ nbr,
+                                                          const int32_t* __restrict__ cnt,
+                                                          const float4* __restrict__ pst,
+                                                          const float4* __restrict__ scr, float4* vel) {
+  surface_of(stage_group(P, n), P, stride, nbr, cnt, pst, scr, vel);
+}
+
+// Without surface tension the force is a sum of zeros, unless something is
+// infinite or none: a few blocks look, and walk the lists only then.
+__global__ void __launch_bounds__(kStageBlock) kt_surface_wild(Dev P, int n, size_t stride,
+                                                               const int32_t* __restrict__ nbr,
+                                                               const int32_t* __restrict__ cnt,
+                                                               const float4* __restrict__ pst,
+                                                               const float4* __restrict__ scr, float4* vel) {
+  if (!P.cell_mark[P.nbins + kWildValues]) return;
+  const int tiles = pbf::tiles_of<kStageGL>(n);
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
+    surface_of(stage_group(P, n, tile), P, stride, nbr, cnt, pst, scr, vel);
 }
 
 // apply_viscosity (particles.h:436-447), Jacobi
@@ -3746,6 +3778,13 @@ int check_launch(pbf_ctx* ctx, const char* what) {
 
 // Build the device constant block from the public parameters (all derived
 // constants are evaluated on the host in the reference's types).
+// Whether the terms of pairs past h are zeros: a lambda of -0 / 0 (no
+// relaxation), densities never computed (no iteration) or a power of s_corr
+// that does not rise make them NaN or more.
+bool zero_terms(const pbf_params& p) {
+  return p.lambda_epsilon > 0.0f && p.solve_steps > 0 && !(p.scorr_k > 0.0f && !(p.scorr_n > 0.0f));
+}
+
 int make_dev(pbf_ctx* ctx, const pbf_params& p, Dev& d, int64_t dims[3]) {
   if (!(p.time_step > 0.0f) || !(p.smoothing_radius > 0.0f) || !(p.neighbor_bin_spacing > 0.0f) ||
       !(p.rest_density > 0.0f) || !(p.rest_mass > 0.0f))
@@ -3831,10 +3870,9 @@ int make_dev(pbf_ctx* ctx, const pbf_params& p, Dev& d, int64_t dims[3]) {
   }
   {
     // near entries (walk_count): within h + kNearMargin * h at the fill, when that is short of s and the
-    // other entries' terms are zeros: a lambda of -0 / 0 (no relaxation), densities never computed (no
-    // iteration) or a power of s_corr that does not rise make them NaN or more
+    // other entries' terms are zeros
     const float near = h + kNearMargin * h;
-    const bool zeros = p.lambda_epsilon > 0.0f && p.solve_steps > 0 && !(p.scorr_k > 0.0f && !(p.scorr_n > 0.0f));
+    const bool zeros = zero_terms(p);
     d.near2 = near < s && zeros ? near * near : d.s2;
     d.near_move = near < s && zeros ? (0.5f * kNearMargin - kNearSlack) * h : FLT_MAX;
   }
@@ -4677,7 +4715,7 @@ void launch_step_t(pbf_ctx* ctx) {
     if (X)
       k_surface<<<g, kBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
     else
-      kt_surface<<<gt, kStageBlock, 0, s>>>(P, F, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
+      kt_surface<<<gt, kStageBlock, 0, s>>>(P, n, st, ctx->nbr, ctx->cnt, ctx->pstS, ctx->scrH, ctx->velS);
   }
   if (X) {
     {
@@ -5380,9 +5418,13 @@ int pbf_apply_surface_tension(pbf_ctx* ctx, size_t cb, size_t ce, size_t sb, siz
   } else {
     kt_color<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(SP, ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->velH, ctx->scrH, true);
     // without surface tension the force is exactly zero, but where a density
-    // not computed yet makes it NaN
-    if (ctx->params.gamma != 0.0f || !ctx->rho_whole)
-      kt_surface<<<blocks_for(ctx->n * (size_t)kStageGL, kStageBlock), kStageBlock, 0, ctx->stream>>>(span_dev(ctx, se), ctx->fast, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+    // not computed yet, an x* that is none or a wild value makes it NaN
+    const Dev SE = span_dev(ctx, se);
+    const int gt = blocks_for(ctx->n * (size_t)kStageGL, kStageBlock);
+    if (ctx->params.gamma == 0.0f && ctx->rho_whole && SE.walk != nullptr && zero_terms(ctx->params))
+      kt_surface_wild<<<std::min(gt, 2 * ctx->sms), kStageBlock, 0, ctx->stream>>>(SE, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
+    else
+      kt_surface<<<gt, kStageBlock, 0, ctx->stream>>>(SE, n, ctx->lstride, ctx->nbr, ctx->cnt, ctx->pstH, ctx->scrH, ctx->velH);
   }
   return check_launch(ctx, "apply_surface_tension");
 }
