@@ -3094,8 +3094,8 @@ __global__ void __launch_bounds__(kStageBlock) kt_lambda(Dev P, Fast F, int n, s
   if (!G.live || G.lane != 0) return;
   const float L2 = F.lam_grad * F.lam_grad;
   const float g2 = pbf::xmul(L2, fmaf(sz, sz, fmaf(sy, sy, sx * sx)));
-  const float C = fmaxf(fmaf(vel[b].w, F.inv_rho0, -1.0f), 0.0f);
-  lam[b] = -C / (fmaf(L2, s2, g2) + F.lambda_eps);
+  const float C = fmaf(vel[b].w, F.inv_rho0, -1.0f);
+  lam[b] = -(C < 0.0f ? 0.0f : C) / (fmaf(L2, s2, g2) + F.lambda_eps);  // of a NaN density NaN
 }
 
 // compute_pressure_dps (particles.h:348-358) -> scratch

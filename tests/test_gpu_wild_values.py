@@ -163,3 +163,22 @@ def test_a_fused_step_from_a_position_out_of_all_bounds(bad, n):
     for a, b, c in zip(got["stages", 1], got["step", 1], got["step", 0]):
         assert np.array_equal(a, b, equal_nan=True)
         assert np.array_equal(np.isfinite(a), np.isfinite(c))
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_a_density(bad):
+    x, v = _state(6)
+
+    def run(g):
+        g.upload(x, v)
+        g.find_neighbors()
+        g.compute_densities()
+        rho = g.densities()
+        rho[300] = bad
+        g.set_array(_abi.ARRAY_DENSITIES, rho)
+        g.compute_pressure_lambdas()
+        out = [g.lambdas()]
+        g.compute_pressure_dps()
+        return out + [g.scratch()]
+
+    _both(run)
